@@ -101,61 +101,6 @@ bool valid_params(const bs_params* p, std::string& why) {
     return true;
 }
 
-// One sphere's tables for the mixed path: real and imaginary float planes of
-// Usp (thetaR x dR) and Uip (thetaR x aR) in CUDA arrays, with a surface
-// object per plane for the build and a texture object per plane for the
-// gathers.  Index k: 0 Usp re, 1 Usp im, 2 Uip re, 3 Uip im.
-struct TexSlot {
-    cudaArray_t arr[4] = {};
-    cudaTextureObject_t tex[4] = {};
-    cudaSurfaceObject_t surf[4] = {};
-    int w = 0, h[4] = {0, 0, 0, 0};
-
-    void release() {
-        for (int k = 0; k < 4; k++) {
-            if (tex[k]) cudaDestroyTextureObject(tex[k]);
-            if (surf[k]) cudaDestroySurfaceObject(surf[k]);
-            if (arr[k]) cudaFreeArray(arr[k]);
-            tex[k] = surf[k] = 0;
-            arr[k] = nullptr;
-            h[k] = 0;
-        }
-        w = 0;
-    }
-
-    // (re)allocate plane k with at least `rows` rows of `width` floats
-    cudaError_t ensure(int k, int width, int rows) {
-        if (arr[k] && w == width && h[k] >= rows) return cudaSuccess;
-        if (tex[k]) cudaDestroyTextureObject(tex[k]);
-        if (surf[k]) cudaDestroySurfaceObject(surf[k]);
-        if (arr[k]) cudaFreeArray(arr[k]);
-        tex[k] = surf[k] = 0;
-        arr[k] = nullptr;
-        cudaChannelFormatDesc fd = cudaCreateChannelDesc<float>();
-        // rows rounded up to a multiple of 256 (reads never pass the spare row): fewer
-        // reallocations, whose cudaFreeArray waits for the whole device
-        rows = (rows + 255) & ~255;
-        cudaError_t e = cudaMallocArray(&arr[k], &fd, width, rows, cudaArraySurfaceLoadStore | cudaArrayTextureGather);
-        if (e != cudaSuccess) return e;
-        cudaResourceDesc rd = {};
-        rd.resType = cudaResourceTypeArray;
-        rd.res.array.array = arr[k];
-        e = cudaCreateSurfaceObject(&surf[k], &rd);
-        if (e != cudaSuccess) return e;
-        cudaTextureDesc td = {};
-        td.addressMode[0] = cudaAddressModeClamp;
-        td.addressMode[1] = cudaAddressModeClamp;
-        td.filterMode = cudaFilterModePoint;
-        td.readMode = cudaReadModeElementType;
-        td.normalizedCoords = 0;
-        e = cudaCreateTextureObject(&tex[k], &rd, &td, nullptr);
-        if (e != cudaSuccess) return e;
-        w = width;
-        h[k] = rows;
-        return cudaSuccess;
-    }
-};
-
 }  // namespace
 
 struct bs_ctx {
@@ -176,7 +121,7 @@ struct bs_ctx {
     bool have = false;
 
     DevBuf d_sph, d_waves, d_kw4, d_ph, d_A, d_B, d_mie, d_tab, d_tabscr, d_legP, d_lut, d_uft, d_uftscr;
-    DevBuf d_cones, d_cnt;  // per-chunk wave cones; staged / total counters of the mixed LUT kernel
+    DevBuf d_cnt;           // staged / total counters of the mixed LUT kernel
     DevBuf d_far;           // far fields Ud, Ufd on request (bs_get_far_field)
     DevBuf d_starts;        // row / coefficient offsets of a coefficient batch
     DevBuf d_lbjobs, d_lbjobs2;  // Usp and Uip tables of a coefficient batch for the mixed LUT build
@@ -188,16 +133,15 @@ struct bs_ctx {
     DevBuf d_fields;  // [2][R*R] U then Uf
     DevBuf d_su, d_sv, d_mask, d_wx, d_wy, d_wix, d_wiy, d_f1, d_f2, d_g1, d_I, d_D, d_img;
     int legP_theta = 0, legP_L = 0;
-    std::vector<TexSlot> slots;  // mixed-path tables, one per sphere of a chunk
-    DevBuf d_texobj;
+    int tab_s0 = 0, tab_s1 = 0;  // spheres whose tables the last run left in d_lut
     int64_t launches = 0;
     int64_t interactions = 0;
     bs_stats stats{};
     // table reuse between runs (bs_set_lut_reuse)
     bool reuse = false;
     int stream_prio = 0;  // bs_set_stream_priority (0: the default priority)
-    int lut_staging = 0;  // bs_set_lut_staging: 0 model-chosen, 1 staged kernel, 2 texture-only kernel
-    int lut_chunk = 0;    // bs_set_lut_wave_chunk: 0 model-chosen, else waves per chunk
+    int lut_staging = 0;  // bs_set_lut_staging: 0, 1 staged kernel, 2 unstaged kernel
+    int lut_chunk = 0;    // bs_set_lut_wave_chunk: 0 default, else waves per counted chunk
     bool bp_on = false;   // bs_set_backpropagation
     double bp_d = 0;
     DevBuf d_bp;          // back-propagation phase on the passband grid
@@ -213,14 +157,12 @@ static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
     return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_mie, &c->d_tab,
             &c->d_tabscr, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
             &c->d_sv, &c->d_mask, &c->d_wx, &c->d_wy, &c->d_wix, &c->d_wiy, &c->d_f1, &c->d_f2,
-            &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cones, &c->d_cnt, &c->d_far,
+            &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_far,
             &c->d_starts, &c->d_lbjobs, &c->d_lbjobs2, &c->d_kcmp, &c->d_fsave, &c->d_dacc, &c->d_line, &c->d_ringcs, &c->d_bp, &c->d_shrec, &c->d_shtab, &c->d_shcoef, &c->d_gscr, &c->d_ufw};
 }
 
 static void release_all(bs_ctx* c) {
     for (DevBuf* b : ctx_bufs(c)) b->release();
-    for (auto& sl : c->slots) sl.release();
-    c->d_texobj.release();
     c->legP_theta = c->legP_L = 0;
     c->lut_valid = false;
     c->have = false;
@@ -251,6 +193,7 @@ static void preload_kernels(int device) {
     std::lock_guard<std::mutex> lock(mu);
     if (std::find(done.begin(), done.end(), device) != done.end()) return;
     preload_nearfield_kernels();
+    preload_uslut_kernels();
     preload_detector_kernels();
     cudaGetLastError();  // a kernel this device cannot load reports at its launch instead
     done.push_back(device);
@@ -267,7 +210,6 @@ bs_status bs_create(const bs_params* params, bs_ctx** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
     for (int i = 0; i < 6 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
     for (DevBuf* b : ctx_bufs(c)) b->st = &c->st;
-    c->d_texobj.st = &c->st;
     if (e != cudaSuccess) {
         delete c;
         return fail(BS_ERR_CUDA, "bs_create: %s", cudaGetErrorString(e));
@@ -411,6 +353,10 @@ static bs_status derive(bs_ctx* c) {
         S.r0 = std::max(in.a, S.dmin);
         S.xs_usp = (S.dR - 1) / (S.dmax - S.r0);
         S.xs_uip = (S.aR - 1) / (S.a - S.dmin);
+        const double tsc = (S.thetaR - 1) / PI_REF, hp = 0.5 * TRUE_PI * tsc;
+        S.tsc = (float)tsc;
+        S.hp_hi = (float)hp;
+        S.hp_lo = (float)(hp - (double)S.hp_hi);
         S.coef_off = coef;
         coef += S.Nl + 1;
         c->Lmax = std::max(c->Lmax, S.Nl + 1);
@@ -566,12 +512,10 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
 // and applied before the next one overwrites the pool).  FP64: one
 // Patch<double> per entry.  Mixed: one float2 per entry in linear rows of
 // thetaR + 1 entries (the last column repeated, rounded up to an even count
-// for 16-byte rows), and a second copy of every entry in the texture planes,
-// which also counts against the budget.
+// for 16-byte rows; a Uip of one row is stored twice).
 static bs_status plan_tables(std::vector<Sphere>& hs, bool mixed, size_t budget, std::vector<int>& chunk_start,
                              size_t& pool, size_t& maxrows, size_t& maxL) {
     const size_t patch = mixed ? sizeof(float2) : sizeof(Patch<double>);
-    const size_t copies = mixed ? 2 : 1;
     const int ns = (int)hs.size();
     chunk_start.clear();
     size_t acc = 0;
@@ -581,11 +525,11 @@ static bs_status plan_tables(std::vector<Sphere>& hs, bool mixed, size_t budget,
     for (int i = 0; i < ns; i++) {
         Sphere& S = hs[i];
         S.lin_stride = mixed ? ((S.thetaR + 2) & ~1) : S.thetaR;
-        size_t need = (size_t)(S.dR + S.aR) * S.lin_stride * patch;
-        if (need * copies > budget)
-            return fail(BS_ERR_NOMEM, "LUT of sphere %d needs %zu bytes, over the budget of %zu", i + 1,
-                        need * copies, budget);
-        if (i == 0 || (acc + need) * copies > budget) {
+        // mixed: two rows or more per table, so that a lookup's row pair needs no clamp
+        size_t need = (size_t)(S.dR + (mixed ? std::max(S.aR, 2) : S.aR)) * S.lin_stride * patch;
+        if (need > budget)
+            return fail(BS_ERR_NOMEM, "LUT of sphere %d needs %zu bytes, over the budget of %zu", i + 1, need, budget);
+        if (i == 0 || acc + need > budget) {
             chunk_start.push_back(i);
             acc = 0;
         }
@@ -645,7 +589,7 @@ static bs_status plan_luts(bs_ctx* c, bool mixed, std::vector<int>& chunk_start,
     if (!budget) {
         size_t free_b = 0, total_b = 0;
         CK(cudaMemGetInfo(&free_b, &total_b));
-        budget = (size_t)(0.80 * (double)(free_b + c->d_lut.n * (mixed ? 2 : 1)));
+        budget = (size_t)(0.80 * (double)(free_b + c->d_lut.n));
     }
     return plan_tables(c->hs, mixed, budget, chunk_start, pool, maxrows, maxL);
 }
@@ -716,173 +660,66 @@ static void sort_waves(std::vector<double>& w, int chunk) {
     w.swap(out);
 }
 
-// Bounding cone (unit axis, half-angle in radians) of every `chunk`
-// consecutive waves, with a small margin for single-precision rounding.  A
-// chunk holding a direction that is not a unit vector gets half-angle pi,
-// which turns the angular window off for it.
-static std::vector<float4> wave_cones(const std::vector<double>& w, int chunk) {
-    size_t nk = w.size() / 3;
-    size_t nch = (nk + chunk - 1) / chunk;
-    std::vector<float4> out(nch);
-    for (size_t ch = 0; ch < nch; ch++) {
-        size_t a = ch * chunk, b = std::min(nk, a + chunk);
-        double m[3] = {0, 0, 0};
-        bool unit = true;
-        for (size_t i = a; i < b; i++) {
-            const double* k = &w[3 * i];
-            double kl = std::sqrt(k[0] * k[0] + k[1] * k[1] + k[2] * k[2]);
-            if (!(std::fabs(kl - 1.0) <= 1e-6)) unit = false;
-            for (int c = 0; c < 3; c++) m[c] += k[c];
-        }
-        double ml = std::sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
-        double beta = 0;
-        if (ml > 1e-3 && unit) {
-            for (int c = 0; c < 3; c++) m[c] /= ml;
-            for (size_t i = a; i < b; i++) {
-                const double* k = &w[3 * i];
-                double cth = k[0] * m[0] + k[1] * m[1] + k[2] * m[2];
-                beta = std::max(beta, std::acos(std::min(1.0, std::max(-1.0, cth))));
-            }
-        } else {
-            m[0] = 0, m[1] = 0, m[2] = 1;
-            beta = TRUE_PI;
-        }
-        out[ch] = make_float4((float)m[0], (float)m[1], (float)m[2], (float)(beta + 1e-4));
+// Bounding cone (unit axis, half-angle in radians, at most 2.9) of all directions; half-angle pi
+// if one of them is not a unit vector, which turns the mixed LUT kernel's angle bounds off.
+static float4 wave_cone(const std::vector<double>& w) {
+    double m[3] = {0, 0, 0};
+    for (size_t i = 0; i < w.size(); i += 3) {
+        const double l = std::sqrt(w[i] * w[i] + w[i + 1] * w[i + 1] + w[i + 2] * w[i + 2]);
+        if (!(std::fabs(l - 1.0) <= 1e-6)) return make_float4(0.f, 0.f, 1.f, (float)TRUE_PI);
+        for (int k = 0; k < 3; k++) m[k] += w[i + k];
     }
-    return out;
+    const double ml = std::sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+    if (!(ml > 1e-3)) return make_float4(0.f, 0.f, 1.f, 2.9f);
+    double c = 1;
+    for (size_t i = 0; i < w.size(); i += 3) c = std::min(c, (w[i] * m[0] + w[i + 1] * m[1] + w[i + 2] * m[2]) / ml);
+    return make_float4((float)(m[0] / ml), (float)(m[1] / ml), (float)(m[2] / ml),
+                       (float)std::min(2.9, std::acos(std::max(-1.0, c))));
 }
 
-// Predicted fraction of (tile, sphere, wave chunk) units whose table window
-// the staged mixed kernel can hold in shared memory, from the kernel's own
-// bounds evaluated on a sample of tiles, spheres and chunks: the tile's
-// distance range (nearest point of the tile rectangle, farthest corner) gives
-// the rows, the corners' angles from the tile-centre direction give gamma.
-// When few windows fit, the texture-only kernel is faster (no shared memory
-// taken from the texture cache).
-// Measured on the config-2 scene at 1536^2 near-field pixels (texture-only
-// kernel 383 ms): staged kernel with 23 % of windows staged 395 ms, 41 %
-// 360 ms, 85 % 329 ms; at 3072^2, 98 % staged 772 ms against 1510 ms.
-// The fraction of windows the staged kernel must fit to beat the texture-only
-// one: its texture fallback runs with the L1 that its shared-memory stage
-// leaves -- 64-wave chunks (51 KB x 4 blocks per SM): 0.3; smaller chunks
-// (72 KB x 3 blocks): 0.7 (served 256^2 - 512^2 requests with 48-62 % of
-// windows staged took 169-320 ms staged against 123-273 ms texture-only;
-// config 3 at 71 % 326 against 383 ms).
-static double staged_min_fraction(int chunk) { return chunk >= WAVE_CHUNK_MAX ? 0.3 : 0.7; }
-static double predict_staged_fraction(const bs_ctx* c, const std::vector<float4>& cones, int s0, int s1, int chunk) {
-    const int cap = lut_stage_entries(chunk);
+// Predicted fraction of the mixed LUT kernel's (tile, sphere, chunk) units whose columns fit
+// its window, from the kernel's own bounds on a sample of tiles and spheres: the tile's angular
+// radius seen from the sphere (its corners) and an even share of the angles between the
+// sampled directions and the tile centre's direction for each group of 32.
+static double predict_staged_fraction(const bs_ctx* c, const std::vector<double>& w) {
     const Scene& sc = c->sc;
-    const int R = sc.R, tiles = (R + LUT_TILE - 1) / LUT_TILE;
-    const int ts = std::max(1, tiles / 16), ss = std::max(1, (s1 - s0) / 32);
-    const int cs = std::max(1, (int)cones.size() / 16);
-    auto pos = [&](double u, double v, double* q) {
-        for (int k = 0; k < 3; k++) q[k] = sc.A[k] + sc.X[k] * (u / R) + sc.Y[k] * (v / R);
-    };
-    const double X2 = sc.X[0] * sc.X[0] + sc.X[1] * sc.X[1] + sc.X[2] * sc.X[2];
-    const double Y2 = sc.Y[0] * sc.Y[0] + sc.Y[1] * sc.Y[1] + sc.Y[2] * sc.Y[2];
+    const int R = sc.R, tiles = (R + LUT_TILE - 1) / LUT_TILE, ns = sc.ns;
+    const int nk = (int)(w.size() / 3), groups = (std::min(nk, 1024) + 31) / 32;
+    if (nk <= LUT_FEW_WAVES) return 0.0;
+    const int ts = std::max(1, tiles / 8), ss = std::max(1, ns / 4), ws = std::max(1, nk / 48);
     long long staged = 0, total = 0;
     for (int ty = 0; ty < tiles; ty += ts)
-        for (int tx = 0; tx < tiles; tx += ts) {
-            const double u0 = tx * LUT_TILE, v0 = ty * LUT_TILE;
-            const double u1 = std::min(u0 + LUT_TILE - 1, (double)R - 1), v1 = std::min(v0 + LUT_TILE - 1, (double)R - 1);
-            for (int si = s0; si < s1; si += ss) {
+        for (int tx = 0; tx < tiles; tx += ts)
+            for (int si = 0; si < ns; si += ss) {
                 const Sphere& S = c->hs[si];
-                double e[3];
-                for (int k = 0; k < 3; k++) e[k] = S.p[k] - sc.A[k];
-                // nearest point of the tile rectangle (X and Y span the plane at right angles)
-                const double un = std::min(std::max((e[0] * sc.X[0] + e[1] * sc.X[1] + e[2] * sc.X[2]) / X2 * R, u0), u1);
-                const double vn = std::min(std::max((e[0] * sc.Y[0] + e[1] * sc.Y[1] + e[2] * sc.Y[2]) / Y2 * R, v0), v1);
-                double q[3], ctr[3];
-                pos(un, vn, q);
-                const double dmin = std::sqrt((q[0] - S.p[0]) * (q[0] - S.p[0]) + (q[1] - S.p[1]) * (q[1] - S.p[1]) +
-                                              (q[2] - S.p[2]) * (q[2] - S.p[2]));
-                const int nch = (int)((cones.size() + cs - 1) / cs);
-                total += nch;
-                if (!(dmin >= S.a) || dmin == 0) continue;
-                pos(u0 + 7.5, v0 + 7.5, ctr);
-                double cl = 0;
-                for (int k = 0; k < 3; k++) {
-                    ctr[k] -= S.p[k];
-                    cl += ctr[k] * ctr[k];
-                }
-                cl = std::sqrt(cl);
-                double dmax = 0, gam = 0;
-                const double cu[4] = {u0, u1, u0, u1}, cv[4] = {v0, v0, v1, v1};
-                for (int k = 0; k < 4; k++) {
-                    pos(cu[k], cv[k], q);
-                    double r[3] = {q[0] - S.p[0], q[1] - S.p[1], q[2] - S.p[2]};
-                    const double d = std::sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-                    dmax = std::max(dmax, d);
-                    const double cosg = (r[0] * ctr[0] + r[1] * ctr[1] + r[2] * ctr[2]) / (d * cl);
-                    gam = std::max(gam, std::acos(std::min(1.0, std::max(-1.0, cosg))));
-                }
-                gam += LUT_STAGE_MARGIN;
-                auto row = [&](double d) {
-                    double x = (d - S.r0) / (S.dmax - S.r0) * (S.dR - 1);
-                    return (int)std::floor(std::min(std::max(x, 0.0), (double)(S.dR - 1)));
+                auto at = [&](double u, double v, double* q) {
+                    double l = 0;
+                    for (int k = 0; k < 3; k++) {
+                        q[k] = sc.A[k] + sc.X[k] * (u / R) + sc.Y[k] * (v / R) - S.p[k];
+                        l += q[k] * q[k];
+                    }
+                    l = std::sqrt(l);
+                    for (int k = 0; k < 3 && l > 0; k++) q[k] /= l;
                 };
-                const int rlo = row(dmin), nrows = std::min(row(dmax) + 1, S.dR - 1) - rlo + 1;
-                const double tsc = (S.thetaR - 1) / PI_REF;
-                for (size_t ch = 0; ch < cones.size(); ch += cs) {
-                    const float4 k = cones[ch];
-                    const double thc =
-                        std::acos(std::min(1.0, std::max(-1.0, (k.x * ctr[0] + k.y * ctr[1] + k.z * ctr[2]) / cl)));
-                    const int t_lo = std::max(0, (int)std::floor((thc - k.w - gam) * tsc) - 1);
-                    const int t_hi = std::min(S.thetaR, (int)std::floor((thc + k.w + gam) * tsc) + 2);
-                    const int W = t_hi - t_lo + 1;
-                    if (W >= 2 && (long long)nrows * lut_stage_stride(W) <= cap) staged++;
+                const double u0 = tx * LUT_TILE, v0 = ty * LUT_TILE, e = LUT_TILE - 1;
+                double ctr[3], q[3], cmin = 1;
+                at(u0 + 7.5, v0 + 7.5, ctr);
+                for (int k = 0; k < 4; k++) {
+                    at((k & 1) ? std::min(u0 + e, R - 1.0) : u0, (k & 2) ? std::min(v0 + e, R - 1.0) : v0, q);
+                    cmin = std::min(cmin, q[0] * ctr[0] + q[1] * ctr[1] + q[2] * ctr[2]);
                 }
+                const double gam = std::acos(std::max(-1.0, cmin)) + LUT_STAGE_MARGIN, tsc = (S.thetaR - 1) / PI_REF;
+                double lo = 1, hi = -1;
+                for (int i = 0; i < nk; i += ws) {
+                    const double d = w[3 * i] * ctr[0] + w[3 * i + 1] * ctr[1] + w[3 * i + 2] * ctr[2];
+                    lo = std::min(lo, d);
+                    hi = std::max(hi, d);
+                }
+                const double range = std::acos(std::max(-1.0, std::min(1.0, lo))) - std::acos(std::max(-1.0, std::min(1.0, hi)));
+                total++;
+                if (gam <= 1.4 && (range / groups + 2 * gam) * tsc + 4.5 <= LUT_WINDOW) staged++;
             }
-        }
     return total ? (double)staged / (double)total : 0.0;
-}
-
-// Waves per chunk for the mixed LUT kernel, with the matching wave order and
-// cones: the largest of 64, 32 and 16 whose predicted staged fraction reaches
-// 0.8, else the one with the largest fraction if that reaches its
-// staged_min_fraction, else the largest fraction among those that reach
-// theirs.  Smaller chunks have narrower cones, so more windows fit, but each
-// chunk pays a window copy, two barriers and a Kahan step.  64 whenever the
-// texture-only kernel will run; bs_set_lut_wave_chunk fixes the chunk instead.
-struct ChunkPlan {
-    int chunk = WAVE_CHUNK_MAX;
-    std::vector<double> w;
-    std::vector<float4> cones;
-    double predicted = 0;
-};
-
-static ChunkPlan choose_chunk(const bs_ctx* c, const std::vector<double>& waves, int ns) {
-    ChunkPlan first, best, viable;  // viable: the best that the staged kernel would run to advantage
-    best.predicted = viable.predicted = -1;
-    if (c->lut_chunk) {
-        best.chunk = c->lut_chunk;
-        best.w = waves;
-        sort_waves(best.w, best.chunk);
-        best.cones = wave_cones(best.w, best.chunk);
-        best.predicted = predict_staged_fraction(c, best.cones, 0, ns, best.chunk);
-        return best;
-    }
-    for (int cand : {WAVE_CHUNK_MAX, WAVE_CHUNK_MAX / 2, WAVE_CHUNK_MAX / 4}) {
-        ChunkPlan cp;
-        cp.chunk = cand;
-        cp.w = waves;
-        sort_waves(cp.w, cand);
-        cp.cones = wave_cones(cp.w, cand);
-        cp.predicted = predict_staged_fraction(c, cp.cones, 0, ns, cand);
-        if (cand == WAVE_CHUNK_MAX) {
-            first = cp;
-            if (c->lut_staging == 2) return first;
-        }
-        const bool enough = cp.predicted >= 0.8;
-        if (cp.predicted >= staged_min_fraction(cand) && cp.predicted > viable.predicted) viable = cp;
-        if (cp.predicted > best.predicted || enough) best = std::move(cp);
-        if (enough) break;
-    }
-    if (c->lut_staging == 0 && best.predicted < staged_min_fraction(best.chunk)) {
-        if (viable.predicted >= 0) return viable;
-        return first;  // 64-wave chunks below their threshold too: the texture-only kernel runs
-    }
-    return best;
 }
 
 // ---------------------------------------------------------------------------
@@ -900,20 +737,13 @@ static bs_status run_nearfield(bs_ctx* c) {
     // upload spheres and waves
     CK(c->d_sph.ensure(std::max(1, ns) * sizeof(Sphere)));
     std::vector<double> w(c->waves);
-    std::vector<float4> cones;
-    int chunk = WAVE_CHUNK_MAX;
-    double predicted = 0;
-    if (p.plane_wave) {
-        w.assign(p.k_dir, p.k_dir + 3);
-    } else if (!fp64 && p.scalar && p.lut_us && ns > 0) {
-        ChunkPlan cp = choose_chunk(c, w, ns);
-        chunk = cp.chunk;
-        w.swap(cp.w);
-        cones.swap(cp.cones);
-        predicted = cp.predicted;
-    } else {
-        sort_waves(w, chunk);
-    }
+    const int chunk = c->lut_chunk ? c->lut_chunk : WAVE_CHUNK_MAX;
+    const bool mixed_lut = !fp64 && p.scalar && p.lut_us && ns > 0;
+    float4 cone = make_float4(0.f, 0.f, 1.f, (float)TRUE_PI);
+    if (p.plane_wave) w.assign(p.k_dir, p.k_dir + 3);
+    if (mixed_lut) cone = wave_cone(w);  // ordered per tile on the device
+    else if (!p.plane_wave) sort_waves(w, WAVE_CHUNK_MAX);
+    const bool unit = cone.w < 3.f;  // the mixed LUT kernel's angle bounds hold
     c->stats.lut_wave_chunk = chunk;
     CK(c->d_waves.ensure(w.size() * sizeof(double)));
     CK(cudaMemcpyAsync(c->d_waves.p, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
@@ -1032,9 +862,7 @@ static bs_status run_nearfield(bs_ctx* c) {
         const int nchunks = (int)chunk_start.size() - 1;
         if (!fp64 && nchunks > 1) CK(c->d_kcmp.ensure((size_t)R * R * sizeof(float2)));
         bool use_stage = false;
-        int max_chunk = 0;
-        for (int ci = 0; ci < nchunks; ci++) max_chunk = std::max(max_chunk, chunk_start[ci + 1] - chunk_start[ci]);
-        // tables of the previous run still in the pool and in the texture slots?
+        // tables of the previous run still in the pool?
         std::vector<double> key;
         if (c->reuse && nchunks == 1) {
             key = {fp64 ? 1.0 : 0.0, sc.kmag, (double)c->Lmax, (double)ns};
@@ -1049,7 +877,7 @@ static bs_status run_nearfield(bs_ctx* c) {
         c->lut_valid = false;  // set again below once this run's tables are complete
         c->stats.lut_tables_built = reuse_now ? 0 : ns;
         if (!fp64 && ns > 0) {
-            // the texture planes are gather-capable 2D CUDA arrays (thetaR wide, rows + 1 high)
+            // tables of the mixed path stay within the GPU's 2D gather extent (thetaR wide, rows + 1 high)
             int maxw = 0, maxh = 0;
             CK(cudaDeviceGetAttribute(&maxw, cudaDevAttrMaxTexture2DGatherWidth, c->device));
             CK(cudaDeviceGetAttribute(&maxh, cudaDevAttrMaxTexture2DGatherHeight, c->device));
@@ -1059,25 +887,14 @@ static bs_status run_nearfield(bs_ctx* c) {
                                 "mixed precision: a %d x %d lookup table exceeds the %d x %d texture limit of this GPU "
                                 "(use BS_PREC_FP64 or fewer table samples)",
                                 std::max(S.dR, S.aR), S.thetaR, maxh - 1, maxw);
-            if ((int)c->slots.size() < max_chunk) c->slots.resize(max_chunk);
-            CK(c->d_texobj.ensure((size_t)4 * max_chunk * sizeof(unsigned long long)));
-            if (cones.empty()) {
-                cones = wave_cones(w, chunk);
-                predicted = predict_staged_fraction(c, cones, 0, ns, chunk);
-            }
-            c->stats.lut_staged_predicted = predicted;
-            use_stage = c->lut_staging == 1 ||
-                        (c->lut_staging == 0 && c->stats.lut_staged_predicted >= staged_min_fraction(chunk));
-            CK(c->d_cones.ensure(cones.size() * sizeof(float4)));
-            CK(cudaMemcpyAsync(c->d_cones.p, cones.data(), cones.size() * sizeof(float4), cudaMemcpyHostToDevice,
-                               c->st));
+            c->stats.lut_staged_predicted = unit ? predict_staged_fraction(c, w) : 0.0;
+            use_stage = unit && c->lut_staging != 2;
             CK(c->d_cnt.ensure(2 * sizeof(unsigned long long)));
             CK(cudaMemsetAsync(c->d_cnt.p, 0, 2 * sizeof(unsigned long long), c->st));
         }
         bool first_build = true;
         for (int ci = 0; ci < std::max(1, nchunks); ci++) {
             int s0 = ns > 0 ? chunk_start[ci] : 0, s1 = ns > 0 ? chunk_start[ci + 1] : 0;
-            std::vector<unsigned long long> handles;
             for (const CoefBatch& b : batches) {
                 if (reuse_now || b.b0 < s0 || b.b1 > s1) continue;
                 CK(cudaMemcpyAsync(c->d_starts.p, b.starts.data(), b.starts.size() * sizeof(long long),
@@ -1094,21 +911,14 @@ static bs_status run_nearfield(bs_ctx* c) {
                     for (int i = b.b0; i < b.b1; i++) {
                         const Sphere& S = c->hs[i];
                         const int L = S.Nl + 1;
-                        TexSlot& sl = c->slots[i - s0];
-                        if (t == 0) {
-                            // one spare row repeats the last, so a gather at the last row clamps as the texture would
-                            const int rows[4] = {S.dR, S.dR, S.aR, S.aR};
-                            for (int k = 0; k < 4; k++) CK(sl.ensure(k, S.thetaR, rows[k] + 1));
-                        }
                         LutBuildJob j{};
                         j.tab_off = b.starts[(size_t)(b.b1 - b.b0) + 1 + (i - b.b0)] + (t ? (long long)S.dR * L : 0);
                         j.lin_off = t ? S.uip_off : S.usp_off;
-                        j.rows = (t ? S.aR : S.dR) + 1;
+                        j.rows = t ? std::max(S.aR, 2) : S.dR;
+                        j.last = (t ? S.aR : S.dR) - 1;
                         j.L = L;
                         j.thetaR = S.thetaR;
                         j.lin_stride = S.lin_stride;
-                        j.sre = sl.surf[2 * t];
-                        j.sim = sl.surf[2 * t + 1];
                         max_rows = std::max(max_rows, j.rows);
                         max_theta = std::max(max_theta, S.thetaR);
                         jobs.push_back(j);
@@ -1119,10 +929,10 @@ static bs_status run_nearfield(bs_ctx* c) {
                     CK(cudaMemcpyAsync(jb.p, jobs.data(), jobs.size() * sizeof(LutBuildJob), cudaMemcpyHostToDevice,
                                        c->st));
                     for (size_t j0 = 0; j0 < jobs.size(); j0 += 65535) {  // the grid's z extent
-                        launch_lut_build_tex_batch(jb.as<LutBuildJob>() + j0,
-                                                   (int)std::min<size_t>(65535, jobs.size() - j0), max_rows, max_theta,
-                                                   c->d_tab.as<zd>(), c->d_legP.as<double>(), c->legP_L,
-                                                   c->d_lut.as<float2>(), c->st);
+                        launch_lut_build_mixed(jb.as<LutBuildJob>() + j0,
+                                               (int)std::min<size_t>(65535, jobs.size() - j0), max_rows, max_theta,
+                                               c->d_tab.as<zd>(), c->d_legP.as<double>(), c->legP_L,
+                                               c->d_lut.as<float2>(), c->st);
                         LAUNCHED(c);
                     }
                 }
@@ -1139,12 +949,6 @@ static bs_status run_nearfield(bs_ctx* c) {
                     LAUNCHED(c);
                 }
             }
-            if (!fp64)
-                for (int i = s0; i < s1; i++)
-                    for (int k = 0; k < 4; k++) handles.push_back(c->slots[i - s0].tex[k]);
-            if (!fp64 && !handles.empty())
-                CK(cudaMemcpyAsync(c->d_texobj.p, handles.data(), handles.size() * sizeof(unsigned long long),
-                                   cudaMemcpyHostToDevice, c->st));
             if (first_build) {
                 cudaEventRecord(c->ev[3], c->st);
                 first_build = false;
@@ -1154,15 +958,14 @@ static bs_status run_nearfield(bs_ctx* c) {
                 launch_us_lut_f64(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_waves.as<double>(),
                                   c->d_ph.as<zd>(), c->d_lut.as<Patch<double>>(), (const zd*)Uf, (zd*)U, c->st);
             } else {
-                launch_us_lut_tex(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_kw4.as<float4>(),
-                                  c->d_cones.as<float4>(), c->d_ph.as<cpx<float>>(),
-                                  c->d_texobj.as<unsigned long long>(), c->d_lut.as<float2>(), (const cpx<float>*)Uf,
-                                  (cpx<float>*)U, ns > 0 ? c->d_cnt.as<unsigned long long>() : nullptr,
-                                  nchunks > 1 ? c->d_kcmp.as<float2>() : nullptr, use_stage, chunk, c->st);
+                launch_us_lut_mixed(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_kw4.as<float4>(),
+                                    c->d_ph.as<cpx<float>>(), c->d_lut.as<float2>(), (const cpx<float>*)Uf,
+                                    (cpx<float>*)U, ns > 0 ? c->d_cnt.as<unsigned long long>() : nullptr,
+                                    nchunks > 1 ? c->d_kcmp.as<float2>() : nullptr, use_stage, chunk, cone, c->st);
             }
             LAUNCHED(c);
-            // the handle list and the table slots are reused by the next chunk
-            if (!fp64 && ci + 1 < std::max(1, nchunks)) CK(cudaStreamSynchronize(c->st));
+            c->tab_s0 = s0;
+            c->tab_s1 = s1;
         }
         if (!key.empty()) {
             c->lut_key.swap(key);
@@ -1217,23 +1020,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         b += B(thetaR * (size_t)c->Lmax * sizeof(double));    // Legendre table
         if (!fp64) {
             if (cs.size() > 2) b += B(R * R * sizeof(float2));  // Kahan carry between chunks
-            // slot k holds the k-th sphere of every chunk: the largest of those tables, plus a spare row each
-            size_t max_chunk = 0;
-            for (size_t ci = 0; ci + 1 < cs.size(); ci++) max_chunk = std::max(max_chunk, (size_t)(cs[ci + 1] - cs[ci]));
-            for (size_t k = 0; k < max_chunk; k++) {
-                size_t hd = 0, ha = 0;
-                for (size_t ci = 0; ci + 1 < cs.size(); ci++) {
-                    const size_t i = cs[ci] + k;
-                    if (i < (size_t)cs[ci + 1]) {
-                        hd = std::max(hd, (size_t)hs[i].dR + 1);
-                        ha = std::max(ha, (size_t)hs[i].aR + 1);
-                    }
-                }
-                // the planes' rows are allocated in multiples of 256 (TexSlot::ensure)
-                b += 2 * thetaR * (((hd + 255) & ~(size_t)255) + ((ha + 255) & ~(size_t)255)) * sizeof(float);
-            }
-            b += B(4 * max_chunk * sizeof(unsigned long long)) + B((nk + 15) / 16 * sizeof(float4)) +
-                 B(2 * sizeof(unsigned long long));
+            b += B(2 * sizeof(unsigned long long));
         }
     }
     std::vector<int> su, sv;
@@ -1841,47 +1628,21 @@ bs_status bs_sweep(bs_ctx* c, const double* lambdas, int32_t nl, const double* n
         if (!(lambdas[l] > 0)) return fail(BS_ERR_ARG, "bs_sweep: wavelength %d is not positive", l + 1);
     const bs_params saved_p = c->prm;
     const std::vector<bs_sphere> saved_s = c->spheres;
-    const int saved_staging = c->lut_staging;
     const size_t npix = (size_t)c->prm.resolution * c->prm.resolution;
-    // Empirical tuning of the mixed LUT kernel: with the choice left to the model
-    // and at least 4 bands, band 0 runs the staged kernel and band 1 the
-    // texture-only one; the faster serves the rest.  Both give the same bits, so
-    // the images do not depend on the choice.
-    const bool tune = saved_staging == 0 && prec == BS_PREC_MIXED && nl >= 4 && c->prm.scalar && c->prm.lut_us &&
-                      ns > 0;
-    float ms_stage = 0, ms_tex = 0;
     bs_status st = BS_OK;
-    // Both trial kernels run at the chunk a single auto-chosen run of this scene uses (the choice
-    // depends on the tile and table geometry, which is the same for every band), so every band has
-    // the bits of a single run.
-    const int saved_chunk = c->lut_chunk;
-    if (tune && saved_chunk == 0) {
-        c->prm.lambda = lambdas[0];
-        for (size_t i = 0; i < ns; i++) {
-            c->spheres[i].n_re = n_table[2 * i];
-            c->spheres[i].n_im = n_table[2 * i + 1];
-        }
-        st = derive(c);
-        if (st == BS_OK) c->lut_chunk = choose_chunk(c, c->waves, (int)ns).chunk;
-    }
     for (int32_t l = 0; l < nl && st == BS_OK; l++) {
         c->prm.lambda = lambdas[l];
         for (size_t i = 0; i < ns; i++) {
             c->spheres[i].n_re = n_table[2 * ((size_t)l * ns + i)];
             c->spheres[i].n_im = n_table[2 * ((size_t)l * ns + i) + 1];
         }
-        if (tune) c->lut_staging = l == 0 ? 1 : (l == 1 ? 2 : (ms_stage <= ms_tex ? 1 : 2));
         st = bs_simulate(c, prec);
-        if (tune && l == 0) ms_stage = c->stats.ms_us;
-        if (tune && l == 1) ms_tex = c->stats.ms_us;
         if (st == BS_OK && images) st = bs_get_image(c, kind, images + (size_t)l * npix, npix);
         if (st == BS_OK && envi_path)
             st = bs_write_envi(c, kind, envi_path, l > 0, band_as_nu ? 1e4 / lambdas[l] : lambdas[l]);
     }
     c->prm = saved_p;
     c->spheres = saved_s;
-    c->lut_staging = saved_staging;
-    c->lut_chunk = saved_chunk;
     c->have = false;
     return st;
 }
@@ -1898,8 +1659,6 @@ bs_status bs_get_info(bs_ctx* c, bs_info* out) {
     out->us_lut_theta = p.us_lut_theta > 0 ? p.us_lut_theta : 1000;
     int64_t tot = 0;
     for (const DevBuf* b : ctx_bufs(c)) tot += (int64_t)b->n;
-    for (const auto& sl : c->slots)
-        for (int k = 0; k < 4; k++) tot += (int64_t)sl.w * sl.h[k] * (int64_t)sizeof(float);
     out->device_bytes = tot;
     return BS_OK;
 }
@@ -1938,17 +1697,14 @@ bs_status bs_get_lut(bs_ctx* c, int32_t sphere, int32_t which, double* host, siz
             host[2 * i + 1] = t[i].v[1];
         }
     } else {
-        int slot = sphere;  // valid when the last run held every sphere in one chunk
-        if (slot >= (int)c->slots.size() || !c->slots[slot].arr[which * 2])
+        if (sphere < c->tab_s0 || sphere >= c->tab_s1)
             return fail(BS_ERR_STATE, "bs_get_lut: table of sphere %d not resident", sphere);
-        std::vector<float> re(n), im(n);
-        CK(cudaMemcpy2DFromArray(re.data(), S.thetaR * sizeof(float), c->slots[slot].arr[which * 2], 0, 0,
-                                 S.thetaR * sizeof(float), rows, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy2DFromArray(im.data(), S.thetaR * sizeof(float), c->slots[slot].arr[which * 2 + 1], 0, 0,
-                                 S.thetaR * sizeof(float), rows, cudaMemcpyDeviceToHost));
+        std::vector<float2> t(n);
+        CK(cudaMemcpy2D(t.data(), S.thetaR * sizeof(float2), c->d_lut.as<float2>() + off, S.lin_stride * sizeof(float2),
+                        S.thetaR * sizeof(float2), rows, cudaMemcpyDeviceToHost));
         for (size_t i = 0; i < n; i++) {
-            host[2 * i] = re[i];
-            host[2 * i + 1] = im[i];
+            host[2 * i] = t[i].x;
+            host[2 * i + 1] = t[i].y;
         }
     }
     return BS_OK;

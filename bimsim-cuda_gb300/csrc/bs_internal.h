@@ -57,6 +57,9 @@ struct Sphere {
     int coef_off;            // first order of this sphere in the coefficient arrays
     int lin_stride;          // mixed path: row stride of the linear float2 tables (thetaR + 1, even)
     double xs_usp, xs_uip;   // (dR - 1) / (dmax - r0) and (aR - 1) / (a - dmin): radial index scales
+    float tsc;               // table columns per radian, (thetaR - 1) / PI_REF
+    float hp_hi, hp_lo;      // pi / 2 in columns, rounded, and the rest
+    float pad_;
 };
 
 // Host helpers (bs_host.cpp).

@@ -9,25 +9,13 @@
 
 namespace bs {
 
-// Plane waves are processed in chunks of 64, 32 or 16 (chosen per run from the
-// predicted fraction of staged windows) after grouping them by direction; the
-// host supplies one bounding cone per chunk.
-constexpr int WAVE_CHUNK_MAX = 64;
-
-// Mixed LUT kernel staging: float2 table values a 16 x 16 pixel tile stages
-// per wave chunk, and the angle margin (radians) added to its window bounds.
-// 64-wave chunks (two pixels per thread, 128 registers): 51 KB, 4 blocks per
-// SM (config 2: 99.6 % of windows staged; 43 KB: 98 %, 730 against 721 ms);
-// 32- and 16-wave chunks (one pixel per thread, coarser pixel pitches): 72 KB,
-// 3 blocks per SM, so that wider windows fit -- config 3 266 against 305 ms
-// per band, config 5 at 512^2 9.9 against 11.7 s, both with 32-wave chunks
-// where 43 KB windows needed 16.
+// Mixed LUT kernel: angle margin (radians) of its window bounds, and the number of
+// directions up to which one thread per pixel reads every cell itself.
+constexpr float LUT_STAGE_MARGIN = 5e-4f;
+constexpr int LUT_FEW_WAVES = 32;
 constexpr int LUT_TILE = 16;
-__host__ __device__ constexpr int lut_stage_entries(int chunk) { return chunk >= 64 ? 6400 : 9000; }
-constexpr float LUT_STAGE_MARGIN = 2e-3f;
-// Shared-memory row stride of a staged window W entries wide: odd, so that
-// lanes reading the same column of different rows fall in different banks.
-__host__ __device__ constexpr int lut_stage_stride(int W) { return W | 1; }
+constexpr int LUT_WINDOW = 64;  // table columns of a staged window
+constexpr int WAVE_CHUNK_MAX = 64;
 
 template <class T>
 struct cpx;
@@ -39,6 +27,7 @@ using zd = cpx<double>;
 // first to use a kernel waited for the long slices on the other workers' streams:
 // p50 8.3 s against 1.9 s with every kernel loaded up front).
 void preload_nearfield_kernels();
+void preload_uslut_kernels();
 void preload_detector_kernels();
 
 // One bilinear LUT cell at (r, t): {T00, T10 - T00, T01 - T00, T11 - T10 - T01 + T00}
@@ -66,34 +55,30 @@ void launch_phase(const Scene& sc, const Sphere* sph, const double* waves, cpx<T
 void launch_us_lut_f64(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
                        const double* waves, const zd* ph, const Patch<double>* lut, const zd* Uf, zd* U,
                        cudaStream_t st);
-// mixed path: tex holds, for sphere s0 + j, the texture objects of
-// {Usp re, Usp im, Uip re, Uip im} at [4 j .. 4 j + 3]
-// lin: linear float2 tables (Sphere::usp_off / uip_off in float2 units, rows
-// of Sphere::lin_stride entries);
-// cones: one {axis, half-angle} per `chunk` waves; counters[0..1] receive
-// the staged and total (sphere, chunk) counts of every block (may be null);
-// kcmp (R x R, or null with a single sphere chunk) carries each pixel's Kahan
+// mixed path.  lin: linear float2 tables (Sphere::usp_off / uip_off in float2 units, rows
+// of Sphere::lin_stride entries, even and 16-byte aligned);
+// counters[0..1] receive the staged and total (tile, sphere, chunk of `chunk` waves) counts
+// (may be null); kcmp (R x R, or null with a single sphere chunk) carries each pixel's Kahan
 // compensation from one sphere chunk's launch to the next, so that chunked
 // tables give the bits of one launch over all spheres;
-// stage = false runs the texture-only variant
-void launch_us_lut_tex(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
-                       const float4* kw4, const float4* cones, const cpx<float>* ph, const unsigned long long* tex,
-                       const float2* lin, const cpx<float>* Uf, cpx<float>* U, unsigned long long* counters,
-                       float2* kcmp, bool stage, int chunk, cudaStream_t st);
-// One table of the mixed path's table build: the rows (one spare) of one
-// sphere's Usp or Uip with their coefficient rows at tab + tab_off, written to
-// the planes sre/sim and the linear rows at lin + lin_off.
+// stage = false reads every cell from the tables; cone: axis and half-angle of a cone that holds
+// every direction (half-angle pi: directions that are not unit vectors)
+void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
+                         const float4* kw4, const cpx<float>* ph, const float2* lin, const cpx<float>* Uf,
+                         cpx<float>* U, unsigned long long* counters, float2* kcmp, bool stage, int chunk,
+                         float4 cone, cudaStream_t st);
+// One table of the mixed path's table build: the rows of one sphere's Usp or Uip with their
+// coefficient rows at tab + tab_off, written to the linear rows at lin + lin_off.
 struct LutBuildJob {
     long long tab_off, lin_off;
     int rows, L, thetaR, lin_stride;
-    cudaSurfaceObject_t sre, sim;
+    int last;  // rows above this one repeat it (a Uip of one row is stored twice)
 };
 // the tables of `jobs` (device array of njobs <= 65535 entries, at most max_rows
 // rows and max_theta angles each) in one launch: the sums of launch_lut_build in
-// double, stored as float in the real and imaginary planes (CUDA arrays, through
-// surfaces) and in the linear rows used for staging
-void launch_lut_build_tex_batch(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab,
-                                const double* P, int Pstride, float2* lin, cudaStream_t st);
+// double, stored as float in linear rows whose last column is repeated
+void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab,
+                            const double* P, int Pstride, float2* lin, cudaStream_t st);
 
 // Direct scattered field through the addition theorem of spherical harmonics:
 // recurrence factors rec, per-wave tables tab (nk x L(L+1)/2), per-sphere

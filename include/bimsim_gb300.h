@@ -120,8 +120,8 @@ typedef struct bs_stats {
     int64_t lut_chunks_staged;
     int64_t lut_chunks_total;
     int64_t lut_tables_built;  /* sphere tables (Usp + Uip) built; 0 when reused */
-    double lut_staged_predicted;  /* the kernel choice's model of lut_chunks_staged / total */
-    int64_t lut_wave_chunk;       /* waves per chunk of the mixed LUT kernel (64, 32 or 16) */
+    double lut_staged_predicted;  /* a host model of lut_chunks_staged / total */
+    int64_t lut_wave_chunk;       /* waves per counted chunk of the mixed LUT kernel (64, 32 or 16) */
 } bs_stats;
 
 typedef struct bs_ctx bs_ctx;
@@ -305,9 +305,7 @@ bs_status bs_plane_point(const bs_params* params, double u, double v, double* xy
  * may be NULL) and, when envi_path is given, to band l of that ENVI file
  * (band value lambda, or 1e4/lambda when band_as_nu).  The context's own
  * wavelength and indices are restored afterwards; results of the last
- * band are dropped.  With bs_set_lut_staging left at 0 and at least 4 mixed
- * bands, bands 0 and 1 time the staged and texture-only LUT kernels and the
- * faster runs the rest (identical bits either way). */
+ * band are dropped. */
 bs_status bs_sweep(bs_ctx* ctx, const double* lambdas, int32_t nl, const double* n_table, bs_precision prec,
                    bs_image_kind kind, float* images, const char* envi_path, int32_t band_as_nu);
 
@@ -320,15 +318,14 @@ bs_status bs_sweep(bs_ctx* ctx, const double* lambdas, int32_t nl, const double*
  * >= k^2).  The incident field Uf is not propagated.  Off by default. */
 bs_status bs_set_backpropagation(bs_ctx* ctx, int32_t enable, double d);
 
-/* Waves per chunk of the mixed LUT kernel: 0 (default) picks 64, 32 or 16 per
- * run from the predicted fraction of staged windows; 16, 32 or 64 fixes it.
- * The staged and texture-only kernels give the same bits at the same chunk. */
+/* Waves per counted chunk of the mixed LUT kernel (lut_chunks_staged and
+ * lut_chunks_total of bs_stats): 0 (default) is 64; 16, 32 or 64 fixes it.
+ * Results do not depend on it. */
 bs_status bs_set_lut_wave_chunk(bs_ctx* ctx, int32_t chunk);
 
-/* Kernel of the mixed-precision LUT stage: 0 (default) chooses from a model
- * of how many table windows fit in shared memory, 1 always stages windows in
- * shared memory (texture gathers where a window does not fit), 2 uses texture
- * gathers only.  All three give the same bits.  No reference counterpart. */
+/* Kernel of the mixed-precision LUT stage: 0 (default) and 1 keep windows of
+ * the tables in shared memory where they fit, 2 reads every cell from the
+ * tables.  All give the same bits.  No reference counterpart. */
 bs_status bs_set_lut_staging(bs_ctx* ctx, int32_t mode);
 
 /* Keep the lookup tables of the last run and skip rebuilding them when the
