@@ -133,6 +133,8 @@ struct bs_ctx {
     DevBuf d_fields;  // [2][R*R] U then Uf
     DevBuf d_su, d_sv, d_mask, d_wx, d_wy, d_wix, d_wiy, d_f1, d_f2, d_g1, d_I, d_D, d_img;
     int legP_theta = 0, legP_L = 0;
+    bool legP_split = false;  // d_legP holds the mixed path's order-major split values
+    DevBuf d_bias;            // mixed path: bias of every coefficient row
     int tab_s0 = 0, tab_s1 = 0;  // spheres whose tables the last run left in d_lut
     int64_t launches = 0;
     int64_t interactions = 0;
@@ -155,7 +157,7 @@ struct bs_ctx {
 // Every linear device buffer of a context.
 static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
     return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_mie, &c->d_tab,
-            &c->d_tabscr, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
+            &c->d_tabscr, &c->d_bias, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
             &c->d_sv, &c->d_mask, &c->d_wx, &c->d_wy, &c->d_wix, &c->d_wiy, &c->d_f1, &c->d_f2,
             &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_far,
             &c->d_starts, &c->d_lbjobs, &c->d_lbjobs2, &c->d_kcmp, &c->d_fsave, &c->d_dacc, &c->d_line, &c->d_ringcs, &c->d_bp, &c->d_shrec, &c->d_shtab, &c->d_shcoef, &c->d_gscr, &c->d_ufw};
@@ -843,18 +845,22 @@ static bs_status run_nearfield(bs_ctx* c) {
         int thetaR = ns > 0 ? c->hs[0].thetaR : 1000;
         if (ns > 0) {
             CK(c->d_lut.ensure(pool));
-            long long maxcoef = 0, maxstarts = 0;
+            long long maxcoef = 0, maxstarts = 0, maxrow = 0;
             for (const CoefBatch& b : batches) {
                 maxcoef = std::max(maxcoef, b.coefs);
+                maxrow = std::max(maxrow, b.rows);
                 maxstarts = std::max(maxstarts, (long long)b.starts.size());
             }
             CK(c->d_tab.ensure((size_t)maxcoef * sizeof(zd)));
             CK(c->d_tabscr.ensure((size_t)maxcoef * 2 * sizeof(double)));
             CK(c->d_starts.ensure((size_t)maxstarts * sizeof(long long)));
-            if (c->legP_theta != thetaR || c->legP_L < c->Lmax) {
+            if (!fp64) CK(c->d_bias.ensure((size_t)maxrow * sizeof(float)));
+            if (c->legP_theta != thetaR || c->legP_L < c->Lmax || c->legP_split != !fp64) {
                 CK(c->d_legP.ensure((size_t)thetaR * c->Lmax * sizeof(double)));
-                launch_legendre_table(thetaR, c->Lmax, c->d_legP.as<double>(), c->st);
+                if (fp64) launch_legendre_table(thetaR, c->Lmax, c->d_legP.as<double>(), c->st);
+                else launch_legendre_split(thetaR, c->Lmax, thetaR, c->d_legP.as<float2>(), c->st);
                 LAUNCHED(c);
+                c->legP_split = !fp64;
                 c->legP_theta = thetaR;
                 c->legP_L = c->Lmax;
             }
@@ -901,7 +907,7 @@ static bs_status run_nearfield(bs_ctx* c) {
                                    cudaMemcpyHostToDevice, c->st));
                 launch_coef_rows_batch(c->d_sph.as<Sphere>(), b.b0, b.b1 - b.b0, c->d_starts.as<long long>(), b.rows,
                                        sc.kmag, c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_tab.as<zd>(),
-                                       c->d_tabscr.as<double>(), c->st);
+                                       c->d_tabscr.as<double>(), fp64 ? nullptr : c->d_bias.as<float>(), c->st);
                 LAUNCHED(c);
                 // mixed path: the tables of every sphere of the batch in two launches (the
                 // dR-row Usp tables, then the shorter Uip tables)
@@ -914,6 +920,7 @@ static bs_status run_nearfield(bs_ctx* c) {
                         LutBuildJob j{};
                         j.tab_off = b.starts[(size_t)(b.b1 - b.b0) + 1 + (i - b.b0)] + (t ? (long long)S.dR * L : 0);
                         j.lin_off = t ? S.uip_off : S.usp_off;
+                        j.row_off = b.starts[i - b.b0] + (t ? S.dR : 0);
                         j.rows = t ? std::max(S.aR, 2) : S.dR;
                         j.last = (t ? S.aR : S.dR) - 1;
                         j.L = L;
@@ -931,8 +938,8 @@ static bs_status run_nearfield(bs_ctx* c) {
                     for (size_t j0 = 0; j0 < jobs.size(); j0 += 65535) {  // the grid's z extent
                         launch_lut_build_mixed(jb.as<LutBuildJob>() + j0,
                                                (int)std::min<size_t>(65535, jobs.size() - j0), max_rows, max_theta,
-                                               c->d_tab.as<zd>(), c->d_legP.as<double>(), c->legP_L,
-                                               c->d_lut.as<float2>(), c->st);
+                                               c->d_tab.as<zd>(), c->d_bias.as<float>(), c->d_legP.as<float2>(),
+                                               thetaR, c->d_lut.as<float2>(), c->st);
                         LAUNCHED(c);
                     }
                 }
@@ -1010,15 +1017,17 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         if (plan_tables(hs, !fp64, lut_budget ? lut_budget : SIZE_MAX / 4, cs, pool, maxrows, maxL) != BS_OK)
             return 0;
         const size_t thetaR = hs[0].thetaR;
-        long long maxcoef = 0, maxstarts = 0;
+        long long maxcoef = 0, maxstarts = 0, maxrow = 0;
         for (const CoefBatch& cb : coef_batches(hs, cs)) {
             maxcoef = std::max(maxcoef, cb.coefs);
+            maxrow = std::max(maxrow, cb.rows);
             maxstarts = std::max(maxstarts, (long long)cb.starts.size());
         }
         b += B(pool) + B((size_t)maxcoef * sizeof(zd)) + B((size_t)maxcoef * 2 * sizeof(double)) +
              B((size_t)maxstarts * sizeof(long long));
         b += B(thetaR * (size_t)c->Lmax * sizeof(double));    // Legendre table
         if (!fp64) {
+            b += B((size_t)maxrow * sizeof(float));
             if (cs.size() > 2) b += B(R * R * sizeof(float2));  // Kahan carry between chunks
             b += B(2 * sizeof(unsigned long long));
         }

@@ -43,9 +43,16 @@ void launch_uf(const Scene& sc, const double* tab, const double* w, cpx<T>* Uf, 
 void launch_uf_table(const Scene& sc, double* tab, double* scratch, cudaStream_t st);
 void launch_mie(const Sphere* sph, int ns, double k, zd* scratch, int lstride, zd* A, zd* B, cudaStream_t st);
 // spheres [s0, s0 + n) in one launch; starts (device): first global row of each
-// sphere (n + 1 values, the last = total_rows) then first coefficient (n values)
+// sphere (n + 1 values, the last = total_rows) then first coefficient (n values);
+// bias (device, one float per row) selects the mixed path's split coefficients
+struct SplitCoef {
+    float hr, hi, lr, li;  // a complex coefficient: nearest floats and the rests; the size of a zd
+};
 void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows,
-                            double k, const zd* A, const zd* B, zd* tab, double* scratch, cudaStream_t st);
+                            double k, const zd* A, const zd* B, zd* tab, double* scratch, float* bias,
+                            cudaStream_t st);
+// Legendre values of the mixed path: P[l * stride + t] = {nearest float, rest}
+void launch_legendre_split(int thetaR, int Lmax, int stride, float2* P, cudaStream_t st);
 void launch_legendre_table(int thetaR, int Lmax, double* P, cudaStream_t st);
 template <class T>
 void launch_lut_build(const zd* tab, int rows, int L, const double* P, int Pstride, int thetaR, Patch<T>* out,
@@ -68,17 +75,17 @@ void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int
                          cpx<float>* U, unsigned long long* counters, float2* kcmp, bool stage, int chunk,
                          float4 cone, cudaStream_t st);
 // One table of the mixed path's table build: the rows of one sphere's Usp or Uip with their
-// coefficient rows at tab + tab_off, written to the linear rows at lin + lin_off.
+// coefficient rows at tab + tab_off and biases at bias + row_off, written to the linear rows at
+// lin + lin_off.
 struct LutBuildJob {
-    long long tab_off, lin_off;
+    long long tab_off, lin_off, row_off;
     int rows, L, thetaR, lin_stride;
     int last;  // rows above this one repeat it (a Uip of one row is stored twice)
 };
-// the tables of `jobs` (device array of njobs <= 65535 entries, at most max_rows
-// rows and max_theta angles each) in one launch: the sums of launch_lut_build in
-// double, stored as float in linear rows whose last column is repeated
+// the tables of `jobs` (device array of njobs <= 65535 entries, at most max_rows rows and max_theta
+// angles each) in one launch; tab holds SplitCoef entries
 void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab,
-                            const double* P, int Pstride, float2* lin, cudaStream_t st);
+                            const float* bias, const float2* P, int Pstride, float2* lin, cudaStream_t st);
 
 // Direct scattered field through the addition theorem of spherical harmonics:
 // recurrence factors rec, per-wave tables tab (nk x L(L+1)/2), per-sphere

@@ -164,11 +164,13 @@ __global__ void mie_kernel(const Sphere* __restrict__ sph, int ns, double k, zd*
 // Thread g takes global row g; starts[i] / starts[n + 1 + i] are sphere i's
 // first global row and its first coefficient in tab (rows of Nl + 1
 // coefficients; starts[n], the total row count, bounds the grid).  The scratch
-// holds 2 (Nl + 1) doubles per row.
+// holds 2 (Nl + 1) doubles per row.  With `bias` (mixed path) every coefficient
+// is stored as SplitCoef instead, and bias[g] is a power of two of at least
+// twice the sum of the row's coefficients, see lut_build_mixed_kernel.
 __global__ void coef_rows_batch_kernel(const Sphere* __restrict__ sph, int s0, int n,
                                        const long long* __restrict__ starts, double k, const zd* __restrict__ A,
                                        const zd* __restrict__ B, zd* __restrict__ tab,
-                                       double* __restrict__ scratch) {
+                                       double* __restrict__ scratch, float* __restrict__ bias) {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= starts[n]) return;
     int lo = 0, hi = n - 1;  // last sphere whose first row is <= g
@@ -189,16 +191,31 @@ __global__ void coef_rows_batch_kernel(const Sphere* __restrict__ sph, int s0, i
         sph_real(S.Nl, k * r, sj, sj + L, 1);
         for (int l = 0; l < L; l++) out[l] = B[S.coef_off + l] * mk(sj[l], sj[L + l]);
     } else {
-        int ia = row - S.dR;
+        const int ia = row - S.dR;
         if (ia == 0) {
             for (int l = 0; l < L; l++) out[l] = (l == 0) ? A[S.coef_off] * mk(1.0, 0.0) : A[S.coef_off + l] * mk(0.0, 0.0);
-            return;
+        } else {
+            double da = S.a / (S.aR - 1);
+            double r = ia * da;
+            zd knr = (mk(S.n_re, S.n_im) * k) * r;
+            sph_complex(S.Nl, knr, true, out, nullptr, nullptr, nullptr);
+            for (int l = 0; l < L; l++) out[l] = A[S.coef_off + l] * out[l];
         }
-        double da = S.a / (S.aR - 1);
-        double r = ia * da;
-        zd knr = (mk(S.n_re, S.n_im) * k) * r;
-        sph_complex(S.Nl, knr, true, out, nullptr, nullptr, nullptr);
-        for (int l = 0; l < L; l++) out[l] = A[S.coef_off + l] * out[l];
+    }
+    if (bias) {
+        float sum = 0.f;
+        SplitCoef* sc = reinterpret_cast<SplitCoef*>(out);
+        for (int l = 0; l < L; l++) {
+            const zd c = out[l];
+            SplitCoef q;
+            q.hr = (float)c.re;
+            q.hi = (float)c.im;
+            q.lr = (float)(c.re - (double)q.hr);
+            q.li = (float)(c.im - (double)q.hi);
+            sc[l] = q;
+            sum += fmaxf(fabsf(q.hr), fabsf(q.hi));
+        }
+        bias[g] = scalbnf(1.f, ilogbf(fmaxf(sum, 1e-30f)) + 2);
     }
 }
 
@@ -217,6 +234,22 @@ __global__ void legendre_table_kernel(int thetaR, int Lmax, double* __restrict__
     for (int l = 2; l < Lmax; l++) {
         legendre_step(l, x, P0, P1);
         row[l] = P1;
+    }
+}
+
+// The mixed path's copy of that table, order-major: P_l of angle t at P[l * stride + t] as the
+// nearest float and the rest.
+__global__ void legendre_split_kernel(int thetaR, int Lmax, int stride, float2* __restrict__ P) {
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= thetaR) return;
+    double dtheta = (double)__fdiv_rn(3.14159f, (float)(thetaR - 1));
+    double x = cos(dtheta * t);
+    double P0 = 1, P1 = x;
+    for (int l = 0; l < Lmax; l++) {
+        if (l > 1) legendre_step(l, x, P0, P1);
+        const double v = l == 0 ? 1.0 : P1;
+        const float h = (float)v;
+        P[(size_t)l * stride + t] = make_float2(h, (float)(v - (double)h));
     }
 }
 
@@ -344,25 +377,116 @@ __global__ void __launch_bounds__(128) us_lut_f64_kernel(Scene sc, const Sphere*
     U[idx] = total;
 }
 
-// Mixed path: the same sums as lut_build_kernel for the tables of a sphere batch in one launch, stored
-// as float2 in linear rows with the last column repeated (a lookup's right neighbour needs no clamp).
-// blockIdx.z picks the table, blockIdx.y its block of 8 rows (blocks past the table's rows return) and
-// blockIdx.x a block of 32 angles.
-__global__ void __launch_bounds__(256) lut_build_mixed_kernel(const LutBuildJob* __restrict__ jobs,
-                                                              const zd* __restrict__ tab,
-                                                              const double* __restrict__ P, int Pstride,
-                                                              float2* __restrict__ lin) {
+// Mixed path: the sums of lut_build_kernel for the tables of a sphere batch in one launch, stored as
+// float2 in linear rows with the last column repeated (a lookup's right neighbour needs no clamp).
+//
+// The sums were bound by the FP64 pipe (2 DFMA per entry and order at 1/64 of the single-precision
+// rate).  Here coefficients and Legendre values are split into two floats each, and a sum is kept as
+// H + lo: H starts at the row's bias, a power of two of at least twice the sum of |coefficients|, so
+// that H + c p rounds to a multiple of ulp(bias), its change (H' - H) is exact, and what the rounding
+// left of the product, c p - (H' - H), comes from one fused multiply-add; lo collects those rests and
+// the cross terms.  H - bias is exact, so the result carries about 46 bits relative to the bias and
+// its float is the double-precision sum's but next to a rounding boundary (6 of 100 000 entries differ in
+// the last bit; the tables' error against double precision is 2.6e-8 either way).  Six packed
+// instructions per (entry, order).  GB300, 50 spheres x 4096 x 1024: 12.4 -> 2.2 ms with the
+// coefficient rows; 120 spheres 25.6 -> 4.3 ms.
+// A block makes 32 rows x 128 angles, a thread 4 rows x 4 angles (angles one warp apart: coalesced
+// rows), with LBM_L orders of both factors in shared memory at a time.
+constexpr int LBM_R = 32, LBM_T = 128, LBM_L = 16;
+
+__device__ __forceinline__ unsigned long long pk2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long pk_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long pk_add(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long pk_sub(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__global__ void __launch_bounds__(256, 2) lut_build_mixed_kernel(const LutBuildJob* __restrict__ jobs,
+                                                                 const SplitCoef* __restrict__ tab,
+                                                                 const float* __restrict__ bias,
+                                                                 const float2* __restrict__ P, int Pstride,
+                                                                 float2* __restrict__ lin) {
+    __shared__ SplitCoef sc[LBM_L][LBM_R];
+    __shared__ float2 sp[LBM_L][LBM_T];
     const LutBuildJob& j = jobs[blockIdx.z];
-    const int r = blockIdx.y * 8 + (threadIdx.x >> 5), t = blockIdx.x * 32 + (threadIdx.x & 31);
-    if (r >= j.rows || t >= j.thetaR) return;
-    const zd* c = tab + j.tab_off + (size_t)min(r, j.last) * j.L;
-    const double* pl = P + (size_t)t * Pstride;
-    zd acc = mk(0.0, 0.0);
-    for (int l = 0; l < j.L; l++) acc = acc + c[l] * pl[l];
-    const float2 v = make_float2((float)acc.re, (float)acc.im);
-    float2* row = lin + j.lin_off + (size_t)r * j.lin_stride;
-    row[t] = v;
-    if (t == j.thetaR - 1) row[j.thetaR] = v;
+    const int r0 = blockIdx.y * LBM_R, t0 = blockIdx.x * LBM_T;
+    if (r0 >= j.rows || t0 >= j.thetaR) return;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, L = j.L, thetaR = j.thetaR, last = j.last;
+    const SplitCoef* c = tab + j.tab_off;
+    unsigned long long H[4][4], lo[4][4];
+    float b[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        b[i] = bias[j.row_off + min(r0 + ty + 8 * i, last)];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            H[i][k] = pk2(b[i], b[i]);
+            lo[i][k] = 0ull;
+        }
+    }
+    for (int l0 = 0; l0 < L; l0 += LBM_L) {
+        const int nl = min(LBM_L, L - l0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < LBM_R * LBM_L; e += 256) {
+            const int l = e % LBM_L, r = e / LBM_L;
+            if (l < nl) sc[l][r] = c[(size_t)min(r0 + r, last) * L + l0 + l];
+        }
+        for (int e = threadIdx.x; e < LBM_T * nl; e += 256) {
+            const int t = e % LBM_T, l = e / LBM_T;
+            sp[l][t] = P[(size_t)(l0 + l) * Pstride + min(t0 + t, thetaR - 1)];
+        }
+        __syncthreads();
+        for (int l = 0; l < nl; l++) {
+            unsigned long long ph[4], pl[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float2 p = sp[l][tx + 32 * k];
+                ph[k] = pk2(p.x, p.x);
+                pl[k] = pk2(p.y, p.y);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const SplitCoef q = sc[l][ty + 8 * i];
+                const unsigned long long ch = pk2(q.hr, q.hi), cl = pk2(q.lr, q.li);
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const unsigned long long h = pk_fma(ch, ph[k], H[i][k]);
+                    const unsigned long long rest = pk_fma(ch, ph[k], pk_sub(H[i][k], h));
+                    H[i][k] = h;
+                    lo[i][k] = pk_fma(cl, ph[k], pk_fma(ch, pl[k], pk_add(lo[i][k], rest)));
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int r = r0 + ty + 8 * i;
+        if (r >= j.rows) continue;
+        float2* row = lin + j.lin_off + (size_t)r * j.lin_stride;
+        const unsigned long long bb = pk2(b[i], b[i]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int t = t0 + tx + 32 * k;
+            if (t >= thetaR) continue;
+            const unsigned long long v = pk_add(pk_sub(H[i][k], bb), lo[i][k]);
+            *reinterpret_cast<unsigned long long*>(row + t) = v;
+            if (t == thetaR - 1) *reinterpret_cast<unsigned long long*>(row + thetaR) = v;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -629,9 +753,14 @@ void launch_mie(const Sphere* sph, int ns, double k, zd* scratch, int lstride, z
 }
 
 void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows,
-                            double k, const zd* A, const zd* B, zd* tab, double* scratch, cudaStream_t st) {
+                            double k, const zd* A, const zd* B, zd* tab, double* scratch, float* bias,
+                            cudaStream_t st) {
     coef_rows_batch_kernel<<<(unsigned)((total_rows + 127) / 128), 128, 0, st>>>(sph, s0, n, starts, k, A, B, tab,
-                                                                               scratch);
+                                                                               scratch, bias);
+}
+
+void launch_legendre_split(int thetaR, int Lmax, int stride, float2* P, cudaStream_t st) {
+    legendre_split_kernel<<<blocks_for(thetaR, 64), 64, 0, st>>>(thetaR, Lmax, stride, P);
 }
 
 void launch_legendre_table(int thetaR, int Lmax, double* P, cudaStream_t st) {
@@ -660,10 +789,10 @@ void launch_us_lut_f64(const Scene& sc, const Sphere* sph, int s0, int s1, int a
 }
 
 void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab,
-                            const double* P, int Pstride, float2* lin, cudaStream_t st) {
+                            const float* bias, const float2* P, int Pstride, float2* lin, cudaStream_t st) {
     if (njobs < 1 || max_rows < 1) return;
-    dim3 grid(blocks_for(max_theta, 32), blocks_for(max_rows, 8), (unsigned)njobs);
-    lut_build_mixed_kernel<<<grid, 256, 0, st>>>(jobs, tab, P, Pstride, lin);
+    dim3 grid(blocks_for(max_theta, LBM_T), blocks_for(max_rows, LBM_R), (unsigned)njobs);
+    lut_build_mixed_kernel<<<grid, 256, 0, st>>>(jobs, reinterpret_cast<const SplitCoef*>(tab), bias, P, Pstride, lin);
 }
 
 void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* waves, double2* rec, double2* tab,
@@ -750,6 +879,7 @@ void preload_nearfield_kernels() {
     cudaFuncGetAttributes(&a, mie_kernel);
     cudaFuncGetAttributes(&a, coef_rows_batch_kernel);
     cudaFuncGetAttributes(&a, legendre_table_kernel);
+    cudaFuncGetAttributes(&a, legendre_split_kernel);
     cudaFuncGetAttributes(&a, us_lut_f64_kernel);
     cudaFuncGetAttributes(&a, lut_build_mixed_kernel);
     cudaFuncGetAttributes(&a, sh_recur_kernel);
