@@ -120,7 +120,7 @@ struct bs_ctx {
     int prec = -1;
     bool have = false;
 
-    DevBuf d_sph, d_waves, d_kw4, d_ph, d_A, d_B, d_mie, d_tab, d_tabscr, d_legP, d_lut, d_uft, d_uftscr;
+    DevBuf d_sph, d_waves, d_kw4, d_ph, d_A, d_B, d_tab, d_tabscr, d_legP, d_lut, d_uft, d_uftscr;
     DevBuf d_cnt;           // staged / total counters of the mixed LUT kernel
     DevBuf d_far;           // far fields Ud, Ufd on request (bs_get_far_field)
     DevBuf d_starts;        // row / coefficient offsets of a coefficient batch
@@ -156,7 +156,7 @@ struct bs_ctx {
 
 // Every linear device buffer of a context.
 static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
-    return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_mie, &c->d_tab,
+    return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_tab,
             &c->d_tabscr, &c->d_bias, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
             &c->d_sv, &c->d_mask, &c->d_wx, &c->d_wy, &c->d_wix, &c->d_wiy, &c->d_f1, &c->d_f2,
             &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_far,
@@ -801,10 +801,8 @@ static bs_status run_nearfield(bs_ctx* c) {
     if (scatter) {
         CK(c->d_A.ensure(ncoef * sizeof(zd)));
         CK(c->d_B.ensure(ncoef * sizeof(zd)));
-        CK(c->d_mie.ensure((size_t)ns * 6 * c->Lmax * sizeof(zd)));
         CK(cudaMemcpyAsync(c->d_sph.p, c->hs.data(), ns * sizeof(Sphere), cudaMemcpyHostToDevice, c->st));
-        launch_mie(c->d_sph.as<Sphere>(), ns, sc.kmag, c->d_mie.as<zd>(), c->Lmax, c->d_A.as<zd>(),
-                   c->d_B.as<zd>(), c->st);
+        launch_mie(c->d_sph.as<Sphere>(), ns, sc.kmag, c->d_A.as<zd>(), c->d_B.as<zd>(), c->st);
         LAUNCHED(c);
         if (p.lut_us) {  // the LUT kernels' phases and float directions (the direct method forms its own)
             CK(c->d_ph.ensure((size_t)ns * nk * sizeof(cpx<T>)));
@@ -1003,7 +1001,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
     if (p.scalar && ns > 0) {
         size_t ncoef = 0;
         for (const Sphere& S : c->hs) ncoef += S.Nl + 1;
-        b += 2 * B(ncoef * sizeof(zd)) + B(ns * 6 * (size_t)c->Lmax * sizeof(zd));
+        b += 2 * B(ncoef * sizeof(zd));
         if (p.lut_us) b += B(ns * nk * cT) + B(nk * sizeof(float4));  // phases, float directions
         if (!p.lut_us) {  // direct method: harmonic recurrences, per-wave and per-sphere tables
             const size_t nlm = (size_t)c->Lmax * (c->Lmax + 1) / 2;

@@ -7,6 +7,7 @@
 #include "bs_geom.cuh"
 #include "bs_kernels.h"
 #include "bs_math.cuh"
+#include "bs_mie.cuh"
 
 namespace bs {
 
@@ -127,35 +128,13 @@ __global__ void uf_table_kernel(Scene sc, double* __restrict__ tab, double* __re
 }
 
 // ---------------------------------------------------------------------------
-// Mie coefficients (sphere::calcCoeff, sphere.cpp:21-97), one thread per sphere
+// Mie coefficients (sphere::calcCoeff, sphere.cpp:21-97), one block per sphere
 // ---------------------------------------------------------------------------
-__global__ void mie_kernel(const Sphere* __restrict__ sph, int ns, double k, zd* __restrict__ scratch, int lstride,
-                           zd* __restrict__ A, zd* __restrict__ B) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= ns) return;
-    Sphere S = sph[s];
-    int N = S.Nl;
-    zd* ja = scratch + (size_t)s * 6 * lstride;
-    zd* ya = ja + lstride;
-    zd* jpa = ya + lstride;
-    zd* ypa = jpa + lstride;
-    zd* jn = ypa + lstride;
-    zd* jpn = jn + lstride;
-    zd n = mk(S.n_re, S.n_im);
-    zd ka = mk(k * S.a, 0.0);
-    zd kna = (n * k) * S.a;
-    sph_complex(N, ka, true, ja, ya, jpa, ypa);
-    sph_complex(N, kna, true, jn, nullptr, jpn, nullptr);
-    for (int l = 0; l <= N; l++) {
-        zd h = mk(ja[l].re - ya[l].im, ja[l].im + ya[l].re);      // j + i y
-        zd hp = mk(jpa[l].re - ypa[l].im, jpa[l].im + ypa[l].re);
-        zd an = ja[l] * hp - jpa[l] * h;
-        zd bn = jn[l] * hp - (h * jpn[l]) * n;
-        zd cn = (ja[l] * jpn[l]) * n - jn[l] * jpa[l];
-        zd f = mk(2.0 * l + 1.0, 0.0) * ipow(l);
-        A[S.coef_off + l] = f * (an / bn);
-        B[S.coef_off + l] = f * (cn / bn);
-    }
+__global__ void __launch_bounds__(MIE_NT) mie_kernel(const Sphere* __restrict__ sph, double k, zd* __restrict__ A,
+                                                     zd* __restrict__ B) {
+    __shared__ MieShared sm;
+    const Sphere& S = sph[blockIdx.x];
+    mie_block(sm, S.Nl, S.a, mk(S.n_re, S.n_im), k, A + S.coef_off, B + S.coef_off);
 }
 
 // Per-row order coefficients of the spheres [s0, s0 + n) in one launch:
@@ -198,7 +177,7 @@ __global__ void coef_rows_batch_kernel(const Sphere* __restrict__ sph, int s0, i
             double da = S.a / (S.aR - 1);
             double r = ia * da;
             zd knr = (mk(S.n_re, S.n_im) * k) * r;
-            sph_complex(S.Nl, knr, true, out, nullptr, nullptr, nullptr);
+            sph_complex(S.Nl, knr, out);
             for (int l = 0; l < L; l++) out[l] = A[S.coef_off + l] * out[l];
         }
     }
@@ -748,8 +727,8 @@ void launch_uf_table(const Scene& sc, double* tab, double* scratch, cudaStream_t
     uf_table_kernel<<<blocks_for(sc.uf_dR, 128), 128, 0, st>>>(sc, tab, scratch);
 }
 
-void launch_mie(const Sphere* sph, int ns, double k, zd* scratch, int lstride, zd* A, zd* B, cudaStream_t st) {
-    mie_kernel<<<blocks_for(ns, 64), 64, 0, st>>>(sph, ns, k, scratch, lstride, A, B);
+void launch_mie(const Sphere* sph, int ns, double k, zd* A, zd* B, cudaStream_t st) {
+    mie_kernel<<<ns, MIE_NT, 0, st>>>(sph, k, A, B);
 }
 
 void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows,

@@ -430,14 +430,8 @@ bs_status bs_server_get_stats(bs_server* srv, bs_server_stats* out);
  *            zeros above, as the context path computes no order beyond Nl_s
  *   stream   cudaStream_t to run on (NULL = legacy default stream); the call is
  *            asynchronous on it.
- * The Bessel work space is a fixed 3 MiB device array inside this library,
- * held by every GPU that loads it; it is fully rewritten before being read,
- * so nothing needs clearing, but every call shares it: calls whose kernels
- * overlap on the GPU (different streams, or threads sharing a device) race.
- * The first call on a device resolves the array's device address, so make it
- * before any stream capture.  That address is kept for the process: do not
- * call cudaDeviceReset on the device after the first call.  Sizes beyond the
- * limits return BS_ERR_ARG. */
+ * The work space is the kernel's shared memory: calls on different streams or
+ * threads may overlap.  Sizes beyond the limits return BS_ERR_ARG. */
 bs_status bs_mie_noalloc(const double* spheres, int32_t ns, int32_t nl, double k, double* A, double* B,
                          void* stream);
 
