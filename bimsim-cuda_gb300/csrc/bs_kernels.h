@@ -88,12 +88,18 @@ void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, in
                             const float* bias, const float2* P, int Pstride, float2* lin, cudaStream_t st);
 
 // Direct scattered field through the addition theorem of spherical harmonics:
-// recurrence factors rec, per-wave tables tab (nk x L(L+1)/2), per-sphere
+// recurrence factors rec (L(L+1)/2), per-wave tables tab (nk x L(L+1)/2), per-sphere
 // coefficients coef (ns x L(L+1)/2 x 2 complex), then the per-pixel sum.
-void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* waves, double2* rec, double2* tab,
+struct ShRec {
+    double a, b, beta, kappa, zero;
+};
+struct ShFrame {
+    double e1[3], e2[3], e3[3];  // the harmonics' axes: e3 the slice's normal
+};
+void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* waves, ShRec* rec, double2* tab,
                       zd* coef, cudaStream_t st);
 template <class T>
-void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const zd* A, const zd* B, const double2* rec,
+void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const zd* A, const zd* B, const ShRec* rec,
                   const zd* coef, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st);
 template <class T>
 void launch_sum_only(const Scene& sc, const Sphere* sph, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st);

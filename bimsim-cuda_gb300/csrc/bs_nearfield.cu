@@ -4,6 +4,8 @@
 // into the epilogue.
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "bs_geom.cuh"
 #include "bs_kernels.h"
 #include "bs_math.cuh"
@@ -477,43 +479,70 @@ __global__ void __launch_bounds__(256, 2) lut_build_mixed_kernel(const LutBuildJ
 // S_l^m(cos t2) cos(m (f1 - f2)), so
 //   Q_l(r^) = sum_m S_l^m(r_z) (cos(m f_r) C_lm + sin(m f_r) S_lm),
 //   (C_lm, S_lm) = sum_w pw_w S_l^m(k_wz) (cos, sin)(m f_w)   per sphere,
-// with f the azimuth about z.  A (pixel, sphere) pair then costs L (L + 1) / 2
+// with f the azimuth about the harmonics' axis.  A (pixel, sphere) pair then costs L (L + 1) / 2
 // terms instead of nk L, and the result is the same sum up to rounding.
+//
+// The axis is the slice's normal (ShFrame): a pixel's cosine is then h / d with the sphere's distance h
+// from the plane, the same for all pixels, and where the plane goes through the sphere's centre (h = 0)
+// every S_l^m is a constant, zero for odd l - m, that goes into the coefficients.
+// FP64 instructions per term (the kernel's bound): the three-term recurrence of the S_l^m in monic form
+// (u_l = x u_{l-1} - beta_l u_{l-2}, scale in the coefficients) 2, its cosine and sine part 2, the sum
+// Q_l 4 -- 8 where summing c_l S_l^m (...) took 13 -- and 4 on half of the terms where h = 0.
 // Tables are in (m, l) order: index(m, l) = m L - m (m - 1) / 2 + (l - m).
 // ---------------------------------------------------------------------------
 __host__ __device__ __forceinline__ int sh_index(int L, int m, int l) { return m * L - m * (m - 1) / 2 + (l - m); }
 
-// Recurrence factors: rec[index(m, l)] = (a, b) with S_l^m = a x S_{l-1}^m - b S_{l-2}^m
-// for l >= m + 2 (a = (2l - 1) / sqrt(l^2 - m^2), b = sqrt((l-1)^2 - m^2) / sqrt(l^2 - m^2)),
-// a = sqrt(2m + 1) for l = m + 1, and for l = m the diagonal factor
-// S_m^m = a sin(t) S_{m-1}^{m-1} (a = 1 for m = 1, sqrt((2m - 1) / (2m)) above).
-__global__ void sh_recur_kernel(int L, double2* __restrict__ rec) {
-    const int m = blockIdx.x, l = m + threadIdx.x;
-    if (m >= L || l >= L) return;
-    double a = 0, b = 0;
-    if (l == m) a = m == 0 ? 1.0 : (m == 1 ? 1.0 : sqrt((2.0 * m - 1.0) / (2.0 * m)));
-    else if (l == m + 1) a = sqrt(2.0 * m + 1.0);
-    else {
-        const double den = sqrt((double)l * l - (double)m * m);
-        a = (2.0 * l - 1.0) / den;
-        b = sqrt((double)(l - 1) * (l - 1) - (double)m * m) / den;
+// Per (m, l): a, b of S_l^m = a x S_{l-1}^m - b S_{l-2}^m for l >= m + 2 (a = (2l - 1) / sqrt(l^2 - m^2),
+// b = sqrt((l-1)^2 - m^2) / sqrt(l^2 - m^2)), a = sqrt(2m + 1) for l = m + 1, and for l = m the diagonal
+// factor S_m^m = a sin(t) S_{m-1}^{m-1} (a = 1 for m = 1, sqrt((2m - 1) / (2m)) above); the monic form
+// S_l^m = kappa u_l, beta = b kappa_{l-2} / kappa_l; and zero = S_l^m at x = 0.
+__global__ void sh_recur_kernel(int L, ShRec* __restrict__ rec) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= L) return;
+    double diag = 1;  // S_m^m at sin t = 1
+    for (int i = 2; i <= m; i++) diag *= sqrt((2.0 * i - 1.0) / (2.0 * i));
+    double a1 = 1, kap = 1, z2 = 0, z1 = diag;
+    for (int l = m; l < L; l++) {
+        ShRec r{0, 0, 0, 1, 0};
+        if (l == m) {
+            r.a = m < 2 ? 1.0 : sqrt((2.0 * m - 1.0) / (2.0 * m));
+            r.zero = diag;
+        } else if (l == m + 1) {
+            r.a = a1 = sqrt(2.0 * m + 1.0);
+            r.kappa = kap = a1;
+            z2 = diag;
+            z1 = 0;
+        } else {
+            const double den = sqrt((double)l * l - (double)m * m);
+            r.a = (2.0 * l - 1.0) / den;
+            r.b = sqrt((double)(l - 1) * (l - 1) - (double)m * m) / den;
+            r.beta = r.b / (r.a * a1);
+            r.kappa = kap = kap * r.a;
+            a1 = r.a;
+            r.zero = -r.b * z2;
+            z2 = z1;
+            z1 = r.zero;
+        }
+        rec[sh_index(L, m, l)] = r;
     }
-    rec[sh_index(L, m, l)] = make_double2(a, b);
 }
 
-// Per wave: tab[w][index(m, l)] = S_l^m(k_z) (cos, sin)(m f_k).
-__global__ void sh_wave_kernel(int nk, int L, const double* __restrict__ waves, const double2* __restrict__ rec,
-                               double2* __restrict__ tab) {
+__device__ __forceinline__ double dot3(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
+
+// Per wave: tab[w][index(m, l)] = S_l^m(k_n) (cos, sin)(m f_k), k_n the component along the normal.
+__global__ void sh_wave_kernel(int nk, int L, ShFrame fr, const double* __restrict__ waves,
+                               const ShRec* __restrict__ rec, double2* __restrict__ tab) {
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= nk) return;
-    const double kx = waves[3 * w], ky = waves[3 * w + 1], kz = waves[3 * w + 2];
+    const double* k = waves + 3 * w;
+    const double kx = dot3(k, fr.e1), ky = dot3(k, fr.e2), kz = dot3(k, fr.e3);
     const double rho = sqrt(kx * kx + ky * ky);
     const double cf = rho > 0 ? kx / rho : 1.0, sf = rho > 0 ? ky / rho : 0.0;
     double2* out = tab + (size_t)w * (L * (L + 1) / 2);
     double cm = 1, sm = 0, smm = 1;  // cos(m f), sin(m f), S_m^m
     for (int m = 0; m < L; m++) {
         if (m > 0) {
-            smm *= rec[sh_index(L, m, m)].x * rho;
+            smm *= rec[sh_index(L, m, m)].a * rho;
             const double c2 = cm * cf - sm * sf;
             sm = sm * cf + cm * sf;
             cm = c2;
@@ -522,10 +551,10 @@ __global__ void sh_wave_kernel(int nk, int L, const double* __restrict__ waves, 
         for (int l = m; l < L; l++) {
             double v;
             if (l == m) v = smm;
-            else if (l == m + 1) v = rec[sh_index(L, m, l)].x * kz * smm;
+            else if (l == m + 1) v = rec[sh_index(L, m, l)].a * kz * smm;
             else {
-                const double2 ab = rec[sh_index(L, m, l)];
-                v = ab.x * kz * p1 - ab.y * p2;
+                const ShRec r = rec[sh_index(L, m, l)];
+                v = r.a * kz * p1 - r.b * p2;
             }
             if (l > m) {
                 p2 = p1;
@@ -536,10 +565,18 @@ __global__ void sh_wave_kernel(int nk, int L, const double* __restrict__ waves, 
     }
 }
 
-// Per sphere s and table index: coef[s][index] = (C, S) = sum_w pw_{s,w} tab[w][index], with the
-// phase pw of phase_kernel in double precision.
+// Whether the slice's plane goes through the sphere's centre, to rounding.
+__device__ __forceinline__ bool sh_in_plane(const Scene& sc, const ShFrame& fr, const Sphere& S, double& h) {
+    const double r[3] = {sc.A[0] - S.p[0], sc.A[1] - S.p[1], sc.A[2] - S.p[2]};
+    h = dot3(r, fr.e3);
+    return fabs(h) <= 4e-16 * (fabs(r[0]) + fabs(r[1]) + fabs(r[2]));
+}
+
+// Per sphere s and table index: coef[s][index] = (C, S) = scale sum_w pw_{s,w} tab[w][index], with the phase pw
+// of phase_kernel in double precision and the scale kappa, or S_l^m(0) for a sphere centred in the plane.
 constexpr int SH_WAVES = 128;
-__global__ void sh_coef_kernel(Scene sc, const Sphere* __restrict__ sph, int L, const double* __restrict__ waves,
+__global__ void sh_coef_kernel(Scene sc, ShFrame fr, const Sphere* __restrict__ sph, int L,
+                               const double* __restrict__ waves, const ShRec* __restrict__ rec,
                                const double2* __restrict__ tab, zd* __restrict__ coef) {
     __shared__ zd s_pw[SH_WAVES];
     const int s = blockIdx.y, nlm = L * (L + 1) / 2;
@@ -565,29 +602,83 @@ __global__ void sh_coef_kernel(Scene sc, const Sphere* __restrict__ sph, int L, 
             }
     }
     if (i < nlm) {
-        coef[((size_t)s * nlm + i) * 2] = ac;
-        coef[((size_t)s * nlm + i) * 2 + 1] = as;
+        double h;
+        const double scale = sh_in_plane(sc, fr, sph[s], h) ? rec[i].zero : rec[i].kappa;
+        coef[((size_t)s * nlm + i) * 2] = ac * scale;
+        coef[((size_t)s * nlm + i) * 2 + 1] = as * scale;
     }
 }
 
-// Per pixel: U = sum_s sum_l c_l(r) Q_l(r^) (+ Uf outside every sphere)
-// (--recursive; nfScalarUs.cu:17-95, 201-245, 333-491).  The Bessel recurrences
-// depend on (pixel, sphere) only, so they run once per pair in double and give
+// The radial factors of one (pixel, sphere) pair, order after order:
 //   outside (d > a):  c_l = B_l (j_l + i y_l)(k d)   with the reference clamps
-//   inside  (d <= a): c_l = A_l j_l(k n d)           (c_0 = A_0 only when
-//                                                      Re(k n d) < 1e-6)
-// where the reference re-runs them for every wave (nfScalarUs.cu:69-93).  All
-// in double precision, stored as T.
+//   inside  (d <= a): c_l = A_l j_l(k n d)           (c_0 = A_0 only when Re(k n d) < 1e-6)
+// (--recursive; nfScalarUs.cu:17-95, 201-245, 333-491).  They depend on (pixel, sphere) only; the
+// reference re-runs them for every wave (nfScalarUs.cu:69-93).  One reciprocal serves all orders.
+struct ShRadial {
+    bool inside, centre;
+    double x, inv;
+    zd z, zinv;
+    zd p0, p1;  // outside: (j, y) of the last two orders; inside: j
+
+    __device__ __forceinline__ void start(const Scene& sc, const Sphere& S, double d) {
+        inside = d <= S.a;
+        centre = false;
+        if (inside) {
+            z = mk(sc.kmag * d * S.n_re, sc.kmag * d * S.n_im);
+            centre = z.re < EPS_FLOAT;
+            if (centre) return;
+            zinv = mk(1.0, 0.0) / z;
+            const zd j0 = zsin(z) / z;
+            p0 = j0;
+            p1 = j0 / z - zcos(z) / z;
+        } else {
+            x = sc.kmag * d;
+            inv = 1.0 / x;
+            double sn, cs;
+            sincos(x, &sn, &cs);
+            const double j0 = sn / x, y0 = -cs / x;
+            p0 = mk(j0, y0);
+            p1 = mk(j0 / x - cs / x, y0 / x - sn / x);
+        }
+    }
+    // c_l for l = 0, 1, 2, ... in turn
+    __device__ __forceinline__ zd next(int l, const zd* __restrict__ A, const zd* __restrict__ B) {
+        if (inside) {
+            if (centre) return l == 0 ? A[0] : mk(0.0, 0.0);
+            if (l < 2) return A[l] * (l == 0 ? p0 : p1);
+            const zd w = (2.0 * l - 1.0) * zinv;
+            zd b = mk(fma(w.re, p1.re, fma(-w.im, p1.im, -p0.re)), fma(w.re, p1.im, fma(w.im, p1.re, -p0.im)));
+            if (l > z.re && (b.re < CONV_MIN || b.re > CONV_MAX)) b = mk(0.0, 0.0);
+            p0 = p1;
+            p1 = b;
+            return A[l] * b;
+        }
+        if (l >= 2) {
+            const double w = quot(2.0 * l - 1.0, x, inv);
+            double j = fma(w, p1.re, -p0.re), y = fma(w, p1.im, -p0.im);
+            if (l > x && (j < CONV_MIN || j > CONV_MAX)) j = 0.0;
+            if (y < Y_FLOOR || (l > x && y > 0)) {
+                y = 0;
+                p1.im = 0;
+            }
+            p0 = p1;
+            p1 = mk(j, y);
+        }
+        return B[l] * (l == 0 ? p0 : p1);
+    }
+};
+
+// Per pixel: U = sum_s sum_l c_l(r) Q_l(r^) (+ Uf outside every sphere).  All in double precision, stored as T.
 constexpr int SH_BLOCK = 64;
 template <class T>
-__global__ void __launch_bounds__(SH_BLOCK) us_sh_kernel(Scene sc, const Sphere* __restrict__ sph, int L,
+__global__ void __launch_bounds__(SH_BLOCK) us_sh_kernel(Scene sc, ShFrame fr, const Sphere* __restrict__ sph, int L,
                                                          const zd* __restrict__ A, const zd* __restrict__ B,
-                                                         const double2* __restrict__ rec, const zd* __restrict__ coef,
+                                                         const ShRec* __restrict__ rec, const zd* __restrict__ coef,
                                                          const cpx<T>* __restrict__ Uf, cpx<T>* __restrict__ U) {
     extern __shared__ unsigned char smem_raw[];
-    zd* cl = reinterpret_cast<zd*>(smem_raw);  // [L][SH_BLOCK]
-    const int tid = threadIdx.x, nlm = L * (L + 1) / 2;
-    int idx = blockIdx.x * SH_BLOCK + tid;
+    zd* col = reinterpret_cast<zd*>(smem_raw) + threadIdx.x;  // the thread's L values, SH_BLOCK apart
+    const int nlm = L * (L + 1) / 2;
+    int idx = blockIdx.x * SH_BLOCK + threadIdx.x;
     const bool valid = idx < sc.R * sc.R;
     if (!valid) idx = sc.R * sc.R - 1;
     double p[3];
@@ -596,93 +687,65 @@ __global__ void __launch_bounds__(SH_BLOCK) us_sh_kernel(Scene sc, const Sphere*
     bool outside = true;
     for (int s = 0; s < sc.ns; s++) {
         const Sphere& S = sph[s];
-        double r[3];
+        double r[3], h;
         const double d = dist_exact(p, S.p, r);
         if (d < S.a) outside = false;
         const int Ls = S.Nl + 1;
-        int Leff = Ls;
-        if (d <= S.a) {
-            const zd* co = A + S.coef_off;
-            const zd knd = mk(sc.kmag * d * S.n_re, sc.kmag * d * S.n_im);
-            if (knd.re < EPS_FLOAT) {
-                Leff = 1;
-                cl[tid] = co[0];
-            } else {
-                zd j0 = zsin(knd) / knd;
-                zd j1 = j0 / knd - zcos(knd) / knd;
-                for (int l = 0; l < Ls; l++) {
-                    zd jl;
-                    if (l == 0) {
-                        jl = j0;
-                    } else {
-                        if (l > 1) sbesselj_step_c(l, knd, j0, j1);
-                        jl = j1;
-                    }
-                    cl[l * SH_BLOCK + tid] = co[l] * jl;
-                }
-            }
-        } else {
-            const zd* co = B + S.coef_off;
-            const double kd = sc.kmag * d;
-            double sn, cs;
-            sincos(kd, &sn, &cs);
-            double j0 = sn / kd, j1 = j0 / kd - cs / kd;
-            double y0 = -cs / kd, y1 = y0 / kd - sn / kd;
-            for (int l = 0; l < Ls; l++) {
-                double jl, yl;
-                if (l == 0) {
-                    jl = j0;
-                    yl = y0;
-                } else {
-                    if (l > 1) {
-                        sbesselj_step(l, kd, j0, j1);
-                        sbessely_step(l, kd, y0, y1);
-                    }
-                    jl = j1;
-                    yl = y1;
-                }
-                cl[l * SH_BLOCK + tid] = co[l] * mk(jl, yl);
-            }
-        }
-        // direction of the pixel from the sphere; at d == 0 only l = 0 remains
-        double x = 0, rho = 0, cf = 1, sf = 0;
-        if (d != 0) {
-            const double rx = r[0] / d, ry = r[1] / d;
-            x = r[2] / d;
-            rho = sqrt(rx * rx + ry * ry);
-            if (rho > 0) {
-                cf = rx / rho;
-                sf = ry / rho;
-            }
-        }
+        const bool in_plane = sh_in_plane(sc, fr, S, h);
+        const double r1 = dot3(r, fr.e1), r2 = dot3(r, fr.e2), rho = sqrt(r1 * r1 + r2 * r2);
+        const double cf = rho > 0 ? r1 / rho : 1.0, sf = rho > 0 ? r2 / rho : 0.0;
         const zd* cs_ = coef + (size_t)s * nlm * 2;
+        ShRadial rad;
+        rad.start(sc, S, d);
+        const zd *Al = A + S.coef_off, *Bl = B + S.coef_off;
         zd acc = mk(0.0, 0.0);
-        double cm = 1, sm = 0, smm = 1;
-        for (int m = 0; m < Leff; m++) {
-            if (m > 0) {
-                smm *= rec[sh_index(L, m, m)].x * rho;
+        if (in_plane) {
+            double cm = 1, sm = 0;
+            for (int m = 0; m < Ls; m++) {  // cos(m f), sin(m f)
+                col[m * SH_BLOCK] = mk(cm, sm);
                 const double c2 = cm * cf - sm * sf;
                 sm = sm * cf + cm * sf;
                 cm = c2;
             }
-            double p2 = 0, p1 = smm;
-            for (int l = m; l < Leff; l++) {
-                double v;
-                if (l == m) v = smm;
-                else if (l == m + 1) v = rec[sh_index(L, m, l)].x * x * smm;
-                else {
-                    const double2 ab = rec[sh_index(L, m, l)];
-                    v = ab.x * x * p1 - ab.y * p2;
+            for (int l = 0; l < Ls; l++) {
+                zd q = mk(0.0, 0.0);
+#pragma unroll 4
+                for (int m = l & 1; m <= l; m += 2) {
+                    const int k = sh_index(L, m, l);
+                    const zd C = cs_[2 * k], Sn = cs_[2 * k + 1], e = col[m * SH_BLOCK];
+                    q = mk(fma(e.re, C.re, fma(e.im, Sn.re, q.re)), fma(e.re, C.im, fma(e.im, Sn.im, q.im)));
                 }
-                if (l > m) {
-                    p2 = p1;
-                    p1 = v;
-                }
-                const int k = sh_index(L, m, l);
-                const zd C = cs_[2 * k], Sn = cs_[2 * k + 1];
-                const zd q = mk(cm * C.re + sm * Sn.re, cm * C.im + sm * Sn.im) * v;
-                acc = acc + cl[l * SH_BLOCK + tid] * q;
+                acc = acc + rad.next(l, Al, Bl) * q;
             }
+        } else {
+            const double x = d != 0 ? h / d : 0.0, st = d != 0 ? rho / d : 0.0;
+            for (int l = 0; l < Ls; l++) col[l * SH_BLOCK] = mk(0.0, 0.0);
+            double cm = 1, sm = 0, smm = 1;
+            for (int m = 0; m < Ls; m++) {
+                if (m > 0) {
+                    smm *= rec[sh_index(L, m, m)].a * st;
+                    const double c2 = cm * cf - sm * sf;
+                    sm = sm * cf + cm * sf;
+                    cm = c2;
+                }
+                const double c = smm * cm, sn = smm * sm;
+                double u2 = 0, u1 = 1;
+                const int k0 = sh_index(L, m, m);
+#pragma unroll 4
+                for (int l = m; l < Ls; l++) {
+                    const int k = k0 + l - m;
+                    if (l > m) {  // beta is 0 for l = m + 1
+                        const double u = fma(x, u1, -rec[k].beta * u2);
+                        u2 = u1;
+                        u1 = u;
+                    }
+                    const zd C = cs_[2 * k], Sn = cs_[2 * k + 1];
+                    const double wc = c * u1, ws = sn * u1;
+                    zd& q = col[l * SH_BLOCK];
+                    q = mk(fma(wc, C.re, fma(ws, Sn.re, q.re)), fma(wc, C.im, fma(ws, Sn.im, q.im)));
+                }
+            }
+            for (int l = 0; l < Ls; l++) acc = acc + rad.next(l, Al, Bl) * col[l * SH_BLOCK];
         }
         // Kahan over spheres
         const zd y = acc - cmp;
@@ -774,25 +837,51 @@ void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, in
     lut_build_mixed_kernel<<<grid, 256, 0, st>>>(jobs, reinterpret_cast<const SplitCoef*>(tab), bias, P, Pstride, lin);
 }
 
-void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* waves, double2* rec, double2* tab,
+// Orthonormal frame of the slice: the u axis and the normal; of a slice that is a line, the line
+// and an axis across it (of a point, the coordinate axes).
+static ShFrame sh_frame(const Scene& sc) {
+    auto len = [](const double* a) { return std::sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]); };
+    auto cross = [](const double* a, const double* b, double* c) {
+        for (int i = 0; i < 3; i++) c[i] = a[(i + 1) % 3] * b[(i + 2) % 3] - a[(i + 2) % 3] * b[(i + 1) % 3];
+    };
+    ShFrame f{{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
+    const double* X = len(sc.X) > 0 ? sc.X : sc.Y;
+    const double lx = len(X);
+    if (!(lx > 0)) return f;
+    for (int i = 0; i < 3; i++) f.e1[i] = X[i] / lx;
+    cross(sc.X, sc.Y, f.e3);
+    if (!(len(f.e3) > 1e-14 * lx * lx)) {
+        int k = 0;  // the coordinate axis farthest from the line
+        for (int i = 1; i < 3; i++)
+            if (std::fabs(f.e1[i]) < std::fabs(f.e1[k])) k = i;
+        const double a[3] = {double(k == 0), double(k == 1), double(k == 2)};
+        cross(f.e1, a, f.e3);
+    }
+    const double ln = len(f.e3);
+    for (int i = 0; i < 3; i++) f.e3[i] /= ln;
+    cross(f.e3, f.e1, f.e2);
+    return f;
+}
+
+void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* waves, ShRec* rec, double2* tab,
                       zd* coef, cudaStream_t st) {
-    sh_recur_kernel<<<L, ((L + 31) / 32) * 32, 0, st>>>(L, rec);
-    sh_wave_kernel<<<blocks_for(sc.nk, 64), 64, 0, st>>>(sc.nk, L, waves, rec, tab);
+    const ShFrame fr = sh_frame(sc);
+    sh_recur_kernel<<<blocks_for(L, 32), 32, 0, st>>>(L, rec);
+    sh_wave_kernel<<<blocks_for(sc.nk, 32), 32, 0, st>>>(sc.nk, L, fr, waves, rec, tab);
     const int nlm = L * (L + 1) / 2;
     dim3 grid(blocks_for(nlm, 128), sc.ns);
-    sh_coef_kernel<<<grid, 128, 0, st>>>(sc, sph, L, waves, tab, coef);
+    sh_coef_kernel<<<grid, 128, 0, st>>>(sc, fr, sph, L, waves, rec, tab, coef);
 }
 
 template <class T>
-void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const zd* A, const zd* B, const double2* rec,
+void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const zd* A, const zd* B, const ShRec* rec,
                   const zd* coef, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st) {
     const size_t smem = (size_t)L * SH_BLOCK * sizeof(zd);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(us_sh_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const long long n = (long long)sc.R * sc.R;
-    us_sh_kernel<T><<<blocks_for(n, SH_BLOCK), SH_BLOCK, smem, st>>>(sc, sph, L, A, B, rec, coef, Uf, U);
+    us_sh_kernel<T><<<blocks_for(n, SH_BLOCK), SH_BLOCK, smem, st>>>(sc, sh_frame(sc), sph, L, A, B, rec, coef, Uf, U);
 }
-
 
 template <class T>
 void launch_sum_only(const Scene& sc, const Sphere* sph, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st) {
@@ -871,7 +960,7 @@ void preload_nearfield_kernels() {
     template void launch_uf<T>(const Scene&, const double*, const double*, cpx<T>*, cudaStream_t);              \
     template void launch_lut_build<T>(const zd*, int, int, const double*, int, int, Patch<T>*, cudaStream_t);   \
     template void launch_phase<T>(const Scene&, const Sphere*, const double*, cpx<T>*, float4*, cudaStream_t);  \
-    template void launch_us_sh<T>(const Scene&, const Sphere*, int, const zd*, const zd*, const double2*,       \
+    template void launch_us_sh<T>(const Scene&, const Sphere*, int, const zd*, const zd*, const ShRec*,         \
                                   const zd*, const cpx<T>*, cpx<T>*, cudaStream_t);                           \
     template void launch_sum_only<T>(const Scene&, const Sphere*, const cpx<T>*, cpx<T>*, cudaStream_t);
 BS_INST(float)
