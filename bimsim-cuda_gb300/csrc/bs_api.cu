@@ -135,6 +135,8 @@ struct bs_ctx {
     int legP_theta = 0, legP_L = 0;
     bool legP_split = false;  // d_legP holds the mixed path's order-major split values
     DevBuf d_bias;            // mixed path: bias of every coefficient row
+    DevBuf d_acos;            // FP64 path: nodes of the arc cosine for acos_theta angles
+    int acos_theta = 0;
     int tab_s0 = 0, tab_s1 = 0;  // spheres whose tables the last run left in d_lut
     int64_t launches = 0;
     int64_t interactions = 0;
@@ -157,7 +159,7 @@ struct bs_ctx {
 // Every linear device buffer of a context.
 static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
     return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_tab,
-            &c->d_tabscr, &c->d_bias, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
+            &c->d_tabscr, &c->d_bias, &c->d_acos, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
             &c->d_sv, &c->d_mask, &c->d_wx, &c->d_wy, &c->d_wix, &c->d_wiy, &c->d_f1, &c->d_f2,
             &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_far,
             &c->d_starts, &c->d_lbjobs, &c->d_lbjobs2, &c->d_kcmp, &c->d_fsave, &c->d_dacc, &c->d_line, &c->d_ringcs, &c->d_bp, &c->d_shrec, &c->d_shtab, &c->d_shcoef, &c->d_gscr, &c->d_ufw};
@@ -165,7 +167,7 @@ static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
 
 static void release_all(bs_ctx* c) {
     for (DevBuf* b : ctx_bufs(c)) b->release();
-    c->legP_theta = c->legP_L = 0;
+    c->legP_theta = c->legP_L = c->acos_theta = 0;
     c->lut_valid = false;
     c->have = false;
 }
@@ -853,6 +855,12 @@ static bs_status run_nearfield(bs_ctx* c) {
             CK(c->d_tabscr.ensure((size_t)maxcoef * 2 * sizeof(double)));
             CK(c->d_starts.ensure((size_t)maxstarts * sizeof(long long)));
             if (!fp64) CK(c->d_bias.ensure((size_t)maxrow * sizeof(float)));
+            if (fp64 && c->acos_theta != thetaR) {
+                CK(c->d_acos.ensure((ACOS_NODES + 1) * sizeof(AcosNode)));
+                launch_acos_nodes(thetaR, c->d_acos.as<AcosNode>(), c->st);
+                LAUNCHED(c);
+                c->acos_theta = thetaR;
+            }
             if (c->legP_theta != thetaR || c->legP_L < c->Lmax || c->legP_split != !fp64) {
                 CK(c->d_legP.ensure((size_t)thetaR * c->Lmax * sizeof(double)));
                 if (fp64) launch_legendre_table(thetaR, c->Lmax, c->d_legP.as<double>(), c->st);
@@ -961,7 +969,8 @@ static bs_status run_nearfield(bs_ctx* c) {
             int finalize = (ci == std::max(1, nchunks) - 1);
             if (fp64) {
                 launch_us_lut_f64(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_waves.as<double>(),
-                                  c->d_ph.as<zd>(), c->d_lut.as<Patch<double>>(), (const zd*)Uf, (zd*)U, c->st);
+                                  c->d_acos.as<AcosNode>(), c->d_ph.as<zd>(), c->d_lut.as<Patch<double>>(),
+                                  (const zd*)Uf, (zd*)U, c->st);
             } else {
                 launch_us_lut_mixed(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_kw4.as<float4>(),
                                     c->d_ph.as<cpx<float>>(), c->d_lut.as<float2>(), (const cpx<float>*)Uf,
@@ -1024,8 +1033,9 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         b += B(pool) + B((size_t)maxcoef * sizeof(zd)) + B((size_t)maxcoef * 2 * sizeof(double)) +
              B((size_t)maxstarts * sizeof(long long));
         b += B(thetaR * (size_t)c->Lmax * sizeof(double));    // Legendre table
+        if (fp64) b += B((ACOS_NODES + 1) * sizeof(AcosNode));
         if (!fp64) {
-            b += B((size_t)maxrow * sizeof(float));
+            b += B((size_t)maxrow * sizeof(float));  // biases
             if (cs.size() > 2) b += B(R * R * sizeof(float2));  // Kahan carry between chunks
             b += B(2 * sizeof(unsigned long long));
         }

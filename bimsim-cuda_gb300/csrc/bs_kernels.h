@@ -59,9 +59,16 @@ void launch_lut_build(const zd* tab, int rows, int L, const double* P, int Pstri
                       cudaStream_t st);
 template <class T>
 void launch_phase(const Scene& sc, const Sphere* sph, const double* waves, cpx<T>* ph, float4* kw4, cudaStream_t st);
+// Nodes of the double-precision arc cosine at j pi / ACOS_NODES: cos, 1 / sin, the angle in columns of a
+// table of thetaR angles, and the series coefficients of the angle around it (us_lut_f64_kernel); ACOS_NODES + 1 of them.
+constexpr int ACOS_NODES = 2048;
+struct alignas(64) AcosNode {
+    double c, is, th, b2, b3, b4, b5, b6;
+};
+void launch_acos_nodes(int thetaR, AcosNode* nodes, cudaStream_t st);
 void launch_us_lut_f64(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
-                       const double* waves, const zd* ph, const Patch<double>* lut, const zd* Uf, zd* U,
-                       cudaStream_t st);
+                       const double* waves, const AcosNode* nodes, const zd* ph, const Patch<double>* lut, const zd* Uf,
+                       zd* U, cudaStream_t st);
 // mixed path.  lin: linear float2 tables (Sphere::usp_off / uip_off in float2 units, rows
 // of Sphere::lin_stride entries, even and 16-byte aligned);
 // counters[0..1] receive the staged and total (tile, sphere, chunk of `chunk` waves) counts
