@@ -473,8 +473,8 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
     T* I = c->d_I.as<T>();
     long long RR = (long long)R * R;
     // split-K scratch for the GEMMs with few output tiles
-    const size_t scr = std::max(std::max(cgemm_scratch_elems(R, Nu, R, 2), cgemm_scratch_elems(Nv, Nu, R, 2)),
-                                std::max(cgemm_scratch_elems(Nv, C, Nu, 2), cgemm_scratch_elems(C, C, Nv, 2)));
+    const size_t scr = std::max(std::max(cgemm_scratch_elems<T>(R, Nu, R, 2), cgemm_scratch_elems<T>(Nv, Nu, R, 2)),
+                                std::max(cgemm_scratch_elems<T>(Nv, C, Nu, 2), cgemm_scratch_elems<T>(C, C, Nv, 2)));
     CK(c->d_gscr.ensure(std::max<size_t>(scr, 1) * ce));
     cpx<T>* gs = c->d_gscr.as<cpx<T>>();
     launch_cgemm<T>(R, Nu, R, 2, fields, R, RR, wx, Nu, 0, f1, Nu, (long long)R * Nu, 0, nullptr, (T)1, nullptr, gs,
@@ -1050,8 +1050,11 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         b += B(R * Nu * cT) + B(Nv * R * cT) + B(Nu * C * cT) + B(C * Nv * cT);
         b += B(2 * R * Nu * cT) + B(2 * Nv * Nu * cT) + B(2 * Nv * C * cT) + B(2 * C * C * rT);
         const int Ri = (int)R, Ui = (int)Nu, Vi = (int)Nv, Ci = (int)C;
-        const size_t scr = std::max(std::max(cgemm_scratch_elems(Ri, Ui, Ri, 2), cgemm_scratch_elems(Vi, Ui, Ri, 2)),
-                                    std::max(cgemm_scratch_elems(Vi, Ci, Ui, 2), cgemm_scratch_elems(Ci, Ci, Vi, 2)));
+        auto elems = [fp64](int M, int N, int K) {
+            return fp64 ? cgemm_scratch_elems<double>(M, N, K, 2) : cgemm_scratch_elems<float>(M, N, K, 2);
+        };
+        const size_t scr = std::max(std::max(elems(Ri, Ui, Ri), elems(Vi, Ui, Ri)),
+                                    std::max(elems(Vi, Ci, Ui), elems(Ci, Ci, Vi)));
         b += B(std::max<size_t>(scr, 1) * cT);  // split-K parts
     }
     b += B(res * res * rT);                                   // image staging

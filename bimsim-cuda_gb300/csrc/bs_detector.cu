@@ -32,10 +32,31 @@ __global__ void twiddle_kernel(int ni, int nj, const int* __restrict__ freq, int
     out[(long long)i * ld_i + (long long)j * ld_j] = mk((T)c, (T)(sign * s));
 }
 
-// Tiled complex GEMM.  Block 16 x 16 threads, tile BM x BN = 64 x 32, each
-// thread 4 x 2 outputs, BK = 16.  Float accumulation is split into per-tile
-// partial sums combined with Kahan compensation.
-constexpr int GB_M = 64, GB_N = 32, GB_K = 16;
+// Tiled complex GEMM.  Block 16 x 16 threads, tile 64 x 16 NJ, each thread
+// 4 x NJ outputs, K tiles of 16.  Accumulation is split into per-tile
+// partial sums combined with Kahan compensation.  Double precision is bound by the
+// FP64 pipe (four multiply-adds per product), so its tile is 16 columns wide: a
+// passband of 41 columns fills 85 % of the tiles' work instead of 64 %.
+// 1280^2 field to 41 columns, two fields: 3.55 -> 1.36 ms.
+constexpr int GB_M = 64, GB_K = 16;
+template <class T>
+__host__ __device__ constexpr int gb_nj() { return sizeof(T) == 8 ? 1 : 2; }
+template <class T>
+__host__ __device__ constexpr int gb_n() { return 16 * gb_nj<T>(); }
+
+// One product a b of a tile's sum (p0 - p1) + i (p2 + p3).  Double precision sums the four products of the
+// parts each on its own, four instructions; single precision is not bound by its pipe and rounds each
+// product's two parts together first (p0 and p2), which leaves the sums 4 to 20 % closer.
+__device__ __forceinline__ void cmac(cpx<double> a, cpx<double> b, double& p0, double& p1, double& p2, double& p3) {
+    p0 = fma(a.re, b.re, p0);
+    p1 = fma(a.im, b.im, p1);
+    p2 = fma(a.re, b.im, p2);
+    p3 = fma(a.im, b.re, p3);
+}
+__device__ __forceinline__ void cmac(cpx<float> a, cpx<float> b, float& p0, float&, float& p2, float&) {
+    p0 += a.re * b.re - a.im * b.im;
+    p2 += a.re * b.im + a.im * b.re;
+}
 
 // Epilogue of one output element c of batch b: epi 0 store, 1 store times the
 // band-pass mask, 2 |scale c|^2 into I, 3 store scale c.
@@ -68,69 +89,66 @@ __global__ void __launch_bounds__(256) cgemm_kernel(int M, int N, int K, const c
                                                     cpx<T>* __restrict__ C, int ldc, long long sC, int epi,
                                                     const float* __restrict__ mask, T scale, T* __restrict__ I,
                                                     int ksplit, cpx<T>* __restrict__ part) {
+    constexpr int NJ = gb_nj<T>(), GN = gb_n<T>();
     __shared__ cpx<T> As[GB_K][GB_M + 1];
-    __shared__ cpx<T> Bs[GB_K][GB_N + 1];
+    __shared__ cpx<T> Bs[GB_K][GN + 1];
     const int b = blockIdx.z / ksplit, ks = blockIdx.z % ksplit;
     A += b * sA;
     B += b * sB;
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * GB_M, n0 = blockIdx.x * GB_N;
+    const int m0 = blockIdx.y * GB_M, n0 = blockIdx.x * GN;
     const int kc = ((K + ksplit - 1) / ksplit + GB_K - 1) / GB_K * GB_K;  // K range per split, whole tiles
     const int kbeg = ks * kc, kend = min(K, kbeg + kc);
-    T accr[4][2], acci[4][2], cr[4][2], ci[4][2];
+    T accr[4][NJ], acci[4][NJ], cr[4][NJ], ci[4][NJ];
+    T p0[4][NJ], p1[4][NJ], p2[4][NJ], p3[4][NJ];  // the tile's sums, see cmac
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 2; j++) accr[i][j] = acci[i][j] = cr[i][j] = ci[i][j] = 0;
+        for (int j = 0; j < NJ; j++) accr[i][j] = acci[i][j] = cr[i][j] = ci[i][j] = p0[i][j] = p1[i][j] = p2[i][j] = p3[i][j] = 0;
     for (int k0 = kbeg; k0 < kend; k0 += GB_K) {
         for (int e = threadIdx.x; e < GB_K * GB_M; e += 256) {
             int kk = e % GB_K, mm = e / GB_K;
             int gm = m0 + mm, gk = k0 + kk;
             As[kk][mm] = (gm < M && gk < kend) ? A[(long long)gm * lda + gk] : mk((T)0, (T)0);
         }
-        for (int e = threadIdx.x; e < GB_K * GB_N; e += 256) {
-            int nn = e % GB_N, kk = e / GB_N;
+        for (int e = threadIdx.x; e < GB_K * GN; e += 256) {
+            int nn = e % GN, kk = e / GN;
             int gn = n0 + nn, gk = k0 + kk;
             Bs[kk][nn] = (gn < N && gk < kend) ? B[(long long)gk * ldb + gn] : mk((T)0, (T)0);
         }
         __syncthreads();
-        T pr[4][2], pi[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 2; j++) pr[i][j] = pi[i][j] = 0;
 #pragma unroll
         for (int kk = 0; kk < GB_K; kk++) {
-            cpx<T> a[4], bb[2];
+            cpx<T> a[4], bb[NJ];
 #pragma unroll
             for (int i = 0; i < 4; i++) a[i] = As[kk][ty + 16 * i];
 #pragma unroll
-            for (int j = 0; j < 2; j++) bb[j] = Bs[kk][tx + 16 * j];
+            for (int j = 0; j < NJ; j++) bb[j] = Bs[kk][tx + 16 * j];
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    pr[i][j] += a[i].re * bb[j].re - a[i].im * bb[j].im;
-                    pi[i][j] += a[i].re * bb[j].im + a[i].im * bb[j].re;
+                for (int j = 0; j < NJ; j++) {
+                    cmac(a[i], bb[j], p0[i][j], p1[i][j], p2[i][j], p3[i][j]);
                 }
         }
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
-            for (int j = 0; j < 2; j++) {  // Kahan step
-                T yr = pr[i][j] - cr[i][j], yi = pi[i][j] - ci[i][j];
+            for (int j = 0; j < NJ; j++) {  // Kahan step
+                T yr = (p0[i][j] - p1[i][j]) - cr[i][j], yi = (p2[i][j] + p3[i][j]) - ci[i][j];
                 T trr = accr[i][j] + yr, tii = acci[i][j] + yi;
                 cr[i][j] = (trr - accr[i][j]) - yr;
                 ci[i][j] = (tii - acci[i][j]) - yi;
                 accr[i][j] = trr;
                 acci[i][j] = tii;
+                p0[i][j] = p1[i][j] = p2[i][j] = p3[i][j] = 0;
             }
         __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
+        for (int j = 0; j < NJ; j++) {
             int gm = m0 + ty + 16 * i, gn = n0 + tx + 16 * j;
             if (gm >= M || gn >= N) continue;
             if (ksplit > 1)
@@ -195,22 +213,26 @@ void launch_twiddle(int ni, int nj, const int* freq, int off_i, int R, int sign,
     twiddle_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ni, nj, freq, off_i, R, sign, ld_i, ld_j, out);
 }
 
-// Splits of K for a GEMM with few output tiles: enough blocks for about two per
-// SM, each split at least 4 K tiles long, at most 64 splits.
+// Splits of K for a GEMM with few output tiles: enough blocks for about two per SM (six in double
+// precision, whose time is the busiest SM's share of the multiply-adds), each split at least 4 K
+// tiles long, at most 64 splits.
+template <class T>
 int cgemm_ksplit(int M, int N, int K, int batch) {
     int dev = 0, n_sm = 1;  // attribute queries are cheap host calls; no shared cache between threads
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) !=
                                                    cudaSuccess)
         n_sm = 1;
-    const long long tiles = (long long)((N + GB_N - 1) / GB_N) * ((M + GB_M - 1) / GB_M) * batch;
-    if (tiles <= 0 || tiles >= n_sm) return 1;
-    long long ks = (2LL * n_sm + tiles - 1) / tiles;
+    const long long tiles = (long long)((N + gb_n<T>() - 1) / gb_n<T>()) * ((M + GB_M - 1) / GB_M) * batch;
+    const long long want = (sizeof(T) == 8 ? 6LL : 2LL) * n_sm;
+    if (tiles <= 0 || 2 * tiles >= want) return 1;
+    long long ks = (want + tiles - 1) / tiles;
     ks = std::min<long long>(ks, std::max(1, K / (4 * GB_K)));
     return (int)std::min<long long>(ks, 64);
 }
 
+template <class T>
 size_t cgemm_scratch_elems(int M, int N, int K, int batch) {
-    const int ks = cgemm_ksplit(M, N, K, batch);
+    const int ks = cgemm_ksplit<T>(M, N, K, batch);
     return ks > 1 ? (size_t)batch * ks * M * N : 0;
 }
 
@@ -218,9 +240,9 @@ template <class T>
 void launch_cgemm(int M, int N, int K, int batch, const cpx<T>* A, int lda, long long sA, const cpx<T>* B, int ldb,
                   long long sB, cpx<T>* C, int ldc, long long sC, int epi, const float* mask, T scale, T* I,
                   cpx<T>* scratch, size_t scratch_elems, cudaStream_t st) {
-    int ks = cgemm_ksplit(M, N, K, batch);
+    int ks = cgemm_ksplit<T>(M, N, K, batch);
     if ((size_t)batch * ks * M * N > scratch_elems || !scratch) ks = 1;
-    dim3 grid((N + GB_N - 1) / GB_N, (M + GB_M - 1) / GB_M, batch * ks);
+    dim3 grid((N + gb_n<T>() - 1) / gb_n<T>(), (M + GB_M - 1) / GB_M, batch * ks);
     cgemm_kernel<T><<<grid, 256, 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, epi, mask, scale, I, ks,
                                           scratch);
     if (ks > 1) {
@@ -427,6 +449,7 @@ void preload_detector_kernels() {
     template void launch_cgemm<T>(int, int, int, int, const cpx<T>*, int, long long, const cpx<T>*, int,       \
                                   long long, cpx<T>*, int, long long, int, const float*, T, T*, cpx<T>*,       \
                                   size_t, cudaStream_t);                                                        \
+    template size_t cgemm_scratch_elems<T>(int, int, int, int);                                                 \
     template void launch_bin<T>(int, int, int, int, const T*, T*, cudaStream_t);                                    \
     template void launch_image<T>(int, int, const T*, const T*, T*, cudaStream_t);                             \
     template void launch_rotate_add_images<T>(int, float, float, const T*, T*, cudaStream_t);                 \

@@ -128,6 +128,7 @@ void launch_twiddle(int ni, int nj, const int* freq, int off_i, int R, int sign,
 // GEMMs with fewer output tiles than SMs split K over more blocks and add the
 // parts in a fixed order (deterministic) when `scratch` holds
 // cgemm_scratch_elems(M, N, K, batch) elements; else one block per tile.
+template <class T>
 size_t cgemm_scratch_elems(int M, int N, int K, int batch);
 template <class T>
 void launch_cgemm(int M, int N, int K, int batch, const cpx<T>* A, int lda, long long sA, const cpx<T>* B, int ldb,
