@@ -330,6 +330,8 @@ static bs_status derive(bs_ctx* c) {
     sc.uf_dmin = quad_dist(nf, f);
     sc.uf_dmax = quad_dist_max(nf, f);
     sc.uf_dR = p.uf_lut_r > 0 ? p.uf_lut_r : 2 * c->R;
+    sc.uf_scale = (sc.uf_dR - 1) / (sc.uf_dmax - sc.uf_dmin);
+    sc.invR = 1.0 / c->R;
     sc.ns = (int)c->spheres.size();
     c->hs.resize(sc.ns);
     double diag = v3_len(V3{nf.X.x + nf.Y.x, nf.X.y + nf.Y.y, nf.X.z + nf.Y.z});
@@ -762,7 +764,8 @@ static bs_status run_nearfield(bs_ctx* c) {
     }
     {
         // condenser aperture factor of each order, the same for every pixel (nfScalarUf.cu:46-175)
-        std::vector<double> w(sc.m + 1);
+        std::vector<UfOrder> w(sc.m + 1);
+        double kap = 1, kap2 = 1;  // P_l = kappa_l u_l, kappa_l = (2l - 1) / l kappa_{l-1}
         double a0 = 1, a1 = sc.cos_a, a2 = 1, b0 = 1, b1 = sc.cos_b, b2 = 1;
         auto step = [](int n, double x, double& q0, double& q1) {  // rts/math/legendre.h:17-25
             const double qn = ((2 * n - 1) * x * q1 - (n - 1) * q0) / n;
@@ -776,11 +779,18 @@ static bs_status run_nearfield(bs_ctx* c) {
                 b2 = b0;
                 step(l + 1, sc.cos_b, b0, b1);
             }
-            w[l] = a1 - a2 - b1 + b2;
+            w[l].beta = 0;
+            if (l > 0) {
+                const double k1 = kap;
+                kap *= (2.0 * l - 1.0) / l;
+                if (l > 1) w[l].beta = (l - 1.0) / l * kap2 / kap;
+                kap2 = k1;
+            }
+            w[l].w = (l & 2 ? -1.0 : 1.0) * kap * (l == 0 ? a1 - b1 : a1 - a2 - b1 + b2) * (2.0 * PI_REF * sc.amp);
         }
-        CK(c->d_ufw.ensure(w.size() * sizeof(double)));
-        CK(cudaMemcpyAsync(c->d_ufw.p, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
-        launch_uf<T>(sc, c->d_uft.as<double>(), c->d_ufw.as<double>(), Uf, c->st);
+        CK(c->d_ufw.ensure(w.size() * sizeof(UfOrder)));
+        CK(cudaMemcpyAsync(c->d_ufw.p, w.data(), w.size() * sizeof(UfOrder), cudaMemcpyHostToDevice, c->st));
+        launch_uf<T>(sc, c->d_uft.as<double>(), c->d_ufw.as<UfOrder>(), Uf, c->st);
         LAUNCHED(c);
         CK(cudaStreamSynchronize(c->st));  // w is a host vector of this scope
     }
@@ -1006,7 +1016,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
     b += B(std::max<size_t>(1, ns) * sizeof(Sphere));
     b += B((p.plane_wave ? 1 : nk) * 3 * sizeof(double));     // directions
     if (p.lut_uf && !p.plane_wave && p.scalar) b += 2 * B((size_t)sc.uf_dR * (sc.m + 1) * sizeof(double));
-    b += B((size_t)(sc.m + 1) * sizeof(double));               // incident-field aperture factors
+    b += B((size_t)(sc.m + 1) * sizeof(UfOrder));              // incident-field order weights
     if (p.scalar && ns > 0) {
         size_t ncoef = 0;
         for (const Sphere& S : c->hs) ncoef += S.Nl + 1;

@@ -10,8 +10,9 @@ namespace bs {
 // restatement, with no fused multiply-add, so the GPU and the double
 // precision reference agree on every boundary pixel.
 __device__ __forceinline__ void pixel_pos(const Scene& sc, int iu, int iv, double p[3]) {
-    // quad::operator()(u, v) = (A + X u) + Y v with u = iu / R (nfScalarUf.cu:66-71)
-    double u = __ddiv_rn((double)iu, (double)sc.R), v = __ddiv_rn((double)iv, (double)sc.R);
+    // quad::operator()(u, v) = (A + X u) + Y v with u = iu / R (nfScalarUf.cu:66-71); quot gives the correctly
+    // rounded quotient, as invR = 1 / R is and R's significand is not all ones
+    const double u = quot((double)iu, (double)sc.R, sc.invR), v = quot((double)iv, (double)sc.R, sc.invR);
 #pragma unroll
     for (int c = 0; c < 3; c++) p[c] = __dadd_rn(__dadd_rn(sc.A[c], __dmul_rn(sc.X[c], u)), __dmul_rn(sc.Y[c], v));
 }

@@ -43,6 +43,14 @@ struct Scene {
     double uf_dmin, uf_dmax;
     int uf_dR;
     int pad_;
+    double uf_scale;          // (uf_dR - 1) / (uf_dmax - uf_dmin)
+    double invR;              // 1 / R
+};
+
+// Per order l of the incident field: the monic Legendre recurrence's factor and the weight
+// +-2 PI A w_l kappa_l (sign of i^l; P_l = kappa_l u_l).
+struct UfOrder {
+    double beta, w;
 };
 
 // Per-sphere data (sphere.h:14-92 plus the LUT geometry of sphere.cpp:222-240).
