@@ -61,6 +61,14 @@ __device__ __forceinline__ f32x2 theta_column2(f32x2 c, f32x2 ntsc, f32x2 hb) {
     return f2_fma(f2_pack(copysignf(w.x, cc.x), copysignf(w.y, cc.y)), ntsc, hb);
 }
 
+// hb of the columns from t_lo on.  From column 0 on it is at least the largest w in columns, rounded up:
+// a direction through the pixel (c = 1) then has column 0 or a little above, where the rounding of hb
+// and tsc alone could leave it below 0 and outside the table or the window.
+__device__ __forceinline__ float column_base(float hp_hi, float hp_lo, float tsc, int t_lo) {
+    const float hb = (hp_hi - (float)t_lo) + hp_lo;
+    return t_lo == 0 ? fmaxf(hb, __fmul_ru(1.570796371f, tsc)) : hb;
+}
+
 // ---------------------------------------------------------------------------
 // The sorted kernel (more than LUT_FEW_WAVES directions)
 //
@@ -431,7 +439,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
                         }
                         __syncwarp();
                     }
-                    const f32x2 ntsc = f2_splat(-tsc), hb = f2_splat((hp_hi - (float)t_lo) + hp_lo);
+                    const f32x2 ntsc = f2_splat(-tsc), hb = f2_splat(column_base(hp_hi, hp_lo, tsc, t_lo));
                     // polynomial coefficients of a direction's column along the row (x = +-(7.5 - i) / 7.5)
                     auto node = [&](float4 k, int n) {
                         const float4 xy = sm.node[warp][r][2 * n];
@@ -643,7 +651,7 @@ __global__ void __launch_bounds__(256) us_lut_few_kernel(Scene sc, const Sphere*
         const float inv = d != 0 ? 1.f / (float)d : 0.f;
         const float rx = (float)r[0] * inv, ry = (float)r[1] * inv, rz = (float)r[2] * inv;
         const float cb = d != 0 ? 0.f : 1.f;  // d == 0: cos(theta) := 1
-        const f32x2 ntsc = f2_splat(-S.tsc), hb = f2_splat(S.hp_hi);
+        const f32x2 ntsc = f2_splat(-S.tsc), hb = f2_splat(column_base(S.hp_hi, 0.f, S.tsc, 0));
         float2 sx = make_float2(0.f, 0.f), sy = make_float2(0.f, 0.f);
         for (int w = 0; w < sc.nk; w++) {
             const float4 k = kw4[w];
