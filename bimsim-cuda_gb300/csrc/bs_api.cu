@@ -126,6 +126,7 @@ struct bs_ctx {
     DevBuf d_starts;        // row / coefficient offsets of a coefficient batch
     DevBuf d_lbjobs, d_lbjobs2;  // Usp and Uip tables of a coefficient batch for the mixed LUT build
     DevBuf d_kcmp;               // Kahan compensation of the mixed LUT sums between sphere chunks
+    DevBuf d_part;               // mixed LUT sums of the spheres' shares (lut_splits)
     DevBuf d_fsave;         // U, Uf of a ring's first source (bs_simulate_ring_interp)
     DevBuf d_dacc;          // detector sum of bs_simulate_ring_detector
     DevBuf d_line, d_ringcs;  // radial lines and ring (cos, sin) of bs_simulate_ring_line
@@ -162,7 +163,7 @@ static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
             &c->d_tabscr, &c->d_bias, &c->d_acos, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
             &c->d_sv, &c->d_mask, &c->d_wx, &c->d_wy, &c->d_wix, &c->d_wiy, &c->d_f1, &c->d_f2,
             &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_far,
-            &c->d_starts, &c->d_lbjobs, &c->d_lbjobs2, &c->d_kcmp, &c->d_fsave, &c->d_dacc, &c->d_line, &c->d_ringcs, &c->d_bp, &c->d_shrec, &c->d_shtab, &c->d_shcoef, &c->d_gscr, &c->d_ufw};
+            &c->d_starts, &c->d_lbjobs, &c->d_lbjobs2, &c->d_kcmp, &c->d_part, &c->d_fsave, &c->d_dacc, &c->d_line, &c->d_ringcs, &c->d_bp, &c->d_shrec, &c->d_shtab, &c->d_shcoef, &c->d_gscr, &c->d_ufw};
 }
 
 static void release_all(bs_ctx* c) {
@@ -882,7 +883,9 @@ static bs_status run_nearfield(bs_ctx* c) {
             }
         }
         const int nchunks = (int)chunk_start.size() - 1;
-        if (!fp64 && nchunks > 1) CK(c->d_kcmp.ensure((size_t)R * R * sizeof(float2)));
+        const int shares = fp64 || ns == 0 ? 1 : lut_splits(R, ns, nk);
+        if (shares > 1) CK(c->d_part.ensure((size_t)shares * 4 * R * R * sizeof(float)));
+        else if (!fp64 && nchunks > 1) CK(c->d_kcmp.ensure((size_t)R * R * sizeof(float2)));
         bool use_stage = false;
         // tables of the previous run still in the pool?
         std::vector<double> key;
@@ -985,7 +988,9 @@ static bs_status run_nearfield(bs_ctx* c) {
                 launch_us_lut_mixed(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_kw4.as<float4>(),
                                     c->d_ph.as<cpx<float>>(), c->d_lut.as<float2>(), (const cpx<float>*)Uf,
                                     (cpx<float>*)U, ns > 0 ? c->d_cnt.as<unsigned long long>() : nullptr,
-                                    nchunks > 1 ? c->d_kcmp.as<float2>() : nullptr, use_stage, chunk, cone, c->st);
+                                    nchunks > 1 ? c->d_kcmp.as<float2>() : nullptr,
+                                    shares > 1 ? c->d_part.as<float>() : nullptr, use_stage, chunk, cone, c->st);
+                if (shares > 1 && finalize) c->launches++;
             }
             LAUNCHED(c);
             c->tab_s0 = s0;
@@ -1046,7 +1051,9 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         if (fp64) b += B((ACOS_NODES + 1) * sizeof(AcosNode));
         if (!fp64) {
             b += B((size_t)maxrow * sizeof(float));  // biases
-            if (cs.size() > 2) b += B(R * R * sizeof(float2));  // Kahan carry between chunks
+            const int shares = lut_splits((int)R, (int)ns, (int)nk);
+            if (shares > 1) b += B((size_t)shares * 4 * R * R * sizeof(float));
+            else if (cs.size() > 2) b += B(R * R * sizeof(float2));  // Kahan carry between chunks
             b += B(2 * sizeof(unsigned long long));
         }
     }

@@ -79,8 +79,12 @@ void launch_us_lut_f64(const Scene& sc, const Sphere* sph, int s0, int s1, int a
 // every direction (half-angle pi: directions that are not unit vectors)
 void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
                          const float4* kw4, const cpx<float>* ph, const float2* lin, const cpx<float>* Uf,
-                         cpx<float>* U, unsigned long long* counters, float2* kcmp, bool stage, int chunk,
+                         cpx<float>* U, unsigned long long* counters, float2* kcmp, float* part, bool stage, int chunk,
                          float4 cone, cudaStream_t st);
+// Shares of the spheres that launch_us_lut_mixed runs side by side; above 1, `part` (else null) holds
+// 4 floats per pixel and share.
+constexpr int GB300_SMS = 152;
+int lut_splits(int R, int ns, int nk);
 // One table of the mixed path's table build: the rows of one sphere's Usp or Uip with their
 // coefficient rows at tab + tab_off and biases at bias + row_off, written to the linear rows at
 // lin + lin_off.

@@ -96,6 +96,20 @@ constexpr int SW_W = 64;         // columns of a pixel's window
 constexpr int SW_GROUPS = SW_WAVES / 32;
 constexpr float SW_HALF = 7.5f;  // half a row, pixels
 
+// Whether a pixel lies outside every sphere (nfSumUf.cu:35).
+__device__ __forceinline__ bool outside_all(const Scene& sc, const Sphere* __restrict__ sph, const double p[3]) {
+    for (int s = 0; s < sc.ns; s++) {
+        const Sphere& S = sph[s];
+        // clearly outside in single precision (0.1 % margin on d^2), else the exact test
+        const float dx = (float)(p[0] - S.p[0]), dy = (float)(p[1] - S.p[1]), dz = (float)(p[2] - S.p[2]);
+        const float af = (float)S.a;
+        if (dx * dx + dy * dy + dz * dz > 1.001f * af * af) continue;
+        double r[3];
+        if (dist_exact(p, S.p, r) < S.a) return false;
+    }
+    return true;
+}
+
 template <int N>
 struct Int {  // a compile-time argument of the kernel's lambdas
     static constexpr int value = N;
@@ -258,12 +272,20 @@ __global__ void __launch_bounds__(SW_NT, 2)
     us_lut_sorted_kernel(Scene sc, const Sphere* __restrict__ sph, int s0, int s1, int accumulate, int finalize,
                          const float4* __restrict__ kw4, const cpx<float>* __restrict__ ph,
                          const float2* __restrict__ lin, const cpx<float>* __restrict__ Uf, cpx<float>* __restrict__ U,
-                         unsigned long long* __restrict__ counters, float2* __restrict__ kcmp, int chunk, float4 cone) {
+                         unsigned long long* __restrict__ counters, float2* __restrict__ kcmp,
+                         float* __restrict__ part, int chunk, float4 cone) {
     extern __shared__ __align__(1024) unsigned char sw_smem[];
     SwShared& sm = *reinterpret_cast<SwShared*>(sw_smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_u = (sc.R + 15) / 16;
     const int tu = (blockIdx.x % tiles_u) * 16, tv = (blockIdx.x / tiles_u) * 16;
+    // blockIdx.y: the block's share of all the spheres (lut_splits), with sums of its own
+    const int share = blockIdx.y, shares = gridDim.y;
+    const int sb = max(s0, (int)((long long)sc.ns * share / shares));
+    const int se = min(s1, (int)((long long)sc.ns * (share + 1) / shares));
+    const size_t plane = 2 * (size_t)sc.R * sc.R;
+    float* sum = part ? part + 2 * share * plane : reinterpret_cast<float*>(U);
+    float* comp = part ? sum + plane : reinterpret_cast<float*>(kcmp);
     // pixel_pos computes (A + X u) + Y v: the terms of the tile's 16 columns and 16 rows, once
     if (threadIdx.x < 32) {
         const int k = threadIdx.x & 15;
@@ -282,8 +304,8 @@ __global__ void __launch_bounds__(SW_NT, 2)
         float2 a = make_float2(0.f, 0.f);
         if (accumulate && opx < sc.R && iv < sc.R) {
             const size_t o = 2 * ((size_t)iv * sc.R + opx) + (lane & 1);
-            a.x = reinterpret_cast<const float*>(U)[o];
-            if (kcmp) a.y = reinterpret_cast<const float*>(kcmp)[o];
+            a.x = sum[o];
+            if (comp) a.y = comp[o];
         }
         sm.acc[warp][r][lane] = a;
     }
@@ -297,7 +319,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
     unsigned staged_units = 0;
     const unsigned win0 = (unsigned)(warp * sizeof(sm.win[0]));
     __syncthreads();
-    for (int s = s0; s < s1; s++) {
+    for (int s = sb; s < se; s++) {
         const Sphere& S = sph[s];
         // ---- the warp's pixels: lanes 0-15 the first row, 16-31 the second ----
         {
@@ -584,7 +606,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
     }
     if (threadIdx.x == 0 && counters) {
         atomicAdd(counters, (unsigned long long)staged_units);
-        atomicAdd(counters + 1, (unsigned long long)(s1 - s0) * ((sc.nk + chunk - 1) / chunk));
+        atomicAdd(counters + 1, (unsigned long long)max(se - sb, 0) * ((sc.nk + chunk - 1) / chunk));
     }
 #pragma unroll
     for (int r = 0; r < 2; r++) {
@@ -592,25 +614,15 @@ __global__ void __launch_bounds__(SW_NT, 2)
         if (opx >= sc.R || iv >= sc.R) continue;
         float2 a = sm.acc[warp][r][lane];
         const size_t o = 2 * ((size_t)iv * sc.R + opx) + (lane & 1);
-        if (finalize) {
+        if (finalize && !part) {
             double p[3];
 #pragma unroll
             for (int c = 0; c < 3; c++) p[c] = __dadd_rn(sm.pa[c][lu], sm.pb[c][lv]);
-            bool outside = true;
-            for (int s = 0; s < sc.ns && outside; s++) {
-                const Sphere& S = sph[s];
-                // clearly outside in single precision (0.1 % margin on d^2), else the exact test
-                const float dx = (float)(p[0] - S.p[0]), dy = (float)(p[1] - S.p[1]), dz = (float)(p[2] - S.p[2]);
-                const float af = (float)S.a;
-                if (dx * dx + dy * dy + dz * dz > 1.001f * af * af) continue;
-                double rr[3];
-                if (dist_exact(p, S.p, rr) < S.a) outside = false;
-            }
-            if (outside) a.x += reinterpret_cast<const float*>(Uf)[o] - a.y;
-        } else if (kcmp) {
-            reinterpret_cast<float*>(kcmp)[o] = a.y;
+            if (outside_all(sc, sph, p)) a.x += reinterpret_cast<const float*>(Uf)[o] - a.y;
+        } else if (comp) {
+            comp[o] = a.y;
         }
-        reinterpret_cast<float*>(U)[o] = a.x;
+        sum[o] = a.x;
     }
 }
 
@@ -674,17 +686,7 @@ __global__ void __launch_bounds__(256) us_lut_few_kernel(Scene sc, const Sphere*
         tot = make_float2(tr, ti);
     }
     if (finalize) {
-        bool outside = true;
-        for (int s = 0; s < sc.ns && outside; s++) {
-            const Sphere& S = sph[s];
-            // clearly outside in single precision (0.1 % margin on d^2), else the exact test
-            const float dx = (float)(p[0] - S.p[0]), dy = (float)(p[1] - S.p[1]), dz = (float)(p[2] - S.p[2]);
-            const float af = (float)S.a;
-            if (dx * dx + dy * dy + dz * dz > 1.001f * af * af) continue;
-            double r[3];
-            if (dist_exact(p, S.p, r) < S.a) outside = false;
-        }
-        if (outside) {
+        if (outside_all(sc, sph, p)) {
             tot.x += Uf[idx].re - cmp.x;
             tot.y += Uf[idx].im - cmp.y;
         }
@@ -694,9 +696,46 @@ __global__ void __launch_bounds__(256) us_lut_few_kernel(Scene sc, const Sphere*
     U[idx] = mk(tot.x, tot.y);
 }
 
+// The shares' sums added in order (Kahan), and Uf where the pixel is outside every sphere.
+__global__ void __launch_bounds__(128) us_lut_join_kernel(Scene sc, const Sphere* __restrict__ sph, int shares,
+                                                          const float* __restrict__ part,
+                                                          const cpx<float>* __restrict__ Uf, cpx<float>* __restrict__ U) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= sc.R * sc.R) return;
+    const size_t plane = (size_t)sc.R * sc.R;
+    const float2* v = reinterpret_cast<const float2*>(part) + idx;
+    float2 tot = make_float2(0.f, 0.f), cmp = tot;
+    auto add = [&](float2 a) {
+        const float yr = a.x - cmp.x, yi = a.y - cmp.y, tr = tot.x + yr, ti = tot.y + yi;
+        cmp = make_float2((tr - tot.x) - yr, (ti - tot.y) - yi);
+        tot = make_float2(tr, ti);
+    };
+    for (int q = 0; q < shares; q++, v += 2 * plane) {
+        add(v[0]);
+        add(make_float2(-v[plane].x, -v[plane].y));
+    }
+    double p[3];
+    pixel_pos(sc, idx % sc.R, idx / sc.R, p);
+    if (outside_all(sc, sph, p)) {
+        tot.x += Uf[idx].re - cmp.x;
+        tot.y += Uf[idx].im - cmp.y;
+    }
+    U[idx] = mk(tot.x, tot.y);
+}
+
+// A slice of fewer tiles than three per SM leaves SMs with one block of 8 warps or none: its spheres are
+// shared out so that there are about four blocks per SM.  A sphere's share depends on the slice alone, so
+// that chunked tables give the bits of one launch.  192^2 pixels, 12 spheres, 400 directions: 1.16 ms a slice
+// in one share, 0.79 ms in five.
+int lut_splits(int R, int ns, int nk) {
+    const int tiles = ((R + 15) / 16) * ((R + 15) / 16);
+    if (nk <= LUT_FEW_WAVES || tiles >= 3 * GB300_SMS) return 1;
+    return std::max(1, std::min({ns, 8, (4 * GB300_SMS + tiles - 1) / tiles}));
+}
+
 void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
                          const float4* kw4, const cpx<float>* ph, const float2* lin, const cpx<float>* Uf,
-                         cpx<float>* U, unsigned long long* counters, float2* kcmp, bool stage, int chunk,
+                         cpx<float>* U, unsigned long long* counters, float2* kcmp, float* part, bool stage, int chunk,
                          float4 cone, cudaStream_t st) {
     const unsigned tiles = (sc.R + 15) / 16;
     if (sc.nk <= LUT_FEW_WAVES) {
@@ -704,11 +743,14 @@ void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int
                                                          counters, kcmp, chunk);
         return;
     }
+    const int shares = part ? lut_splits(sc.R, sc.ns, sc.nk) : 1;
     // per device and cheap; a failure shows up as the launch error
     auto kernel = stage ? us_lut_sorted_kernel<true> : us_lut_sorted_kernel<false>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SwShared));
-    kernel<<<tiles * tiles, SW_NT, sizeof(SwShared), st>>>(sc, sph, s0, s1, accumulate, finalize, kw4, ph, lin, Uf, U,
-                                                           counters, kcmp, chunk, cone);
+    kernel<<<dim3(tiles * tiles, shares), SW_NT, sizeof(SwShared), st>>>(sc, sph, s0, s1, accumulate, finalize, kw4, ph,
+                                                                         lin, Uf, U, counters, kcmp, part, chunk, cone);
+    if (part && finalize)
+        us_lut_join_kernel<<<(sc.R * sc.R + 127) / 128, 128, 0, st>>>(sc, sph, shares, part, Uf, U);
 }
 
 // Loads every kernel of this file (cudaFuncGetAttributes), see preload_nearfield_kernels.
@@ -717,6 +759,7 @@ void preload_uslut_kernels() {
     cudaFuncGetAttributes(&a, us_lut_sorted_kernel<true>);
     cudaFuncGetAttributes(&a, us_lut_sorted_kernel<false>);
     cudaFuncGetAttributes(&a, us_lut_few_kernel);
+    cudaFuncGetAttributes(&a, us_lut_join_kernel);
 }
 
 }  // namespace bs
