@@ -14,7 +14,7 @@ namespace bs {
 constexpr float LUT_STAGE_MARGIN = 5e-4f;
 constexpr int LUT_FEW_WAVES = 32;
 constexpr int LUT_TILE = 16;
-constexpr int LUT_WINDOW = 64;  // table columns of a staged window
+constexpr int LUT_WINDOW = 256;  // table columns of the widest staged window
 constexpr int WAVE_CHUNK_MAX = 64;
 
 template <class T>

@@ -77,10 +77,11 @@ __device__ __forceinline__ float column_base(float hp_hi, float hp_lo, float tsc
 //    from the sphere; up to SW_WAVES at a time), so that 32 consecutive directions, one per
 //    lane, fall into neighbouring table columns for every pixel of the tile: a warp's load
 //    touches a few contiguous words instead of 32 scattered ones;
-//  * a warp takes bands of consecutive groups of 32 directions whose columns fit a window of
-//    SW_W columns, blends each pixel's two table rows over that window (the radial weight is
-//    the same for every direction) and keeps the blended row in shared memory: a lookup then
-//    reads two values instead of four.  Groups whose window does not fit read the table itself;
+//  * a warp takes bands of consecutive groups of 32 directions whose columns fit a window (64
+//    columns of 16 pixels, or more columns of fewer pixels at a time, see plan_bands), blends
+//    each pixel's two table rows over that window (the radial weight is the same for every
+//    direction) and keeps the blended row in shared memory: a lookup then reads two values
+//    instead of four.  Groups whose window does not fit read the table itself;
 //  * a lane walks its direction over the row's 16 pixels.  The column t along the row is
 //    smooth, so far from the poles it is a polynomial through 4 or 6 Chebyshev points of the
 //    row instead of 16 arc cosines (row_mode below), and evaluating it for the pixels +-s
@@ -89,7 +90,7 @@ __device__ __forceinline__ float column_base(float hp_hi, float hp_lo, float tsc
 // over spheres with Kahan compensation: the same for the staged and the unstaged kernel, whose
 // results are therefore identical.
 // ---------------------------------------------------------------------------
-constexpr int SW_BATCH = 4;  // pixels whose table rows a lane loads together
+constexpr int SW_BATCH = 4;      // pixels whose table rows a lane loads together
 constexpr int SW_NT = 256;       // threads per block
 constexpr int SW_WAVES = 1024;   // directions sorted at a time
 constexpr int SW_W = 64;         // columns of a pixel's window
@@ -229,36 +230,62 @@ __device__ __forceinline__ void order_waves(SwShared& sm, const float4* __restri
 }
 
 // Warp 0: lane g finds the band that starts at group g, the groups [g, nx) whose columns, seen from
-// anywhere in the tile, fit one window: band[g] = {first column, nx | fits << 8 | columns << 16,
+// anywhere in the tile, fit one window: band[g] = {first column, nx | shape << 8 | columns << 16,
 // (half row length) / (smallest sine of the angles between the band's directions and the tile's
-// pixels), 0}.  A group that fits no window is a band of its own.  Returns the number of chunks of
-// `chunk` directions (64, 32 or 16) in the bands that fit (lane 0; chunk 0: none).
-__device__ __forceinline__ unsigned plan_bands(SwShared& sm, int G, int nkb, int thetaR, float tsc, float gam, int chunk) {
+// pixels), 0}.  The window holds 16 pixels x 64 columns, half the row's pixels x 128 or a quarter x 256
+// (shapes 1, 2, 3): wider ones take in more groups per blended row, but a row's polynomials are made
+// again for each part.  The shape of least cost per (pixel, group) is taken, in instructions and their
+// shared-memory share: 24 per 64 columns blended, and the row's polynomial (3.5 or 5.5 a pixel, 16 pixels)
+// or arc cosine (11); none (shape 0: a band of one group, cells from the table) where all are above 40.
+// Measured with 16 x 64 alone and with all three: 768^2 pixels of 0.39 um, 120 spheres, 1000 directions 144
+// and 120 ms; 906^2 of 0.13 um, NA 0.9 18.7 and 17.0 ms; 3072^2 of 0.1 um (narrow windows throughout) the same.
+// Returns the number of chunks of `chunk` directions (64, 32 or 16) in the bands with a window (lane 0;
+// chunk 0: none).
+__device__ __forceinline__ unsigned plan_bands(SwShared& sm, int G, int nkb, int thetaR, float tsc, float gam, float rdist,
+                                               int chunk) {
     const int lane = threadIdx.x & 31;
     const float gcol = gam * tsc;
     int info = 0;
     if (lane < G) {
+        const int t_lo = max(0, (int)floorf(sm.gb[lane].x - gcol) - 1) & ~1;
+        float best = 40.f, bq = 0.f;
+        info = (lane + 1);
         float lo = sm.gb[lane].x, hi = sm.gb[lane].y;
-        const int t_lo = max(0, (int)floorf(lo - gcol) - 1) & ~1;
+        auto quotient = [&]() {  // (half row length) / (smallest sine)
+            const float rt = 1.f / tsc, th0 = lo * rt - gam, th1 = hi * rt + gam;
+            const float sn = th0 > 0.f && th1 < (float)TRUE_PI ? fminf(__sinf(th0), __sinf(th1)) : 0.f;
+            return sm.half / fmaxf(sn, 1e-30f);
+        };
+        bq = quotient();
         int nx = lane, t_hi = t_lo;
-        while (nx < G) {
-            const float2 b = sm.gb[nx];
-            const int th = min(thetaR, (int)floorf(b.y + gcol) + 2);
-            if (th - t_lo > SW_W - 1 || max(0, (int)floorf(b.x - gcol) - 1) < t_lo) break;
-            t_hi = max(t_hi, th);
-            lo = fminf(lo, b.x);
-            hi = fmaxf(hi, b.y);
-            nx++;
+        for (int s = 0; s < 3; s++) {  // the groups that fit a wider window continue those of the narrower
+            while (nx < G) {
+                const float2 b = sm.gb[nx];
+                const int th = min(thetaR, (int)floorf(b.y + gcol) + 2);
+                if (th - t_lo > (SW_W << s) - 1 || max(0, (int)floorf(b.x - gcol) - 1) < t_lo) break;
+                t_hi = max(t_hi, th);
+                lo = fminf(lo, b.x);
+                hi = fmaxf(hi, b.y);
+                nx++;
+            }
+            if (nx == lane) continue;
+            const float q = quotient();
+            const int mode = row_mode(q * rdist);
+            const float cost = 24.f * (1 << s) / (nx - lane) +
+                               (mode == 4 && s == 0 ? 3.5f : mode != 0 ? 5.5f * (1 << s) : 11.f);
+            if (cost < best) {
+                best = cost;
+                bq = q;
+                info = nx | (s + 1) << 8 | (t_hi - t_lo) << 16;
+            }
+            if (nx == G) break;
         }
-        info = (nx > lane ? nx | 256 : lane + 1) | (t_hi - t_lo) << 16;
-        const float rt = 1.f / tsc, th0 = lo * rt - gam, th1 = hi * rt + gam;
-        const float sn = th0 > 0.f && th1 < (float)TRUE_PI ? fminf(__sinf(th0), __sinf(th1)) : 0.f;
-        sm.band[lane] = make_int4(t_lo, info, __float_as_int(sm.half / fmaxf(sn, 1e-30f)), 0);
+        sm.band[lane] = make_int4(t_lo, info, __float_as_int(bq), 0);
     }
     unsigned mask = 0;  // groups in bands that fit
     for (int g = 0; g < G;) {
         const int i = __shfl_sync(0xffffffffu, info, g), nx = i & 255;
-        if (i & 256) mask |= (nx < 32 ? (1u << nx) - 1u : 0xffffffffu) & ~((1u << g) - 1u);
+        if (i & 0x300) mask |= (nx < 32 ? (1u << nx) - 1u : 0xffffffffu) & ~((1u << g) - 1u);
         g = nx;
     }
     const unsigned last = mask >> (G - 1) & 1u;
@@ -370,7 +397,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
             const cpx<float>* phs = ph + (size_t)s * sc.nk + w0;
             // ---- the tile seen from the sphere: centre direction, angular radius gamma ----
             float3 ctr;
-            float gam;
+            float gam, tile_rdist = 0.f;  // 1 / distance of the tile's centre
             {
                 const float3 A = sm.A, X = sm.X, Y = sm.Y, P = make_float3((float)S.p[0], (float)S.p[1], (float)S.p[2]);
                 const float iR = sm.iR;
@@ -383,6 +410,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
                 gam = (float)TRUE_PI;
                 if (cl2 > 0.f) {
                     const float ci = 1.f / sqrtf(cl2);
+                    tile_rdist = ci;
                     ctr = make_float3(ctr.x * ci, ctr.y * ci, ctr.z * ci);
                     const float3 q = at((float)((lane & 1) ? min(tu + 15, sc.R - 1) : tu),
                                         (float)((lane & 2) ? min(tv + 15, sc.R - 1) : tv));
@@ -417,7 +445,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
                 if (lane == 0) sm.gb[g] = t;
             }
             __syncthreads();
-            if (warp == 0) staged_units += plan_bands(sm, G, nkb, thetaR, tsc, gam, STAGE ? chunk : 0);
+            if (warp == 0) staged_units += plan_bands(sm, G, nkb, thetaR, tsc, gam, tile_rdist, STAGE ? chunk : 0);
             __syncthreads();
 #pragma unroll 1
             for (int r = 0; r < 2; r++) {
@@ -429,38 +457,42 @@ __global__ void __launch_bounds__(SW_NT, 2)
                 int g0 = 0;
                 while (g0 < G) {
                     const int4 band = sm.band[g0];
-                    const int t_lo = band.x, g1 = band.y & 255, width = band.y >> 16;
-                    const int mode = row_mode(__int_as_float(band.z) * sm.rdist[warp][r]);
-                    const bool staged = STAGE && (band.y & 256);
-                    if (staged) {
+                    const int t_lo = band.x, g1 = band.y & 255, shape = band.y >> 8 & 3, width = band.y >> 16;
+                    int mode = row_mode(__int_as_float(band.z) * sm.rdist[warp][r]);
+                    if (shape > 1 && mode == 4) mode = 6;  // one polynomial for the wider windows
+                    // the blended rows of part h of the row: pixels i and 15 - i, i in [8 h / parts, 8 (h + 1) / parts)
+                    auto stage = [&](auto sh, int h) {
+                        constexpr int S = decltype(sh)::value, NP = 16 >> S, W = SW_W << S;
                         __syncwarp();  // readers of the previous window are done
-                        const int col = t_lo + 2 * lane;
-                        if (2 * lane <= width && col + 2 <= row_len) {
-                            float2* dst = &sm.win[warp][2 * lane];
 #pragma unroll 1
-                            for (int j0 = 0; j0 < 16; j0 += SW_BATCH) {
+                        for (int c = 2 * lane; c <= width; c += 64) {
+                            if (t_lo + c + 2 > row_len) break;
+                            const float2* src = tab + t_lo + c;
+                            float2* dst = &sm.win[warp][c];
+#pragma unroll 1
+                            for (int e0 = 0; e0 < NP; e0 += SW_BATCH) {
                                 ulonglong2 a[SW_BATCH], b[SW_BATCH];
                                 float al_[SW_BATCH];
 #pragma unroll
-                                for (int j = 0; j < SW_BATCH; j++) {
-                                    const PixRow q = px[j0 + j];
-                                    const float2* src = tab + (size_t)(q.off + (unsigned)col);
-                                    a[j] = __ldg(reinterpret_cast<const ulonglong2*>(src));
-                                    b[j] = __ldg(reinterpret_cast<const ulonglong2*>(src + row_len));
-                                    al_[j] = q.al;
+                                for (int q = 0; q < SW_BATCH; q++) {
+                                    const int sl = e0 + q, i = h * (NP / 2) + (sl >> 1);
+                                    const PixRow pr = px[sl & 1 ? 15 - i : i];
+                                    a[q] = __ldg(reinterpret_cast<const ulonglong2*>(src + pr.off));
+                                    b[q] = __ldg(reinterpret_cast<const ulonglong2*>(src + pr.off + row_len));
+                                    al_[q] = pr.al;
                                 }
 #pragma unroll
-                                for (int j = 0; j < SW_BATCH; j++) {
-                                    const f32x2 al = f2_splat(al_[j]);
+                                for (int q = 0; q < SW_BATCH; q++) {
+                                    const f32x2 al = f2_splat(al_[q]);
                                     ulonglong2 v;
-                                    v.x = f2_fma(al, f2_sub(b[j].x, a[j].x), a[j].x);
-                                    v.y = f2_fma(al, f2_sub(b[j].y, a[j].y), a[j].y);
-                                    *reinterpret_cast<ulonglong2*>(dst + (j0 + j) * SW_W) = v;
+                                    v.x = f2_fma(al, f2_sub(b[q].x, a[q].x), a[q].x);
+                                    v.y = f2_fma(al, f2_sub(b[q].y, a[q].y), a[q].y);
+                                    *reinterpret_cast<ulonglong2*>(dst + (e0 + q) * W) = v;
                                 }
                             }
                         }
                         __syncwarp();
-                    }
+                    };
                     const f32x2 ntsc = f2_splat(-tsc), hb = f2_splat(column_base(hp_hi, hp_lo, tsc, t_lo));
                     // polynomial coefficients of a direction's column along the row (x = +-(7.5 - i) / 7.5)
                     auto node = [&](float4 k, int n) {
@@ -478,7 +510,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
                             const float o0 = (u.x - u.y) * 0.541196100f, o1 = (v.x - v.y) * 1.306562965f;
                             a[2] = (e0 - e1) * 1.414213562f, a[0] = fmaf(a[2], -0.146446609f, e1);
                             a[3] = (o0 - o1) * 1.414213562f, a[1] = fmaf(a[3], -0.146446609f, o1);
-                        } else {
+                        } else if constexpr (decltype(nc)::value == 6) {
                             const float2 u = node(k, 2), v = node(k, 3), w = node(k, 4);
                             const float y0 = 0.933012702f, y1 = 0.5f, y2 = 0.066987298f;
                             auto poly = [&](float f0, float f1, float f2, float& c0_, float& c2_, float& c4_) {
@@ -492,14 +524,21 @@ __global__ void __launch_bounds__(SW_NT, 2)
                                  a[3], a[5]);
                         }
                     };
-                    auto column = [&](auto nc, const float (&a)[6], int i) {
+                    auto column = [&](auto nc, const float (&a)[6], float4 k, int i) {
                         const float x = (SW_HALF - i) / SW_HALF;
-                        float ev, od;
+                        float ev = 0.f, od = 0.f;
                         if constexpr (decltype(nc)::value == 4) {
                             ev = fmaf(a[2], x * x, a[0]), od = fmaf(a[3], x * x, a[1]);
-                        } else {
+                        } else if constexpr (decltype(nc)::value == 6) {
                             ev = fmaf(fmaf(a[4], x * x, a[2]), x * x, a[0]);
                             od = fmaf(fmaf(a[5], x * x, a[3]), x * x, a[1]);
+                        } else {  // an arc cosine per pixel
+                            const float4 xy = sm.dir[warp][r][2 * i], zc = sm.dir[warp][r][2 * i + 1];
+                            return f2_unpack(theta_column2(
+                                f2_fma(f2_splat(k.x), f2_pack(xy.x, xy.y),
+                                       f2_fma(f2_splat(k.y), f2_pack(xy.z, xy.w),
+                                              f2_fma(f2_splat(k.z), f2_pack(zc.x, zc.y), f2_pack(zc.z, zc.w)))),
+                                ntsc, hb));
                         }
                         return make_float2(fmaf(-x, od, ev), fmaf(x, od, ev));
                     };
@@ -508,7 +547,8 @@ __global__ void __launch_bounds__(SW_NT, 2)
                         ar[j] = fmaf(-pw.y, vi, fmaf(pw.x, vr, ar[j]));
                         ai[j] = fmaf(pw.y, vr, fmaf(pw.x, vi, ai[j]));
                     };
-                    auto look = [&](float2 pw, int i, float2 tt) {  // pixels i and 15 - i from the window
+                    auto look = [&](auto sh, float2 pw, int i, float2 tt) {  // pixels i and 15 - i from the window
+                        constexpr int S = decltype(sh)::value, NP = 16 >> S, W = SW_W << S;
 #pragma unroll
                         for (int h = 0; h < 2; h++) {
                             const int j = h ? 15 - i : i;
@@ -517,27 +557,52 @@ __global__ void __launch_bounds__(SW_NT, 2)
                             // the low bits but the last three.  Inside the window by construction; the mask
                             // keeps any column in it
                             const float be = tj - (__fadd_rd(tj, 12582912.f) - 12582912.f);
-                            const unsigned o = (__float_as_uint(__fadd_rd(tj, 1572864.f)) & (8u * (SW_W - 1))) | win0;
+                            const unsigned o = (__float_as_uint(__fadd_rd(tj, 1572864.f)) & (8u * (W - 1))) | win0;
                             const float2* e = reinterpret_cast<const float2*>(
-                                reinterpret_cast<const char*>(&sm.win[0][0]) + o + 8 * SW_W * j);
+                                reinterpret_cast<const char*>(&sm.win[0][0]) + o + 8 * W * (2 * (i % (NP / 2)) + h));
                             add(pw, j, e[0], e[1], be);
                         }
                     };
-                    auto rows = [&](auto nc) {
-                        int g = g0;
+                    auto part = [&](auto nc, auto sh, auto hh) {
+                        constexpr int NI = 8 >> decltype(sh)::value, I0 = decltype(hh)::value * NI;
+                        stage(sh, decltype(hh)::value);
 #pragma unroll 1
-                        for (; g < g1; g++) {
+                        for (int g = g0; g < g1; g++) {
+                            // keeps the row's node and pixel directions in shared memory: held in registers over
+                            // this loop they spill the sums (24.6 against 22.6 ms, 3072^2 pixels x 2 spheres)
+                            asm volatile("" ::: "memory");
                             float a[6];
                             const float2 pa = sm.p[32 * g + lane];
-                            coefs(nc, sm.k[32 * g + lane], a);
+                            const float4 k = sm.k[32 * g + lane];
+                            coefs(nc, k, a);
 #pragma unroll
-                            for (int i = 0; i < 8; i++) look(pa, i, column(nc, a, i));
+                            for (int i = 0; i < NI; i++) look(sh, pa, I0 + i, column(nc, a, k, I0 + i));
                         }
                     };
-                    if (staged && mode == 4) {
-                        rows(Int<4>{});
-                    } else if (staged && mode == 6) {
-                        rows(Int<6>{});
+                    auto rows = [&](auto nc, auto sh) {
+                        constexpr int S = decltype(sh)::value;
+                        part(nc, sh, Int<0>{});
+                        if constexpr (S > 0) part(nc, sh, Int<1>{});
+                        if constexpr (S > 1) {
+                            part(nc, sh, Int<2>{});
+                            part(nc, sh, Int<3>{});
+                        }
+                    };
+                    auto by_mode = [&](auto sh) {
+                        if constexpr (decltype(sh)::value == 0)
+                            if (mode == 4) {
+                                rows(Int<4>{}, sh);
+                                return;
+                            }
+                        if (mode == 6) rows(Int<6>{}, sh);
+                        else rows(Int<0>{}, sh);
+                    };
+                    if (STAGE && shape == 1) {
+                        by_mode(Int<0>{});
+                    } else if (STAGE && shape == 2) {
+                        by_mode(Int<1>{});
+                    } else if (STAGE && shape == 3) {
+                        by_mode(Int<2>{});
                     } else {
 #pragma unroll 1
                         for (int g = g0; g < g1; g++) {
@@ -548,23 +613,8 @@ __global__ void __launch_bounds__(SW_NT, 2)
                             if (mode == 6) coefs(Int<6>{}, k, a);
 #pragma unroll
                             for (int i = 0; i < 8; i++) {
-                                float2 t;
-                                if (mode == 4) {
-                                    t = column(Int<4>{}, a, i);
-                                } else if (mode == 6) {
-                                    t = column(Int<6>{}, a, i);
-                                } else {
-                                    const float4 xy = sm.dir[warp][r][2 * i], zc = sm.dir[warp][r][2 * i + 1];
-                                    t = f2_unpack(theta_column2(f2_fma(f2_splat(k.x), f2_pack(xy.x, xy.y),
-                                                             f2_fma(f2_splat(k.y), f2_pack(xy.z, xy.w),
-                                                                    f2_fma(f2_splat(k.z), f2_pack(zc.x, zc.y),
-                                                                           f2_pack(zc.z, zc.w)))),
-                                                      ntsc, hb));
-                                }
-                                if (staged) {
-                                    look(pw, i, t);
-                                    continue;
-                                }
+                                const float2 t = mode == 4 ? column(Int<4>{}, a, k, i)
+                                                           : mode == 6 ? column(Int<6>{}, a, k, i) : column(Int<0>{}, a, k, i);
 #pragma unroll
                                 for (int h = 0; h < 2; h++) {
                                     const int j = h ? 15 - i : i;
@@ -574,7 +624,8 @@ __global__ void __launch_bounds__(SW_NT, 2)
                                     const f32x2* e = reinterpret_cast<const f32x2*>(tab + (size_t)(q.off + (unsigned)n));
                                     const f32x2 al = f2_splat(q.al);
                                     const f32x2 e00 = e[0], e01 = e[1], e10 = e[row_len], e11 = e[row_len + 1];
-                                    add(pw, j, f2_unpack(f2_fma(al, f2_sub(e10, e00), e00)), f2_unpack(f2_fma(al, f2_sub(e11, e01), e01)), tj - tf);
+                                    add(pw, j, f2_unpack(f2_fma(al, f2_sub(e10, e00), e00)),
+                                        f2_unpack(f2_fma(al, f2_sub(e11, e01), e01)), tj - tf);
                                 }
                             }
                         }
