@@ -417,6 +417,46 @@ static void passbands(const bs_ctx* c, std::vector<int>& su, std::vector<int>& s
     }
 }
 
+// The folded forward transforms: fields [R][R] along x to f1 [Nu][R], f1 along y to f2 [Nv][Nu].  A passband is
+// the bins 0 .. npos - 1 and R - nneg .. R - 1 (bin_freq is monotonic on both sides).
+static FoldDft fold_dft(int R, const std::vector<int>& bins) {
+    FoldDft f{};
+    f.R = f.lda = R;
+    while (f.npos < (int)bins.size() && bins[f.npos] <= R / 2) f.npos++;
+    f.nneg = (int)bins.size() - f.npos;
+    f.nh = std::max(f.npos, f.nneg + 1);
+    return f;
+}
+static FoldDft fold_x(int R, const std::vector<int>& su, const std::vector<int>& sv) {
+    FoldDft f = fold_dft(R, su);
+    f.M = R;
+    f.ldt = std::max(f.nh, fold_dft(R, sv).nh);
+    f.row_stride = 1;
+    f.bin_stride = R;
+    f.sA = (long long)R * R;
+    f.sC = (long long)su.size() * R;
+    return f;
+}
+static FoldDft fold_y(int R, const std::vector<int>& su, const std::vector<int>& sv) {
+    FoldDft f = fold_dft(R, sv);
+    f.M = (int)su.size();
+    f.ldt = std::max(f.nh, fold_dft(R, su).nh);
+    f.row_stride = 1;
+    f.bin_stride = (int)su.size();
+    f.sA = (long long)su.size() * R;
+    f.sC = (long long)su.size() * sv.size();
+    return f;
+}
+
+// Elements of the split-K scratch of a slice's transforms
+template <class T>
+static size_t detector_scratch_elems(const FoldDft& fx, const FoldDft& fy, int Nu, int Nv, int C) {
+    const int R = fx.R;
+    const size_t fwd = sizeof(T) == 8 ? std::max(fold_scratch_elems(fx, 2), fold_scratch_elems(fy, 2))
+                                      : std::max(cgemm_scratch_elems<T>(R, Nu, R, 2), cgemm_scratch_elems<T>(Nv, Nu, R, 2));
+    return std::max(fwd, std::max(cgemm_scratch_elems<T>(Nv, C, Nu, 2), cgemm_scratch_elems<T>(C, C, Nv, 2)));
+}
+
 template <class T>
 static bs_status run_detector(bs_ctx* c, bool accumulate) {
     const bs_params& p = c->prm;
@@ -444,8 +484,14 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
     CK(c->d_su.ensure(Nu * sizeof(int)));
     CK(c->d_sv.ensure(Nv * sizeof(int)));
     CK(c->d_mask.ensure(mask.size() * sizeof(float)));
-    CK(c->d_wx.ensure((size_t)R * Nu * ce));
-    CK(c->d_wy.ensure((size_t)Nv * R * ce));
+    constexpr bool fp64 = sizeof(T) == 8;
+    const FoldDft fx = fold_x(R, su, sv), fy = fold_y(R, su, sv);
+    if (fp64) {
+        CK(c->d_wx.ensure((size_t)(R / 2 + 1) * fx.ldt * ce));
+    } else {
+        CK(c->d_wx.ensure((size_t)R * Nu * ce));
+        CK(c->d_wy.ensure((size_t)Nv * R * ce));
+    }
     CK(c->d_wix.ensure((size_t)Nu * C * ce));
     CK(c->d_wiy.ensure((size_t)C * Nv * ce));
     CK(c->d_f1.ensure(2 * (size_t)R * Nu * ce));
@@ -460,10 +506,15 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
     cpx<T>* wix = c->d_wix.as<cpx<T>>();
     cpx<T>* wiy = c->d_wiy.as<cpx<T>>();
     // forward x: Wx[x][k] = e^{-2 pi i x su_k / R}; forward y: Wy[j][y] = e^{-2 pi i y sv_j / R}
-    launch_twiddle<T>(R, Nu, c->d_su.as<int>(), 0, R, -1, Nu, 1, wx, c->st);
-    LAUNCHED(c);
-    launch_twiddle<T>(R, Nv, c->d_sv.as<int>(), 0, R, -1, 1, R, wy, c->st);
-    LAUNCHED(c);
+    if constexpr (fp64) {
+        launch_fold_table(R, fx.ldt, wx, c->st);
+        LAUNCHED(c);
+    } else {
+        launch_twiddle<T>(R, Nu, c->d_su.as<int>(), 0, R, -1, Nu, 1, wx, c->st);
+        LAUNCHED(c);
+        launch_twiddle<T>(R, Nv, c->d_sv.as<int>(), 0, R, -1, 1, R, wy, c->st);
+        LAUNCHED(c);
+    }
     // inverse on the crop only: Wix[k][x] = e^{+2 pi i (off+x) su_k / R}, Wiy[y][j] likewise
     launch_twiddle<T>(C, Nu, c->d_su.as<int>(), c->off, R, +1, 1, C, wix, c->st);
     LAUNCHED(c);
@@ -476,16 +527,22 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
     T* I = c->d_I.as<T>();
     long long RR = (long long)R * R;
     // split-K scratch for the GEMMs with few output tiles
-    const size_t scr = std::max(std::max(cgemm_scratch_elems<T>(R, Nu, R, 2), cgemm_scratch_elems<T>(Nv, Nu, R, 2)),
-                                std::max(cgemm_scratch_elems<T>(Nv, C, Nu, 2), cgemm_scratch_elems<T>(C, C, Nv, 2)));
+    const size_t scr = detector_scratch_elems<T>(fx, fy, Nu, Nv, C);
     CK(c->d_gscr.ensure(std::max<size_t>(scr, 1) * ce));
     cpx<T>* gs = c->d_gscr.as<cpx<T>>();
-    launch_cgemm<T>(R, Nu, R, 2, fields, R, RR, wx, Nu, 0, f1, Nu, (long long)R * Nu, 0, nullptr, (T)1, nullptr, gs,
-                    scr, c->st);
-    LAUNCHED(c);
-    launch_cgemm<T>(Nv, Nu, R, 2, wy, R, 0, f1, Nu, (long long)R * Nu, f2, Nu, (long long)Nv * Nu, 1,
-                    c->d_mask.as<float>(), (T)1, nullptr, gs, scr, c->st);
-    LAUNCHED(c);
+    if constexpr (fp64) {  // f1 transposed: [Nu][R]
+        launch_fold_dft(fx, 2, fields, wx, f1, nullptr, gs, c->st);
+        LAUNCHED(c);
+        launch_fold_dft(fy, 2, f1, wx, f2, c->d_mask.as<float>(), gs, c->st);
+        LAUNCHED(c);
+    } else {
+        launch_cgemm<T>(R, Nu, R, 2, fields, R, RR, wx, Nu, 0, f1, Nu, (long long)R * Nu, 0, nullptr, (T)1, nullptr, gs,
+                        scr, c->st);
+        LAUNCHED(c);
+        launch_cgemm<T>(Nv, Nu, R, 2, wy, R, 0, f1, Nu, (long long)R * Nu, f2, Nu, (long long)Nv * Nu, 1,
+                        c->d_mask.as<float>(), (T)1, nullptr, gs, scr, c->st);
+        LAUNCHED(c);
+    }
     if (c->bp_on) {
         // applyBackpropagation (microscope.cu:423-488, 592-605) on U only: -exp(i kz d) with
         // kz = sqrt(k^2 - kx^2 - ky^2), k = 2 PI / lambda, kx = 2 PI u; zero where kx^2 + ky^2 >= k^2
@@ -1064,14 +1121,12 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
     b += B(2 * res * res * rT);                               // D, Di
     if (Nu && Nv) {
         b += B(Nu * sizeof(int)) + B(Nv * sizeof(int)) + B(Nv * Nu * sizeof(float));
-        b += B(R * Nu * cT) + B(Nv * R * cT) + B(Nu * C * cT) + B(C * Nv * cT);
+        const FoldDft fx = fold_x((int)R, su, sv), fy = fold_y((int)R, su, sv);
+        b += fp64 ? B((R / 2 + 1) * fx.ldt * cT) : B(R * Nu * cT) + B(Nv * R * cT);
+        b += B(Nu * C * cT) + B(C * Nv * cT);
         b += B(2 * R * Nu * cT) + B(2 * Nv * Nu * cT) + B(2 * Nv * C * cT) + B(2 * C * C * rT);
-        const int Ri = (int)R, Ui = (int)Nu, Vi = (int)Nv, Ci = (int)C;
-        auto elems = [fp64](int M, int N, int K) {
-            return fp64 ? cgemm_scratch_elems<double>(M, N, K, 2) : cgemm_scratch_elems<float>(M, N, K, 2);
-        };
-        const size_t scr = std::max(std::max(elems(Ri, Ui, Ri), elems(Vi, Ui, Ri)),
-                                    std::max(elems(Vi, Ci, Ui), elems(Ci, Ci, Vi)));
+        const size_t scr = fp64 ? detector_scratch_elems<double>(fx, fy, (int)Nu, (int)Nv, (int)C)
+                                : detector_scratch_elems<float>(fx, fy, (int)Nu, (int)Nv, (int)C);
         b += B(std::max<size_t>(scr, 1) * cT);  // split-K parts
     }
     b += B(res * res * rT);                                   // image staging

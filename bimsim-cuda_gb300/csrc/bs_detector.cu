@@ -32,17 +32,23 @@ __global__ void twiddle_kernel(int ni, int nj, const int* __restrict__ freq, int
     out[(long long)i * ld_i + (long long)j * ld_j] = mk((T)c, (T)(sign * s));
 }
 
-// Tiled complex GEMM.  Block 16 x 16 threads, tile 64 x 16 NJ, each thread
-// 4 x NJ outputs, K tiles of 16.  Accumulation is split into per-tile
-// partial sums combined with Kahan compensation.  Double precision is bound by the
-// FP64 pipe (four multiply-adds per product), so its tile is 16 columns wide: a
-// passband of 41 columns fills 85 % of the tiles' work instead of 64 %.
-// 1280^2 field to 41 columns, two fields: 3.55 -> 1.36 ms.
-constexpr int GB_M = 64, GB_K = 16;
+// Tiled complex GEMM: tile GM x GN, K tiles of 16, accumulation split into per-tile
+// partial sums combined with Kahan compensation.  Single precision: 16 x 16 threads of
+// 4 x 2 outputs, 64 x 32.  Double precision is bound by the FP64 pipe (four multiply-adds
+// per product) and, on the inverse transforms' few output tiles, by one SM's share of it:
+// 8 x 16 threads (a warp for each quarter of the pipe) of 2 x 1 outputs, 32 x 8.  96 x 25 and
+// 96 x 96 outputs, K = 25, two fields: 44 and 46 us in tiles of 64 x 16, 17 and 17 us now.
+constexpr int GB_K = 16;
+template <class T>
+__host__ __device__ constexpr int gb_tx() { return sizeof(T) == 8 ? 8 : 16; }  // 16 threads along M
+template <class T>
+__host__ __device__ constexpr int gb_ni() { return sizeof(T) == 8 ? 2 : 4; }
 template <class T>
 __host__ __device__ constexpr int gb_nj() { return sizeof(T) == 8 ? 1 : 2; }
 template <class T>
-__host__ __device__ constexpr int gb_n() { return 16 * gb_nj<T>(); }
+__host__ __device__ constexpr int gb_m() { return 16 * gb_ni<T>(); }
+template <class T>
+__host__ __device__ constexpr int gb_n() { return gb_tx<T>() * gb_nj<T>(); }
 
 // One product a b of a tile's sum (p0 - p1) + i (p2 + p3).  Double precision sums the four products of the
 // parts each on its own, four instructions; single precision is not bound by its pipe and rounds each
@@ -84,34 +90,34 @@ __device__ __forceinline__ void cgemm_store(int epi, long long o, int gm, int gn
 // ks-th of ksplit equal K ranges into part[b][ks][M][N]; cgemm_reduce_kernel
 // adds the ranges in order (deterministic) and applies the epilogue.
 template <class T>
-__global__ void __launch_bounds__(256) cgemm_kernel(int M, int N, int K, const cpx<T>* __restrict__ A, int lda,
+__global__ void __launch_bounds__(16 * gb_tx<T>()) cgemm_kernel(int M, int N, int K, const cpx<T>* __restrict__ A, int lda,
                                                     long long sA, const cpx<T>* __restrict__ B, int ldb, long long sB,
                                                     cpx<T>* __restrict__ C, int ldc, long long sC, int epi,
                                                     const float* __restrict__ mask, T scale, T* __restrict__ I,
                                                     int ksplit, cpx<T>* __restrict__ part) {
-    constexpr int NJ = gb_nj<T>(), GN = gb_n<T>();
-    __shared__ cpx<T> As[GB_K][GB_M + 1];
+    constexpr int NT = gb_tx<T>(), NI = gb_ni<T>(), NJ = gb_nj<T>(), GM = gb_m<T>(), GN = gb_n<T>();
+    __shared__ cpx<T> As[GB_K][GM + 1];
     __shared__ cpx<T> Bs[GB_K][GN + 1];
     const int b = blockIdx.z / ksplit, ks = blockIdx.z % ksplit;
     A += b * sA;
     B += b * sB;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * GB_M, n0 = blockIdx.x * GN;
+    const int tx = threadIdx.x % NT, ty = threadIdx.x / NT;
+    const int m0 = blockIdx.y * GM, n0 = blockIdx.x * GN;
     const int kc = ((K + ksplit - 1) / ksplit + GB_K - 1) / GB_K * GB_K;  // K range per split, whole tiles
     const int kbeg = ks * kc, kend = min(K, kbeg + kc);
-    T accr[4][NJ], acci[4][NJ], cr[4][NJ], ci[4][NJ];
-    T p0[4][NJ], p1[4][NJ], p2[4][NJ], p3[4][NJ];  // the tile's sums, see cmac
+    T accr[NI][NJ], acci[NI][NJ], cr[NI][NJ], ci[NI][NJ];
+    T p0[NI][NJ], p1[NI][NJ], p2[NI][NJ], p3[NI][NJ];  // the tile's sums, see cmac
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < NI; i++)
 #pragma unroll
         for (int j = 0; j < NJ; j++) accr[i][j] = acci[i][j] = cr[i][j] = ci[i][j] = p0[i][j] = p1[i][j] = p2[i][j] = p3[i][j] = 0;
     for (int k0 = kbeg; k0 < kend; k0 += GB_K) {
-        for (int e = threadIdx.x; e < GB_K * GB_M; e += 256) {
+        for (int e = threadIdx.x; e < GB_K * GM; e += 16 * NT) {
             int kk = e % GB_K, mm = e / GB_K;
             int gm = m0 + mm, gk = k0 + kk;
             As[kk][mm] = (gm < M && gk < kend) ? A[(long long)gm * lda + gk] : mk((T)0, (T)0);
         }
-        for (int e = threadIdx.x; e < GB_K * GN; e += 256) {
+        for (int e = threadIdx.x; e < GB_K * GN; e += 16 * NT) {
             int nn = e % GN, kk = e / GN;
             int gn = n0 + nn, gk = k0 + kk;
             Bs[kk][nn] = (gn < N && gk < kend) ? B[(long long)gk * ldb + gn] : mk((T)0, (T)0);
@@ -119,20 +125,20 @@ __global__ void __launch_bounds__(256) cgemm_kernel(int M, int N, int K, const c
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < GB_K; kk++) {
-            cpx<T> a[4], bb[NJ];
+            cpx<T> a[NI], bb[NJ];
 #pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty + 16 * i];
+            for (int i = 0; i < NI; i++) a[i] = As[kk][ty + 16 * i];
 #pragma unroll
-            for (int j = 0; j < NJ; j++) bb[j] = Bs[kk][tx + 16 * j];
+            for (int j = 0; j < NJ; j++) bb[j] = Bs[kk][tx + NT * j];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < NI; i++)
 #pragma unroll
                 for (int j = 0; j < NJ; j++) {
                     cmac(a[i], bb[j], p0[i][j], p1[i][j], p2[i][j], p3[i][j]);
                 }
         }
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < NI; i++)
 #pragma unroll
             for (int j = 0; j < NJ; j++) {  // Kahan step
                 T yr = (p0[i][j] - p1[i][j]) - cr[i][j], yi = (p2[i][j] + p3[i][j]) - ci[i][j];
@@ -146,10 +152,10 @@ __global__ void __launch_bounds__(256) cgemm_kernel(int M, int N, int K, const c
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < NI; i++)
 #pragma unroll
         for (int j = 0; j < NJ; j++) {
-            int gm = m0 + ty + 16 * i, gn = n0 + tx + 16 * j;
+            int gm = m0 + ty + 16 * i, gn = n0 + tx + NT * j;
             if (gm >= M || gn >= N) continue;
             if (ksplit > 1)
                 part[((long long)blockIdx.z * M + gm) * N + gn] = mk(accr[i][j], acci[i][j]);
@@ -177,6 +183,135 @@ __global__ void cgemm_reduce_kernel(int M, int N, int batch, int ksplit, const c
         si = ti;
     }
     cgemm_store(epi, b * sC + (long long)gm * ldc + gn, gm, gn, N, sr, si, C, mask, scale, I);
+}
+
+// ---------------------------------------------------------------------------
+// The double-precision forward transforms, folded.  With e_n = x_n + x_{R-n} and o_n = x_n - x_{R-n},
+//   X(+-h) = sum_n e_n cos(2 pi n h / R) -+ i sum_n o_n sin(2 pi n h / R),   n = 0 .. R / 2,
+// so two bins and two samples share four multiply-adds where the plain product takes sixteen; the FP64
+// pipe bounds both.  Tile 32 rows x 8 bins, 8 x 16 threads of 2 x 1 (a warp for each quarter of the
+// pipe), 16 folded samples at a time: a tile small enough that a small slice's few tiles,
+// split along the samples, still reach every SM.  Sums of two tiles are combined with Kahan compensation.
+// 1280^2 field to 42 columns, two fields: 1.36 ms as a plain product, 0.36 ms folded; 288^2 to
+// 26 columns and on to 26 rows: 111 + 106 us, 23 + 12 us (and 12 us each for the splits).
+// ---------------------------------------------------------------------------
+constexpr int FD_M = 32, FD_H = 8;
+
+// tab[n][h] = (cos, sin)(2 pi n h / R), n = 0 .. R / 2
+__global__ void fold_table_kernel(int R, int nh, zd* __restrict__ tab) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (R / 2 + 1) * nh) return;
+    const long long m = (long long)(e / nh) * (e % nh) % R;
+    double s, c;
+    sincospi(2.0 * (double)m / (double)R, &s, &c);
+    tab[e] = mk(c, s);
+}
+
+// Where the bins +-h of row gm go, and their values from the sums q = (sum e cos, sum o sin).
+__device__ __forceinline__ void fold_store(const FoldDft& f, int b, int gm, int h, zd ec, zd os, zd* __restrict__ C,
+                                           const float* __restrict__ mask) {
+    auto put = [&](int pos, zd v) {
+        const long long o = (long long)gm * f.row_stride + (long long)pos * f.bin_stride;
+        if (mask) {
+            const double w = (double)mask[o];
+            v = mk(v.re * w, v.im * w);
+        }
+        C[b * f.sC + o] = v;
+    };
+    if (h < f.npos) put(h, mk(ec.re + os.im, ec.im - os.re));
+    if (h >= 1 && h <= f.nneg) put(f.npos + f.nneg - h, mk(ec.re - os.im, ec.im + os.re));
+}
+
+__global__ void __launch_bounds__(128) fold_dft_kernel(FoldDft f, const zd* __restrict__ A, const zd* __restrict__ tab,
+                                                      zd* __restrict__ C, const float* __restrict__ mask, int ksplit,
+                                                      zd* __restrict__ part) {
+    __shared__ zd Es[GB_K][FD_M + 1], Os[GB_K][FD_M + 1], Ws[GB_K][FD_H + 1];
+    const int b = blockIdx.z / ksplit, ks = blockIdx.z % ksplit;
+    const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;
+    const int m0 = blockIdx.y * FD_M, h0 = blockIdx.x * FD_H, K = f.R / 2 + 1;
+    const int kc = ((K + GB_K - 1) / GB_K + ksplit - 1) / ksplit * GB_K;  // folded samples per split, whole tiles
+    const int kbeg = ks * kc, kend = min(K, kbeg + kc);
+    A += b * f.sA;
+    double acc[2][4], cmp[2][4], p[2][4];  // per row: sums of e.re cos, e.im cos, o.re sin, o.im sin
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[i][q] = cmp[i][q] = p[i][q] = 0;
+    for (int k0 = kbeg; k0 < kend; k0 += GB_K) {
+#pragma unroll 4
+        for (int e = threadIdx.x; e < GB_K * FD_M; e += 128) {
+            const int kk = e % GB_K, mm = e / GB_K, gm = m0 + mm, n = k0 + kk;
+            zd x = mk(0.0, 0.0), y = x;
+            if (gm < f.M && n < kend) {
+                x = A[(long long)gm * f.lda + n];
+                if (n > 0 && 2 * n < f.R) y = A[(long long)gm * f.lda + f.R - n];  // the samples 0 and R / 2 are alone
+            }
+            Es[kk][mm] = x + y;
+            Os[kk][mm] = x - y;
+        }
+        for (int e = threadIdx.x; e < GB_K * FD_H; e += 128) {
+            const int hh = e % FD_H, kk = e / FD_H;
+            Ws[kk][hh] = h0 + hh < f.nh && k0 + kk < kend ? tab[(long long)(k0 + kk) * f.ldt + h0 + hh] : mk(0.0, 0.0);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < GB_K; kk++) {
+            const zd w = Ws[kk][tx];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const zd ev = Es[kk][ty + 16 * i], ov = Os[kk][ty + 16 * i];
+                p[i][0] = fma(ev.re, w.re, p[i][0]);
+                p[i][1] = fma(ev.im, w.re, p[i][1]);
+                p[i][2] = fma(ov.re, w.im, p[i][2]);
+                p[i][3] = fma(ov.im, w.im, p[i][3]);
+            }
+        }
+        if (((k0 - kbeg) / GB_K & 1) || k0 + GB_K >= kend) {
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) {  // Kahan step
+                    const double v = p[i][q] - cmp[i][q], t = acc[i][q] + v;
+                    cmp[i][q] = (t - acc[i][q]) - v;
+                    acc[i][q] = t;
+                    p[i][q] = 0;
+                }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int gm = m0 + ty + 16 * i, h = h0 + tx;
+        if (gm >= f.M || h >= f.nh) continue;
+        const zd ec = mk(acc[i][0], acc[i][1]), os = mk(acc[i][2], acc[i][3]);
+        if (ksplit > 1) {
+            zd* o = part + 2 * (((long long)blockIdx.z * f.nh + h) * f.M + gm);
+            o[0] = ec;
+            o[1] = os;
+        } else {
+            fold_store(f, b, gm, h, ec, os, C, mask);
+        }
+    }
+}
+
+// The splits' sums added in order (Kahan).
+__global__ void __launch_bounds__(128) fold_reduce_kernel(FoldDft f, int batch, int ksplit, const zd* __restrict__ part,
+                                                          zd* __restrict__ C, const float* __restrict__ mask) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x, per = (long long)f.nh * f.M;
+    if (e >= batch * per) return;
+    const int b = (int)(e / per);
+    zd s[2] = {mk(0.0, 0.0), mk(0.0, 0.0)}, c[2] = {s[0], s[0]};
+#pragma unroll 4
+    for (int ks = 0; ks < ksplit; ks++) {
+        const zd* v = part + 2 * ((b * (long long)ksplit + ks) * per + e % per);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const zd y = v[q] - c[q], t = s[q] + y;
+            c[q] = (t - s[q]) - y;
+            s[q] = t;
+        }
+    }
+    fold_store(f, b, (int)(e % f.M), (int)(e % per / f.M), s[0], s[1], C, mask);
 }
 
 template <class T>
@@ -222,7 +357,7 @@ int cgemm_ksplit(int M, int N, int K, int batch) {
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) !=
                                                    cudaSuccess)
         n_sm = 1;
-    const long long tiles = (long long)((N + gb_n<T>() - 1) / gb_n<T>()) * ((M + GB_M - 1) / GB_M) * batch;
+    const long long tiles = (long long)((N + gb_n<T>() - 1) / gb_n<T>()) * ((M + gb_m<T>() - 1) / gb_m<T>()) * batch;
     const long long want = (sizeof(T) == 8 ? 6LL : 2LL) * n_sm;
     if (tiles <= 0 || 2 * tiles >= want) return 1;
     long long ks = (want + tiles - 1) / tiles;
@@ -242,13 +377,42 @@ void launch_cgemm(int M, int N, int K, int batch, const cpx<T>* A, int lda, long
                   cpx<T>* scratch, size_t scratch_elems, cudaStream_t st) {
     int ks = cgemm_ksplit<T>(M, N, K, batch);
     if ((size_t)batch * ks * M * N > scratch_elems || !scratch) ks = 1;
-    dim3 grid((N + gb_n<T>() - 1) / gb_n<T>(), (M + GB_M - 1) / GB_M, batch * ks);
-    cgemm_kernel<T><<<grid, 256, 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, epi, mask, scale, I, ks,
+    dim3 grid((N + gb_n<T>() - 1) / gb_n<T>(), (M + gb_m<T>() - 1) / gb_m<T>(), batch * ks);
+    cgemm_kernel<T><<<grid, 16 * gb_tx<T>(), 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, epi, mask, scale, I, ks,
                                           scratch);
     if (ks > 1) {
         const long long n = (long long)batch * M * N;
         cgemm_reduce_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(M, N, batch, ks, scratch, C, ldc, sC, epi,
                                                                             mask, scale, I);
+    }
+}
+
+// Blocks for about eight per SM, since the busiest SM's share is the time.  At most 16 splits, whose sums
+// are added one after the other (0.8 us each).
+static int fold_ksplit(const FoldDft& f, int batch) {
+    const int tiles = (f.nh + FD_H - 1) / FD_H * ((f.M + FD_M - 1) / FD_M) * batch, kt = (f.R / 2 + GB_K) / GB_K;
+    const int ks = std::min(std::min((8 * GB300_SMS + tiles - 1) / tiles, kt), 16);
+    const int per = (kt + ks - 1) / ks;  // tiles per split: no split without any
+    return (kt + per - 1) / per;
+}
+
+size_t fold_scratch_elems(const FoldDft& f, int batch) {
+    const int ks = fold_ksplit(f, batch);
+    return ks > 1 ? (size_t)2 * batch * ks * f.nh * f.M : 0;
+}
+
+void launch_fold_table(int R, int nh, zd* tab, cudaStream_t st) {
+    fold_table_kernel<<<(unsigned)(((R / 2 + 1) * nh + 127) / 128), 128, 0, st>>>(R, nh, tab);
+}
+
+void launch_fold_dft(const FoldDft& f, int batch, const zd* A, const zd* tab, zd* C, const float* mask, zd* scratch,
+                     cudaStream_t st) {
+    const int ks = fold_ksplit(f, batch);
+    dim3 grid((f.nh + FD_H - 1) / FD_H, (f.M + FD_M - 1) / FD_M, batch * ks);
+    fold_dft_kernel<<<grid, 128, 0, st>>>(f, A, tab, C, mask, ks, scratch);
+    if (ks > 1) {
+        const long long n = (long long)batch * f.nh * f.M;
+        fold_reduce_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(f, batch, ks, scratch, C, mask);
     }
 }
 
@@ -437,9 +601,12 @@ static void preload_detector_t() {
     cudaFuncGetAttributes(&a, cmul_kernel<T>);
 }
 void preload_detector_kernels() {
+    cudaFuncAttributes a;
+    cudaFuncGetAttributes(&a, fold_table_kernel);
+    cudaFuncGetAttributes(&a, fold_dft_kernel);
+    cudaFuncGetAttributes(&a, fold_reduce_kernel);
     preload_detector_t<float>();
     preload_detector_t<double>();
-    cudaFuncAttributes a;
     cudaFuncGetAttributes(&a, kk_kernel_g);
     cudaFuncGetAttributes(&a, kk_kernel_conv);
 }

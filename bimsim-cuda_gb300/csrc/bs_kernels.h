@@ -12,6 +12,7 @@ namespace bs {
 // Mixed LUT kernel: angle margin (radians) of its window bounds, and the number of
 // directions up to which one thread per pixel reads every cell itself.
 constexpr float LUT_STAGE_MARGIN = 5e-4f;
+constexpr int GB300_SMS = 152;
 constexpr int LUT_FEW_WAVES = 32;
 constexpr int LUT_TILE = 16;
 constexpr int LUT_WINDOW = 256;  // table columns of the widest staged window
@@ -83,7 +84,6 @@ void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int
                          float4 cone, cudaStream_t st);
 // Shares of the spheres that launch_us_lut_mixed runs side by side; above 1, `part` (else null) holds
 // 4 floats per pixel and share.
-constexpr int GB300_SMS = 152;
 int lut_splits(int R, int ns, int nk);
 // One table of the mixed path's table build: the rows of one sphere's Usp or Uip with their
 // coefficient rows at tab + tab_off and biases at bias + row_off, written to the linear rows at
@@ -138,6 +138,19 @@ template <class T>
 void launch_cgemm(int M, int N, int K, int batch, const cpx<T>* A, int lda, long long sA, const cpx<T>* B, int ldb,
                   long long sB, cpx<T>* C, int ldc, long long sC, int epi, const float* mask, T scale, T* I,
                   cpx<T>* scratch, size_t scratch_elems, cudaStream_t st);
+
+// Double-precision forward transform of the rows x_0 .. x_{R-1} of a batch of M x R arrays, the bins 0 .. npos - 1
+// and R - nneg .. R - 1 (stored in that order): bin j of row m to C[b sC + m row_stride + j bin_stride], times
+// mask[m row_stride + j bin_stride] unless mask is null.  nh = max(npos, nneg + 1); tab of launch_fold_table holds
+// ldt >= nh columns; scratch fold_scratch_elems.
+struct FoldDft {
+    int M, R, npos, nneg, nh, lda, ldt, row_stride, bin_stride;
+    long long sA, sC;
+};
+void launch_fold_table(int R, int nh, zd* tab, cudaStream_t st);
+size_t fold_scratch_elems(const FoldDft& f, int batch);
+void launch_fold_dft(const FoldDft& f, int batch, const zd* A, const zd* tab, zd* C, const float* mask, zd* scratch,
+                     cudaStream_t st);
 
 // D[b][iv][iu] (+)= sum over the ss x ss block of I[b] / ss^2 (fieldslice.cu:71-108);
 // accumulate adds to D (the detector sums point sources)
