@@ -900,12 +900,11 @@ static bs_status run_nearfield(bs_ctx* c) {
             const int L = c->Lmax, nlm = L * (L + 1) / 2;
             CK(c->d_shrec.ensure((size_t)nlm * sizeof(ShRec)));
             CK(c->d_shtab.ensure((size_t)nk * nlm * sizeof(double2)));
-            CK(c->d_shcoef.ensure((size_t)ns * nlm * 2 * sizeof(zd)));
+            CK(c->d_shcoef.ensure((size_t)ns * nlm * 4 * sizeof(zd)));
             launch_sh_tables(sc, c->d_sph.as<Sphere>(), L, c->d_waves.as<double>(), c->d_shrec.as<ShRec>(),
-                             c->d_shtab.as<double2>(), c->d_shcoef.as<zd>(), c->st);
+                             c->d_shtab.as<double2>(), c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_shcoef.as<zd>(), c->st);
             c->launches += 3;
-            launch_us_sh<T>(sc, c->d_sph.as<Sphere>(), L, c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_shrec.as<ShRec>(),
-                            c->d_shcoef.as<zd>(), Uf, U, c->st);
+            launch_us_sh<T>(sc, c->d_sph.as<Sphere>(), L, c->d_shrec.as<ShRec>(), c->d_shcoef.as<zd>(), Uf, U, c->st);
             LAUNCHED(c);
         }
         c->interactions = (long long)R * R * ns * nk;
@@ -1086,7 +1085,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         if (p.lut_us) b += B(ns * nk * cT) + B(nk * sizeof(float4));  // phases, float directions
         if (!p.lut_us) {  // direct method: harmonic recurrences, per-wave and per-sphere tables
             const size_t nlm = (size_t)c->Lmax * (c->Lmax + 1) / 2;
-            b += B(nlm * sizeof(ShRec)) + B(nk * nlm * sizeof(double2)) + B(ns * nlm * 2 * sizeof(zd));
+            b += B(nlm * sizeof(ShRec)) + B(nk * nlm * sizeof(double2)) + B(ns * nlm * 4 * sizeof(zd));
         }
     }
     if (p.scalar && p.lut_us && ns > 0) {

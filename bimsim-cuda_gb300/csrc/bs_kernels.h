@@ -100,7 +100,8 @@ void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, in
 
 // Direct scattered field through the addition theorem of spherical harmonics:
 // recurrence factors rec (L(L+1)/2), per-wave tables tab (nk x L(L+1)/2), per-sphere
-// coefficients coef (ns x L(L+1)/2 x 2 complex), then the per-pixel sum.
+// coefficients coef (ns x {outside, inside} x L(L+1)/2 x 2 complex, with the Mie
+// coefficients B, A), then the per-pixel sum.
 struct ShRec {
     double a, b, beta, kappa, zero;
 };
@@ -108,10 +109,9 @@ struct ShFrame {
     double e1[3], e2[3], e3[3];  // the harmonics' axes: e3 the slice's normal
 };
 void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* waves, ShRec* rec, double2* tab,
-                      zd* coef, cudaStream_t st);
+                      const zd* A, const zd* B, zd* coef, cudaStream_t st);
 template <class T>
-void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const zd* A, const zd* B, const ShRec* rec,
-                  const zd* coef, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st);
+void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const ShRec* rec, const zd* coef, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st);
 template <class T>
 void launch_sum_only(const Scene& sc, const Sphere* sph, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st);
 // U and Uf (src: U then Uf, R x R each) rotated about the slice centre into dst;

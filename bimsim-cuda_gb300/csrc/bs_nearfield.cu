@@ -618,12 +618,14 @@ __device__ __forceinline__ bool sh_in_plane(const Scene& sc, const ShFrame& fr, 
     return fabs(h) <= 4e-16 * (fabs(r[0]) + fabs(r[1]) + fabs(r[2]));
 }
 
-// Per sphere s and table index: coef[s][index] = (C, S) = scale sum_w pw_{s,w} tab[w][index], with the phase pw
-// of phase_kernel in double precision and the scale kappa, or S_l^m(0) for a sphere centred in the plane.
+// Per sphere s and table index: coef[s][0][index] = (C, S) = B_l scale sum_w pw_{s,w} tab[w][index], with the phase
+// pw of phase_kernel in double precision and the scale kappa, or S_l^m(0) for a sphere centred in the plane;
+// coef[s][1] with A_l for the pixels inside the sphere.
 constexpr int SH_WAVES = 128;
 __global__ void sh_coef_kernel(Scene sc, ShFrame fr, const Sphere* __restrict__ sph, int L,
                                const double* __restrict__ waves, const ShRec* __restrict__ rec,
-                               const double2* __restrict__ tab, zd* __restrict__ coef) {
+                               const double2* __restrict__ tab, const zd* __restrict__ A, const zd* __restrict__ B,
+                               zd* __restrict__ coef) {
     __shared__ zd s_pw[SH_WAVES];
     const int s = blockIdx.y, nlm = L * (L + 1) / 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -650,19 +652,31 @@ __global__ void sh_coef_kernel(Scene sc, ShFrame fr, const Sphere* __restrict__ 
     if (i < nlm) {
         double h;
         const double scale = sh_in_plane(sc, fr, sph[s], h) ? rec[i].zero : rec[i].kappa;
-        coef[((size_t)s * nlm + i) * 2] = ac * scale;
-        coef[((size_t)s * nlm + i) * 2 + 1] = as * scale;
+        int m = 0, k = i;  // i = index(m, l)
+        while (k >= L - m) k -= L - m++;
+        const int l = m + k;
+        const bool have = l <= sph[s].Nl;
+        const zd b = have ? B[sph[s].coef_off + l] : mk(0.0, 0.0), a = have ? A[sph[s].coef_off + l] : b;
+        zd* o = coef + (size_t)4 * s * nlm + 2 * i;
+        o[0] = (ac * scale) * b;
+        o[1] = (as * scale) * b;
+        o[2 * nlm] = (ac * scale) * a;
+        o[2 * nlm + 1] = (as * scale) * a;
     }
 }
 
-// The radial factors of one (pixel, sphere) pair, order after order:
-//   outside (d > a):  c_l = B_l (j_l + i y_l)(k d)   with the reference clamps
-//   inside  (d <= a): c_l = A_l j_l(k n d)           (c_0 = A_0 only when Re(k n d) < 1e-6)
-// (--recursive; nfScalarUs.cu:17-95, 201-245, 333-491).  They depend on (pixel, sphere) only; the
-// reference re-runs them for every wave (nfScalarUs.cu:69-93).  One reciprocal serves all orders.
+// The radial functions of one (pixel, sphere) pair, order after order:
+//   outside (d > a):  j_l + i y_l (k d)   with the reference clamps
+//   inside  (d <= a): j_l(k n d)          (1 for l = 0 and else 0 when Re(k n d) < 1e-6)
+// (--recursive; nfScalarUs.cu:17-95, 201-245, 333-491); their factors B_l and A_l are in the coefficients.
+// They depend on (pixel, sphere) only; the reference re-runs them for every wave (nfScalarUs.cu:69-93).
+// One reciprocal serves all orders, and outside the clamps compare high words, off the FP64 pipe: ten
+// FP64 instructions per order with the sum over l, where twenty-one took 4.72 ms of a 1280^2 slice with one sphere
+// (3.63 ms now).
 struct ShRadial {
     bool inside, centre;
-    double x, inv;
+    int xi;  // outside: l > x when l > xi
+    double x, inv, odd;
     zd z, zinv;
     zd p0, p1;  // outside: (j, y) of the last two orders; inside: j
 
@@ -679,38 +693,45 @@ struct ShRadial {
             p1 = j0 / z - zcos(z) / z;
         } else {
             x = sc.kmag * d;
+            xi = (int)floor(x);
             inv = 1.0 / x;
+            odd = 1.0;
             double sn, cs;
             sincos(x, &sn, &cs);
-            const double j0 = sn / x, y0 = -cs / x;
-            p0 = mk(j0, y0);
-            p1 = mk(j0 / x - cs / x, y0 / x - sn / x);
+            const double s1 = quot(sn, x, inv), c1 = quot(cs, x, inv);
+            p0 = mk(s1, -c1);
+            p1 = mk(quot(s1, x, inv) - c1, quot(-c1, x, inv) - s1);
         }
     }
-    // c_l for l = 0, 1, 2, ... in turn
-    __device__ __forceinline__ zd next(int l, const zd* __restrict__ A, const zd* __restrict__ B) {
+    // The function of order l = 0, 1, 2, ... in turn
+    __device__ __forceinline__ zd next(int l) {
         if (inside) {
-            if (centre) return l == 0 ? A[0] : mk(0.0, 0.0);
-            if (l < 2) return A[l] * (l == 0 ? p0 : p1);
+            if (centre) return mk(l == 0 ? 1.0 : 0.0, 0.0);
+            if (l < 2) return l == 0 ? p0 : p1;
             const zd w = (2.0 * l - 1.0) * zinv;
             zd b = mk(fma(w.re, p1.re, fma(-w.im, p1.im, -p0.re)), fma(w.re, p1.im, fma(w.im, p1.re, -p0.im)));
             if (l > z.re && (b.re < CONV_MIN || b.re > CONV_MAX)) b = mk(0.0, 0.0);
             p0 = p1;
             p1 = b;
-            return A[l] * b;
+            return b;
         }
-        if (l >= 2) {
-            const double w = quot(2.0 * l - 1.0, x, inv);
-            double j = fma(w, p1.re, -p0.re), y = fma(w, p1.im, -p0.im);
-            if (l > x && (j < CONV_MIN || j > CONV_MAX)) j = 0.0;
-            if (y < Y_FLOOR || (l > x && y > 0)) {
-                y = 0;
-                p1.im = 0;
-            }
-            p0 = p1;
-            p1 = mk(j, y);
+        if (l < 2) return l == 0 ? p0 : p1;
+        odd += 2.0;
+        const double w = quot(odd, x, inv);
+        double j = fma(w, p1.re, -p0.re), y = fma(w, p1.im, -p0.im);
+        // high words of CONV_MIN, CONV_MAX and Y_FLOOR decide, but where they are equal
+        constexpr int LO = 0x3f8db22d, HI = 0x3fd99999;
+        constexpr unsigned FLOOR = 0xc6c8a6e3u;
+        const int hj = __double2hiint(j), hy = __double2hiint(y);
+        const bool beyond = l > xi;
+        if (beyond && (hj <= LO || hj >= HI) && (hj < LO || hj > HI || j < CONV_MIN || j > CONV_MAX)) j = 0.0;
+        if ((beyond && hy > 0) || ((unsigned)hy >= FLOOR && ((unsigned)hy > FLOOR || y < Y_FLOOR))) {
+            y = 0;
+            p1.im = 0;
         }
-        return B[l] * (l == 0 ? p0 : p1);
+        p0 = p1;
+        p1 = mk(j, y);
+        return p1;
     }
 };
 
@@ -718,7 +739,6 @@ struct ShRadial {
 constexpr int SH_BLOCK = 64;
 template <class T>
 __global__ void __launch_bounds__(SH_BLOCK) us_sh_kernel(Scene sc, ShFrame fr, const Sphere* __restrict__ sph, int L,
-                                                         const zd* __restrict__ A, const zd* __restrict__ B,
                                                          const ShRec* __restrict__ rec, const zd* __restrict__ coef,
                                                          const cpx<T>* __restrict__ Uf, cpx<T>* __restrict__ U) {
     extern __shared__ unsigned char smem_raw[];
@@ -739,12 +759,15 @@ __global__ void __launch_bounds__(SH_BLOCK) us_sh_kernel(Scene sc, ShFrame fr, c
         const int Ls = S.Nl + 1;
         const bool in_plane = sh_in_plane(sc, fr, S, h);
         const double r1 = dot3(r, fr.e1), r2 = dot3(r, fr.e2), rho = sqrt(r1 * r1 + r2 * r2);
-        const double cf = rho > 0 ? r1 / rho : 1.0, sf = rho > 0 ? r2 / rho : 0.0;
-        const zd* cs_ = coef + (size_t)s * nlm * 2;
+        const double irho = 1.0 / rho;
+        const double cf = rho > 0 ? quot(r1, rho, irho) : 1.0, sf = rho > 0 ? quot(r2, rho, irho) : 0.0;
         ShRadial rad;
         rad.start(sc, S, d);
-        const zd *Al = A + S.coef_off, *Bl = B + S.coef_off;
+        const zd* cs_ = coef + ((size_t)2 * s + (rad.inside ? 1 : 0)) * nlm * 2;
         zd acc = mk(0.0, 0.0);
+        auto add = [&](zd f, zd q) {
+            acc = mk(fma(f.re, q.re, fma(-f.im, q.im, acc.re)), fma(f.re, q.im, fma(f.im, q.re, acc.im)));
+        };
         if (in_plane) {
             double cm = 1, sm = 0;
             for (int m = 0; m < Ls; m++) {  // cos(m f), sin(m f)
@@ -761,7 +784,7 @@ __global__ void __launch_bounds__(SH_BLOCK) us_sh_kernel(Scene sc, ShFrame fr, c
                     const zd C = cs_[2 * k], Sn = cs_[2 * k + 1], e = col[m * SH_BLOCK];
                     q = mk(fma(e.re, C.re, fma(e.im, Sn.re, q.re)), fma(e.re, C.im, fma(e.im, Sn.im, q.im)));
                 }
-                acc = acc + rad.next(l, Al, Bl) * q;
+                add(rad.next(l), q);
             }
         } else {
             const double x = d != 0 ? h / d : 0.0, st = d != 0 ? rho / d : 0.0;
@@ -791,7 +814,7 @@ __global__ void __launch_bounds__(SH_BLOCK) us_sh_kernel(Scene sc, ShFrame fr, c
                     q = mk(fma(wc, C.re, fma(ws, Sn.re, q.re)), fma(wc, C.im, fma(ws, Sn.im, q.im)));
                 }
             }
-            for (int l = 0; l < Ls; l++) acc = acc + rad.next(l, Al, Bl) * col[l * SH_BLOCK];
+            for (int l = 0; l < Ls; l++) add(rad.next(l), col[l * SH_BLOCK]);
         }
         // Kahan over spheres
         const zd y = acc - cmp;
@@ -914,23 +937,22 @@ static ShFrame sh_frame(const Scene& sc) {
 }
 
 void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* waves, ShRec* rec, double2* tab,
-                      zd* coef, cudaStream_t st) {
+                      const zd* A, const zd* B, zd* coef, cudaStream_t st) {
     const ShFrame fr = sh_frame(sc);
     sh_recur_kernel<<<blocks_for(L, 32), 32, 0, st>>>(L, rec);
     sh_wave_kernel<<<blocks_for(sc.nk, 32), 32, 0, st>>>(sc.nk, L, fr, waves, rec, tab);
     const int nlm = L * (L + 1) / 2;
     dim3 grid(blocks_for(nlm, 128), sc.ns);
-    sh_coef_kernel<<<grid, 128, 0, st>>>(sc, fr, sph, L, waves, rec, tab, coef);
+    sh_coef_kernel<<<grid, 128, 0, st>>>(sc, fr, sph, L, waves, rec, tab, A, B, coef);
 }
 
 template <class T>
-void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const zd* A, const zd* B, const ShRec* rec,
-                  const zd* coef, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st) {
+void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const ShRec* rec, const zd* coef, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st) {
     const size_t smem = (size_t)L * SH_BLOCK * sizeof(zd);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(us_sh_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const long long n = (long long)sc.R * sc.R;
-    us_sh_kernel<T><<<blocks_for(n, SH_BLOCK), SH_BLOCK, smem, st>>>(sc, sh_frame(sc), sph, L, A, B, rec, coef, Uf, U);
+    us_sh_kernel<T><<<blocks_for(n, SH_BLOCK), SH_BLOCK, smem, st>>>(sc, sh_frame(sc), sph, L, rec, coef, Uf, U);
 }
 
 template <class T>
@@ -1011,7 +1033,7 @@ void preload_nearfield_kernels() {
     template void launch_uf<T>(const Scene&, const double*, const UfOrder*, cpx<T>*, cudaStream_t);             \
     template void launch_lut_build<T>(const zd*, int, int, const double*, int, int, Patch<T>*, cudaStream_t);   \
     template void launch_phase<T>(const Scene&, const Sphere*, const double*, cpx<T>*, float4*, cudaStream_t);  \
-    template void launch_us_sh<T>(const Scene&, const Sphere*, int, const zd*, const zd*, const ShRec*,         \
+    template void launch_us_sh<T>(const Scene&, const Sphere*, int, const ShRec*,         \
                                   const zd*, const cpx<T>*, cpx<T>*, cudaStream_t);                           \
     template void launch_sum_only<T>(const Scene&, const Sphere*, const cpx<T>*, cpx<T>*, cudaStream_t);
 BS_INST(float)
