@@ -120,7 +120,7 @@ struct bs_ctx {
     int prec = -1;
     bool have = false;
 
-    DevBuf d_sph, d_waves, d_kw4, d_ph, d_A, d_B, d_tab, d_tabscr, d_legP, d_lut, d_uft, d_uftscr;
+    DevBuf d_sph, d_waves, d_kw4, d_ph, d_A, d_B, d_tab, d_legP, d_lut, d_uft, d_uftscr;
     DevBuf d_cnt;           // staged / total counters of the mixed LUT kernel
     DevBuf d_far;           // far fields Ud, Ufd on request (bs_get_far_field)
     DevBuf d_starts;        // row / coefficient offsets of a coefficient batch
@@ -160,7 +160,7 @@ struct bs_ctx {
 // Every linear device buffer of a context.
 static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
     return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_tab,
-            &c->d_tabscr, &c->d_bias, &c->d_acos, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
+            &c->d_bias, &c->d_acos, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
             &c->d_sv, &c->d_mask, &c->d_wx, &c->d_wy, &c->d_wix, &c->d_wiy, &c->d_f1, &c->d_f2,
             &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_far,
             &c->d_starts, &c->d_lbjobs, &c->d_lbjobs2, &c->d_kcmp, &c->d_part, &c->d_fsave, &c->d_dacc, &c->d_line, &c->d_ringcs, &c->d_bp, &c->d_shrec, &c->d_shtab, &c->d_shcoef, &c->d_gscr, &c->d_ufw};
@@ -899,7 +899,7 @@ static bs_status run_nearfield(bs_ctx* c) {
             // the addition theorem turns the per-wave Legendre sums into per-sphere coefficients
             const int L = c->Lmax, nlm = L * (L + 1) / 2;
             CK(c->d_shrec.ensure((size_t)nlm * sizeof(ShRec)));
-            CK(c->d_shtab.ensure((size_t)nk * nlm * sizeof(double2)));
+            CK(c->d_shtab.ensure((size_t)nk * (nlm + ns) * sizeof(double2)));
             CK(c->d_shcoef.ensure((size_t)ns * nlm * 4 * sizeof(zd)));
             launch_sh_tables(sc, c->d_sph.as<Sphere>(), L, c->d_waves.as<double>(), c->d_shrec.as<ShRec>(),
                              c->d_shtab.as<double2>(), c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_shcoef.as<zd>(), c->st);
@@ -919,7 +919,6 @@ static bs_status run_nearfield(bs_ctx* c) {
                 maxstarts = std::max(maxstarts, (long long)b.starts.size());
             }
             CK(c->d_tab.ensure((size_t)maxcoef * sizeof(zd)));
-            CK(c->d_tabscr.ensure((size_t)maxcoef * 2 * sizeof(double)));
             CK(c->d_starts.ensure((size_t)maxstarts * sizeof(long long)));
             if (!fp64) CK(c->d_bias.ensure((size_t)maxrow * sizeof(float)));
             if (fp64 && c->acos_theta != thetaR) {
@@ -981,8 +980,8 @@ static bs_status run_nearfield(bs_ctx* c) {
                 CK(cudaMemcpyAsync(c->d_starts.p, b.starts.data(), b.starts.size() * sizeof(long long),
                                    cudaMemcpyHostToDevice, c->st));
                 launch_coef_rows_batch(c->d_sph.as<Sphere>(), b.b0, b.b1 - b.b0, c->d_starts.as<long long>(), b.rows,
-                                       sc.kmag, c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_tab.as<zd>(),
-                                       c->d_tabscr.as<double>(), fp64 ? nullptr : c->d_bias.as<float>(), c->st);
+                                       c->Lmax, sc.kmag, c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_tab.as<zd>(),
+                                       fp64 ? nullptr : c->d_bias.as<float>(), c->st);
                 LAUNCHED(c);
                 // mixed path: the tables of every sphere of the batch in two launches (the
                 // dR-row Usp tables, then the shorter Uip tables)
@@ -1085,7 +1084,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         if (p.lut_us) b += B(ns * nk * cT) + B(nk * sizeof(float4));  // phases, float directions
         if (!p.lut_us) {  // direct method: harmonic recurrences, per-wave and per-sphere tables
             const size_t nlm = (size_t)c->Lmax * (c->Lmax + 1) / 2;
-            b += B(nlm * sizeof(ShRec)) + B(nk * nlm * sizeof(double2)) + B(ns * nlm * 4 * sizeof(zd));
+            b += B(nlm * sizeof(ShRec)) + B(nk * (nlm + ns) * sizeof(double2)) + B(ns * nlm * 4 * sizeof(zd));
         }
     }
     if (p.scalar && p.lut_us && ns > 0) {
@@ -1101,7 +1100,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
             maxrow = std::max(maxrow, cb.rows);
             maxstarts = std::max(maxstarts, (long long)cb.starts.size());
         }
-        b += B(pool) + B((size_t)maxcoef * sizeof(zd)) + B((size_t)maxcoef * 2 * sizeof(double)) +
+        b += B(pool) + B((size_t)maxcoef * sizeof(zd)) +
              B((size_t)maxstarts * sizeof(long long));
         b += B(thetaR * (size_t)c->Lmax * sizeof(double));    // Legendre table
         if (fp64) b += B((ACOS_NODES + 1) * sizeof(AcosNode));

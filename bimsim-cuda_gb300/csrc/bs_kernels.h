@@ -49,9 +49,8 @@ void launch_mie(const Sphere* sph, int ns, double k, zd* A, zd* B, cudaStream_t 
 struct SplitCoef {
     float hr, hi, lr, li;  // a complex coefficient: nearest floats and the rests; the size of a zd
 };
-void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows,
-                            double k, const zd* A, const zd* B, zd* tab, double* scratch, float* bias,
-                            cudaStream_t st);
+void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows, int Lmax,
+                            double k, const zd* A, const zd* B, zd* tab, float* bias, cudaStream_t st);
 // Legendre values of the mixed path: P[l * stride + t] = {nearest float, rest}
 void launch_legendre_split(int thetaR, int Lmax, int stride, float2* P, cudaStream_t st);
 void launch_legendre_table(int thetaR, int Lmax, double* P, cudaStream_t st);
@@ -99,7 +98,8 @@ void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, in
                             const float* bias, const float2* P, int Pstride, float2* lin, cudaStream_t st);
 
 // Direct scattered field through the addition theorem of spherical harmonics:
-// recurrence factors rec (L(L+1)/2), per-wave tables tab (nk x L(L+1)/2), per-sphere
+// recurrence factors rec (L(L+1)/2), per-wave tables tab (nk x L(L+1)/2, then the ns x nk
+// phases), per-sphere
 // coefficients coef (ns x {outside, inside} x L(L+1)/2 x 2 complex, with the Mie
 // coefficients B, A), then the per-pixel sum.
 struct ShRec {

@@ -114,10 +114,19 @@ __device__ __forceinline__ void sbessely_step(int n, double x, double& b0, doubl
 // Its Zhang & Jin routines stop at the order where J falls below 1e-200 (the
 // MSTA1 estimate) and leave higher entries unset; those entries are zero here.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int miller_start(int N, double ax) {
-    double m = fmax((double)N, ax);
-    return (int)(m + 16.0 + sqrt(60.0 * (m + 1.0)));
+// Start order of Miller's recurrence for the orders up to N of an argument of modulus ax and imaginary part im.
+// What the start leaves in order l is of relative size exp(-2 eta), eta = M acosh(M / m) - sqrt(M^2 - m^2) from
+// m = max(N, ax) on (Debye's expansion), below 2^-60 for M = m + 6 + 8 m^(1/3): 57 steps where m + 16 +
+// sqrt(60 (m + 1)) took 80 at m = 25.  Far from the real axis, where j_0 is large beside the start value, the longer
+// run keeps the scale in range.
+__device__ __forceinline__ int miller_start(int N, double ax, double im = 0.0) {
+    const double m = fmax((double)N, ax);
+    if (fabs(im) > 20.0) return (int)(m + 16.0 + sqrt(60.0 * (m + 1.0)));
+    return (int)m + 7 + (int)(8.f * cbrtf((float)m));
 }
+
+// |v| above 2^830 (7e249), from the high word: a comparison off the FP64 pipe
+__device__ __forceinline__ bool beyond_2_830(double v) { return (__double2hiint(v) & 0x7fffffff) >= 0x73d00000; }
 
 __device__ __forceinline__ double digits_at(int n, double x) {
     return 0.5 * log10(6.28 * n) - n * log10(1.36 * x / n);
@@ -199,7 +208,7 @@ __device__ inline void sph_real(int N, double x, double* j, double* y, int st) {
             fp = fc;
             fc = fm;
             if (l - 1 <= Nv) j[(l - 1) * st] = fm;
-            if (fabs(fc) > 1e250) {
+            if (beyond_2_830(fc)) {
                 for (int q = l - 1; q <= Nv; q++) j[q * st] *= 1e-250;
                 fc *= 1e-250;
                 fp *= 1e-250;
@@ -226,35 +235,6 @@ __device__ inline void sph_real(int N, double x, double* j, double* y, int st) {
             y[l * st] *= cs;
         }
     }
-}
-
-// j[l], l = 0..N, of a complex argument.
-__device__ inline void sph_complex(int N, zd z, zd* j) {
-    const double cs = sqrt(PI_BES / TRUE_PI);
-    double az = zabs(z);
-    int Nv = N;
-    if (N >= 2 && N > (int)(0.25 * az)) Nv = orders_kept(N, az);
-    const zd inv = mk(1.0, 0.0) / z;
-    zd s = zsin(z), c = zcos(z);
-    zd j0 = s / z, j1 = s / (z * z) - c / z;
-    int M = miller_start(N, az);
-    zd fp = mk(0.0, 0.0), fc = mk(1e-300, 0.0);
-    if (M <= N) j[M] = fc;
-    for (int l = M; l >= 1; l--) {
-        const zd w = (double)(2 * l + 1) * inv;
-        const zd fm = mk(fma(w.re, fc.re, fma(-w.im, fc.im, -fp.re)), fma(w.re, fc.im, fma(w.im, fc.re, -fp.im)));
-        fp = fc;
-        fc = fm;
-        if (l - 1 <= N) j[l - 1] = fm;
-        if (fmax(fabs(fc.re), fabs(fc.im)) > 1e250) {
-            for (int q = l - 1; q <= N; q++) j[q] = j[q] * 1e-250;
-            fc = fc * 1e-250;
-            fp = fp * 1e-250;
-        }
-    }
-    zd sc = (zabs(j0) >= zabs(j1)) ? j0 / j[0] : j1 / j[1 <= N ? 1 : 0];
-    for (int l = 0; l <= N; l++) j[l] = j[l] * sc;
-    for (int l = 0; l <= N; l++) j[l] = l > Nv ? mk(0.0, 0.0) : j[l] * cs;
 }
 
 }  // namespace bs

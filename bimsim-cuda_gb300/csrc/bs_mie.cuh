@@ -12,7 +12,10 @@ namespace bs {
 // for 200.  Here the step factors (2l + 1) / z are divided out beforehand by all threads, each chain
 // runs on a warp of its own at one or two fused multiply-adds per step, the trigonometric start
 // values and the order cut-offs on two more warps, and everything per order (derivatives,
-// coefficients) in parallel.  All in shared memory.
+// coefficients) in parallel.  All in shared memory.  A warp's FP64 instruction takes 64 cycles of its
+// quarter of the SM's pipe whatever its lanes do, so a chain's time is its count of them: the parts of the
+// complex recurrence run on two lanes, and the rescaling tests look at high words (one sphere of 24
+// orders: 59 us with both parts on one lane and comparisons in FP64, 38 us now).
 constexpr int MIE_NT = 160;
 constexpr int MIE_N = MAX_ORDER + 1;  // orders 0 .. MAX_ORDER
 constexpr int MIE_W = 768;            // step factors kept; beyond (large |n| k a) they are divided per step
@@ -38,7 +41,7 @@ __device__ inline void mie_block(MieShared& sm, int N, double a, zd n, double k,
     const double ka = k * a, cs = sqrt(PI_BES / TRUE_PI);
     const zd kna = (n * k) * a;
     const double az = fabs(ka), anz = zabs(kna);
-    const int M1 = miller_start(N, az), M2 = miller_start(N, anz);
+    const int M1 = miller_start(N, az), M2 = miller_start(N, anz, kna.im);
     for (int l = tid; l < min(max(M1, M2) + 1, MIE_W); l += MIE_NT) {
         sm.w1[l] = (2.0 * l + 1.0) / ka;
         sm.w2[l] = mk(2.0 * l + 1.0, 0.0) / kna;
@@ -56,29 +59,31 @@ __device__ inline void mie_block(MieShared& sm, int N, double a, zd n, double k,
                 sm.j[l - 1] = fm;
                 sm.sj[l - 1] = (short)s;
             }
-            if (fabs(fc) > 1e250) {
+            if (beyond_2_830(fc)) {
                 fc *= 1e-250;
                 fp *= 1e-250;
                 s++;
             }
         }
         sm.tj = s;
-    } else if (tid == 32) {  // j of k n a
-        zd fp = mk(0.0, 0.0), fc = mk(1e-300, 0.0);
+    } else if (tid == 32 || tid == 33) {  // j of k n a, one part on each lane
+        const int im = tid & 1;
+        double fp = 0.0, fc = im ? 0.0 : 1e-300;
         int s = 0;
 #pragma unroll 4
         for (int l = M2; l >= 1; l--) {
             const zd w = l < MIE_W ? sm.w2[l] : mk(2.0 * l + 1.0, 0.0) / kna;
-            const zd fm = mk(fma(w.re, fc.re, fma(-w.im, fc.im, -fp.re)), fma(w.re, fc.im, fma(w.im, fc.re, -fp.im)));
+            const double other = __shfl_xor_sync(3u, fc, 1);
+            const double fm = fma(w.re, fc, fma(im ? w.im : -w.im, other, -fp));
             fp = fc;
             fc = fm;
             if (l - 1 <= N) {
-                sm.jn[l - 1] = fm;
+                reinterpret_cast<double*>(&sm.jn[l - 1])[im] = fm;
                 sm.sn[l - 1] = (short)s;
             }
-            if (fmax(fabs(fc.re), fabs(fc.im)) > 1e250) {
-                fc = fc * 1e-250;
-                fp = fp * 1e-250;
+            if (__any_sync(3u, beyond_2_830(fc))) {
+                fc *= 1e-250;
+                fp *= 1e-250;
                 s++;
             }
         }

@@ -151,18 +151,29 @@ __global__ void __launch_bounds__(MIE_NT) mie_kernel(const Sphere* __restrict__ 
 // Per-row order coefficients of the spheres [s0, s0 + n) in one launch:
 //   rows [0, dR):  C_l(r) = B_l (j_l + i y_l)(k r),  r in [r0, dmax]  (sphere.cpp:154-203)
 //   rows [dR, dR+aR): D_l(r) = A_l j_l(k n r),       r in [0, a]      (sphere.cpp:99-152)
-// Thread g takes global row g; starts[i] / starts[n + 1 + i] are sphere i's
-// first global row and its first coefficient in tab (rows of Nl + 1
-// coefficients; starts[n], the total row count, bounds the grid).  The scratch
-// holds 2 (Nl + 1) doubles per row.  With `bias` (mixed path) every coefficient
-// is stored as SplitCoef instead, and bias[g] is a power of two of at least
-// twice the sum of the row's coefficients, see lut_build_mixed_kernel.
-__global__ void coef_rows_batch_kernel(const Sphere* __restrict__ sph, int s0, int n,
-                                       const long long* __restrict__ starts, double k, const zd* __restrict__ A,
-                                       const zd* __restrict__ B, zd* __restrict__ tab,
-                                       double* __restrict__ scratch, float* __restrict__ bias) {
-    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= starts[n]) return;
+// starts[i] / starts[n + 1 + i] are sphere i's first global row and its first coefficient in tab (rows of
+// Nl + 1 coefficients; starts[n] is the total row count).  With `bias` (mixed path) every coefficient is
+// stored as SplitCoef instead, and bias[g] is a power of two of at least twice the sum of the row's
+// coefficients, see lut_build_mixed_kernel.
+//
+// A block takes 32 rows, one per lane.  The time of a small slice is the count of FP64 instructions on one
+// warp's chain (64 cycles each), so the four warps share it: the first runs the j recurrence, the second
+// that of y (with j where that runs upwards too) or, inside, the trigonometric start values, and all four finish the orders l = warp (mod 4), in
+// shared memory, from where whole rows are written.  1600 rows of 25 orders: 77 us with a thread per row
+// and its values in global memory, 44 us now; 205 000 rows of 21 orders, bound by the pipe: 230 and 213 us.
+constexpr int CR_ROWS = 32, CR_PAD = CR_ROWS + 1;
+__global__ void __launch_bounds__(128) coef_rows_batch_kernel(const Sphere* __restrict__ sph, int s0, int n,
+                                                              const long long* __restrict__ starts, double k,
+                                                              const zd* __restrict__ A, const zd* __restrict__ B,
+                                                              zd* __restrict__ tab, float* __restrict__ bias) {
+    extern __shared__ zd cr_val[];  // [order][row]: (j, y) or j of a complex argument, then the coefficients
+    __shared__ zd s_j0[CR_ROWS], s_j1[CR_ROWS];
+    __shared__ int s_nv[CR_ROWS], s_len[CR_ROWS];
+    __shared__ long long s_out[CR_ROWS];
+    __shared__ float s_sum[4][CR_ROWS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long g = (long long)blockIdx.x * CR_ROWS + lane;
+    const bool live = g < starts[n];
     int lo = 0, hi = n - 1;  // last sphere whose first row is <= g
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -170,42 +181,144 @@ __global__ void coef_rows_batch_kernel(const Sphere* __restrict__ sph, int s0, i
         else hi = mid - 1;
     }
     const Sphere& S = sph[s0 + lo];
-    const int row = (int)(g - starts[lo]);
-    const int L = S.Nl + 1;
-    const long long c0 = starts[n + 1 + lo] + (long long)row * L;
-    zd* out = tab + c0;
-    double* sj = scratch + 2 * c0;
-    if (row < S.dR) {
-        double dr = (S.dmax - S.r0) / (S.dR - 1);
-        double r = row * dr + S.r0;
-        sph_real(S.Nl, k * r, sj, sj + L, 1);
-        for (int l = 0; l < L; l++) out[l] = B[S.coef_off + l] * mk(sj[l], sj[L + l]);
-    } else {
-        const int ia = row - S.dR;
-        if (ia == 0) {
-            for (int l = 0; l < L; l++) out[l] = (l == 0) ? A[S.coef_off] * mk(1.0, 0.0) : A[S.coef_off + l] * mk(0.0, 0.0);
-        } else {
-            double da = S.a / (S.aR - 1);
-            double r = ia * da;
-            zd knr = (mk(S.n_re, S.n_im) * k) * r;
-            sph_complex(S.Nl, knr, out);
-            for (int l = 0; l < L; l++) out[l] = A[S.coef_off + l] * out[l];
+    const int row = live ? (int)(g - starts[lo]) : 0, N = S.Nl, L = N + 1;
+    const bool outer = row < S.dR, centre = row == S.dR;  // centre: r = 0, the order 0 alone
+    zd* v = cr_val + lane;                                // order l at v[l * CR_PAD]
+    const double cs = sqrt(PI_BES / TRUE_PI);
+    double x = 1.0;
+    zd z = mk(1.0, 0.0);
+    if (outer) {
+        const double dr = (S.dmax - S.r0) / (S.dR - 1);
+        x = k * (row * dr + S.r0);
+    } else if (!centre) {
+        const double da = S.a / (S.aR - 1);
+        z = (mk(S.n_re, S.n_im) * k) * ((row - S.dR) * da);
+    }
+    int Nv = N;
+    if (outer && !(x < 1e-15) && N >= 2 && N > (int)(0.9 * x)) Nv = orders_kept(N, x);
+    const bool upward = Nv < x;  // j upwards too, with y and its factors
+    if (warp == 0) {
+        s_len[lane] = live ? L : 0;
+        s_out[lane] = starts[n + 1 + lo] + (long long)row * L;
+        if (outer && !(x < 1e-15)) {
+            if (!upward) {
+                const double inv = 1.0 / x;
+                double fp = 0.0, fc = 1e-300;
+                for (int l = miller_start(Nv, x); l >= 1; l--) {
+                    const double fm = fma(quot(2 * l + 1, x, inv), fc, -fp);
+                    fp = fc;
+                    fc = fm;
+                    if (l - 1 <= Nv) v[(l - 1) * CR_PAD].re = fm;
+                    if (beyond_2_830(fc)) {
+                        for (int q = l - 1; q <= Nv; q++) v[q * CR_PAD].re *= 1e-250;
+                        fc *= 1e-250;
+                        fp *= 1e-250;
+                    }
+                }
+            }
+        } else if (!outer && !centre) {
+            const double az = zabs(z);
+            if (N >= 2 && N > (int)(0.25 * az)) Nv = orders_kept(N, az);
+            s_nv[lane] = Nv;
+            const zd inv = mk(1.0, 0.0) / z;
+            zd fp = mk(0.0, 0.0), fc = mk(1e-300, 0.0);
+            for (int l = miller_start(N, az, z.im); l >= 1; l--) {
+                const zd w = (double)(2 * l + 1) * inv;
+                const zd fm =
+                    mk(fma(w.re, fc.re, fma(-w.im, fc.im, -fp.re)), fma(w.re, fc.im, fma(w.im, fc.re, -fp.im)));
+                fp = fc;
+                fc = fm;
+                if (l - 1 <= N) v[(l - 1) * CR_PAD] = fm;
+                if (beyond_2_830(fc.re) || beyond_2_830(fc.im)) {
+                    for (int q = l - 1; q <= N; q++) v[q * CR_PAD] = v[q * CR_PAD] * 1e-250;
+                    fc = fc * 1e-250;
+                    fp = fp * 1e-250;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (outer && !(x < 1e-15)) {
+            const double inv = 1.0 / x;
+            double sn, c;
+            sincos(x, &sn, &c);
+            const double ix = quot(c, x, inv), ja = quot(sn, x, inv), xx = x * x;
+            double pj = ja, j = sn / xx - ix, py = -ix, y = -c / xx - ja;
+            s_j0[lane] = mk(pj, 0.0);
+            s_j1[lane] = mk(j, 0.0);
+            v[0].im = py;
+            if (N >= 1) v[CR_PAD].im = y;
+            if (upward) {
+                v[0].re = pj;
+                if (N >= 1) v[CR_PAD].re = j;
+            }
+            for (int l = 2; l <= Nv; l++) {
+                const double w = quot(2 * l - 1, x, inv), t = fma(w, y, -py);
+                py = y;
+                y = t;
+                v[l * CR_PAD].im = t;
+                if (upward) {
+                    const double u = fma(w, j, -pj);
+                    pj = j;
+                    j = u;
+                    v[l * CR_PAD].re = u;
+                }
+            }
+        } else if (!outer && !centre) {
+            const zd sn = zsin(z), c = zcos(z);
+            s_j0[lane] = sn / z;
+            s_j1[lane] = sn / (z * z) - c / z;
         }
     }
-    if (bias) {
-        float sum = 0.f;
-        SplitCoef* sc = reinterpret_cast<SplitCoef*>(out);
-        for (int l = 0; l < L; l++) {
-            const zd c = out[l];
+    __syncthreads();
+    if (!outer && !centre) Nv = s_nv[lane];
+    const zd f0 = v[0], f1 = v[N >= 1 ? CR_PAD : 0];
+    __syncthreads();
+    float sum = 0.f;
+    zd sc = mk(1.0, 0.0);  // what the downward recurrence lacks
+    if (outer) {
+        if (!(x < 1e-15) && !upward) {
+            const double j0 = s_j0[lane].re, j1 = s_j1[lane].re;
+            sc.re = fabs(j0) >= fabs(j1) ? j0 / f0.re : j1 / f1.re;
+        }
+    } else if (!centre) {
+        const zd j0 = s_j0[lane], j1 = s_j1[lane];
+        sc = zabs(j0) >= zabs(j1) ? j0 / f0 : j1 / f1;
+    }
+    for (int l = warp; l < L; l += 4) {
+        zd c;
+        if (outer) {
+            zd jy = mk(0.0, 0.0);
+            if (x < 1e-15) {
+                const double big = sqrt(PI_BES / (x * 2.0));
+                jy = mk(0.0 * big, -1e308 * big);
+            } else if (l <= Nv) {
+                jy = mk(v[l * CR_PAD].re * sc.re * cs, v[l * CR_PAD].im * cs);
+            }
+            c = B[S.coef_off + l] * jy;
+        } else if (centre) {
+            c = A[S.coef_off + l] * mk(l == 0 ? 1.0 : 0.0, 0.0);
+        } else {
+            c = A[S.coef_off + l] * (l > Nv ? mk(0.0, 0.0) : (v[l * CR_PAD] * sc) * cs);
+        }
+        if (bias) {
             SplitCoef q;
             q.hr = (float)c.re;
             q.hi = (float)c.im;
             q.lr = (float)(c.re - (double)q.hr);
             q.li = (float)(c.im - (double)q.hi);
-            sc[l] = q;
             sum += fmaxf(fabsf(q.hr), fabsf(q.hi));
+            reinterpret_cast<SplitCoef&>(v[l * CR_PAD]) = q;
+        } else {
+            v[l * CR_PAD] = c;
         }
-        bias[g] = scalbnf(1.f, ilogbf(fmaxf(sum, 1e-30f)) + 2);
+    }
+    s_sum[warp][lane] = sum;
+    __syncthreads();
+    for (int r = warp; r < CR_ROWS; r += 4)
+        for (int l = lane; l < s_len[r]; l += 32) tab[s_out[r] + l] = cr_val[l * CR_PAD + r];
+    if (bias && warp == 0 && live) {
+        const float all = (s_sum[0][lane] + s_sum[1][lane]) + (s_sum[2][lane] + s_sum[3][lane]);
+        bias[g] = scalbnf(1.f, ilogbf(fmaxf(all, 1e-30f)) + 2);
     }
 }
 
@@ -535,6 +648,9 @@ __global__ void __launch_bounds__(256, 2) lut_build_mixed_kernel(const LutBuildJ
 // (u_l = x u_{l-1} - beta_l u_{l-2}, scale in the coefficients) 2, its cosine and sine part 2, the sum
 // Q_l 4 -- 8 where summing c_l S_l^m (...) took 13 -- and 4 on half of the terms where h = 0.
 // Tables are in (m, l) order: index(m, l) = m L - m (m - 1) / 2 + (l - m).
+// The tables' kernels are bound by the FP64 instructions on one warp's chain (64 cycles each), so they run a warp
+// per m, a thread per (wave, m) and a thread per index and sixteenth of the waves: 25 orders, 400 directions, one
+// sphere 6 + 9 + 23 us, where a thread per m, per wave and per index took 64 + 128 + 103 us.
 // ---------------------------------------------------------------------------
 __host__ __device__ __forceinline__ int sh_index(int L, int m, int l) { return m * L - m * (m - 1) / 2 + (l - m); }
 
@@ -542,72 +658,84 @@ __host__ __device__ __forceinline__ int sh_index(int L, int m, int l) { return m
 // b = sqrt((l-1)^2 - m^2) / sqrt(l^2 - m^2)), a = sqrt(2m + 1) for l = m + 1, and for l = m the diagonal
 // factor S_m^m = a sin(t) S_{m-1}^{m-1} (a = 1 for m = 1, sqrt((2m - 1) / (2m)) above); the monic form
 // S_l^m = kappa u_l, beta = b kappa_{l-2} / kappa_l; and zero = S_l^m at x = 0.
-__global__ void sh_recur_kernel(int L, ShRec* __restrict__ rec) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= L) return;
+// A warp per m, a lane per l: roots and quotients side by side, the products over l (kappa, zero) as scans.
+__global__ void __launch_bounds__(32) sh_recur_kernel(int L, ShRec* __restrict__ rec) {
+    const int m = blockIdx.x, lane = threadIdx.x;
+    const unsigned all = 0xffffffffu;
     double diag = 1;  // S_m^m at sin t = 1
-    for (int i = 2; i <= m; i++) diag *= sqrt((2.0 * i - 1.0) / (2.0 * i));
-    double a1 = 1, kap = 1, z2 = 0, z1 = diag;
-    for (int l = m; l < L; l++) {
-        ShRec r{0, 0, 0, 1, 0};
-        if (l == m) {
-            r.a = m < 2 ? 1.0 : sqrt((2.0 * m - 1.0) / (2.0 * m));
-            r.zero = diag;
-        } else if (l == m + 1) {
-            r.a = a1 = sqrt(2.0 * m + 1.0);
-            r.kappa = kap = a1;
-            z2 = diag;
-            z1 = 0;
-        } else {
-            const double den = sqrt((double)l * l - (double)m * m);
-            r.a = (2.0 * l - 1.0) / den;
-            r.b = sqrt((double)(l - 1) * (l - 1) - (double)m * m) / den;
-            r.beta = r.b / (r.a * a1);
-            r.kappa = kap = kap * r.a;
-            a1 = r.a;
-            r.zero = -r.b * z2;
-            z2 = z1;
-            z1 = r.zero;
+    for (int i = 2 + lane; i <= m; i += 32) diag *= sqrt((2.0 * i - 1.0) / (2.0 * i));
+    for (int d = 16; d >= 1; d >>= 1) diag *= __shfl_xor_sync(all, diag, d);
+    const double m2 = (double)m * m;
+    double kap0 = 1, z_even = diag, z_odd = 0;  // kappa of the order before the 32, and zero at the last even, odd l - m
+    double a_before = 1;
+    for (int l0 = m; l0 < L; l0 += 32) {
+        const int l = l0 + lane, q = l - m;
+        const double den = sqrt((double)l * l - m2);
+        const double a = q == 0 ? 1.0 : (2.0 * l - 1.0) / den;
+        const double b = q < 2 ? 0.0 : sqrt((double)(l - 1) * (l - 1) - m2) / den;
+        double a1 = __shfl_up_sync(all, a, 1);
+        if (lane == 0) a1 = a_before;
+        double kap = a, z = q < 2 ? 1.0 : -b;
+        for (int d = 1; d < 32; d <<= 1) {
+            const double k2 = __shfl_up_sync(all, kap, d), z2 = __shfl_up_sync(all, z, 2 * d);
+            if (lane >= d) kap *= k2;
+            if (lane >= 2 * d) z *= z2;
         }
-        rec[sh_index(L, m, l)] = r;
+        kap *= kap0;
+        z *= q & 1 ? z_odd : z_even;
+        if (l < L) {
+            ShRec r;
+            r.a = q == 0 ? (m < 2 ? 1.0 : sqrt((2.0 * m - 1.0) / (2.0 * m))) : a;
+            r.b = b;
+            r.beta = q < 2 ? 0.0 : b / (a * a1);
+            r.kappa = kap;
+            r.zero = z;
+            rec[sh_index(L, m, l)] = r;
+        }
+        kap0 = __shfl_sync(all, kap, 31);
+        a_before = __shfl_sync(all, a, 31);
+        z_even = __shfl_sync(all, z, 30);
+        z_odd = 0;
     }
 }
 
 __device__ __forceinline__ double dot3(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 
-// Per wave: tab[w][index(m, l)] = S_l^m(k_n) (cos, sin)(m f_k), k_n the component along the normal.
-__global__ void sh_wave_kernel(int nk, int L, ShFrame fr, const double* __restrict__ waves,
-                               const ShRec* __restrict__ rec, double2* __restrict__ tab) {
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= nk) return;
+// Per wave: tab[w][index(m, l)] = S_l^m(k_n) (cos, sin)(m f_k), k_n the component along the normal: a thread per
+// (wave, m), from S_m^m (cos, sin)(m f) = S_m^m(0) (k_x + i k_y)^m.  The ns last values of m: the phases
+// pw[s][w] as phase_kernel's, in double precision.
+__global__ void __launch_bounds__(32) sh_wave_kernel(Scene sc, ShFrame fr, const Sphere* __restrict__ sph, int L,
+                                                     const double* __restrict__ waves, const ShRec* __restrict__ rec,
+                                                     double2* __restrict__ tab, zd* __restrict__ pw) {
+    const int m = blockIdx.x % (L + sc.ns), w = blockIdx.x / (L + sc.ns) * 32 + threadIdx.x;
+    if (w >= sc.nk) return;
     const double* k = waves + 3 * w;
-    const double kx = dot3(k, fr.e1), ky = dot3(k, fr.e2), kz = dot3(k, fr.e3);
-    const double rho = sqrt(kx * kx + ky * ky);
-    const double cf = rho > 0 ? kx / rho : 1.0, sf = rho > 0 ? ky / rho : 0.0;
-    double2* out = tab + (size_t)w * (L * (L + 1) / 2);
-    double cm = 1, sm = 0, smm = 1;  // cos(m f), sin(m f), S_m^m
-    for (int m = 0; m < L; m++) {
-        if (m > 0) {
-            smm *= rec[sh_index(L, m, m)].a * rho;
-            const double c2 = cm * cf - sm * sf;
-            sm = sm * cf + cm * sf;
-            cm = c2;
-        }
-        double p2 = 0, p1 = smm;
-        for (int l = m; l < L; l++) {
-            double v;
-            if (l == m) v = smm;
-            else if (l == m + 1) v = rec[sh_index(L, m, l)].a * kz * smm;
-            else {
-                const ShRec r = rec[sh_index(L, m, l)];
-                v = r.a * kz * p1 - r.b * p2;
-            }
-            if (l > m) {
-                p2 = p1;
-                p1 = v;
-            }
-            out[sh_index(L, m, l)] = make_double2(v * cm, v * sm);
-        }
+    if (m >= L) {
+        const Sphere& S = sph[m - L];
+        const double arg =
+            sc.kmag * (k[0] * (S.p[0] - sc.focus[0]) + k[1] * (S.p[1] - sc.focus[1]) + k[2] * (S.p[2] - sc.focus[2]));
+        double sn, cs;
+        sincos(arg, &sn, &cs);
+        pw[(size_t)(m - L) * sc.nk + w] = mk(sc.wave_amp * cs, sc.wave_amp * sn);
+        return;
+    }
+    const double kz = dot3(k, fr.e3);
+    zd b = mk(dot3(k, fr.e1), dot3(k, fr.e2)), e = mk(1.0, 0.0);
+    for (int i = m; i; i >>= 1) {
+        if (i & 1) e = mk(e.re * b.re - e.im * b.im, e.re * b.im + e.im * b.re);
+        b = mk(b.re * b.re - b.im * b.im, 2.0 * b.re * b.im);
+    }
+    const ShRec* r = rec + sh_index(L, m, m);
+    e = e * r[0].zero;
+    double2* out = tab + (size_t)w * (L * (L + 1) / 2) + sh_index(L, m, m);
+    double p2 = 0, p1 = 1;
+    out[0] = make_double2(e.re, e.im);
+#pragma unroll 4
+    for (int q = 1; q < L - m; q++) {  // b is 0 for q = 1
+        const double v = fma(r[q].a * kz, p1, -r[q].b * p2);
+        p2 = p1;
+        p1 = v;
+        out[q] = make_double2(v * e.re, v * e.im);
     }
 }
 
@@ -618,51 +746,49 @@ __device__ __forceinline__ bool sh_in_plane(const Scene& sc, const ShFrame& fr, 
     return fabs(h) <= 4e-16 * (fabs(r[0]) + fabs(r[1]) + fabs(r[2]));
 }
 
-// Per sphere s and table index: coef[s][0][index] = (C, S) = B_l scale sum_w pw_{s,w} tab[w][index], with the phase
-// pw of phase_kernel in double precision and the scale kappa, or S_l^m(0) for a sphere centred in the plane;
-// coef[s][1] with A_l for the pixels inside the sphere.
-constexpr int SH_WAVES = 128;
-__global__ void sh_coef_kernel(Scene sc, ShFrame fr, const Sphere* __restrict__ sph, int L,
-                               const double* __restrict__ waves, const ShRec* __restrict__ rec,
-                               const double2* __restrict__ tab, const zd* __restrict__ A, const zd* __restrict__ B,
-                               zd* __restrict__ coef) {
-    __shared__ zd s_pw[SH_WAVES];
+// Per sphere s and table index: coef[s][0][index] = (C, S) = B_l scale sum_w pw[s][w] tab[w][index], with the scale
+// kappa, or S_l^m(0) for a sphere centred in the plane; coef[s][1] with A_l for the pixels inside the sphere.
+// A block takes 8 indices, thread t every 16th wave of index t mod 8.
+constexpr int SC_I = 8, SC_W = 16;
+__global__ void __launch_bounds__(SC_I* SC_W) sh_coef_kernel(Scene sc, ShFrame fr, const Sphere* __restrict__ sph, int L,
+                                                             const ShRec* __restrict__ rec,
+                                                             const double2* __restrict__ tab,
+                                                             const zd* __restrict__ pw, const zd* __restrict__ A,
+                                                             const zd* __restrict__ B, zd* __restrict__ coef) {
+    __shared__ zd s_c[SC_W][SC_I], s_s[SC_W][SC_I];
     const int s = blockIdx.y, nlm = L * (L + 1) / 2;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const double c0 = sph[s].p[0] - sc.focus[0], c1 = sph[s].p[1] - sc.focus[1], c2 = sph[s].p[2] - sc.focus[2];
+    const int ti = threadIdx.x % SC_I, tw = threadIdx.x / SC_I, i = blockIdx.x * SC_I + ti;
     zd ac = mk(0.0, 0.0), as = mk(0.0, 0.0);
-    for (int w0 = 0; w0 < sc.nk; w0 += SH_WAVES) {
-        const int nw = min(SH_WAVES, sc.nk - w0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nw; t += blockDim.x) {
-            const double* k = waves + 3 * (w0 + t);
-            const double arg = sc.kmag * (k[0] * c0 + k[1] * c1 + k[2] * c2);
-            double sn, cs;
-            sincos(arg, &sn, &cs);
-            s_pw[t] = mk(sc.wave_amp * cs, sc.wave_amp * sn);
-        }
-        __syncthreads();
-        if (i < nlm)
-            for (int t = 0; t < nw; t++) {
-                const double2 v = tab[(size_t)(w0 + t) * nlm + i];
-                ac = ac + s_pw[t] * v.x;
-                as = as + s_pw[t] * v.y;
-            }
-    }
     if (i < nlm) {
-        double h;
-        const double scale = sh_in_plane(sc, fr, sph[s], h) ? rec[i].zero : rec[i].kappa;
-        int m = 0, k = i;  // i = index(m, l)
-        while (k >= L - m) k -= L - m++;
-        const int l = m + k;
-        const bool have = l <= sph[s].Nl;
-        const zd b = have ? B[sph[s].coef_off + l] : mk(0.0, 0.0), a = have ? A[sph[s].coef_off + l] : b;
-        zd* o = coef + (size_t)4 * s * nlm + 2 * i;
-        o[0] = (ac * scale) * b;
-        o[1] = (as * scale) * b;
-        o[2 * nlm] = (ac * scale) * a;
-        o[2 * nlm + 1] = (as * scale) * a;
+        const zd* p = pw + (size_t)s * sc.nk;
+#pragma unroll 4
+        for (int w = tw; w < sc.nk; w += SC_W) {
+            const double2 v = tab[(size_t)w * nlm + i];
+            const zd f = p[w];
+            ac = mk(fma(f.re, v.x, ac.re), fma(f.im, v.x, ac.im));
+            as = mk(fma(f.re, v.y, as.re), fma(f.im, v.y, as.im));
+        }
     }
+    s_c[tw][ti] = ac;
+    s_s[tw][ti] = as;
+    __syncthreads();
+    if (tw != 0 || i >= nlm) return;
+    for (int q = 1; q < SC_W; q++) {
+        ac = ac + s_c[q][ti];
+        as = as + s_s[q][ti];
+    }
+    double h;
+    const double scale = sh_in_plane(sc, fr, sph[s], h) ? rec[i].zero : rec[i].kappa;
+    int m = 0, k = i;  // i = index(m, l)
+    while (k >= L - m) k -= L - m++;
+    const int l = m + k;
+    const bool have = l <= sph[s].Nl;
+    const zd b = have ? B[sph[s].coef_off + l] : mk(0.0, 0.0), a = have ? A[sph[s].coef_off + l] : b;
+    zd* o = coef + (size_t)4 * s * nlm + 2 * i;
+    o[0] = (ac * scale) * b;
+    o[1] = (as * scale) * b;
+    o[2 * nlm] = (ac * scale) * a;
+    o[2 * nlm + 1] = (as * scale) * a;
 }
 
 // The radial functions of one (pixel, sphere) pair, order after order:
@@ -863,11 +989,13 @@ void launch_mie(const Sphere* sph, int ns, double k, zd* A, zd* B, cudaStream_t 
     mie_kernel<<<ns, MIE_NT, 0, st>>>(sph, k, A, B);
 }
 
-void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows,
-                            double k, const zd* A, const zd* B, zd* tab, double* scratch, float* bias,
-                            cudaStream_t st) {
-    coef_rows_batch_kernel<<<(unsigned)((total_rows + 127) / 128), 128, 0, st>>>(sph, s0, n, starts, k, A, B, tab,
-                                                                               scratch, bias);
+void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows, int Lmax,
+                            double k, const zd* A, const zd* B, zd* tab, float* bias, cudaStream_t st) {
+    const size_t smem = (size_t)Lmax * CR_PAD * sizeof(zd);  // 68 KB at 128 orders
+    if (smem > 44 * 1024)
+        cudaFuncSetAttribute(coef_rows_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    coef_rows_batch_kernel<<<(unsigned)((total_rows + CR_ROWS - 1) / CR_ROWS), 128, smem, st>>>(sph, s0, n, starts, k,
+                                                                                              A, B, tab, bias);
 }
 
 void launch_legendre_split(int thetaR, int Lmax, int stride, float2* P, cudaStream_t st) {
@@ -939,11 +1067,11 @@ static ShFrame sh_frame(const Scene& sc) {
 void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* waves, ShRec* rec, double2* tab,
                       const zd* A, const zd* B, zd* coef, cudaStream_t st) {
     const ShFrame fr = sh_frame(sc);
-    sh_recur_kernel<<<blocks_for(L, 32), 32, 0, st>>>(L, rec);
-    sh_wave_kernel<<<blocks_for(sc.nk, 32), 32, 0, st>>>(sc.nk, L, fr, waves, rec, tab);
     const int nlm = L * (L + 1) / 2;
-    dim3 grid(blocks_for(nlm, 128), sc.ns);
-    sh_coef_kernel<<<grid, 128, 0, st>>>(sc, fr, sph, L, waves, rec, tab, A, B, coef);
+    zd* pw = reinterpret_cast<zd*>(tab + (size_t)sc.nk * nlm);
+    sh_recur_kernel<<<L, 32, 0, st>>>(L, rec);
+    sh_wave_kernel<<<blocks_for(sc.nk, 32) * (unsigned)(L + sc.ns), 32, 0, st>>>(sc, fr, sph, L, waves, rec, tab, pw);
+    sh_coef_kernel<<<dim3(blocks_for(nlm, SC_I), sc.ns), SC_I * SC_W, 0, st>>>(sc, fr, sph, L, rec, tab, pw, A, B, coef);
 }
 
 template <class T>
