@@ -111,6 +111,10 @@ struct bs_ctx {
     int device = 0;
     cudaStream_t st = nullptr;
     cudaEvent_t ev[6] = {};
+    // The incident field and the transforms' tables, which the scattered field does not need, run beside the
+    // Mie coefficients and lookup tables on a second stream (SideWork, made by the first run).
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, uf_ev[2] = {};
     size_t budget = 0;  // LUT bytes allowed; 0 = automatic
 
     // derived per simulate
@@ -204,6 +208,15 @@ static void preload_kernels(int device) {
     done.push_back(device);
 }
 
+static void free_streams(bs_ctx* c) {
+    for (cudaEvent_t e : c->ev)
+        if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : {c->uf_ev[0], c->uf_ev[1], c->fork, c->join})
+        if (e) cudaEventDestroy(e);
+    if (c->side) cudaStreamDestroy(c->side);
+    if (c->st) cudaStreamDestroy(c->st);
+}
+
 bs_status bs_create(const bs_params* params, bs_ctx** out) {
     if (!params || !out) return fail(BS_ERR_ARG, "bs_create: null argument");
     std::string why;
@@ -216,6 +229,7 @@ bs_status bs_create(const bs_params* params, bs_ctx** out) {
     for (int i = 0; i < 6 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
     for (DevBuf* b : ctx_bufs(c)) b->st = &c->st;
     if (e != cudaSuccess) {
+        free_streams(c);
         delete c;
         return fail(BS_ERR_CUDA, "bs_create: %s", cudaGetErrorString(e));
     }
@@ -228,9 +242,7 @@ bs_status bs_destroy(bs_ctx* c) {
     if (c->st) cudaStreamSynchronize(c->st);
     release_all(c);
     if (c->st) cudaStreamSynchronize(c->st);  // the stream-ordered frees
-    for (int i = 0; i < 6; i++)
-        if (c->ev[i]) cudaEventDestroy(c->ev[i]);
-    if (c->st) cudaStreamDestroy(c->st);
+    free_streams(c);
     delete c;
     return BS_OK;
 }
@@ -457,8 +469,9 @@ static size_t detector_scratch_elems(const FoldDft& fx, const FoldDft& fy, int N
     return std::max(fwd, std::max(cgemm_scratch_elems<T>(Nv, C, Nu, 2), cgemm_scratch_elems<T>(C, C, Nv, 2)));
 }
 
+// The detector's device buffers and small host tables (passbands, mask), before the streams part.
 template <class T>
-static bs_status run_detector(bs_ctx* c, bool accumulate) {
+static bs_status detector_buffers(bs_ctx* c) {
     const bs_params& p = c->prm;
     const int R = c->R;
     double du, dv;
@@ -469,10 +482,7 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
     const int Nu = (int)su.size(), Nv = (int)sv.size(), C = c->crop, res = c->res;
     c->det_Nv = (Nu == 0) ? 0 : Nv;
     CK(c->d_D.ensure(2 * (size_t)res * res * sizeof(T)));
-    if (Nu == 0 || Nv == 0) {
-        if (!accumulate) CK(cudaMemsetAsync(c->d_D.p, 0, 2 * (size_t)res * res * sizeof(T), c->st));
-        return BS_OK;
-    }
+    if (Nu == 0 || Nv == 0) return BS_OK;
     std::vector<float> mask((size_t)Nv * Nu);
     for (int j = 0; j < Nv; j++)
         for (int k = 0; k < Nu; k++) {
@@ -484,9 +494,8 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
     CK(c->d_su.ensure(Nu * sizeof(int)));
     CK(c->d_sv.ensure(Nv * sizeof(int)));
     CK(c->d_mask.ensure(mask.size() * sizeof(float)));
-    constexpr bool fp64 = sizeof(T) == 8;
     const FoldDft fx = fold_x(R, su, sv), fy = fold_y(R, su, sv);
-    if (fp64) {
+    if (sizeof(T) == 8) {
         CK(c->d_wx.ensure((size_t)(R / 2 + 1) * fx.ldt * ce));
     } else {
         CK(c->d_wx.ensure((size_t)R * Nu * ce));
@@ -498,37 +507,68 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
     CK(c->d_f2.ensure(2 * (size_t)Nv * Nu * ce));
     CK(c->d_g1.ensure(2 * (size_t)Nv * C * ce));
     CK(c->d_I.ensure(2 * (size_t)C * C * sizeof(T)));
+    // split-K scratch for the GEMMs with few output tiles
+    CK(c->d_gscr.ensure(std::max<size_t>(detector_scratch_elems<T>(fx, fy, Nu, Nv, C), 1) * ce));
     CK(cudaMemcpyAsync(c->d_su.p, su.data(), Nu * sizeof(int), cudaMemcpyHostToDevice, c->st));
     CK(cudaMemcpyAsync(c->d_sv.p, sv.data(), Nv * sizeof(int), cudaMemcpyHostToDevice, c->st));
     CK(cudaMemcpyAsync(c->d_mask.p, mask.data(), mask.size() * sizeof(float), cudaMemcpyHostToDevice, c->st));
+    return BS_OK;
+}
+
+// The transforms' tables, on the stream st.
+template <class T>
+static bs_status detector_tables(bs_ctx* c, cudaStream_t st) {
+    const int R = c->R, C = c->crop;
+    double du, dv;
+    std::vector<int> su, sv;
+    passbands(c, su, sv, du, dv);
+    const int Nu = (int)su.size(), Nv = (int)sv.size();
+    if (Nu == 0 || Nv == 0) return BS_OK;
+    const int *fu = c->d_su.as<int>(), *fv = c->d_sv.as<int>();
+    // forward x: Wx[x][k] = e^{-2 pi i x su_k / R}; forward y: Wy[j][y] = e^{-2 pi i y sv_j / R}
+    if constexpr (sizeof(T) == 8) {
+        launch_fold_table(R, fold_x(R, su, sv).ldt, c->d_wx.as<zd>(), st);
+        LAUNCHED(c);
+    } else {
+        launch_twiddle<T>(R, Nu, fu, 0, R, -1, Nu, 1, c->d_wx.as<cpx<T>>(), st);
+        LAUNCHED(c);
+        launch_twiddle<T>(R, Nv, fv, 0, R, -1, 1, R, c->d_wy.as<cpx<T>>(), st);
+        LAUNCHED(c);
+    }
+    // inverse on the crop only: Wix[k][x] = e^{+2 pi i (off+x) su_k / R}, Wiy[y][j] likewise
+    launch_twiddle<T>(C, Nu, fu, c->off, R, +1, 1, C, c->d_wix.as<cpx<T>>(), st);
+    LAUNCHED(c);
+    launch_twiddle<T>(C, Nv, fv, c->off, R, +1, Nv, 1, c->d_wiy.as<cpx<T>>(), st);
+    LAUNCHED(c);
+    return BS_OK;
+}
+
+// The detector images of the fields in d_fields, with the buffers and tables of the slice's near field.
+template <class T>
+static bs_status run_detector(bs_ctx* c, bool accumulate) {
+    const bs_params& p = c->prm;
+    const int R = c->R;
+    double du, dv;
+    std::vector<int> su, sv;
+    passbands(c, su, sv, du, dv);
+    const int Nu = (int)su.size(), Nv = (int)sv.size(), C = c->crop, res = c->res;
+    if (Nu == 0 || Nv == 0) {
+        if (!accumulate) CK(cudaMemsetAsync(c->d_D.p, 0, 2 * (size_t)res * res * sizeof(T), c->st));
+        return BS_OK;
+    }
+    constexpr bool fp64 = sizeof(T) == 8;
+    const FoldDft fx = fold_x(R, su, sv), fy = fold_y(R, su, sv);
     cpx<T>* wx = c->d_wx.as<cpx<T>>();
     cpx<T>* wy = c->d_wy.as<cpx<T>>();
     cpx<T>* wix = c->d_wix.as<cpx<T>>();
     cpx<T>* wiy = c->d_wiy.as<cpx<T>>();
-    // forward x: Wx[x][k] = e^{-2 pi i x su_k / R}; forward y: Wy[j][y] = e^{-2 pi i y sv_j / R}
-    if constexpr (fp64) {
-        launch_fold_table(R, fx.ldt, wx, c->st);
-        LAUNCHED(c);
-    } else {
-        launch_twiddle<T>(R, Nu, c->d_su.as<int>(), 0, R, -1, Nu, 1, wx, c->st);
-        LAUNCHED(c);
-        launch_twiddle<T>(R, Nv, c->d_sv.as<int>(), 0, R, -1, 1, R, wy, c->st);
-        LAUNCHED(c);
-    }
-    // inverse on the crop only: Wix[k][x] = e^{+2 pi i (off+x) su_k / R}, Wiy[y][j] likewise
-    launch_twiddle<T>(C, Nu, c->d_su.as<int>(), c->off, R, +1, 1, C, wix, c->st);
-    LAUNCHED(c);
-    launch_twiddle<T>(C, Nv, c->d_sv.as<int>(), c->off, R, +1, Nv, 1, wiy, c->st);
-    LAUNCHED(c);
     const cpx<T>* fields = c->d_fields.as<cpx<T>>();
     cpx<T>* f1 = c->d_f1.as<cpx<T>>();
     cpx<T>* f2 = c->d_f2.as<cpx<T>>();
     cpx<T>* g1 = c->d_g1.as<cpx<T>>();
     T* I = c->d_I.as<T>();
     long long RR = (long long)R * R;
-    // split-K scratch for the GEMMs with few output tiles
     const size_t scr = detector_scratch_elems<T>(fx, fy, Nu, Nv, C);
-    CK(c->d_gscr.ensure(std::max<size_t>(scr, 1) * ce));
     cpx<T>* gs = c->d_gscr.as<cpx<T>>();
     if constexpr (fp64) {  // f1 transposed: [Nu][R]
         launch_fold_dft(fx, 2, fields, wx, f1, nullptr, gs, c->st);
@@ -789,6 +829,33 @@ static double predict_staged_fraction(const bs_ctx* c, const std::vector<double>
 // ---------------------------------------------------------------------------
 // The near field
 // ---------------------------------------------------------------------------
+// Work on the context's second stream, from what was on the first at the fork on.  The first waits for it at
+// join(), or when a failed run leaves the scope.
+struct SideWork {
+    bs_ctx* c;
+    bool open = false;
+    cudaError_t fork() {
+        cudaError_t e = cudaSuccess;
+        if (!c->side) e = cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, c->stream_prio);
+        for (cudaEvent_t* v : {&c->uf_ev[0], &c->uf_ev[1]})
+            if (e == cudaSuccess && !*v) e = cudaEventCreate(v);
+        for (cudaEvent_t* v : {&c->fork, &c->join})
+            if (e == cudaSuccess && !*v) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventRecord(c->fork, c->st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->fork, 0);
+        open = e == cudaSuccess;
+        return e;
+    }
+    cudaError_t join() {
+        open = false;
+        cudaError_t e = cudaEventRecord(c->join, c->side);
+        return e == cudaSuccess ? cudaStreamWaitEvent(c->st, c->join, 0) : e;
+    }
+    ~SideWork() {
+        if (open) join();
+    }
+};
+
 template <class T>
 static bs_status run_nearfield(bs_ctx* c) {
     Scene& sc = c->sc;
@@ -812,17 +879,16 @@ static bs_status run_nearfield(bs_ctx* c) {
     CK(c->d_waves.ensure(w.size() * sizeof(double)));
     CK(cudaMemcpyAsync(c->d_waves.p, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
 
-    // ---- incident field ----
+    // ---- what the second stream needs ----
     cudaEventRecord(c->ev[0], c->st);
-    if (p.lut_uf && !p.plane_wave && p.scalar) {
+    const bool uf_table = p.lut_uf && !p.plane_wave && p.scalar;
+    if (uf_table) {
         CK(c->d_uft.ensure((size_t)sc.uf_dR * (sc.m + 1) * sizeof(double)));
         CK(c->d_uftscr.ensure((size_t)sc.uf_dR * (sc.m + 1) * sizeof(double)));
-        launch_uf_table(sc, c->d_uft.as<double>(), c->d_uftscr.as<double>(), c->st);
-        LAUNCHED(c);
     }
+    std::vector<UfOrder> ufw(sc.m + 1);
     {
         // condenser aperture factor of each order, the same for every pixel (nfScalarUf.cu:46-175)
-        std::vector<UfOrder> w(sc.m + 1);
         double kap = 1, kap2 = 1;  // P_l = kappa_l u_l, kappa_l = (2l - 1) / l kappa_{l-1}
         double a0 = 1, a1 = sc.cos_a, a2 = 1, b0 = 1, b1 = sc.cos_b, b2 = 1;
         auto step = [](int n, double x, double& q0, double& q1) {  // rts/math/legendre.h:17-25
@@ -837,21 +903,22 @@ static bs_status run_nearfield(bs_ctx* c) {
                 b2 = b0;
                 step(l + 1, sc.cos_b, b0, b1);
             }
-            w[l].beta = 0;
+            ufw[l].beta = 0;
             if (l > 0) {
                 const double k1 = kap;
                 kap *= (2.0 * l - 1.0) / l;
-                if (l > 1) w[l].beta = (l - 1.0) / l * kap2 / kap;
+                if (l > 1) ufw[l].beta = (l - 1.0) / l * kap2 / kap;
                 kap2 = k1;
             }
-            w[l].w = (l & 2 ? -1.0 : 1.0) * kap * (l == 0 ? a1 - b1 : a1 - a2 - b1 + b2) * (2.0 * PI_REF * sc.amp);
+            ufw[l].w = (l & 2 ? -1.0 : 1.0) * kap * (l == 0 ? a1 - b1 : a1 - a2 - b1 + b2) * (2.0 * PI_REF * sc.amp);
         }
-        CK(c->d_ufw.ensure(w.size() * sizeof(UfOrder)));
-        CK(cudaMemcpyAsync(c->d_ufw.p, w.data(), w.size() * sizeof(UfOrder), cudaMemcpyHostToDevice, c->st));
-        launch_uf<T>(sc, c->d_uft.as<double>(), c->d_ufw.as<UfOrder>(), Uf, c->st);
-        LAUNCHED(c);
-        CK(cudaStreamSynchronize(c->st));  // w is a host vector of this scope
+        CK(c->d_ufw.ensure(ufw.size() * sizeof(UfOrder)));
+        CK(cudaMemcpyAsync(c->d_ufw.p, ufw.data(), ufw.size() * sizeof(UfOrder), cudaMemcpyHostToDevice, c->st));
     }
+    bs_status det = detector_buffers<T>(c);
+    if (det != BS_OK) return det;
+    SideWork side{c};
+    CK(side.fork());
     cudaEventRecord(c->ev[1], c->st);
 
     // ---- LUT placement (before the sphere table goes to the device) ----
@@ -885,15 +952,29 @@ static bs_status run_nearfield(bs_ctx* c) {
         CK(cudaMemcpyAsync(c->d_sph.p, c->hs.data(), ns * sizeof(Sphere), cudaMemcpyHostToDevice, c->st));
     }
     cudaEventRecord(c->ev[2], c->st);
+
+    // ---- incident field and the transforms' tables, beside the Mie coefficients and lookup tables ----
+    cudaEventRecord(c->uf_ev[0], c->side);
+    if (uf_table) {
+        launch_uf_table(sc, c->d_uft.as<double>(), c->d_uftscr.as<double>(), c->side);
+        LAUNCHED(c);
+    }
+    launch_uf<T>(sc, c->d_uft.as<double>(), c->d_ufw.as<UfOrder>(), Uf, c->side);
+    LAUNCHED(c);
+    cudaEventRecord(c->uf_ev[1], c->side);
+    det = detector_tables<T>(c, c->side);
+    if (det != BS_OK) return det;
     c->interactions = 0;
 
     if (!p.scalar) {
+        CK(side.join());
         launch_sum_only<T>(sc, c->d_sph.as<Sphere>(), Uf, U, c->st);
         LAUNCHED(c);
         cudaEventRecord(c->ev[3], c->st);
     } else if (!p.lut_us) {
         cudaEventRecord(c->ev[3], c->st);
         if (ns == 0) {
+            CK(side.join());
             CK(cudaMemcpyAsync(U, Uf, (size_t)R * R * sizeof(cpx<T>), cudaMemcpyDeviceToDevice, c->st));
         } else {
             // the addition theorem turns the per-wave Legendre sums into per-sphere coefficients
@@ -904,6 +985,7 @@ static bs_status run_nearfield(bs_ctx* c) {
             launch_sh_tables(sc, c->d_sph.as<Sphere>(), L, c->d_waves.as<double>(), c->d_shrec.as<ShRec>(),
                              c->d_shtab.as<double2>(), c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_shcoef.as<zd>(), c->st);
             c->launches += 3;
+            CK(side.join());
             launch_us_sh<T>(sc, c->d_sph.as<Sphere>(), L, c->d_shrec.as<ShRec>(), c->d_shcoef.as<zd>(), Uf, U, c->st);
             LAUNCHED(c);
         }
@@ -1033,6 +1115,7 @@ static bs_status run_nearfield(bs_ctx* c) {
             if (first_build) {
                 cudaEventRecord(c->ev[3], c->st);
                 first_build = false;
+                CK(side.join());
             }
             int finalize = (ci == std::max(1, nchunks) - 1);
             if (fp64) {
@@ -1167,6 +1250,8 @@ bs_status bs_set_stream_priority(bs_ctx* c, int32_t priority) {
     if (e != cudaSuccess) return fail(BS_ERR_CUDA, "bs_set_stream_priority: %s", cudaGetErrorString(e));
     cudaStreamDestroy(c->st);
     c->st = st;
+    if (c->side) cudaStreamDestroy(c->side);  // made anew by the next run
+    c->side = nullptr;
     c->stream_prio = prio;
     return BS_OK;
 }
@@ -1223,10 +1308,14 @@ static bs_status simulate_impl(bs_ctx* c, bs_precision prec, bool accumulate) {
     st = (prec == BS_PREC_FP64) ? run_detector<double>(c, accumulate) : run_detector<float>(c, accumulate);
     if (st != BS_OK) return st;
     cudaEventRecord(c->ev[5], c->st);
+    const bool counted = prec == BS_PREC_MIXED && c->prm.scalar && c->prm.lut_us && !c->hs.empty();
+    unsigned long long cnt[2] = {0, 0};
+    if (counted) CK(cudaMemcpyAsync(cnt, c->d_cnt.p, sizeof(cnt), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     CK(cudaGetLastError());
     float t[5] = {0, 0, 0, 0, 0};
     for (int i = 0; i < 5; i++) cudaEventElapsedTime(&t[i], c->ev[i], c->ev[i + 1]);
+    cudaEventElapsedTime(&t[0], c->uf_ev[0], c->uf_ev[1]);  // beside the next two
     c->stats.ms_uf = t[0];
     c->stats.ms_mie = t[1];
     c->stats.ms_lut = t[2];
@@ -1238,9 +1327,7 @@ static bs_status simulate_impl(bs_ctx* c, bs_precision prec, bool accumulate) {
     c->stats.kernel_launches = c->launches - l0;
     c->stats.us_interactions = c->interactions;
     c->stats.lut_chunks_staged = c->stats.lut_chunks_total = 0;
-    if (prec == BS_PREC_MIXED && c->prm.scalar && c->prm.lut_us && !c->hs.empty()) {
-        unsigned long long cnt[2] = {0, 0};
-        CK(cudaMemcpy(cnt, c->d_cnt.p, sizeof(cnt), cudaMemcpyDeviceToHost));
+    if (counted) {
         c->stats.lut_chunks_staged = (int64_t)cnt[0];
         c->stats.lut_chunks_total = (int64_t)cnt[1];
     }
@@ -1621,52 +1708,56 @@ bs_status bs_plane_point(const bs_params* params, double u, double v, double* xy
     return BS_OK;
 }
 
-static bs_status image_to_host(bs_ctx* c, bs_image_kind kind, std::vector<double>& out) {
-    if (!c) return fail(BS_ERR_ARG, "null context");
-    if (!c->have) return fail(BS_ERR_STATE, "no simulation result (call bs_simulate first)");
-    if (kind < BS_IMG_INTENSITY || kind > BS_IMG_TRANSMITTANCE) return fail(BS_ERR_ARG, "unknown image kind");
-    int n = c->res * c->res;
-    size_t es = elem_r(c->prec);
-    CK(c->d_img.ensure((size_t)n * es));
-    if (c->prec == BS_PREC_FP64) {
-        const double* D = c->d_D.as<double>();
-        launch_image<double>(n, kind, D, D + n, c->d_img.as<double>(), c->st);
-    } else {
-        const float* D = c->d_D.as<float>();
-        launch_image<float>(n, kind, D, D + n, c->d_img.as<float>(), c->st);
+extern "C++" {
+
+// An image into the caller's res x res values of type H; the detector images themselves need no kernel, and
+// values of the run's own type no staging.
+template <class T, class H>
+static bs_status image_values(bs_ctx* c, bs_image_kind kind, H* host) {
+    const size_t n = (size_t)c->res * c->res;
+    const T* img = c->d_D.as<T>() + (kind == BS_IMG_INCIDENT ? n : 0);
+    if (kind > BS_IMG_INCIDENT) {
+        CK(c->d_img.ensure(n * sizeof(T)));
+        launch_image<T>((int)n, kind, img, img + n, c->d_img.as<T>(), c->st);
+        LAUNCHED(c);
+        img = c->d_img.as<T>();
     }
-    LAUNCHED(c);
-    out.resize(n);
-    if (c->prec == BS_PREC_FP64) {
-        CK(cudaMemcpyAsync(out.data(), c->d_img.p, n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-        CK(cudaStreamSynchronize(c->st));
-    } else {
-        std::vector<float> tmp(n);
-        CK(cudaMemcpyAsync(tmp.data(), c->d_img.p, n * sizeof(float), cudaMemcpyDeviceToHost, c->st));
-        CK(cudaStreamSynchronize(c->st));
-        for (int i = 0; i < n; i++) out[i] = tmp[i];
-    }
+    std::vector<T> tmp(sizeof(T) > sizeof(H) ? n : 0);
+    // floats for a double buffer go to its upper half and are widened from the front
+    T* to = sizeof(T) > sizeof(H) ? tmp.data() : reinterpret_cast<T*>(host) + (sizeof(H) / sizeof(T) - 1) * n;
+    CK(cudaMemcpyAsync(to, img, n * sizeof(T), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    if (sizeof(T) != sizeof(H))
+        for (size_t k = 0; k < n; k++) {
+            T v;
+            std::memcpy(&v, to + k, sizeof(T));
+            const H h = (H)v;
+            std::memcpy(host + k, &h, sizeof(H));
+        }
     return BS_OK;
 }
+
+template <class H>
+static bs_status image_to_host(bs_ctx* c, bs_image_kind kind, H* host) {
+    if (!c->have) return fail(BS_ERR_STATE, "no simulation result (call bs_simulate first)");
+    if (kind < BS_IMG_INTENSITY || kind > BS_IMG_TRANSMITTANCE) return fail(BS_ERR_ARG, "unknown image kind");
+    return c->prec == BS_PREC_FP64 ? image_values<double>(c, kind, host) : image_values<float>(c, kind, host);
+}
+
+}  // extern "C++"
 
 bs_status bs_get_image(bs_ctx* c, bs_image_kind kind, float* host, size_t count) {
     if (!host) return fail(BS_ERR_ARG, "bs_get_image: null buffer");
     if (c && count < (size_t)c->res * c->res) return fail(BS_ERR_ARG, "bs_get_image: buffer holds %zu of %d values", count, c->res * c->res);
-    std::vector<double> v;
-    bs_status st = image_to_host(c, kind, v);
-    if (st != BS_OK) return st;
-    for (size_t i = 0; i < v.size(); i++) host[i] = (float)v[i];
-    return BS_OK;
+    if (!c) return fail(BS_ERR_ARG, "null context");
+    return image_to_host(c, kind, host);
 }
 
 bs_status bs_get_image_f64(bs_ctx* c, bs_image_kind kind, double* host, size_t count) {
     if (!host) return fail(BS_ERR_ARG, "bs_get_image_f64: null buffer");
     if (c && count < (size_t)c->res * c->res) return fail(BS_ERR_ARG, "bs_get_image_f64: buffer too small");
-    std::vector<double> v;
-    bs_status st = image_to_host(c, kind, v);
-    if (st != BS_OK) return st;
-    std::memcpy(host, v.data(), v.size() * sizeof(double));
-    return BS_OK;
+    if (!c) return fail(BS_ERR_ARG, "null context");
+    return image_to_host(c, kind, host);
 }
 
 bs_status bs_get_field(bs_ctx* c, bs_field_kind kind, double* host, size_t count) {
@@ -1690,10 +1781,10 @@ bs_status bs_get_field(bs_ctx* c, bs_field_kind kind, double* host, size_t count
 
 bs_status bs_write_envi(bs_ctx* c, bs_image_kind kind, const char* path, int32_t append, double band_value) {
     if (!path) return fail(BS_ERR_ARG, "bs_write_envi: null path");
-    std::vector<double> v;
-    bs_status st = image_to_host(c, kind, v);
+    if (!c) return fail(BS_ERR_ARG, "null context");
+    std::vector<float> f((size_t)c->res * c->res);
+    bs_status st = image_to_host(c, kind, f.data());
     if (st != BS_OK) return st;
-    std::vector<float> f(v.begin(), v.end());
     char err[512] = {0};
     if (envi_add_band(path, f.data(), c->res, c->res, band_value, append, err, sizeof(err)) != 0)
         return fail(BS_ERR_IO, "%s", err);

@@ -108,7 +108,7 @@ typedef struct bs_info {
 /* Per-stage device timings (ms) and launch count of the last bs_simulate. */
 typedef struct bs_stats {
     double ms_total;
-    double ms_uf;
+    double ms_uf;        /* on a second stream, beside ms_mie and ms_lut */
     double ms_mie;
     double ms_lut;
     double ms_us;
