@@ -138,6 +138,7 @@ struct bs_server {
     std::vector<std::unique_ptr<Worker>> workers;
     uint64_t next_id = 1;
     bool stop = false;
+    int ready = 0;  // workers waiting for their first request
     int64_t submitted = 0, completed = 0, failed = 0, reuses = 0, running = 0;
     std::vector<double> latencies;
     size_t peak = 0;
@@ -258,6 +259,8 @@ size_t bs_server::run(Worker& w, Request& r) {
 void bs_server::loop(Worker& w) {
     if (!cfg.dry_run) cudaSetDevice(device);
     std::unique_lock<std::mutex> lk(mu);
+    ready++;
+    cv_done.notify_all();
     for (;;) {
         Request* r = nullptr;
         cv_work.wait(lk, [&] {
@@ -361,6 +364,12 @@ bs_status bs_server_create(const bs_server_config* cfg, bs_server** out) {
     for (auto& w : srv->workers) {
         Worker* wp = w.get();
         wp->th = std::thread([srv, wp] { srv->loop(*wp); });
+    }
+    {
+        // every worker up before the first request: short requests would otherwise all go to the first
+        // one that is, whose launches hold up the others' cudaSetDevice
+        std::unique_lock<std::mutex> lk(srv->mu);
+        srv->cv_done.wait(lk, [&] { return srv->ready == nw; });
     }
     *out = srv;
     return BS_OK;
