@@ -1004,7 +1004,7 @@ static bs_status run_nearfield(bs_ctx* c) {
             CK(c->d_starts.ensure((size_t)maxstarts * sizeof(long long)));
             if (!fp64) CK(c->d_bias.ensure((size_t)maxrow * sizeof(float)));
             if (fp64 && c->acos_theta != thetaR) {
-                CK(c->d_acos.ensure((ACOS_NODES + 1) * sizeof(AcosNode)));
+                CK(c->d_acos.ensure((ACOS_NODES + 1) * sizeof(AcosNode) + thetaR * sizeof(double)));
                 launch_acos_nodes(thetaR, c->d_acos.as<AcosNode>(), c->st);
                 LAUNCHED(c);
                 c->acos_theta = thetaR;
@@ -1186,7 +1186,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         b += B(pool) + B((size_t)maxcoef * sizeof(zd)) +
              B((size_t)maxstarts * sizeof(long long));
         b += B(thetaR * (size_t)c->Lmax * sizeof(double));    // Legendre table
-        if (fp64) b += B((ACOS_NODES + 1) * sizeof(AcosNode));
+        if (fp64) b += B((ACOS_NODES + 1) * sizeof(AcosNode) + c->hs[0].thetaR * sizeof(double));
         if (!fp64) {
             b += B((size_t)maxrow * sizeof(float));  // biases
             const int shares = lut_splits((int)R, (int)ns, (int)nk);

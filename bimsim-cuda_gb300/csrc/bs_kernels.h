@@ -59,11 +59,12 @@ void launch_lut_build(const zd* tab, int rows, int L, const double* P, int Pstri
                       cudaStream_t st);
 template <class T>
 void launch_phase(const Scene& sc, const Sphere* sph, const double* waves, cpx<T>* ph, float4* kw4, cudaStream_t st);
-// Nodes of the double-precision arc cosine at j pi / ACOS_NODES: cos, 1 / sin, the angle in columns of a
-// table of thetaR angles, and the series coefficients of the angle around it (us_lut_f64_kernel); ACOS_NODES + 1 of them.
-constexpr int ACOS_NODES = 2048;
-struct alignas(64) AcosNode {
-    double c, is, th, b2, b3, b4, b5, b6;
+// Nodes of the double-precision arc cosine at j pi / ACOS_NODES: the cosine c, the angle t in columns of a table of
+// thetaR angles, and d1 .. d4 of the column t + d1 y + d2 y^2 + d3 y^3 + d4 y^4 at the cosine c - y
+// (us_lut_f64_kernel); ACOS_NODES + 1 of them, then the numbers 0 .. thetaR - 1 as doubles.
+constexpr int ACOS_NODES = 16384;
+struct alignas(16) AcosNode {
+    double c, t, d1, d2, d3, d4;
 };
 void launch_acos_nodes(int thetaR, AcosNode* nodes, cudaStream_t st);
 void launch_us_lut_f64(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,

@@ -428,25 +428,31 @@ __global__ void phase_kernel(Scene sc, const Sphere* __restrict__ sph, const dou
 // picks the nearest of ACOS_NODES equal steps of [0, pi], and the rest is the inverse series of
 // cos(theta_j + e) = c: with x = (cos theta_j - c) / sin theta_j and kappa = cot theta_j,
 //   e = x - kappa/2 x^2 + (3 kappa^2 + 1)/6 x^3 - kappa (5 kappa^2 + 3)/8 x^4
-//         + (35 kappa^4 + 30 kappa^2 + 3)/40 x^5 - kappa (63 kappa^4 + 70 kappa^2 + 15)/48 x^6 + ...
-// whose next term is below 2e-17 for |x| <= pi/4096 and |kappa| <= 6; closer to the poles (9.5 degrees)
-// acos itself is called.  26 instructions per lookup; 8 spheres, 288^2 pixels, 200 directions: 12.8 ms
-// before, 6.6 ms now.  Blocks of 64 pixels: at 128 the last wave of that slice is a quarter full (7.5 ms).
+//         + (35 kappa^4 + 30 kappa^2 + 3)/40 x^5 - ...
+// whose next term is below 2e-17 for |x| <= pi/30000 and |kappa| <= 6; closer to the poles (9.5 degrees)
+// acos itself is called.  The nodes hold the coefficients in columns and powers of cos theta_j - c, so that the
+// column costs five instructions, and conversions, which share the pipe, are left out: the float cosine is
+// put together from c's high word, and a table gives the column's number as a double.  20 instructions per
+// lookup.  8 spheres, 288^2 pixels, 200 directions: 12.8 ms with acos, 6.57 ms with 2048 nodes of six terms
+// (nine instructions), 5.54 ms with these nodes, 4.94 ms without the conversions.  The nodes' 0.8 MB are
+// read by neighbouring pixels at neighbouring angles.  Blocks of 64 pixels: at 128 the last wave of that slice is a
+// quarter full.
 // ---------------------------------------------------------------------------
-__global__ void acos_node_kernel(double tsc, AcosNode* __restrict__ nodes) {
+__global__ void acos_node_kernel(int thetaR, double tsc, AcosNode* __restrict__ nodes) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    double* cols = reinterpret_cast<double*>(nodes + ACOS_NODES + 1);
+    for (int i = j; i < thetaR; i += gridDim.x * blockDim.x) cols[i] = i;
     if (j > ACOS_NODES) return;
     AcosNode n;
     double sn;
     sincospi((double)j / ACOS_NODES, &sn, &n.c);
-    const double k = j == 0 || j == ACOS_NODES ? 0.0 : n.c / sn, k2 = k * k;
-    n.is = j == 0 || j == ACOS_NODES ? 0.0 : 1.0 / sn;
-    n.th = j * (TRUE_PI / ACOS_NODES) * tsc;
-    n.b2 = -0.5 * k;
-    n.b3 = (3.0 * k2 + 1.0) / 6.0;
-    n.b4 = -k * (5.0 * k2 + 3.0) / 8.0;
-    n.b5 = ((35.0 * k2 + 30.0) * k2 + 3.0) / 40.0;
-    n.b6 = -k * ((63.0 * k2 + 70.0) * k2 + 15.0) / 48.0;
+    const bool pole = j == 0 || j == ACOS_NODES;
+    const double k = pole ? 0.0 : n.c / sn, k2 = k * k, is = pole ? 0.0 : 1.0 / sn, is2 = is * is;
+    n.t = j * (TRUE_PI / ACOS_NODES) * tsc;
+    n.d1 = tsc * is;
+    n.d2 = -0.5 * k * tsc * is2;
+    n.d3 = (3.0 * k2 + 1.0) / 6.0 * tsc * (is2 * is);
+    n.d4 = -k * (5.0 * k2 + 3.0) / 8.0 * tsc * (is2 * is2);
     nodes[j] = n;
 }
 
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(F64_BLOCK) us_lut_f64_kernel(Scene sc, const S
                                                           const AcosNode* __restrict__ nodes,
                                                           const zd* __restrict__ ph, const Patch<double>* __restrict__ lut,
                                                           const zd* __restrict__ Uf, zd* __restrict__ U) {
-    constexpr int POLE = 108;  // nodes within 9.5 degrees of a pole
+    constexpr int POLE = 864;  // nodes within 9.5 degrees of a pole
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= sc.R * sc.R) return;
     double p[3];
@@ -479,24 +485,26 @@ __global__ void __launch_bounds__(F64_BLOCK) us_lut_f64_kernel(Scene sc, const S
             cb = 0.0;
         }
         const double tmax = S.thetaR - 1, tsc = tmax * (1.0 / PI_REF);
+        const double* cols = reinterpret_cast<const double*>(nodes + ACOS_NODES + 1);
         zd sum = mk(0.0, 0.0);
         const zd* phs = ph + (size_t)s * sc.nk;
-#pragma unroll 2
+#pragma unroll 4
         for (int w = 0; w < sc.nk; w++) {
             const double* k = waves + 3 * w;
             const double c = fma(k[0], rn[0], fma(k[1], rn[1], fma(k[2], rn[2], cb)));
-            const int j = __float2int_rn(acosf(fminf(fmaxf((float)c, -1.f), 1.f)) * (float)(ACOS_NODES / TRUE_PI));
+            const int hc = __double2hiint(c), mag = min(hc & 0x7fffffff, 0x47e00000) - 0x38000000;
+            const float cf = __int_as_float((hc & 0x80000000) | max(mag, 0) << 3);  // c, its high word's 20 bits
+            const int j = __float2int_rn(acosf(fminf(fmaxf(cf, -1.f), 1.f)) * (float)(ACOS_NODES / TRUE_PI));
             double t;
             if (j > POLE && j < ACOS_NODES - POLE) {
-                const AcosNode& n = nodes[j];
-                const double x = (n.c - c) * n.is;
-                const double q = fma(fma(fma(fma(n.b6, x, n.b5), x, n.b4), x, n.b3), x, n.b2);
-                t = fma(fma(q * x, x, x), tsc, n.th);
+                const AcosNode n = nodes[j];
+                const double y = n.c - c;
+                t = fma(fma(fma(fma(n.d4, y, n.d3), y, n.d2), y, n.d1), y, n.t);
             } else {
                 t = fmin(acos(fmin(fmax(c, -1.0), 1.0)) * tsc, tmax);
             }
             const double u = __dadd_rd(t, 6755399441055744.0);  // 1.5 2^52: the sum's low word is floor(t)
-            const double be = t - (u - 6755399441055744.0);
+            const double be = t - cols[__double2loint(u)];
             const Patch<double>& q = row[__double2loint(u)];
             const double vr = fma(be, fma(al, q.v[6], q.v[4]), fma(al, q.v[2], q.v[0]));
             const double vi = fma(be, fma(al, q.v[7], q.v[5]), fma(al, q.v[3], q.v[1]));
@@ -1020,7 +1028,7 @@ void launch_phase(const Scene& sc, const Sphere* sph, const double* waves, cpx<T
 }
 
 void launch_acos_nodes(int thetaR, AcosNode* nodes, cudaStream_t st) {
-    acos_node_kernel<<<blocks_for(ACOS_NODES + 1, 64), 64, 0, st>>>((thetaR - 1) * (1.0 / PI_REF), nodes);
+    acos_node_kernel<<<blocks_for(ACOS_NODES + 1, 64), 64, 0, st>>>(thetaR, (thetaR - 1) * (1.0 / PI_REF), nodes);
 }
 
 void launch_us_lut_f64(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,

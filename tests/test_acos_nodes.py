@@ -24,3 +24,19 @@ def test_angles(z, theta):
         ctx.simulate(BS_PREC_FP64)
         err = np.linalg.norm(ctx.field() - U) / np.linalg.norm(U)
     assert err <= 1e-10, err
+
+
+def test_directions_that_are_not_unit_vectors():
+    """Cosines beyond 1, up to and past the range of a float: the angle clamps at 0 and pi."""
+    p = abi.make_params(lam=2.5, condenser=(0, 0.5), objective=(0, 0.5), xy=(8, 0), resolution=11, padding=1,
+                        supersample=1, us_lut_r=60, us_lut_theta=90)
+    s = [(0.0, 0.0, 0.0, 1.0, 1.45, 0.03)]
+    scale = np.concatenate([np.linspace(0.8, 1.3, 56), [1e3, 1e30, 1e39, 1e60]])
+    w = scenes.mc_waves(60, 0, 0.5, seed=43) * scale[:, None]
+    U = oracle_lib.simulate(p, *abi.sphere_array(s), w)[0]
+    with Context(p) as ctx:
+        ctx.set_spheres(s)
+        ctx.set_waves(w)
+        ctx.simulate(BS_PREC_FP64)
+        err = np.linalg.norm(ctx.field() - U) / np.linalg.norm(U)
+    assert err <= 1e-10, err
