@@ -152,6 +152,12 @@ __constant__ float c_nodes[10] = {0.923879533f, -0.923879533f, 0.382683432f, -0.
 // largest over 4e4 random geometries per decade of q.  Both limits keep it under 6e-8 rad,
 // half of what single precision leaves of the arc cosine itself.
 __device__ __forceinline__ int row_mode(float q) { return q <= 0.037f ? 4 : (q <= 0.148f ? 6 : 0); }
+// In windows of 8 pixels (shape 2) the polynomial is made twice, of 4 (shape 3) four times: 4 points still cost
+// less than 8 arc cosines, 6 do not, and nothing less than 4.
+__device__ __forceinline__ int band_mode(float q, int shape) {
+    const int mode = row_mode(q);
+    return shape < 2 || (shape == 2 && mode == 4) ? mode : 0;
+}
 
 // Order the nkb directions kw[0 .. nkb) by their angle to `ctr` and write them, with their
 // phases, to sm.k and sm.p: a stable counting sort over SW_BUCKETS equal steps of the cosine
@@ -235,10 +241,11 @@ __device__ __forceinline__ void order_waves(SwShared& sm, const float4* __restri
 // pixels), 0}.  The window holds 16 pixels x 64 columns, half the row's pixels x 128 or a quarter x 256
 // (shapes 1, 2, 3): wider ones take in more groups per blended row, but a row's polynomials are made
 // again for each part.  The shape of least cost per (pixel, group) is taken, in instructions and their
-// shared-memory share: 24 per 64 columns blended, and the row's polynomial (3.5 or 5.5 a pixel, 16 pixels)
-// or arc cosine (11); none (shape 0: a band of one group, cells from the table) where all are above 40.
-// Measured with 16 x 64 alone and with all three: 768^2 pixels of 0.39 um, 120 spheres, 1000 directions 144
-// and 120 ms; 906^2 of 0.13 um, NA 0.9 18.7 and 17.0 ms; 3072^2 of 0.1 um (narrow windows throughout) the same.
+// shared-memory share: 24 per 64 columns blended, and the row's polynomial (3.5 or 5.5 a pixel each time it is made)
+// or arc cosine (11); none (shape 0: a band of one group, cells from the table) where all are above 34.
+// Measured with 16 x 64 alone, with all three and polynomials of 6 points in all, and now: 768^2 pixels of 0.39 um,
+// 120 spheres, 1000 directions 144, 120 and 115 ms; 906^2 of 0.13 um, NA 0.9 18.7, 17.0 and 16.0 ms; 3072^2 of 0.1 um
+// (narrow windows throughout) the same.
 // Returns the number of chunks of `chunk` directions (64, 32 or 16) in the bands with a window (lane 0;
 // chunk 0: none).
 __device__ __forceinline__ unsigned plan_bands(SwShared& sm, int G, int nkb, int thetaR, float tsc, float gam, float rdist,
@@ -248,7 +255,7 @@ __device__ __forceinline__ unsigned plan_bands(SwShared& sm, int G, int nkb, int
     int info = 0;
     if (lane < G) {
         const int t_lo = max(0, (int)floorf(sm.gb[lane].x - gcol) - 1) & ~1;
-        float best = 40.f, bq = 0.f;
+        float best = 34.f, bq = 0.f;
         info = (lane + 1);
         float lo = sm.gb[lane].x, hi = sm.gb[lane].y;
         auto quotient = [&]() {  // (half row length) / (smallest sine)
@@ -270,9 +277,8 @@ __device__ __forceinline__ unsigned plan_bands(SwShared& sm, int G, int nkb, int
             }
             if (nx == lane) continue;
             const float q = quotient();
-            const int mode = row_mode(q * rdist);
-            const float cost = 24.f * (1 << s) / (nx - lane) +
-                               (mode == 4 && s == 0 ? 3.5f : mode != 0 ? 5.5f * (1 << s) : 11.f);
+            const int mode = band_mode(q * rdist, s + 1);
+            const float cost = 24.f * (1 << s) / (nx - lane) + (mode == 4 ? 3.5f * (1 << s) : mode == 6 ? 5.5f : 11.f);
             if (cost < best) {
                 best = cost;
                 bq = q;
@@ -458,8 +464,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
                 while (g0 < G) {
                     const int4 band = sm.band[g0];
                     const int t_lo = band.x, g1 = band.y & 255, shape = band.y >> 8 & 3, width = band.y >> 16;
-                    int mode = row_mode(__int_as_float(band.z) * sm.rdist[warp][r]);
-                    if (shape > 1 && mode == 4) mode = 6;  // one polynomial for the wider windows
+                    const int mode = band_mode(__int_as_float(band.z) * sm.rdist[warp][r], shape);
                     // the blended rows of part h of the row: pixels i and 15 - i, i in [8 h / parts, 8 (h + 1) / parts)
                     auto stage = [&](auto sh, int h) {
                         constexpr int S = decltype(sh)::value, NP = 16 >> S, W = SW_W << S;
@@ -589,13 +594,18 @@ __global__ void __launch_bounds__(SW_NT, 2)
                         }
                     };
                     auto by_mode = [&](auto sh) {
-                        if constexpr (decltype(sh)::value == 0)
+                        constexpr int S = decltype(sh)::value;
+                        if constexpr (S < 2)
                             if (mode == 4) {
                                 rows(Int<4>{}, sh);
                                 return;
                             }
-                        if (mode == 6) rows(Int<6>{}, sh);
-                        else rows(Int<0>{}, sh);
+                        if constexpr (S == 0)
+                            if (mode == 6) {
+                                rows(Int<6>{}, sh);
+                                return;
+                            }
+                        rows(Int<0>{}, sh);
                     };
                     if (STAGE && shape == 1) {
                         by_mode(Int<0>{});
