@@ -1022,7 +1022,9 @@ static bs_status run_nearfield(bs_ctx* c) {
         const int nchunks = (int)chunk_start.size() - 1;
         const int shares = fp64 || ns == 0 ? 1 : lut_splits(R, ns, nk);
         if (shares > 1) CK(c->d_part.ensure((size_t)shares * 4 * R * R * sizeof(float)));
-        else if (!fp64 && nchunks > 1) CK(c->d_kcmp.ensure((size_t)R * R * sizeof(float2)));
+        const int ranges = fp64 || ns == 0 ? 1 : lut_ranges(R, ns, nk, pool);
+        const bool carry = shares == 1 && (nchunks > 1 || ranges > 1);
+        if (!fp64 && carry) CK(c->d_kcmp.ensure((size_t)R * R * sizeof(float2)));
         bool use_stage = false;
         // tables of the previous run still in the pool?
         std::vector<double> key;
@@ -1123,11 +1125,18 @@ static bs_status run_nearfield(bs_ctx* c) {
                                   c->d_acos.as<AcosNode>(), c->d_ph.as<zd>(), c->d_lut.as<Patch<double>>(),
                                   (const zd*)Uf, (zd*)U, c->st);
             } else {
-                launch_us_lut_mixed(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_kw4.as<float4>(),
-                                    c->d_ph.as<cpx<float>>(), c->d_lut.as<float2>(), (const cpx<float>*)Uf,
-                                    (cpx<float>*)U, ns > 0 ? c->d_cnt.as<unsigned long long>() : nullptr,
-                                    nchunks > 1 ? c->d_kcmp.as<float2>() : nullptr,
-                                    shares > 1 ? c->d_part.as<float>() : nullptr, use_stage, chunk, cone, c->st);
+                for (int q = 0; q < ranges; q++) {
+                    const int r0 = s0 + (int)((long long)(s1 - s0) * q / ranges);
+                    const int r1 = s0 + (int)((long long)(s1 - s0) * (q + 1) / ranges);
+                    const int last = q == ranges - 1;
+                    launch_us_lut_mixed(sc, c->d_sph.as<Sphere>(), r0, r1, ci > 0 || q > 0, finalize && last,
+                                        c->d_kw4.as<float4>(), c->d_ph.as<cpx<float>>(), c->d_lut.as<float2>(),
+                                        (const cpx<float>*)Uf, (cpx<float>*)U,
+                                        ns > 0 ? c->d_cnt.as<unsigned long long>() : nullptr,
+                                        carry ? c->d_kcmp.as<float2>() : nullptr,
+                                        shares > 1 ? c->d_part.as<float>() : nullptr, use_stage, chunk, cone, c->st);
+                    if (!last) LAUNCHED(c);
+                }
                 if (shares > 1 && finalize) c->launches++;
             }
             LAUNCHED(c);
@@ -1191,7 +1200,8 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
             b += B((size_t)maxrow * sizeof(float));  // biases
             const int shares = lut_splits((int)R, (int)ns, (int)nk);
             if (shares > 1) b += B((size_t)shares * 4 * R * R * sizeof(float));
-            else if (cs.size() > 2) b += B(R * R * sizeof(float2));  // Kahan carry between chunks
+            else if (cs.size() > 2 || lut_ranges((int)R, (int)ns, (int)nk, pool) > 1)
+                b += B(R * R * sizeof(float2));  // Kahan carry between chunks
             b += B(2 * sizeof(unsigned long long));
         }
     }

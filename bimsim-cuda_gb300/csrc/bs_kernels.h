@@ -85,6 +85,8 @@ void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int
 // Shares of the spheres that launch_us_lut_mixed runs side by side; above 1, `part` (else null) holds
 // 4 floats per pixel and share.
 int lut_splits(int R, int ns, int nk);
+// Launches of launch_us_lut_mixed, over parts of the spheres, for spheres with `table_bytes` of tables in all.
+int lut_ranges(int R, int ns, int nk, size_t table_bytes);
 // One table of the mixed path's table build: the rows of one sphere's Usp or Uip with their
 // coefficient rows at tab + tab_off and biases at bias + row_off, written to the linear rows at
 // lin + lin_off.

@@ -784,14 +784,24 @@ __global__ void __launch_bounds__(128) us_lut_join_kernel(Scene sc, const Sphere
     U[idx] = mk(tot.x, tot.y);
 }
 
-// A slice of fewer tiles than three per SM leaves SMs with one block of 8 warps or none: its spheres are
-// shared out so that there are about four blocks per SM.  A sphere's share depends on the slice alone, so
-// that chunked tables give the bits of one launch.  192^2 pixels, 12 spheres, 400 directions: 1.16 ms a slice
-// in one share, 0.79 ms in five.
+// The spheres of a slice are shared out over blocks: a small grid leaves SMs with one block of 8 warps or none,
+// the tiles' work differs and two blocks at a time leave a long tail on grids of a few rounds, and blocks that
+// work on the same few spheres find their tables (34 MB each at 4096 x 1024) in L2.  About 128 blocks per SM;
+// from 64 tiles per SM on the sums' memory (16 bytes a pixel and share) is not worth it, see lut_ranges.  A
+// sphere's share depends on the slice alone, so that chunked tables give the bits of one launch.  Scattered
+// field in one share, 4 blocks per SM and 128: 192^2 pixels, 12 spheres, 400 directions 1.16, 0.70 and 0.59 ms;
+// 384^2, 50, 200: 7.2, 7.2 and 6.0 ms; 768^2, 120, 1000: 115, 115 and 102 ms.
 int lut_splits(int R, int ns, int nk) {
-    const int tiles = ((R + 15) / 16) * ((R + 15) / 16);
-    if (nk <= LUT_FEW_WAVES || tiles >= 3 * GB300_SMS) return 1;
-    return std::max(1, std::min({ns, 8, (4 * GB300_SMS + tiles - 1) / tiles}));
+    const long long tiles = (long long)((R + 15) / 16) * ((R + 15) / 16);
+    if (nk <= LUT_FEW_WAVES || tiles >= 64 * GB300_SMS) return 1;
+    return (int)std::max(1LL, std::min({(long long)ns, 16LL, (128 * GB300_SMS + tiles - 1) / tiles}));
+}
+
+// Launches the spheres of a chunk are spread over where lut_splits gives one share: each with about twice the L2
+// cache's size of tables, up to 8.  3072^2 pixels, 50 spheres with 34 MB each: 576 ms in one launch, 563 in 6.
+int lut_ranges(int R, int ns, int nk, size_t table_bytes) {
+    if (nk <= LUT_FEW_WAVES || lut_splits(R, ns, nk) > 1) return 1;
+    return (int)std::max<size_t>(1, std::min<size_t>(std::min(ns, 8), table_bytes >> 28));
 }
 
 void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,

@@ -38,3 +38,22 @@ def test_shares(ns, fov, pieces):
             got.append((ctx.field(), ctx.image(BS_IMG_INTENSITY, f64=True)))
     assert rel(got[0][0], U) <= 1e-4 and rel(got[0][1], D) <= 1e-5, (rel(got[0][0], U), rel(got[0][1], D))
     assert np.array_equal(got[0][0], got[1][0])
+
+
+def test_ranges():
+    """A grid too large for shares with tables of twice 256 MB: two launches, the bits of a table at a time."""
+    p = abi.make_params(lam=3.0, condenser=(0, 0.5), objective=(0, 0.5), xy=(60, 0), resolution=529, padding=1,
+                        supersample=1, us_lut_r=4096, us_lut_theta=1024)
+    s = [(14 * (i % 4) - 21.0, 14 * (i // 4) - 22.0, 0.0, 1.0, 1.3 + 0.01 * i, 0.01) for i in range(16)]
+    w = scenes.mc_waves(40, 0, 0.5, seed=32)
+    got = []
+    for budget in (0, 40 << 20):
+        with Context(p) as ctx:
+            ctx.set_spheres(s)
+            ctx.set_waves(w)
+            if budget:
+                ctx.set_lut_budget(budget)
+            ctx.simulate(BS_PREC_MIXED)
+            got.append((ctx.field(), ctx.stats().kernel_launches))
+    assert got[0][1] < got[1][1]
+    assert np.array_equal(got[0][0], got[1][0])
