@@ -903,6 +903,7 @@ static bs_status run_nearfield(bs_ctx* c) {
                 b2 = b0;
                 step(l + 1, sc.cos_b, b0, b1);
             }
+            ufw[l].odd = 2.0 * l - 1.0;
             ufw[l].beta = 0;
             if (l > 0) {
                 const double k1 = kap;

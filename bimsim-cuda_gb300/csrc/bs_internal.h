@@ -48,9 +48,9 @@ struct Scene {
 };
 
 // Per order l of the incident field: the monic Legendre recurrence's factor and the weight
-// +-2 PI A w_l kappa_l (sign of i^l; P_l = kappa_l u_l).
+// +-2 PI A w_l kappa_l (sign of i^l; P_l = kappa_l u_l); 2 l - 1.
 struct UfOrder {
-    double beta, w;
+    double beta, w, odd;
 };
 
 // Per-sphere data (sphere.h:14-92 plus the LUT geometry of sphere.cpp:222-240).

@@ -22,7 +22,8 @@ namespace bs {
 // every pixel.  The kernel is bound by the FP64 pipe, so the host's UfOrder carries all that depends on the order
 // alone: P_l runs in monic form (u_l = x u_{l-1} - beta_l u_{l-2}, two instructions), its scale, w_l and
 // the sign of i^l in one weight; even orders sum into the real part, odd ones into the imaginary part.
-// 3072^2 pixels, 11 orders, table mode: 6.0 -> 2.4 ms; direct mode at 1280^2: 1.43 -> 0.72 ms.
+// 3072^2 pixels, 11 orders, table mode: 6.0 -> 2.4 ms; direct mode at 1280^2: 1.43 -> 0.72 ms, and 0.57 ms with the
+// clamps, the order's factors and four of the five divisions off the pipe as well.
 struct UfLegendre {  // u_l(x), l = 0, 1, 2, ... in turn
     double u2 = 0, u1 = 1;
     __device__ __forceinline__ double next(int l, double x, double beta) {
@@ -34,35 +35,41 @@ struct UfLegendre {  // u_l(x), l = 0, 1, 2, ... in turn
     }
 };
 
-// The clamped upward j_l recurrence (sbesselj_step) with one reciprocal for all orders.
+// The clamp of sbesselj_step off the FP64 pipe: the high words of CONV_MIN and CONV_MAX decide, but where they are equal.
+__device__ __forceinline__ double clamp_j(double j, bool beyond) {
+    constexpr int LO = 0x3f8db22d, HI = 0x3fd99999;
+    const int h = __double2hiint(j);
+    return beyond && (h <= LO || h >= HI) && (h < LO || h > HI || j < CONV_MIN || j > CONV_MAX) ? 0.0 : j;
+}
+
+// The clamped upward j_l recurrence (sbesselj_step), one reciprocal for all quotients and orders.
 __device__ zd uf_direct(const Scene& sc, const UfOrder* __restrict__ w, const double p[3]) {
     double r[3];
     double d = dist_exact(p, sc.focus, r);
     if (d < EPS_FLOAT) return mk(sc.amp * 2 * PI_REF * (sc.cos_a - sc.cos_b), 0.0);
-    const double cth = (sc.kdir[0] * r[0] + sc.kdir[1] * r[1] + sc.kdir[2] * r[2]) / d;
+    const double cth = quot(sc.kdir[0] * r[0] + sc.kdir[1] * r[1] + sc.kdir[2] * r[2], d, 1.0 / d);
     const double kd = sc.kmag * d, inv = 1.0 / kd;
     double s, c;
     sincos(kd, &s, &c);
-    double j0 = s / kd, j1 = j0 / kd - c / kd;
+    double j0 = quot(s, kd, inv), j1 = quot(j0, kd, inv) - quot(c, kd, inv);
     const int lclamp = kd < (double)MAX_ORDER ? (int)kd : MAX_ORDER;  // l > kd exactly for l > lclamp
-    UfLegendre P;
-    zd sum = mk(0.0, 0.0);
-    for (int l = 0; l <= sc.m; l += 2) {
-        double jl = l == 0 ? j0 : fma(quot(2.0 * l - 1.0, kd, inv), j1, -j0);
-        if (l > 0) {
-            if (l > lclamp && (jl < CONV_MIN || jl > CONV_MAX)) jl = 0.0;
-            j0 = j1;
-            j1 = jl;
-        }
-        sum.re = fma(jl * P.next(l, cth, w[l].beta), w[l].w, sum.re);
+    zd sum = mk(j0 * w[0].w, 0.0);
+    if (sc.m == 0) return sum;
+    double u2 = 1.0, u1 = cth;  // u_{l-1} and u_l, see UfLegendre
+    sum.im = j1 * u1 * w[1].w;
+    auto step = [&](int l) {  // j_l u_l
+        const double jl = clamp_j(fma(quot(w[l].odd, kd, inv), j1, -j0), l > lclamp);
+        j0 = j1;
+        j1 = jl;
+        const double u = fma(cth, u1, -w[l].beta * u2);
+        u2 = u1;
+        u1 = u;
+        return jl * u;
+    };
+    for (int l = 2; l <= sc.m; l += 2) {
+        sum.re = fma(step(l), w[l].w, sum.re);
         if (l + 1 > sc.m) break;
-        jl = l == 0 ? j1 : fma(quot(2.0 * l + 1.0, kd, inv), j1, -j0);
-        if (l > 0) {
-            if (l + 1 > lclamp && (jl < CONV_MIN || jl > CONV_MAX)) jl = 0.0;
-            j0 = j1;
-            j1 = jl;
-        }
-        sum.im = fma(jl * P.next(l + 1, cth, w[l + 1].beta), w[l + 1].w, sum.im);
+        sum.im = fma(step(l + 1), w[l + 1].w, sum.im);
     }
     return sum;
 }
@@ -827,7 +834,7 @@ struct ShRadial {
             p1 = j0 / z - zcos(z) / z;
         } else {
             x = sc.kmag * d;
-            xi = (int)floor(x);
+            xi = x < (double)MAX_ORDER ? (int)x : MAX_ORDER;
             inv = 1.0 / x;
             odd = 1.0;
             double sn, cs;
@@ -852,13 +859,11 @@ struct ShRadial {
         if (l < 2) return l == 0 ? p0 : p1;
         odd += 2.0;
         const double w = quot(odd, x, inv);
-        double j = fma(w, p1.re, -p0.re), y = fma(w, p1.im, -p0.im);
-        // high words of CONV_MIN, CONV_MAX and Y_FLOOR decide, but where they are equal
-        constexpr int LO = 0x3f8db22d, HI = 0x3fd99999;
-        constexpr unsigned FLOOR = 0xc6c8a6e3u;
-        const int hj = __double2hiint(j), hy = __double2hiint(y);
         const bool beyond = l > xi;
-        if (beyond && (hj <= LO || hj >= HI) && (hj < LO || hj > HI || j < CONV_MIN || j > CONV_MAX)) j = 0.0;
+        const double j = clamp_j(fma(w, p1.re, -p0.re), beyond);
+        double y = fma(w, p1.im, -p0.im);
+        constexpr unsigned FLOOR = 0xc6c8a6e3u;  // Y_FLOOR's high word
+        const int hy = __double2hiint(y);
         if ((beyond && hy > 0) || ((unsigned)hy >= FLOOR && ((unsigned)hy > FLOOR || y < Y_FLOOR))) {
             y = 0;
             p1.im = 0;
