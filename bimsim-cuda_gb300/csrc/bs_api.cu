@@ -836,9 +836,9 @@ struct SideWork {
     bool open = false;
     cudaError_t fork() {
         cudaError_t e = cudaSuccess;
-        if (!c->side) e = cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, c->stream_prio);
         for (cudaEvent_t* v : {&c->uf_ev[0], &c->uf_ev[1]})
             if (e == cudaSuccess && !*v) e = cudaEventCreate(v);
+        if (!c->side) e = cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, c->stream_prio);
         for (cudaEvent_t* v : {&c->fork, &c->join})
             if (e == cudaSuccess && !*v) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventRecord(c->fork, c->st);
@@ -1155,8 +1155,7 @@ static bs_status run_nearfield(bs_ctx* c) {
 }
 
 // Device bytes the buffers of run_nearfield and run_detector reach for the
-// derived scene of `c` (each DevBuf at least 256 bytes; texture planes as
-// width x height floats, as bs_get_info counts them).  0 if the tables do not
+// derived scene of `c` (each DevBuf at least 256 bytes).  0 if the tables do not
 // fit lut_budget.
 static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
     const bs_params& p = c->prm;
@@ -1320,8 +1319,6 @@ static bs_status simulate_impl(bs_ctx* c, bs_precision prec, bool accumulate) {
     if (st != BS_OK) return st;
     cudaEventRecord(c->ev[5], c->st);
     const bool counted = prec == BS_PREC_MIXED && c->prm.scalar && c->prm.lut_us && !c->hs.empty();
-    unsigned long long cnt[2] = {0, 0};
-    if (counted) CK(cudaMemcpyAsync(cnt, c->d_cnt.p, sizeof(cnt), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     CK(cudaGetLastError());
     float t[5] = {0, 0, 0, 0, 0};
@@ -1338,7 +1335,9 @@ static bs_status simulate_impl(bs_ctx* c, bs_precision prec, bool accumulate) {
     c->stats.kernel_launches = c->launches - l0;
     c->stats.us_interactions = c->interactions;
     c->stats.lut_chunks_staged = c->stats.lut_chunks_total = 0;
-    if (counted) {
+    if (counted) {  // after the wait: a copy to pageable memory that waits itself holds up other threads' calls
+        unsigned long long cnt[2] = {0, 0};
+        CK(cudaMemcpy(cnt, c->d_cnt.p, sizeof(cnt), cudaMemcpyDeviceToHost));
         c->stats.lut_chunks_staged = (int64_t)cnt[0];
         c->stats.lut_chunks_total = (int64_t)cnt[1];
     }
