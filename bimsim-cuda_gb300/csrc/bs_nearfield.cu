@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(128) coef_rows_batch_kernel(const Sphere* __re
                                                               const zd* __restrict__ A, const zd* __restrict__ B,
                                                               zd* __restrict__ tab, float* __restrict__ bias) {
     extern __shared__ zd cr_val[];  // [order][row]: (j, y) or j of a complex argument, then the coefficients
-    __shared__ zd s_j0[CR_ROWS], s_j1[CR_ROWS];
+    __shared__ zd s_j0[CR_ROWS], s_j1[CR_ROWS], s_sc[CR_ROWS];
     __shared__ int s_nv[CR_ROWS], s_len[CR_ROWS];
     __shared__ long long s_out[CR_ROWS];
     __shared__ float s_sum[4][CR_ROWS];
@@ -277,20 +277,21 @@ __global__ void __launch_bounds__(128) coef_rows_batch_kernel(const Sphere* __re
         }
     }
     __syncthreads();
-    if (!outer && !centre) Nv = s_nv[lane];
-    const zd f0 = v[0], f1 = v[N >= 1 ? CR_PAD : 0];
-    __syncthreads();
-    float sum = 0.f;
-    zd sc = mk(1.0, 0.0);  // what the downward recurrence lacks
-    if (outer) {
-        if (!(x < 1e-15) && !upward) {
-            const double j0 = s_j0[lane].re, j1 = s_j1[lane].re;
-            sc.re = fabs(j0) >= fabs(j1) ? j0 / f0.re : j1 / f1.re;
+    if (warp == 0) {  // what the downward recurrence lacks
+        zd sc = mk(1.0, 0.0);
+        const zd j0 = s_j0[lane], j1 = s_j1[lane], f0 = v[0], f1 = v[N >= 1 ? CR_PAD : 0];
+        if (outer) {
+            if (!(x < 1e-15) && !upward) sc.re = fabs(j0.re) >= fabs(j1.re) ? j0.re / f0.re : j1.re / f1.re;
+        } else if (!centre) {
+            const bool first = zabs(j0) >= zabs(j1);
+            sc = (first ? j0 : j1) / (first ? f0 : f1);
         }
-    } else if (!centre) {
-        const zd j0 = s_j0[lane], j1 = s_j1[lane];
-        sc = zabs(j0) >= zabs(j1) ? j0 / f0 : j1 / f1;
+        s_sc[lane] = sc;
     }
+    __syncthreads();
+    if (!outer && !centre) Nv = s_nv[lane];
+    const zd sc = s_sc[lane];
+    float sum = 0.f;
     for (int l = warp; l < L; l += 4) {
         zd c;
         if (outer) {

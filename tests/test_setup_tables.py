@@ -46,3 +46,18 @@ def test_rows(s, fov, z):
                                         ([LARGE], 40, 1.5, 5)])
 def test_harmonics(s, fov, z, nk):
     check(s, nk, xy=(fov, z), lut_us=False, lut_uf=False)
+
+
+# scenes of eight spheres whose inner rows, those scaled by j_1, share blocks with other spheres' outer rows
+@pytest.mark.parametrize("seed", [16, 21, 23])
+def test_rows_of_many_spheres(seed):
+    p = abi.make_params(lam=3.0, condenser=(0, 0.5), objective=(0, 0.5), xy=(24, 0), resolution=96, padding=1,
+                        supersample=1)
+    s = scenes.random_spheres(8, 24.0, 0.8, 2.5, seed=seed * 1009 + 2, z_slab=0.0)
+    w = scenes.mc_waves(6, 0, 0.5, seed=seed)
+    U = oracle_lib.simulate(p, *abi.sphere_array(s), w)[0]
+    with Context(p) as ctx:
+        ctx.set_spheres(s)
+        ctx.set_waves(w)
+        ctx.simulate(BS_PREC_FP64)
+        assert rel(ctx.field(), U) <= 1e-10
