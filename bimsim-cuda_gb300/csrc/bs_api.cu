@@ -128,7 +128,7 @@ struct bs_ctx {
     DevBuf d_cnt;           // staged / total counters of the mixed LUT kernel
     DevBuf d_far;           // far fields Ud, Ufd on request (bs_get_far_field)
     DevBuf d_starts;        // row / coefficient offsets of a coefficient batch
-    DevBuf d_lbjobs, d_lbjobs2;  // Usp and Uip tables of a coefficient batch for the mixed LUT build
+    DevBuf d_lbjobs, d_lbjobs2;  // Usp and Uip tables of a coefficient batch for the LUT builds
     DevBuf d_kcmp;               // Kahan compensation of the mixed LUT sums between sphere chunks
     DevBuf d_part;               // mixed LUT sums of the spheres' shares (lut_splits)
     DevBuf d_fsave;         // U, Uf of a ring's first source (bs_simulate_ring_interp)
@@ -1068,9 +1068,9 @@ static bs_status run_nearfield(bs_ctx* c) {
                                        c->Lmax, sc.kmag, c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_tab.as<zd>(),
                                        fp64 ? nullptr : c->d_bias.as<float>(), c->st);
                 LAUNCHED(c);
-                // mixed path: the tables of every sphere of the batch in two launches (the
-                // dR-row Usp tables, then the shorter Uip tables)
-                for (int t = 0; t < 2 && !fp64; t++) {
+                // the tables of every sphere of the batch in two launches (the dR-row Usp tables,
+                // then the shorter Uip tables)
+                for (int t = 0; t < 2; t++) {
                     std::vector<LutBuildJob> jobs;
                     int max_rows = 0, max_theta = 1;
                     for (int i = b.b0; i < b.b1; i++) {
@@ -1080,7 +1080,7 @@ static bs_status run_nearfield(bs_ctx* c) {
                         j.tab_off = b.starts[(size_t)(b.b1 - b.b0) + 1 + (i - b.b0)] + (t ? (long long)S.dR * L : 0);
                         j.lin_off = t ? S.uip_off : S.usp_off;
                         j.row_off = b.starts[i - b.b0] + (t ? S.dR : 0);
-                        j.rows = t ? std::max(S.aR, 2) : S.dR;
+                        j.rows = t ? (fp64 ? S.aR : std::max(S.aR, 2)) : S.dR;
                         j.last = (t ? S.aR : S.dR) - 1;
                         j.L = L;
                         j.thetaR = S.thetaR;
@@ -1095,24 +1095,16 @@ static bs_status run_nearfield(bs_ctx* c) {
                     CK(cudaMemcpyAsync(jb.p, jobs.data(), jobs.size() * sizeof(LutBuildJob), cudaMemcpyHostToDevice,
                                        c->st));
                     for (size_t j0 = 0; j0 < jobs.size(); j0 += 65535) {  // the grid's z extent
-                        launch_lut_build_mixed(jb.as<LutBuildJob>() + j0,
-                                               (int)std::min<size_t>(65535, jobs.size() - j0), max_rows, max_theta,
-                                               c->d_tab.as<zd>(), c->d_bias.as<float>(), c->d_legP.as<float2>(),
-                                               thetaR, c->d_lut.as<float2>(), c->st);
+                        const int nj = (int)std::min<size_t>(65535, jobs.size() - j0);
+                        if (fp64)
+                            launch_lut_build(jb.as<LutBuildJob>() + j0, nj, max_rows, max_theta, c->d_tab.as<zd>(),
+                                             c->d_legP.as<double>(), c->legP_L, c->d_lut.as<Patch<double>>(), c->st);
+                        else
+                            launch_lut_build_mixed(jb.as<LutBuildJob>() + j0, nj, max_rows, max_theta,
+                                                   c->d_tab.as<zd>(), c->d_bias.as<float>(), c->d_legP.as<float2>(),
+                                                   thetaR, c->d_lut.as<float2>(), c->st);
                         LAUNCHED(c);
                     }
-                }
-                for (int i = b.b0; i < b.b1 && fp64; i++) {
-                    const Sphere& S = c->hs[i];
-                    const int L = S.Nl + 1;
-                    const zd* tab = c->d_tab.as<zd>() + b.starts[(size_t)(b.b1 - b.b0) + 1 + (i - b.b0)];
-                    Patch<double>* lut = c->d_lut.as<Patch<double>>();
-                    launch_lut_build<double>(tab, S.dR, L, c->d_legP.as<double>(), c->legP_L, S.thetaR,
-                                             lut + S.usp_off, c->st);
-                    LAUNCHED(c);
-                    launch_lut_build<double>(tab + (size_t)S.dR * L, S.aR, L, c->d_legP.as<double>(), c->legP_L,
-                                             S.thetaR, lut + S.uip_off, c->st);
-                    LAUNCHED(c);
                 }
             }
             if (first_build) {
@@ -1192,7 +1184,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
             maxrow = std::max(maxrow, cb.rows);
             maxstarts = std::max(maxstarts, (long long)cb.starts.size());
         }
-        b += B(pool) + B((size_t)maxcoef * sizeof(zd)) +
+        b += 2 * B(ns * sizeof(LutBuildJob)) + B(pool) + B((size_t)maxcoef * sizeof(zd)) +
              B((size_t)maxstarts * sizeof(long long));
         b += B(thetaR * (size_t)c->Lmax * sizeof(double));    // Legendre table
         if (fp64) b += B((ACOS_NODES + 1) * sizeof(AcosNode) + c->hs[0].thetaR * sizeof(double));

@@ -55,9 +55,6 @@ void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* s
 void launch_legendre_split(int thetaR, int Lmax, int stride, float2* P, cudaStream_t st);
 void launch_legendre_table(int thetaR, int Lmax, double* P, cudaStream_t st);
 template <class T>
-void launch_lut_build(const zd* tab, int rows, int L, const double* P, int Pstride, int thetaR, Patch<T>* out,
-                      cudaStream_t st);
-template <class T>
 void launch_phase(const Scene& sc, const Sphere* sph, const double* waves, cpx<T>* ph, float4* kw4, cudaStream_t st);
 // Nodes of the double-precision arc cosine at j pi / ACOS_NODES: the cosine c, the angle t in columns of a table of
 // thetaR angles, and d1 .. d4 of the column t + d1 y + d2 y^2 + d3 y^3 + d4 y^4 at the cosine c - y
@@ -99,6 +96,10 @@ struct LutBuildJob {
 // angles each) in one launch; tab holds SplitCoef entries
 void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab,
                             const float* bias, const float2* P, int Pstride, float2* lin, cudaStream_t st);
+
+// the same in double precision, as bilinear patches at out + lin_off
+void launch_lut_build(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab, const double* P,
+                      int Pstride, Patch<double>* out, cudaStream_t st);
 
 // Direct scattered field through the addition theorem of spherical harmonics:
 // recurrence factors rec (L(L+1)/2), per-wave tables tab (nk x L(L+1)/2, then the ns x nk
