@@ -93,10 +93,10 @@ class ClockSampler:
 
 
 def profile_record():
-    """Per-launch DRAM bytes and shared-memory wavefronts of the dominant kernel, from the ncu
-    capture recorded in profiles/us_lut_tex_config2.json (written beside its summary)."""
+    """DRAM bytes and shared-memory wavefronts of the dominant kernel's launches of one slice, from the ncu
+    capture recorded in profiles/us_lut_sorted_config2.json (written beside its summary)."""
     try:
-        return json.load(open(os.path.join(REPO, "profiles", "us_lut_tex_config2.json")))
+        return json.load(open(os.path.join(REPO, "profiles", "us_lut_sorted_config2.json")))
     except (OSError, ValueError):
         return {}
 
@@ -540,37 +540,36 @@ def run_gb300(args):
                    "parallelism": f"replicas x{ws}"},
         "e2e": {"value": e2e_value, "unit": "pixels/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "gpu_launches": launches,
-        "roofline": {"bound": "fp32", "kernel": "us_lut_tex_kernel", "achieved": achieved,
+        "roofline": {"bound": "fp32", "kernel": "us_lut_sorted_kernel", "achieved": achieved,
                      "peak": fp32_tf, "unit": "TFLOP/s", "frac": achieved / fp32_tf,
                      "traffic": profile_traffic(),
                      "peak_source": "measured FP32 FMA loop on this GPU (bs_measure_fma_peak)",
-                     "work": f"{FLOP_PER_LOOKUP} flop x {lookups} (pixel, sphere, wave) lookups per launch",
+                     "work": f"{FLOP_PER_LOOKUP} flop x {lookups} (pixel, sphere, wave) lookups per slice (one launch per range of spheres)",
                      "launch_ms": us_s * 1e3, "lookups_per_s": lookups / us_s,
                      "staged_fraction": staged, "wave_chunk": wave_chunk,
                      "hbm_peak_gbs": peaks.get("hbm_gbs"), "fp64_peak_tflops": fp64_tf,
                      "why_not_hbm_or_tensor": "no step is a dense contraction (no tensor-core use) and the kernel "
-                                              "reads ~0.14 TB/s of DRAM: it is bound by the shared-memory (L1TEX) "
-                                              "pipe feeding its FP32 arithmetic, so the roofline is the measured "
-                                              "FP32 FMA peak; the DRAM view is roofline_hbm, the shared-memory "
-                                              "pipe roofline_l1"},
+                                              "reads ~0.013 TB/s of DRAM: it is bound by instruction issue, half of "
+                                              "it FP32 arithmetic, so the roofline is the measured FP32 FMA peak; "
+                                              "the DRAM view is roofline_hbm, the shared-memory pipe roofline_l1"},
         "roofline_hbm": (None if not (profile_traffic() and peaks.get("hbm_gbs")) else
-                         {"bound": "hbm", "kernel": "us_lut_tex_kernel", "unit": "GB/s",
+                         {"bound": "hbm", "kernel": "us_lut_sorted_kernel", "unit": "GB/s",
                           "achieved": profile_traffic() / us_s / 1e9, "peak": peaks["hbm_gbs"],
                           "frac": profile_traffic() / us_s / 1e9 / peaks["hbm_gbs"],
                           "traffic": profile_traffic(), "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)",
-                          "note": "DRAM bytes of one full launch (ncu, profiles/us_lut_tex_config2.json) over this "
-                                  "run's launch time"}),
+                          "note": "DRAM bytes of one slice (ncu, profiles/us_lut_sorted_config2.json) over this "
+                                  "run's time of the kernel"}),
         # the shared-memory (L1TEX data) pipe retires one 128-byte wavefront per SM per cycle
         "roofline_l1": (None if not (profile_wavefronts() and not args.small and clocks.get("sm_mhz")) else
-                        {"bound": "shared-memory wavefronts", "kernel": "us_lut_tex_kernel",
+                        {"bound": "shared-memory wavefronts", "kernel": "us_lut_sorted_kernel",
                          "unit": "wavefronts per SM per cycle",
                          "achieved": profile_wavefronts() / (us_s * clocks["sm_mhz"] * 1e6 * n_sm),
                          "peak": 1.0,
                          "frac": profile_wavefronts() / (us_s * clocks["sm_mhz"] * 1e6 * n_sm),
                          "wavefronts": profile_wavefronts(),
                          "wavefronts_per_warp_lookup": profile_wavefronts() / (lookups / 32),
-                         "note": "shared wavefronts of one full launch (ncu, profiles/us_lut_tex_config2.json) "
-                                 "over this run's launch time at the sampled SM clock"}),
+                         "note": "shared wavefronts of one slice (ncu, profiles/us_lut_sorted_config2.json) "
+                                 "over this run's time of the kernel at the sampled SM clock"}),
         "mixed_vs_fp64_rel_l2": {"value": rel, "absorbance": rel_a, "tolerance": 1e-5, "case": case},
         "mixed_vs_oracle_rows_rel_l2": vs_oracle,
         "fp64_plain": fp64,
