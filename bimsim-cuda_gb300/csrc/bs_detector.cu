@@ -33,15 +33,14 @@ __global__ void twiddle_kernel(int ni, int nj, const int* __restrict__ freq, int
 }
 
 // Tiled complex GEMM: tile GM x GN, K tiles of 16, accumulation split into per-tile
-// partial sums combined with Kahan compensation.  Partial sums of 16 products, of 4 for single-precision transforms
-// of at most GEMM_SHORT rows, columns and products: a sum of three or four partial sums of 16 averages little out, and
-// the absorbance of a 48^2 near field comes 15 % closer to double precision (mean of 8 seeds); a 303^2 one would go
-// 57 % further off.
+// partial sums of 16 products combined with Kahan compensation, at every size and in both precisions: the
+// absorbance of a slice with little contrast is the difference of two such transforms, so a rule that changed the
+// partial sums with the size would change that image by more than its own rounding.
 // Single precision: 16 x 16 threads of 4 x 2 outputs, 64 x 32.  Double precision is bound by the FP64 pipe (four multiply-adds
 // per product) and, on the inverse transforms' few output tiles, by one SM's share of it:
 // 8 x 16 threads (a warp for each quarter of the pipe) of 2 x 1 outputs, 32 x 8.  96 x 25 and
 // 96 x 96 outputs, K = 25, two fields: 44 and 46 us in tiles of 64 x 16, 17 and 17 us now.
-constexpr int GB_K = 16, GEMM_SHORT = 64;
+constexpr int GB_K = 16;
 template <class T>
 __host__ __device__ constexpr int gb_tx() { return sizeof(T) == 8 ? 8 : 16; }  // 16 threads along M
 template <class T>
@@ -93,7 +92,7 @@ __device__ __forceinline__ void cgemm_store(int epi, long long o, int gm, int gn
 // ksplit > 1 (few output tiles, long K): block z = b * ksplit + ks sums the
 // ks-th of ksplit equal K ranges into part[b][ks][M][N]; cgemm_reduce_kernel
 // adds the ranges in order (deterministic) and applies the epilogue.
-template <class T, int KP>  // KP: products between Kahan steps
+template <class T>
 __global__ void __launch_bounds__(16 * gb_tx<T>()) cgemm_kernel(int M, int N, int K, const cpx<T>* __restrict__ A, int lda,
                                                     long long sA, const cpx<T>* __restrict__ B, int ldb, long long sB,
                                                     cpx<T>* __restrict__ C, int ldc, long long sC, int epi,
@@ -128,32 +127,29 @@ __global__ void __launch_bounds__(16 * gb_tx<T>()) cgemm_kernel(int M, int N, in
         }
         __syncthreads();
 #pragma unroll
-        for (int k1 = 0; k1 < GB_K; k1 += KP) {
+        for (int kk = 0; kk < GB_K; kk++) {
+            cpx<T> a[NI], bb[NJ];
 #pragma unroll
-            for (int kk = k1; kk < k1 + KP; kk++) {
-                cpx<T> a[NI], bb[NJ];
+            for (int i = 0; i < NI; i++) a[i] = As[kk][ty + 16 * i];
 #pragma unroll
-                for (int i = 0; i < NI; i++) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-                for (int j = 0; j < NJ; j++) bb[j] = Bs[kk][tx + NT * j];
-#pragma unroll
-                for (int i = 0; i < NI; i++)
-#pragma unroll
-                    for (int j = 0; j < NJ; j++) cmac(a[i], bb[j], p0[i][j], p1[i][j], p2[i][j], p3[i][j]);
-            }
+            for (int j = 0; j < NJ; j++) bb[j] = Bs[kk][tx + NT * j];
 #pragma unroll
             for (int i = 0; i < NI; i++)
 #pragma unroll
-                for (int j = 0; j < NJ; j++) {  // Kahan step
-                    T yr = (p0[i][j] - p1[i][j]) - cr[i][j], yi = (p2[i][j] + p3[i][j]) - ci[i][j];
-                    T trr = accr[i][j] + yr, tii = acci[i][j] + yi;
-                    cr[i][j] = (trr - accr[i][j]) - yr;
-                    ci[i][j] = (tii - acci[i][j]) - yi;
-                    accr[i][j] = trr;
-                    acci[i][j] = tii;
-                    p0[i][j] = p1[i][j] = p2[i][j] = p3[i][j] = 0;
-                }
+                for (int j = 0; j < NJ; j++) cmac(a[i], bb[j], p0[i][j], p1[i][j], p2[i][j], p3[i][j]);
         }
+#pragma unroll
+        for (int i = 0; i < NI; i++)
+#pragma unroll
+            for (int j = 0; j < NJ; j++) {  // Kahan step
+                T yr = (p0[i][j] - p1[i][j]) - cr[i][j], yi = (p2[i][j] + p3[i][j]) - ci[i][j];
+                T trr = accr[i][j] + yr, tii = acci[i][j] + yi;
+                cr[i][j] = (trr - accr[i][j]) - yr;
+                ci[i][j] = (tii - acci[i][j]) - yi;
+                accr[i][j] = trr;
+                acci[i][j] = tii;
+                p0[i][j] = p1[i][j] = p2[i][j] = p3[i][j] = 0;
+            }
         __syncthreads();
     }
 #pragma unroll
@@ -383,12 +379,8 @@ void launch_cgemm(int M, int N, int K, int batch, const cpx<T>* A, int lda, long
     int ks = cgemm_ksplit<T>(M, N, K, batch);
     if ((size_t)batch * ks * M * N > scratch_elems || !scratch) ks = 1;
     dim3 grid((N + gb_n<T>() - 1) / gb_n<T>(), (M + gb_m<T>() - 1) / gb_m<T>(), batch * ks);
-    if (sizeof(T) == 4 && std::max({M, N, K}) <= GEMM_SHORT)
-        cgemm_kernel<T, 4><<<grid, 16 * gb_tx<T>(), 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, epi, mask, scale, I,
-                                                            ks, scratch);
-    else
-        cgemm_kernel<T, GB_K><<<grid, 16 * gb_tx<T>(), 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, epi, mask,
-                                                               scale, I, ks, scratch);
+    cgemm_kernel<T><<<grid, 16 * gb_tx<T>(), 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, epi, mask, scale, I,
+                                                      ks, scratch);
     if (ks > 1) {
         const long long n = (long long)batch * M * N;
         cgemm_reduce_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(M, N, batch, ks, scratch, C, ldc, sC, epi,
@@ -600,8 +592,7 @@ template <class T>
 static void preload_detector_t() {
     cudaFuncAttributes a;
     cudaFuncGetAttributes(&a, twiddle_kernel<T>);
-    cudaFuncGetAttributes(&a, cgemm_kernel<T, 4>);
-    cudaFuncGetAttributes(&a, cgemm_kernel<T, GB_K>);
+    cudaFuncGetAttributes(&a, cgemm_kernel<T>);
     cudaFuncGetAttributes(&a, cgemm_reduce_kernel<T>);
     cudaFuncGetAttributes(&a, bin_kernel<T>);
     cudaFuncGetAttributes(&a, image_kernel<T>);
