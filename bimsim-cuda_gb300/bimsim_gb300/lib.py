@@ -228,7 +228,7 @@ class Context:
         self.params = params
 
     def set_lut_staging(self, mode):
-        """0, 1: windows in shared memory where they fit; 2: every cell from the tables (same results)."""
+        """0 chosen by the library, 1: windows in shared memory where they fit, 2: every cell from the tables (same results)."""
         self._check(self.lib.bs_set_lut_staging(self.h, mode))
 
     def set_backpropagation(self, enable, d=0.0):
@@ -236,7 +236,7 @@ class Context:
         self._check(self.lib.bs_set_backpropagation(self.h, int(bool(enable)), float(d)))
 
     def set_lut_wave_chunk(self, chunk):
-        """Waves per counted chunk of the mixed LUT kernel: 0 is 64, else 16, 32 or 64."""
+        """Waves per chunk of the mixed LUT kernels: 0 chooses per run, else 16, 32 or 64."""
         self._check(self.lib.bs_set_lut_wave_chunk(self.h, chunk))
 
     def set_lut_reuse(self, enable):

@@ -125,7 +125,8 @@ struct bs_ctx {
     bool have = false;
 
     DevBuf d_sph, d_waves, d_kw4, d_ph, d_A, d_B, d_tab, d_legP, d_lut, d_uft, d_uftscr;
-    DevBuf d_cnt;           // staged / total counters of the mixed LUT kernel
+    DevBuf d_cnt;           // staged / total counters of the mixed LUT kernels
+    DevBuf d_cones;         // bounding cones of the plain mixed LUT kernel's wave chunks
     DevBuf d_far;           // far fields Ud, Ufd on request (bs_get_far_field)
     DevBuf d_starts;        // row / coefficient offsets of a coefficient batch
     DevBuf d_lbjobs, d_lbjobs2;  // Usp and Uip tables of a coefficient batch for the LUT builds
@@ -166,7 +167,7 @@ static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
     return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_tab,
             &c->d_bias, &c->d_acos, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
             &c->d_sv, &c->d_mask, &c->d_wx, &c->d_wy, &c->d_wix, &c->d_wiy, &c->d_f1, &c->d_f2,
-            &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_far,
+            &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_cones, &c->d_far,
             &c->d_starts, &c->d_lbjobs, &c->d_lbjobs2, &c->d_kcmp, &c->d_part, &c->d_fsave, &c->d_dacc, &c->d_line, &c->d_ringcs, &c->d_bp, &c->d_shrec, &c->d_shtab, &c->d_shcoef, &c->d_gscr, &c->d_ufw};
 }
 
@@ -203,6 +204,7 @@ static void preload_kernels(int device) {
     if (std::find(done.begin(), done.end(), device) != done.end()) return;
     preload_nearfield_kernels();
     preload_uslut_kernels();
+    preload_uslut_plain_kernels();
     preload_detector_kernels();
     cudaGetLastError();  // a kernel this device cannot load reports at its launch instead
     done.push_back(device);
@@ -781,7 +783,7 @@ static float4 wave_cone(const std::vector<double>& w) {
                        (float)std::min(2.9, std::acos(std::max(-1.0, c))));
 }
 
-// Predicted fraction of the mixed LUT kernel's (tile, sphere, chunk) units whose columns fit
+// Predicted fraction of the sorted mixed LUT kernel's (tile, sphere, chunk) units whose columns fit
 // its window, from the kernel's own bounds on a sample of tiles and spheres: the tile's angular
 // radius seen from the sphere (its corners) and an even share of the angles between the
 // sampled directions and the tile centre's direction for each group of 32.
@@ -789,7 +791,6 @@ static double predict_staged_fraction(const bs_ctx* c, const std::vector<double>
     const Scene& sc = c->sc;
     const int R = sc.R, tiles = (R + LUT_TILE - 1) / LUT_TILE, ns = sc.ns;
     const int nk = (int)(w.size() / 3), groups = (std::min(nk, 1024) + 31) / 32;
-    if (nk <= LUT_FEW_WAVES) return 0.0;
     const int ts = std::max(1, tiles / 8), ss = std::max(1, ns / 4), ws = std::max(1, nk / 48);
     long long staged = 0, total = 0;
     for (int ty = 0; ty < tiles; ty += ts)
@@ -824,6 +825,154 @@ static double predict_staged_fraction(const bs_ctx* c, const std::vector<double>
                 if (gam <= 1.4 && (range / groups + 2 * gam) * tsc + 4.5 <= LUT_WINDOW) staged++;
             }
     return total ? (double)staged / (double)total : 0.0;
+}
+
+// Bounding cone (unit axis, half-angle in radians) of every `chunk`
+// consecutive waves, with a small margin for single-precision rounding.  A
+// chunk holding a direction that is not a unit vector gets half-angle pi,
+// which turns the angular window off for it.
+static std::vector<float4> wave_cones(const std::vector<double>& w, int chunk) {
+    size_t nk = w.size() / 3;
+    size_t nch = (nk + chunk - 1) / chunk;
+    std::vector<float4> out(nch);
+    for (size_t ch = 0; ch < nch; ch++) {
+        size_t a = ch * chunk, b = std::min(nk, a + chunk);
+        double m[3] = {0, 0, 0};
+        bool unit = true;
+        for (size_t i = a; i < b; i++) {
+            const double* k = &w[3 * i];
+            double kl = std::sqrt(k[0] * k[0] + k[1] * k[1] + k[2] * k[2]);
+            if (!(std::fabs(kl - 1.0) <= 1e-6)) unit = false;
+            for (int c = 0; c < 3; c++) m[c] += k[c];
+        }
+        double ml = std::sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+        double beta = 0;
+        if (ml > 1e-3 && unit) {
+            for (int c = 0; c < 3; c++) m[c] /= ml;
+            for (size_t i = a; i < b; i++) {
+                const double* k = &w[3 * i];
+                double cth = k[0] * m[0] + k[1] * m[1] + k[2] * m[2];
+                beta = std::max(beta, std::acos(std::min(1.0, std::max(-1.0, cth))));
+            }
+        } else {
+            m[0] = 0, m[1] = 0, m[2] = 1;
+            beta = TRUE_PI;
+        }
+        out[ch] = make_float4((float)m[0], (float)m[1], (float)m[2], (float)(beta + 1e-4));
+    }
+    return out;
+}
+
+// Predicted fraction of (tile, sphere, wave chunk) units whose table window the plain mixed LUT kernel can hold in
+// shared memory, from the kernel's own bounds evaluated on a sample of tiles, spheres and chunks: the tile's
+// distance range (nearest point of the tile rectangle, farthest corner) gives the rows, the corners' angles from
+// the tile-centre direction give gamma.  Below staged_min_fraction the kernel without windows is faster: reads
+// that do not fit one run with the L1 that the staged kernel's shared memory leaves.
+static double staged_min_fraction(int chunk) { return chunk >= WAVE_CHUNK_MAX ? 0.3 : 0.7; }
+static double plain_staged_fraction(const bs_ctx* c, const std::vector<float4>& cones, int s0, int s1, int chunk) {
+    const int cap = lut_plain_entries(chunk);
+    const Scene& sc = c->sc;
+    const int R = sc.R, tiles = (R + LUT_TILE - 1) / LUT_TILE;
+    const int ts = std::max(1, tiles / 16), ss = std::max(1, (s1 - s0) / 32);
+    const int cs = std::max(1, (int)cones.size() / 16);
+    auto pos = [&](double u, double v, double* q) {
+        for (int k = 0; k < 3; k++) q[k] = sc.A[k] + sc.X[k] * (u / R) + sc.Y[k] * (v / R);
+    };
+    const double X2 = sc.X[0] * sc.X[0] + sc.X[1] * sc.X[1] + sc.X[2] * sc.X[2];
+    const double Y2 = sc.Y[0] * sc.Y[0] + sc.Y[1] * sc.Y[1] + sc.Y[2] * sc.Y[2];
+    long long staged = 0, total = 0;
+    for (int ty = 0; ty < tiles; ty += ts)
+        for (int tx = 0; tx < tiles; tx += ts) {
+            const double u0 = tx * LUT_TILE, v0 = ty * LUT_TILE;
+            const double u1 = std::min(u0 + LUT_TILE - 1, (double)R - 1), v1 = std::min(v0 + LUT_TILE - 1, (double)R - 1);
+            for (int si = s0; si < s1; si += ss) {
+                const Sphere& S = c->hs[si];
+                double e[3];
+                for (int k = 0; k < 3; k++) e[k] = S.p[k] - sc.A[k];
+                // nearest point of the tile rectangle (X and Y span the plane at right angles)
+                const double un = std::min(std::max((e[0] * sc.X[0] + e[1] * sc.X[1] + e[2] * sc.X[2]) / X2 * R, u0), u1);
+                const double vn = std::min(std::max((e[0] * sc.Y[0] + e[1] * sc.Y[1] + e[2] * sc.Y[2]) / Y2 * R, v0), v1);
+                double q[3], ctr[3];
+                pos(un, vn, q);
+                const double dmin = std::sqrt((q[0] - S.p[0]) * (q[0] - S.p[0]) + (q[1] - S.p[1]) * (q[1] - S.p[1]) +
+                                              (q[2] - S.p[2]) * (q[2] - S.p[2]));
+                const int nch = (int)((cones.size() + cs - 1) / cs);
+                total += nch;
+                if (!(dmin >= S.a) || dmin == 0) continue;
+                pos(u0 + 7.5, v0 + 7.5, ctr);
+                double cl = 0;
+                for (int k = 0; k < 3; k++) {
+                    ctr[k] -= S.p[k];
+                    cl += ctr[k] * ctr[k];
+                }
+                cl = std::sqrt(cl);
+                double dmax = 0, gam = 0;
+                const double cu[4] = {u0, u1, u0, u1}, cv[4] = {v0, v0, v1, v1};
+                for (int k = 0; k < 4; k++) {
+                    pos(cu[k], cv[k], q);
+                    double r[3] = {q[0] - S.p[0], q[1] - S.p[1], q[2] - S.p[2]};
+                    const double d = std::sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+                    dmax = std::max(dmax, d);
+                    const double cosg = (r[0] * ctr[0] + r[1] * ctr[1] + r[2] * ctr[2]) / (d * cl);
+                    gam = std::max(gam, std::acos(std::min(1.0, std::max(-1.0, cosg))));
+                }
+                gam += LUT_PLAIN_MARGIN;
+                auto row = [&](double d) {
+                    double x = (d - S.r0) / (S.dmax - S.r0) * (S.dR - 1);
+                    return (int)std::floor(std::min(std::max(x, 0.0), (double)(S.dR - 1)));
+                };
+                const int rlo = row(dmin), nrows = std::min(row(dmax) + 1, S.dR - 1) - rlo + 1;
+                const double tsc = (S.thetaR - 1) / PI_REF;
+                for (size_t ch = 0; ch < cones.size(); ch += cs) {
+                    const float4 k = cones[ch];
+                    const double thc =
+                        std::acos(std::min(1.0, std::max(-1.0, (k.x * ctr[0] + k.y * ctr[1] + k.z * ctr[2]) / cl)));
+                    const int t_lo = std::max(0, (int)std::floor((thc - k.w - gam) * tsc) - 1);
+                    const int t_hi = std::min(S.thetaR, (int)std::floor((thc + k.w + gam) * tsc) + 2);
+                    const int W = t_hi - t_lo + 1;
+                    if (W >= 2 && (long long)nrows * lut_plain_stride(W) <= cap) staged++;
+                }
+            }
+        }
+    return total ? (double)staged / (double)total : 0.0;
+}
+
+// Waves per chunk of the plain mixed LUT kernel, with the matching wave order and cones: the largest of 64, 32 and
+// 16 whose predicted staged fraction reaches 0.8, else the one with the largest fraction if that reaches its
+// staged_min_fraction, else the largest fraction among those that reach theirs, else 64.  Smaller chunks have
+// narrower cones, so more windows fit, but each chunk pays a window copy, two barriers and a Kahan step.  The
+// chunk and the order of the waves in it decide the last bits of the sums, so bs_set_lut_staging has no say here;
+// bs_set_lut_wave_chunk fixes the chunk instead.
+struct ChunkPlan {
+    int chunk = WAVE_CHUNK_MAX;
+    std::vector<double> w;
+    std::vector<float4> cones;
+    double predicted = 0;
+};
+
+static ChunkPlan chunk_plan(const bs_ctx* c, const std::vector<double>& waves, int chunk) {
+    ChunkPlan cp;
+    cp.chunk = chunk;
+    cp.w = waves;
+    if (!c->prm.plane_wave) sort_waves(cp.w, chunk);
+    cp.cones = wave_cones(cp.w, chunk);
+    cp.predicted = plain_staged_fraction(c, cp.cones, 0, c->sc.ns, chunk);
+    return cp;
+}
+
+static ChunkPlan choose_chunk(const bs_ctx* c, const std::vector<double>& waves) {
+    if (c->lut_chunk) return chunk_plan(c, waves, c->lut_chunk);
+    ChunkPlan first = chunk_plan(c, waves, WAVE_CHUNK_MAX), best = first, viable;
+    if (c->prm.plane_wave) return first;
+    viable.predicted = best.predicted >= staged_min_fraction(best.chunk) ? best.predicted : -1;
+    if (viable.predicted >= 0) viable = best;  // the best that the staged kernel would run to advantage
+    for (int cand = WAVE_CHUNK_MAX / 2; cand >= WAVE_CHUNK_MAX / 4 && best.predicted < 0.8; cand /= 2) {
+        ChunkPlan cp = chunk_plan(c, waves, cand);
+        if (cp.predicted >= staged_min_fraction(cand) && cp.predicted > viable.predicted) viable = cp;
+        if (cp.predicted > best.predicted || cp.predicted >= 0.8) best = std::move(cp);
+    }
+    if (best.predicted >= staged_min_fraction(best.chunk)) return best;
+    return viable.predicted >= 0 ? viable : first;
 }
 
 // ---------------------------------------------------------------------------
@@ -868,14 +1017,29 @@ static bs_status run_nearfield(bs_ctx* c) {
     // upload spheres and waves
     CK(c->d_sph.ensure(std::max(1, ns) * sizeof(Sphere)));
     std::vector<double> w(c->waves);
-    const int chunk = c->lut_chunk ? c->lut_chunk : WAVE_CHUNK_MAX;
+    int chunk = c->lut_chunk ? c->lut_chunk : WAVE_CHUNK_MAX;
     const bool mixed_lut = !fp64 && p.scalar && p.lut_us && ns > 0;
+    const bool plain = mixed_lut && lut_plain(ns), few = mixed_lut && lut_few(ns, nk);
+    const bool split = mixed_lut && !plain;  // tables of the split single-precision build
     float4 cone = make_float4(0.f, 0.f, 1.f, (float)TRUE_PI);
+    std::vector<float4> cones;
+    double predicted = 0;
     if (p.plane_wave) w.assign(p.k_dir, p.k_dir + 3);
-    if (mixed_lut) cone = wave_cone(w);  // ordered per tile on the device
-    else if (!p.plane_wave) sort_waves(w, WAVE_CHUNK_MAX);
-    const bool unit = cone.w < 3.f;  // the mixed LUT kernel's angle bounds hold
-    c->stats.lut_wave_chunk = chunk;
+    if (plain) {
+        ChunkPlan cp = choose_chunk(c, w);
+        chunk = cp.chunk;
+        w.swap(cp.w);
+        cones.swap(cp.cones);
+        predicted = cp.predicted;
+    } else if (split) {
+        cone = wave_cone(w);  // ordered per tile on the device
+    } else if (!p.plane_wave) {
+        sort_waves(w, WAVE_CHUNK_MAX);
+    }
+    const bool unit = cone.w < 3.f;  // the sorted LUT kernel's angle bounds hold
+    // waves per counted chunk; without windows the chunks are counted in 64s
+    const int counted_chunk = !c->lut_chunk && c->lut_staging == 2 ? WAVE_CHUNK_MAX : chunk;
+    c->stats.lut_wave_chunk = counted_chunk;
     CK(c->d_waves.ensure(w.size() * sizeof(double)));
     CK(cudaMemcpyAsync(c->d_waves.p, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
 
@@ -1003,19 +1167,19 @@ static bs_status run_nearfield(bs_ctx* c) {
             }
             CK(c->d_tab.ensure((size_t)maxcoef * sizeof(zd)));
             CK(c->d_starts.ensure((size_t)maxstarts * sizeof(long long)));
-            if (!fp64) CK(c->d_bias.ensure((size_t)maxrow * sizeof(float)));
+            if (split) CK(c->d_bias.ensure((size_t)maxrow * sizeof(float)));
             if (fp64 && c->acos_theta != thetaR) {
                 CK(c->d_acos.ensure((ACOS_NODES + 1) * sizeof(AcosNode) + thetaR * sizeof(double)));
                 launch_acos_nodes(thetaR, c->d_acos.as<AcosNode>(), c->st);
                 LAUNCHED(c);
                 c->acos_theta = thetaR;
             }
-            if (c->legP_theta != thetaR || c->legP_L < c->Lmax || c->legP_split != !fp64) {
+            if (c->legP_theta != thetaR || c->legP_L < c->Lmax || c->legP_split != split) {
                 CK(c->d_legP.ensure((size_t)thetaR * c->Lmax * sizeof(double)));
-                if (fp64) launch_legendre_table(thetaR, c->Lmax, c->d_legP.as<double>(), c->st);
+                if (!split) launch_legendre_table(thetaR, c->Lmax, c->d_legP.as<double>(), c->st);
                 else launch_legendre_split(thetaR, c->Lmax, thetaR, c->d_legP.as<float2>(), c->st);
                 LAUNCHED(c);
-                c->legP_split = !fp64;
+                c->legP_split = split;
                 c->legP_theta = thetaR;
                 c->legP_L = c->Lmax;
             }
@@ -1030,7 +1194,7 @@ static bs_status run_nearfield(bs_ctx* c) {
         // tables of the previous run still in the pool?
         std::vector<double> key;
         if (c->reuse && nchunks == 1) {
-            key = {fp64 ? 1.0 : 0.0, sc.kmag, (double)c->Lmax, (double)ns};
+            key = {fp64 ? 1.0 : plain ? 2.0 : 0.0, sc.kmag, (double)c->Lmax, (double)ns};
             for (const Sphere& S : c->hs) {
                 const double v[] = {S.p[0], S.p[1], S.p[2], S.a, S.n_re, S.n_im, S.dmin, S.dmax, S.r0,
                                     (double)S.Nl, (double)S.aR, (double)S.dR, (double)S.thetaR,
@@ -1052,8 +1216,16 @@ static bs_status run_nearfield(bs_ctx* c) {
                                 "mixed precision: a %d x %d lookup table exceeds the %d x %d texture limit of this GPU "
                                 "(use BS_PREC_FP64 or fewer table samples)",
                                 std::max(S.dR, S.aR), S.thetaR, maxh - 1, maxw);
-            c->stats.lut_staged_predicted = unit ? predict_staged_fraction(c, w) : 0.0;
-            use_stage = unit && c->lut_staging != 2;
+            if (plain) {
+                use_stage = c->lut_staging == 1 || (c->lut_staging == 0 && predicted >= staged_min_fraction(chunk));
+                CK(c->d_cones.ensure(cones.size() * sizeof(float4)));
+                CK(cudaMemcpyAsync(c->d_cones.p, cones.data(), cones.size() * sizeof(float4), cudaMemcpyHostToDevice,
+                                   c->st));
+            } else if (!few) {
+                predicted = unit ? predict_staged_fraction(c, w) : 0.0;
+                use_stage = unit && c->lut_staging != 2;
+            }
+            c->stats.lut_staged_predicted = predicted;
             CK(c->d_cnt.ensure(2 * sizeof(unsigned long long)));
             CK(cudaMemsetAsync(c->d_cnt.p, 0, 2 * sizeof(unsigned long long), c->st));
         }
@@ -1066,7 +1238,7 @@ static bs_status run_nearfield(bs_ctx* c) {
                                    cudaMemcpyHostToDevice, c->st));
                 launch_coef_rows_batch(c->d_sph.as<Sphere>(), b.b0, b.b1 - b.b0, c->d_starts.as<long long>(), b.rows,
                                        c->Lmax, sc.kmag, c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_tab.as<zd>(),
-                                       fp64 ? nullptr : c->d_bias.as<float>(), c->st);
+                                       split ? c->d_bias.as<float>() : nullptr, c->st);
                 LAUNCHED(c);
                 // the tables of every sphere of the batch in two launches (the dR-row Usp tables,
                 // then the shorter Uip tables)
@@ -1099,6 +1271,10 @@ static bs_status run_nearfield(bs_ctx* c) {
                         if (fp64)
                             launch_lut_build(jb.as<LutBuildJob>() + j0, nj, max_rows, max_theta, c->d_tab.as<zd>(),
                                              c->d_legP.as<double>(), c->legP_L, c->d_lut.as<Patch<double>>(), c->st);
+                        else if (plain)
+                            launch_lut_build_plain(jb.as<LutBuildJob>() + j0, nj, max_rows, max_theta,
+                                                   c->d_tab.as<zd>(), c->d_legP.as<double>(), c->legP_L,
+                                                   c->d_lut.as<float2>(), c->st);
                         else
                             launch_lut_build_mixed(jb.as<LutBuildJob>() + j0, nj, max_rows, max_theta,
                                                    c->d_tab.as<zd>(), c->d_bias.as<float>(), c->d_legP.as<float2>(),
@@ -1117,6 +1293,11 @@ static bs_status run_nearfield(bs_ctx* c) {
                 launch_us_lut_f64(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_waves.as<double>(),
                                   c->d_acos.as<AcosNode>(), c->d_ph.as<zd>(), c->d_lut.as<Patch<double>>(),
                                   (const zd*)Uf, (zd*)U, c->st);
+            } else if (plain || few) {
+                launch_us_lut_plain(sc, c->d_sph.as<Sphere>(), s0, s1, ci > 0, finalize, c->d_kw4.as<float4>(),
+                                    c->d_cones.as<float4>(), c->d_ph.as<cpx<float>>(), c->d_lut.as<float2>(),
+                                    (const cpx<float>*)Uf, (cpx<float>*)U, c->d_cnt.as<unsigned long long>(),
+                                    carry ? c->d_kcmp.as<float2>() : nullptr, use_stage, chunk, counted_chunk, c->st);
             } else {
                 for (int q = 0; q < ranges; q++) {
                     const int r0 = s0 + (int)((long long)(s1 - s0) * q / ranges);
@@ -1189,7 +1370,8 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
         b += B(thetaR * (size_t)c->Lmax * sizeof(double));    // Legendre table
         if (fp64) b += B((ACOS_NODES + 1) * sizeof(AcosNode) + c->hs[0].thetaR * sizeof(double));
         if (!fp64) {
-            b += B((size_t)maxrow * sizeof(float));  // biases
+            if (lut_plain((int)ns)) b += B((nk + 15) / 16 * sizeof(float4));  // cones
+            else b += B((size_t)maxrow * sizeof(float));                      // biases
             const int shares = lut_splits((int)R, (int)ns, (int)nk);
             if (shares > 1) b += B((size_t)shares * 4 * R * R * sizeof(float));
             else if (cs.size() > 2 || lut_ranges((int)R, (int)ns, (int)nk, pool) > 1)

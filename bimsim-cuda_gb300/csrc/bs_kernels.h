@@ -9,14 +9,29 @@
 
 namespace bs {
 
-// Mixed LUT kernel: angle margin (radians) of its window bounds, and the number of
-// directions up to which one thread per pixel reads every cell itself.
+// Mixed LUT kernels: angle margins (radians) of the sorted and of the plain kernel's window bounds.
 constexpr float LUT_STAGE_MARGIN = 5e-4f;
+constexpr float LUT_PLAIN_MARGIN = 2e-3f;
 constexpr int GB300_SMS = 152;
-constexpr int LUT_FEW_WAVES = 32;
 constexpr int LUT_TILE = 16;
 constexpr int LUT_WINDOW = 256;  // table columns of the widest staged window
 constexpr int WAVE_CHUNK_MAX = 64;
+// Slices whose mixed scattered field the plain kernel sums (bs_uslut_plain.cu), from tables summed in double
+// precision, with the directions' order and chunks.  The absorbance of a slice with little contrast is a small
+// difference of two float images, and hangs on the order of the sums: with the sorted kernel's, over lanes, it moves
+// by more than 2e-5 in 17 of 782 drawn slices, all of at most 4 spheres (699 slices of more than 8: by 1.6e-5 at
+// most).  768^2 pixels, one sphere, 400 directions: 1.08 ms sorted, 1.73 ms plain.
+constexpr int LUT_PLAIN_SPHERES = 8;
+inline bool lut_plain(int ns) { return ns <= LUT_PLAIN_SPHERES; }
+// More spheres with few directions: the plain kernel too, without windows and from the sorted kernel's tables.
+constexpr int LUT_FEW_WAVES = 32;
+inline bool lut_few(int ns, int nk) { return !lut_plain(ns) && nk <= LUT_FEW_WAVES; }
+// Float2 values of the plain kernel's staged windows: 51 KB with 64-wave chunks (4 blocks per SM), 72 KB (3) with
+// smaller ones.
+__host__ __device__ constexpr int lut_plain_entries(int chunk) { return chunk >= 64 ? 6400 : 9000; }
+// Shared-memory row stride of such a window W entries wide: odd, so that lanes reading the same column of different
+// rows fall in different banks.
+__host__ __device__ constexpr int lut_plain_stride(int W) { return W | 1; }
 
 template <class T>
 struct cpx;
@@ -29,6 +44,7 @@ using zd = cpx<double>;
 // p50 8.3 s against 1.9 s with every kernel loaded up front).
 void preload_nearfield_kernels();
 void preload_uslut_kernels();
+void preload_uslut_plain_kernels();
 void preload_detector_kernels();
 
 // One bilinear LUT cell at (r, t): {T00, T10 - T00, T01 - T00, T11 - T10 - T01 + T00}
@@ -79,6 +95,12 @@ void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int
                          const float4* kw4, const cpx<float>* ph, const float2* lin, const cpx<float>* Uf,
                          cpx<float>* U, unsigned long long* counters, float2* kcmp, float* part, bool stage, int chunk,
                          float4 cone, cudaStream_t st);
+// the same field by the plain kernel (lut_plain, lut_few): the waves in chunks of `chunk`, one bounding cone {axis,
+// half-angle} per chunk (read with `stage` only); counters in chunks of counted_chunk waves
+void launch_us_lut_plain(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
+                         const float4* kw4, const float4* cones, const cpx<float>* ph, const float2* lin,
+                         const cpx<float>* Uf, cpx<float>* U, unsigned long long* counters, float2* kcmp, bool stage,
+                         int chunk, int counted_chunk, cudaStream_t st);
 // Shares of the spheres that launch_us_lut_mixed runs side by side; above 1, `part` (else null) holds
 // 4 floats per pixel and share.
 int lut_splits(int R, int ns, int nk);
@@ -97,6 +119,9 @@ struct LutBuildJob {
 void launch_lut_build_mixed(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab,
                             const float* bias, const float2* P, int Pstride, float2* lin, cudaStream_t st);
 
+// the same in double precision, rounded, for the plain kernel's tables; tab holds zd entries
+void launch_lut_build_plain(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab,
+                            const double* P, int Pstride, float2* lin, cudaStream_t st);
 // the same in double precision, as bilinear patches at out + lin_off
 void launch_lut_build(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab, const double* P,
                       int Pstride, Patch<double>* out, cudaStream_t st);

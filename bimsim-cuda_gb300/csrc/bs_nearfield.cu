@@ -414,6 +414,24 @@ __global__ void __launch_bounds__(256) lut_build_kernel(const LutBuildJob* __res
     }
 }
 
+// The tables of the plain mixed kernel: the same sums, rounded to float2 in linear rows with the last column repeated.
+// A thread per entry, 8 rows x 32 angles per block.
+__global__ void __launch_bounds__(256) lut_build_plain_kernel(const LutBuildJob* __restrict__ jobs,
+                                                              const zd* __restrict__ tab, const double* __restrict__ P,
+                                                              int Pstride, float2* __restrict__ lin) {
+    const LutBuildJob& j = jobs[blockIdx.z];
+    const int r = blockIdx.y * 8 + (threadIdx.x >> 5), t = blockIdx.x * 32 + (threadIdx.x & 31);
+    if (r >= j.rows || t >= j.thetaR) return;
+    const zd* c = tab + j.tab_off + (size_t)min(r, j.last) * j.L;
+    const double* pl = P + (size_t)t * Pstride;
+    zd acc = mk(0.0, 0.0);
+    for (int l = 0; l < j.L; l++) acc = acc + c[l] * pl[l];
+    const float2 v = make_float2((float)acc.re, (float)acc.im);
+    float2* row = lin + j.lin_off + (size_t)r * j.lin_stride;
+    row[t] = v;
+    if (t == j.thetaR - 1) row[j.thetaR] = v;  // clamped neighbour of the last column
+}
+
 // Per (sphere, wave): (subA / nk) exp(i k k_w . (p_s - f)) (nfScalarUpLut.cu:71,84,90)
 template <class T>
 __global__ void phase_kernel(Scene sc, const Sphere* __restrict__ sph, const double* __restrict__ waves,
@@ -1033,6 +1051,12 @@ void launch_lut_build(const LutBuildJob* jobs, int njobs, int max_rows, int max_
     lut_build_kernel<<<grid, 256, 0, st>>>(jobs, tab, P, Pstride, out);
 }
 
+void launch_lut_build_plain(const LutBuildJob* jobs, int njobs, int max_rows, int max_theta, const zd* tab,
+                            const double* P, int Pstride, float2* lin, cudaStream_t st) {
+    dim3 grid(blocks_for(max_theta, 32), blocks_for(max_rows, 8), (unsigned)njobs);
+    lut_build_plain_kernel<<<grid, 256, 0, st>>>(jobs, tab, P, Pstride, lin);
+}
+
 template <class T>
 void launch_phase(const Scene& sc, const Sphere* sph, const double* waves, cpx<T>* ph, float4* kw4, cudaStream_t st) {
     long long n = std::max<long long>((long long)sc.ns * sc.nk, sc.nk);
@@ -1171,6 +1195,7 @@ void preload_nearfield_kernels() {
     cudaFuncGetAttributes(&a, us_lut_f64_kernel);
     cudaFuncGetAttributes(&a, lut_build_kernel);
     cudaFuncGetAttributes(&a, lut_build_mixed_kernel);
+    cudaFuncGetAttributes(&a, lut_build_plain_kernel);
     cudaFuncGetAttributes(&a, sh_recur_kernel);
     cudaFuncGetAttributes(&a, sh_wave_kernel);
     cudaFuncGetAttributes(&a, sh_coef_kernel);

@@ -5,35 +5,10 @@
 // single precision, per-sphere sums combined with Kahan compensation.
 #include <cuda_runtime.h>
 
-#include "bs_geom.cuh"
 #include "bs_kernels.h"
+#include "bs_lut.cuh"
 
 namespace bs {
-
-// Two single-precision lanes in one 64-bit register pair (low lane first), worked
-// on by packed f32x2 instructions; each lane rounds exactly like the scalar one.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 f2_splat(float a) { return f2_pack(a, a); }
-__device__ __forceinline__ float2 f2_unpack(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 
 // Fractional table columns of two directions: t = acos(c) tsc - t0, with c clamped to
 // [-1, 1] and hb = (pi / 2) tsc - t0.  acos(x) = sqrt(1 - x) g(x) on [0, 1] with g analytic
@@ -70,7 +45,7 @@ __device__ __forceinline__ float column_base(float hp_hi, float hp_lo, float tsc
 }
 
 // ---------------------------------------------------------------------------
-// The sorted kernel (more than LUT_FEW_WAVES directions)
+// The sorted kernel (where neither lut_plain nor lut_few applies)
 //
 // A block owns a 16 x 16 pixel tile, each of its 8 warps two rows of 16 pixels.  Per sphere:
 //  * the block sorts the directions by their angle to the tile centre's direction (as seen
@@ -96,20 +71,6 @@ constexpr int SW_WAVES = 1024;   // directions sorted at a time
 constexpr int SW_W = 64;         // columns of a pixel's window
 constexpr int SW_GROUPS = SW_WAVES / 32;
 constexpr float SW_HALF = 7.5f;  // half a row, pixels
-
-// Whether a pixel lies outside every sphere (nfSumUf.cu:35).
-__device__ __forceinline__ bool outside_all(const Scene& sc, const Sphere* __restrict__ sph, const double p[3]) {
-    for (int s = 0; s < sc.ns; s++) {
-        const Sphere& S = sph[s];
-        // clearly outside in single precision (0.1 % margin on d^2), else the exact test
-        const float dx = (float)(p[0] - S.p[0]), dy = (float)(p[1] - S.p[1]), dz = (float)(p[2] - S.p[2]);
-        const float af = (float)S.a;
-        if (dx * dx + dy * dy + dz * dz > 1.001f * af * af) continue;
-        double r[3];
-        if (dist_exact(p, S.p, r) < S.a) return false;
-    }
-    return true;
-}
 
 template <int N>
 struct Int {  // a compile-time argument of the kernel's lambdas
@@ -687,76 +648,6 @@ __global__ void __launch_bounds__(SW_NT, 2)
     }
 }
 
-// ---------------------------------------------------------------------------
-// Few directions (at most LUT_FEW_WAVES, the plane-wave illumination among them): one thread per
-// pixel, every direction's cell read from the table itself.  The sorted kernel needs a warp's
-// worth of directions per pixel to fill its lanes.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) us_lut_few_kernel(Scene sc, const Sphere* __restrict__ sph, int s0, int s1,
-                                                         int accumulate, int finalize, const float4* __restrict__ kw4,
-                                                         const cpx<float>* __restrict__ ph,
-                                                         const float2* __restrict__ lin,
-                                                         const cpx<float>* __restrict__ Uf, cpx<float>* __restrict__ U,
-                                                         unsigned long long* __restrict__ counters,
-                                                         float2* __restrict__ kcmp, int chunk) {
-    const int tiles_u = (sc.R + 15) / 16;
-    const int iu = (blockIdx.x % tiles_u) * 16 + (threadIdx.x & 15), iv = (blockIdx.x / tiles_u) * 16 + (threadIdx.x >> 4);
-    if (threadIdx.x == 0 && counters)
-        atomicAdd(counters + 1, (unsigned long long)(s1 - s0) * ((sc.nk + chunk - 1) / chunk));
-    if (iu >= sc.R || iv >= sc.R) return;
-    const size_t idx = (size_t)iv * sc.R + iu;
-    double p[3];
-    pixel_pos(sc, iu, iv, p);
-    float2 tot = make_float2(0.f, 0.f), cmp = make_float2(0.f, 0.f);
-    if (accumulate) {
-        tot = make_float2(U[idx].re, U[idx].im);
-        if (kcmp) cmp = kcmp[idx];
-    }
-    for (int s = s0; s < s1; s++) {
-        const Sphere& S = sph[s];
-        double r[3];
-        const double d = dist_exact(p, S.p, r);
-        const TableSel ts = select_table_scaled(S, d);
-        const int ir = min((int)ts.x, max(ts.rows, 2) - 2);
-        const f32x2 al = f2_splat((float)(ts.x - ir));
-        const float2* row = lin + ts.off + (long long)ir * S.lin_stride;
-        const int d1 = S.lin_stride;
-        const float inv = d != 0 ? 1.f / (float)d : 0.f;
-        const float rx = (float)r[0] * inv, ry = (float)r[1] * inv, rz = (float)r[2] * inv;
-        const float cb = d != 0 ? 0.f : 1.f;  // d == 0: cos(theta) := 1
-        const f32x2 ntsc = f2_splat(-S.tsc), hb = f2_splat(column_base(S.hp_hi, 0.f, S.tsc, 0));
-        float2 sx = make_float2(0.f, 0.f), sy = make_float2(0.f, 0.f);
-        for (int w = 0; w < sc.nk; w++) {
-            const float4 k = kw4[w];
-            const cpx<float> pw = ph[(size_t)s * sc.nk + w];
-            const float t =
-                f2_unpack(theta_column2(f2_splat(fmaf(k.x, rx, fmaf(k.y, ry, fmaf(k.z, rz, cb)))), ntsc, hb)).x;
-            const float tf = floorf(t), be = t - tf;
-            const int n = min(max((int)tf, 0), S.thetaR - 1);
-            const f32x2* e = reinterpret_cast<const f32x2*>(row + n);
-            const f32x2 e00 = e[0], e01 = e[1], e10 = e[d1], e11 = e[d1 + 1];
-            const f32x2 v0 = f2_fma(al, f2_sub(e10, e00), e00), v1 = f2_fma(al, f2_sub(e11, e01), e01);
-            const float2 v = f2_unpack(f2_fma(f2_splat(be), f2_sub(v1, v0), v0));
-            sx = make_float2(fmaf(pw.re, v.x, sx.x), fmaf(pw.re, v.y, sx.y));
-            sy = make_float2(fmaf(pw.im, v.x, sy.x), fmaf(pw.im, v.y, sy.y));
-        }
-        // Kahan over spheres
-        const float yr = (sx.x - sy.y) - cmp.x, yi = (sx.y + sy.x) - cmp.y;
-        const float tr = tot.x + yr, ti = tot.y + yi;
-        cmp = make_float2((tr - tot.x) - yr, (ti - tot.y) - yi);
-        tot = make_float2(tr, ti);
-    }
-    if (finalize) {
-        if (outside_all(sc, sph, p)) {
-            tot.x += Uf[idx].re - cmp.x;
-            tot.y += Uf[idx].im - cmp.y;
-        }
-    } else if (kcmp) {
-        kcmp[idx] = cmp;
-    }
-    U[idx] = mk(tot.x, tot.y);
-}
-
 // The shares' sums added in order (Kahan), and Uf where the pixel is outside every sphere.
 __global__ void __launch_bounds__(128) us_lut_join_kernel(Scene sc, const Sphere* __restrict__ sph, int shares,
                                                           const float* __restrict__ part,
@@ -793,14 +684,14 @@ __global__ void __launch_bounds__(128) us_lut_join_kernel(Scene sc, const Sphere
 // 384^2, 50, 200: 7.2, 7.2 and 6.0 ms; 768^2, 120, 1000: 115, 115 and 102 ms.
 int lut_splits(int R, int ns, int nk) {
     const long long tiles = (long long)((R + 15) / 16) * ((R + 15) / 16);
-    if (nk <= LUT_FEW_WAVES || tiles >= 64 * GB300_SMS) return 1;
+    if (lut_plain(ns) || lut_few(ns, nk) || tiles >= 64 * GB300_SMS) return 1;
     return (int)std::max(1LL, std::min({(long long)ns, 16LL, (128 * GB300_SMS + tiles - 1) / tiles}));
 }
 
 // Launches the spheres of a chunk are spread over where lut_splits gives one share: each with about twice the L2
 // cache's size of tables, up to 8.  3072^2 pixels, 50 spheres with 34 MB each: 576 ms in one launch, 563 in 6.
 int lut_ranges(int R, int ns, int nk, size_t table_bytes) {
-    if (nk <= LUT_FEW_WAVES || lut_splits(R, ns, nk) > 1) return 1;
+    if (lut_plain(ns) || lut_few(ns, nk) || lut_splits(R, ns, nk) > 1) return 1;
     return (int)std::max<size_t>(1, std::min<size_t>(std::min(ns, 8), table_bytes >> 28));
 }
 
@@ -809,11 +700,6 @@ void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int
                          cpx<float>* U, unsigned long long* counters, float2* kcmp, float* part, bool stage, int chunk,
                          float4 cone, cudaStream_t st) {
     const unsigned tiles = (sc.R + 15) / 16;
-    if (sc.nk <= LUT_FEW_WAVES) {
-        us_lut_few_kernel<<<tiles * tiles, 256, 0, st>>>(sc, sph, s0, s1, accumulate, finalize, kw4, ph, lin, Uf, U,
-                                                         counters, kcmp, chunk);
-        return;
-    }
     const int shares = part ? lut_splits(sc.R, sc.ns, sc.nk) : 1;
     // per device and cheap; a failure shows up as the launch error
     auto kernel = stage ? us_lut_sorted_kernel<true> : us_lut_sorted_kernel<false>;
@@ -829,7 +715,6 @@ void preload_uslut_kernels() {
     cudaFuncAttributes a;
     cudaFuncGetAttributes(&a, us_lut_sorted_kernel<true>);
     cudaFuncGetAttributes(&a, us_lut_sorted_kernel<false>);
-    cudaFuncGetAttributes(&a, us_lut_few_kernel);
     cudaFuncGetAttributes(&a, us_lut_join_kernel);
 }
 

@@ -121,7 +121,7 @@ typedef struct bs_stats {
     int64_t lut_chunks_total;
     int64_t lut_tables_built;  /* sphere tables (Usp + Uip) built; 0 when reused */
     double lut_staged_predicted;  /* a host model of lut_chunks_staged / total */
-    int64_t lut_wave_chunk;       /* waves per counted chunk of the mixed LUT kernel (64, 32 or 16) */
+    int64_t lut_wave_chunk;       /* waves per counted chunk of the mixed LUT kernels (64, 32 or 16) */
 } bs_stats;
 
 typedef struct bs_ctx bs_ctx;
@@ -318,14 +318,17 @@ bs_status bs_sweep(bs_ctx* ctx, const double* lambdas, int32_t nl, const double*
  * >= k^2).  The incident field Uf is not propagated.  Off by default. */
 bs_status bs_set_backpropagation(bs_ctx* ctx, int32_t enable, double d);
 
-/* Waves per counted chunk of the mixed LUT kernel (lut_chunks_staged and
- * lut_chunks_total of bs_stats): 0 (default) is 64; 16, 32 or 64 fixes it.
- * Results do not depend on it. */
+/* Waves per chunk of the mixed LUT kernels.  Slices of at most 8 spheres sum
+ * a pixel's waves chunk by chunk: 0 (default) picks 64, 32 or 16 per run from
+ * the predicted fraction of staged windows, 16, 32 or 64 fixes it, and the
+ * last bits of the sums depend on it.  With more spheres it is only the unit
+ * of lut_chunks_staged and lut_chunks_total (0: 64). */
 bs_status bs_set_lut_wave_chunk(bs_ctx* ctx, int32_t chunk);
 
-/* Kernel of the mixed-precision LUT stage: 0 (default) and 1 keep windows of
- * the tables in shared memory where they fit, 2 reads every cell from the
- * tables.  All give the same bits.  No reference counterpart. */
+/* Kernel of the mixed-precision LUT stage: 1 keeps windows of the tables in
+ * shared memory where they fit, 2 reads every cell from the tables, 0 (default)
+ * is 1 but for slices of at most 8 spheres few of whose windows fit.  All give
+ * the same bits.  No reference counterpart. */
 bs_status bs_set_lut_staging(bs_ctx* ctx, int32_t mode);
 
 /* Keep the lookup tables of the last run and skip rebuilding them when the
