@@ -124,7 +124,7 @@ struct bs_ctx {
     int prec = -1;
     bool have = false;
 
-    DevBuf d_sph, d_waves, d_kw4, d_ph, d_A, d_B, d_tab, d_legP, d_lut, d_uft, d_uftscr;
+    DevBuf d_sph, d_waves, d_kw4, d_ph, d_A, d_B, d_tab, d_tabscr, d_legP, d_lut, d_uft, d_uftscr;
     DevBuf d_cnt;           // staged / total counters of the mixed LUT kernels
     DevBuf d_cones;         // bounding cones of the plain mixed LUT kernel's wave chunks
     DevBuf d_far;           // far fields Ud, Ufd on request (bs_get_far_field)
@@ -164,7 +164,7 @@ struct bs_ctx {
 
 // Every linear device buffer of a context.
 static std::vector<DevBuf*> ctx_bufs(bs_ctx* c) {
-    return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_tab,
+    return {&c->d_sph, &c->d_waves, &c->d_kw4, &c->d_ph, &c->d_A, &c->d_B, &c->d_tab, &c->d_tabscr,
             &c->d_bias, &c->d_acos, &c->d_legP, &c->d_lut, &c->d_uft, &c->d_uftscr, &c->d_fields, &c->d_su,
             &c->d_sv, &c->d_mask, &c->d_wx, &c->d_wy, &c->d_wix, &c->d_wiy, &c->d_f1, &c->d_f2,
             &c->d_g1, &c->d_I, &c->d_D, &c->d_img, &c->d_cnt, &c->d_cones, &c->d_far,
@@ -1166,6 +1166,7 @@ static bs_status run_nearfield(bs_ctx* c) {
                 maxstarts = std::max(maxstarts, (long long)b.starts.size());
             }
             CK(c->d_tab.ensure((size_t)maxcoef * sizeof(zd)));
+            CK(c->d_tabscr.ensure((size_t)maxcoef * 2 * sizeof(double)));
             CK(c->d_starts.ensure((size_t)maxstarts * sizeof(long long)));
             if (split) CK(c->d_bias.ensure((size_t)maxrow * sizeof(float)));
             if (fp64 && c->acos_theta != thetaR) {
@@ -1237,8 +1238,8 @@ static bs_status run_nearfield(bs_ctx* c) {
                 CK(cudaMemcpyAsync(c->d_starts.p, b.starts.data(), b.starts.size() * sizeof(long long),
                                    cudaMemcpyHostToDevice, c->st));
                 launch_coef_rows_batch(c->d_sph.as<Sphere>(), b.b0, b.b1 - b.b0, c->d_starts.as<long long>(), b.rows,
-                                       c->Lmax, sc.kmag, c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_tab.as<zd>(),
-                                       split ? c->d_bias.as<float>() : nullptr, c->st);
+                                       sc.kmag, c->d_A.as<zd>(), c->d_B.as<zd>(), c->d_tab.as<zd>(),
+                                       c->d_tabscr.as<double>(), split ? c->d_bias.as<float>() : nullptr, c->st);
                 LAUNCHED(c);
                 // the tables of every sphere of the batch in two launches (the dR-row Usp tables,
                 // then the shorter Uip tables)
@@ -1365,7 +1366,7 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
             maxrow = std::max(maxrow, cb.rows);
             maxstarts = std::max(maxstarts, (long long)cb.starts.size());
         }
-        b += 2 * B(ns * sizeof(LutBuildJob)) + B(pool) + B((size_t)maxcoef * sizeof(zd)) +
+        b += 2 * B(ns * sizeof(LutBuildJob)) + B(pool) + 2 * B((size_t)maxcoef * sizeof(zd)) +
              B((size_t)maxstarts * sizeof(long long));
         b += B(thetaR * (size_t)c->Lmax * sizeof(double));    // Legendre table
         if (fp64) b += B((ACOS_NODES + 1) * sizeof(AcosNode) + c->hs[0].thetaR * sizeof(double));

@@ -64,12 +64,12 @@ void launch_uf_table(const Scene& sc, double* tab, double* scratch, cudaStream_t
 void launch_mie(const Sphere* sph, int ns, double k, zd* A, zd* B, cudaStream_t st);
 // spheres [s0, s0 + n) in one launch; starts (device): first global row of each
 // sphere (n + 1 values, the last = total_rows) then first coefficient (n values);
-// bias (device, one float per row) selects the mixed path's split coefficients
+// scratch: 2 doubles per coefficient; bias (device, one float per row) selects the mixed path's split coefficients
 struct SplitCoef {
     float hr, hi, lr, li;  // a complex coefficient: nearest floats and the rests; the size of a zd
 };
-void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows, int Lmax,
-                            double k, const zd* A, const zd* B, zd* tab, float* bias, cudaStream_t st);
+void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows, double k,
+                            const zd* A, const zd* B, zd* tab, double* scratch, float* bias, cudaStream_t st);
 // Legendre values of the mixed path: P[l * stride + t] = {nearest float, rest}
 void launch_legendre_split(int thetaR, int Lmax, int stride, float2* P, cudaStream_t st);
 void launch_legendre_table(int thetaR, int Lmax, double* P, cudaStream_t st);

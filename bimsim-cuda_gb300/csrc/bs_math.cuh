@@ -237,4 +237,33 @@ __device__ inline void sph_real(int N, double x, double* j, double* y, int st) {
     }
 }
 
+// j[l], l = 0..N, of a complex argument.
+__device__ inline void sph_complex(int N, zd z, zd* j) {
+    const double cs = sqrt(PI_BES / TRUE_PI);
+    double az = zabs(z);
+    int Nv = N;
+    if (N >= 2 && N > (int)(0.25 * az)) Nv = orders_kept(N, az);
+    const zd inv = mk(1.0, 0.0) / z;
+    zd s = zsin(z), c = zcos(z);
+    zd j0 = s / z, j1 = s / (z * z) - c / z;
+    int M = miller_start(N, az, z.im);
+    zd fp = mk(0.0, 0.0), fc = mk(1e-300, 0.0);
+    if (M <= N) j[M] = fc;
+    for (int l = M; l >= 1; l--) {
+        const zd w = (double)(2 * l + 1) * inv;
+        const zd fm = mk(fma(w.re, fc.re, fma(-w.im, fc.im, -fp.re)), fma(w.re, fc.im, fma(w.im, fc.re, -fp.im)));
+        fp = fc;
+        fc = fm;
+        if (l - 1 <= N) j[l - 1] = fm;
+        if (beyond_2_830(fc.re) || beyond_2_830(fc.im)) {
+            for (int q = l - 1; q <= N; q++) j[q] = j[q] * 1e-250;
+            fc = fc * 1e-250;
+            fp = fp * 1e-250;
+        }
+    }
+    zd sc = (zabs(j0) >= zabs(j1)) ? j0 / j[0] : j1 / j[1 <= N ? 1 : 0];
+    for (int l = 0; l <= N; l++) j[l] = j[l] * sc;
+    for (int l = 0; l <= N; l++) j[l] = l > Nv ? mk(0.0, 0.0) : j[l] * cs;
+}
+
 }  // namespace bs

@@ -158,29 +158,23 @@ __global__ void __launch_bounds__(MIE_NT) mie_kernel(const Sphere* __restrict__ 
 // Per-row order coefficients of the spheres [s0, s0 + n) in one launch:
 //   rows [0, dR):  C_l(r) = B_l (j_l + i y_l)(k r),  r in [r0, dmax]  (sphere.cpp:154-203)
 //   rows [dR, dR+aR): D_l(r) = A_l j_l(k n r),       r in [0, a]      (sphere.cpp:99-152)
-// starts[i] / starts[n + 1 + i] are sphere i's first global row and its first coefficient in tab (rows of
-// Nl + 1 coefficients; starts[n] is the total row count).  With `bias` (mixed path) every coefficient is
-// stored as SplitCoef instead, and bias[g] is a power of two of at least twice the sum of the row's
-// coefficients, see lut_build_mixed_kernel.
-//
-// A block takes 32 rows, one per lane.  The time of a small slice is the count of FP64 instructions on one
-// warp's chain (64 cycles each), so the four warps share it: the first runs the j recurrence, the second
-// that of y (with j where that runs upwards too) or, inside, the trigonometric start values, and all four finish the orders l = warp (mod 4), in
-// shared memory, from where whole rows are written.  1600 rows of 25 orders: 77 us with a thread per row
-// and its values in global memory, 44 us now; 205 000 rows of 21 orders, bound by the pipe: 230 and 213 us.
-constexpr int CR_ROWS = 32, CR_PAD = CR_ROWS + 1;
+// Thread g takes global row g; starts[i] / starts[n + 1 + i] are sphere i's first global row and its first
+// coefficient in tab (rows of Nl + 1 coefficients; starts[n], the total row count, bounds the grid).  The scratch
+// holds 2 (Nl + 1) doubles per row: every order up to MAX_ORDER fits, whatever the sphere.  With `bias` (mixed path)
+// every coefficient is stored as SplitCoef instead, and bias[g] is a power of two of at least twice the sum of the
+// row's coefficients, see lut_build_mixed_kernel.
+// Bound by the FP64 instructions on one thread's chain: 1600 rows of 25 orders 77 us, 205 000 rows of 21 orders 230 us.
+// Four warps sharing 32 rows through shared memory took 44 and 213 us, but orders above 434 did not fit it, and in
+// some blocks with rows of two spheres two of the warps formed a wrong scale, for no reason that the source shows (run
+// on the CPU with its barriers it has no race and no dependence on what the memory held before).  Here a
+// thread reads only what it has written itself.
 __global__ void __launch_bounds__(128) coef_rows_batch_kernel(const Sphere* __restrict__ sph, int s0, int n,
                                                               const long long* __restrict__ starts, double k,
                                                               const zd* __restrict__ A, const zd* __restrict__ B,
-                                                              zd* __restrict__ tab, float* __restrict__ bias) {
-    extern __shared__ zd cr_val[];  // [order][row]: (j, y) or j of a complex argument, then the coefficients
-    __shared__ zd s_j0[CR_ROWS], s_j1[CR_ROWS], s_sc[CR_ROWS];
-    __shared__ int s_nv[CR_ROWS], s_len[CR_ROWS];
-    __shared__ long long s_out[CR_ROWS];
-    __shared__ float s_sum[4][CR_ROWS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long g = (long long)blockIdx.x * CR_ROWS + lane;
-    const bool live = g < starts[n];
+                                                              zd* __restrict__ tab, double* __restrict__ scratch,
+                                                              float* __restrict__ bias) {
+    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= starts[n]) return;
     int lo = 0, hi = n - 1;  // last sphere whose first row is <= g
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -188,146 +182,34 @@ __global__ void __launch_bounds__(128) coef_rows_batch_kernel(const Sphere* __re
         else hi = mid - 1;
     }
     const Sphere& S = sph[s0 + lo];
-    const int row = live ? (int)(g - starts[lo]) : 0, N = S.Nl, L = N + 1;
-    const bool outer = row < S.dR, centre = row == S.dR;  // centre: r = 0, the order 0 alone
-    zd* v = cr_val + lane;                                // order l at v[l * CR_PAD]
-    const double cs = sqrt(PI_BES / TRUE_PI);
-    double x = 1.0;
-    zd z = mk(1.0, 0.0);
-    if (outer) {
+    const int row = (int)(g - starts[lo]), L = S.Nl + 1;
+    const long long c0 = starts[n + 1 + lo] + (long long)row * L;
+    zd* out = tab + c0;
+    double* sj = scratch + 2 * c0;
+    const zd* a = (row < S.dR ? B : A) + S.coef_off;
+    if (row < S.dR) {
         const double dr = (S.dmax - S.r0) / (S.dR - 1);
-        x = k * (row * dr + S.r0);
-    } else if (!centre) {
+        sph_real(S.Nl, k * (row * dr + S.r0), sj, sj + L, 1);
+    } else if (row > S.dR) {  // the centre, row dR, has the order 0 alone
         const double da = S.a / (S.aR - 1);
-        z = (mk(S.n_re, S.n_im) * k) * ((row - S.dR) * da);
+        sph_complex(S.Nl, (mk(S.n_re, S.n_im) * k) * ((row - S.dR) * da), reinterpret_cast<zd*>(sj));
     }
-    int Nv = N;
-    if (outer && !(x < 1e-15) && N >= 2 && N > (int)(0.9 * x)) Nv = orders_kept(N, x);
-    const bool upward = Nv < x;  // j upwards too, with y and its factors
-    if (warp == 0) {
-        s_len[lane] = live ? L : 0;
-        s_out[lane] = starts[n + 1 + lo] + (long long)row * L;
-        if (outer && !(x < 1e-15)) {
-            if (!upward) {
-                const double inv = 1.0 / x;
-                double fp = 0.0, fc = 1e-300;
-                for (int l = miller_start(Nv, x); l >= 1; l--) {
-                    const double fm = fma(quot(2 * l + 1, x, inv), fc, -fp);
-                    fp = fc;
-                    fc = fm;
-                    if (l - 1 <= Nv) v[(l - 1) * CR_PAD].re = fm;
-                    if (beyond_2_830(fc)) {
-                        for (int q = l - 1; q <= Nv; q++) v[q * CR_PAD].re *= 1e-250;
-                        fc *= 1e-250;
-                        fp *= 1e-250;
-                    }
-                }
-            }
-        } else if (!outer && !centre) {
-            const double az = zabs(z);
-            if (N >= 2 && N > (int)(0.25 * az)) Nv = orders_kept(N, az);
-            s_nv[lane] = Nv;
-            const zd inv = mk(1.0, 0.0) / z;
-            zd fp = mk(0.0, 0.0), fc = mk(1e-300, 0.0);
-            for (int l = miller_start(N, az, z.im); l >= 1; l--) {
-                const zd w = (double)(2 * l + 1) * inv;
-                const zd fm =
-                    mk(fma(w.re, fc.re, fma(-w.im, fc.im, -fp.re)), fma(w.re, fc.im, fma(w.im, fc.re, -fp.im)));
-                fp = fc;
-                fc = fm;
-                if (l - 1 <= N) v[(l - 1) * CR_PAD] = fm;
-                if (beyond_2_830(fc.re) || beyond_2_830(fc.im)) {
-                    for (int q = l - 1; q <= N; q++) v[q * CR_PAD] = v[q * CR_PAD] * 1e-250;
-                    fc = fc * 1e-250;
-                    fp = fp * 1e-250;
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (outer && !(x < 1e-15)) {
-            const double inv = 1.0 / x;
-            double sn, c;
-            sincos(x, &sn, &c);
-            const double ix = quot(c, x, inv), ja = quot(sn, x, inv), xx = x * x;
-            double pj = ja, j = sn / xx - ix, py = -ix, y = -c / xx - ja;
-            s_j0[lane] = mk(pj, 0.0);
-            s_j1[lane] = mk(j, 0.0);
-            v[0].im = py;
-            if (N >= 1) v[CR_PAD].im = y;
-            if (upward) {
-                v[0].re = pj;
-                if (N >= 1) v[CR_PAD].re = j;
-            }
-            for (int l = 2; l <= Nv; l++) {
-                const double w = quot(2 * l - 1, x, inv), t = fma(w, y, -py);
-                py = y;
-                y = t;
-                v[l * CR_PAD].im = t;
-                if (upward) {
-                    const double u = fma(w, j, -pj);
-                    pj = j;
-                    j = u;
-                    v[l * CR_PAD].re = u;
-                }
-            }
-        } else if (!outer && !centre) {
-            const zd sn = zsin(z), c = zcos(z);
-            s_j0[lane] = sn / z;
-            s_j1[lane] = sn / (z * z) - c / z;
-        }
-    }
-    __syncthreads();
-    if (warp == 0) {  // what the downward recurrence lacks
-        zd sc = mk(1.0, 0.0);
-        const zd j0 = s_j0[lane], j1 = s_j1[lane], f0 = v[0], f1 = v[N >= 1 ? CR_PAD : 0];
-        if (outer) {
-            if (!(x < 1e-15) && !upward) sc.re = fabs(j0.re) >= fabs(j1.re) ? j0.re / f0.re : j1.re / f1.re;
-        } else if (!centre) {
-            const bool first = zabs(j0) >= zabs(j1);
-            sc = (first ? j0 : j1) / (first ? f0 : f1);
-        }
-        s_sc[lane] = sc;
-    }
-    __syncthreads();
-    if (!outer && !centre) Nv = s_nv[lane];
-    const zd sc = s_sc[lane];
     float sum = 0.f;
-    for (int l = warp; l < L; l += 4) {
+    for (int l = 0; l < L; l++) {
         zd c;
-        if (outer) {
-            zd jy = mk(0.0, 0.0);
-            if (x < 1e-15) {
-                const double big = sqrt(PI_BES / (x * 2.0));
-                jy = mk(0.0 * big, -1e308 * big);
-            } else if (l <= Nv) {
-                jy = mk(v[l * CR_PAD].re * sc.re * cs, v[l * CR_PAD].im * cs);
-            }
-            c = B[S.coef_off + l] * jy;
-        } else if (centre) {
-            c = A[S.coef_off + l] * mk(l == 0 ? 1.0 : 0.0, 0.0);
-        } else {
-            c = A[S.coef_off + l] * (l > Nv ? mk(0.0, 0.0) : (v[l * CR_PAD] * sc) * cs);
+        if (row < S.dR) c = a[l] * mk(sj[l], sj[L + l]);
+        else if (row > S.dR) c = a[l] * mk(sj[2 * l], sj[2 * l + 1]);
+        else c = a[l] * mk(l == 0 ? 1.0 : 0.0, 0.0);
+        if (bias) {  // {hr, hi, lr, li} of SplitCoef, in the bits of two doubles
+            const float hr = (float)c.re, hi = (float)c.im;
+            const float lr = (float)(c.re - (double)hr), li = (float)(c.im - (double)hi);
+            sum += fmaxf(fabsf(hr), fabsf(hi));
+            c = mk(__hiloint2double(__float_as_int(hi), __float_as_int(hr)),
+                   __hiloint2double(__float_as_int(li), __float_as_int(lr)));
         }
-        if (bias) {
-            SplitCoef q;
-            q.hr = (float)c.re;
-            q.hi = (float)c.im;
-            q.lr = (float)(c.re - (double)q.hr);
-            q.li = (float)(c.im - (double)q.hi);
-            sum += fmaxf(fabsf(q.hr), fabsf(q.hi));
-            reinterpret_cast<SplitCoef&>(v[l * CR_PAD]) = q;
-        } else {
-            v[l * CR_PAD] = c;
-        }
+        out[l] = c;
     }
-    s_sum[warp][lane] = sum;
-    __syncthreads();
-    for (int r = warp; r < CR_ROWS; r += 4)
-        for (int l = lane; l < s_len[r]; l += 32) tab[s_out[r] + l] = cr_val[l * CR_PAD + r];
-    if (bias && warp == 0 && live) {
-        const float all = (s_sum[0][lane] + s_sum[1][lane]) + (s_sum[2][lane] + s_sum[3][lane]);
-        bias[g] = scalbnf(1.f, ilogbf(fmaxf(all, 1e-30f)) + 2);
-    }
+    if (bias) bias[g] = scalbnf(1.f, ilogbf(fmaxf(sum, 1e-30f)) + 2);
 }
 
 // P_l(cos theta_t), theta_t = t * dtheta (sphere.cu:16-21).  The reference's step
@@ -1028,13 +910,9 @@ void launch_mie(const Sphere* sph, int ns, double k, zd* A, zd* B, cudaStream_t 
     mie_kernel<<<ns, MIE_NT, 0, st>>>(sph, k, A, B);
 }
 
-void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows, int Lmax,
-                            double k, const zd* A, const zd* B, zd* tab, float* bias, cudaStream_t st) {
-    const size_t smem = (size_t)Lmax * CR_PAD * sizeof(zd);  // 68 KB at 128 orders
-    if (smem > 44 * 1024)
-        cudaFuncSetAttribute(coef_rows_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    coef_rows_batch_kernel<<<(unsigned)((total_rows + CR_ROWS - 1) / CR_ROWS), 128, smem, st>>>(sph, s0, n, starts, k,
-                                                                                              A, B, tab, bias);
+void launch_coef_rows_batch(const Sphere* sph, int s0, int n, const long long* starts, long long total_rows, double k,
+                            const zd* A, const zd* B, zd* tab, double* scratch, float* bias, cudaStream_t st) {
+    coef_rows_batch_kernel<<<blocks_for(total_rows, 128), 128, 0, st>>>(sph, s0, n, starts, k, A, B, tab, scratch, bias);
 }
 
 void launch_legendre_split(int thetaR, int Lmax, int stride, float2* P, cudaStream_t st) {
