@@ -13,6 +13,7 @@ namespace bs {
 constexpr float LUT_STAGE_MARGIN = 5e-4f;
 constexpr float LUT_PLAIN_MARGIN = 2e-3f;
 constexpr int GB300_SMS = 152;
+constexpr int SMEM_OPTIN = 227 * 1024;  // most shared memory of a block
 constexpr int LUT_TILE = 16;
 constexpr int LUT_WINDOW = 256;  // table columns of the widest staged window
 constexpr int WAVE_CHUNK_MAX = 64;

@@ -999,8 +999,9 @@ void launch_sh_tables(const Scene& sc, const Sphere* sph, int L, const double* w
 template <class T>
 void launch_us_sh(const Scene& sc, const Sphere* sph, int L, const ShRec* rec, const zd* coef, const cpx<T>* Uf, cpx<T>* U, cudaStream_t st) {
     const size_t smem = (size_t)L * SH_BLOCK * sizeof(zd);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(us_sh_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the kernel's attribute is one for all threads of the process: the largest size on every call, so that another
+    // context cannot lower it before this launch
+    cudaFuncSetAttribute(us_sh_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN);
     const long long n = (long long)sc.R * sc.R;
     us_sh_kernel<T><<<blocks_for(n, SH_BLOCK), SH_BLOCK, smem, st>>>(sc, sh_frame(sc), sph, L, rec, coef, Uf, U);
 }

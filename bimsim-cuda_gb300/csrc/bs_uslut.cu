@@ -102,6 +102,8 @@ struct SwShared {
     double pa[3][16], pb[3][16];  // pixel position = pa[.][column] + pb[.][row]
 };
 
+constexpr int SW_SMEM = (int)sizeof(SwShared);
+
 // +-cos of the Chebyshev angles of 4 and of 6 points
 __constant__ float c_nodes[10] = {0.923879533f, -0.923879533f, 0.382683432f, -0.382683432f, 0.965925826f,
                                   -0.965925826f, 0.707106781f, -0.707106781f, 0.258819045f, -0.258819045f};
@@ -703,8 +705,8 @@ void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int
     const int shares = part ? lut_splits(sc.R, sc.ns, sc.nk) : 1;
     // per device and cheap; a failure shows up as the launch error
     auto kernel = stage ? us_lut_sorted_kernel<true> : us_lut_sorted_kernel<false>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SwShared));
-    kernel<<<dim3(tiles * tiles, shares), SW_NT, sizeof(SwShared), st>>>(sc, sph, s0, s1, accumulate, finalize, kw4, ph,
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM);
+    kernel<<<dim3(tiles * tiles, shares), SW_NT, SW_SMEM, st>>>(sc, sph, s0, s1, accumulate, finalize, kw4, ph,
                                                                          lin, Uf, U, counters, kcmp, part, chunk, cone);
     if (part && finalize)
         us_lut_join_kernel<<<(sc.R * sc.R + 127) / 128, 128, 0, st>>>(sc, sph, shares, part, Uf, U);

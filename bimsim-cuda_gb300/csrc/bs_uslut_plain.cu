@@ -32,6 +32,7 @@ constexpr int UP_TILE = 256;  // 16 x 16 pixel tile
 // whose barriers and window copies weigh more, one on 8 warps (307 against 366 ms with 16-wave chunks on a 1536^2
 // slice).
 constexpr int UP_TWO_PIXEL_MIN_CHUNK = 64;
+constexpr int UP_SMEM = lut_plain_entries(16) * (int)sizeof(float2);  // the larger of the windows
 
 // Fractional LUT angle index t = acos(c) tsc for c in [-1, 1] (c is clamped),
 // tsc = (thetaR - 1) / PI_REF, tscpi = tsc * pi.  acos(x) = sqrt(1 - x) g(x)
@@ -473,7 +474,7 @@ void launch_us_lut_plain(const Scene& sc, const Sphere* sph, int s0, int s1, int
     const int cap = stage ? lut_plain_entries(chunk) : 0, smem = cap * (int)sizeof(float2);
     auto kernel = !stage ? us_lut_plain_kernel<false, 1> : two ? us_lut_plain_kernel<true, 2> : us_lut_plain_kernel<true, 1>;
     // per device, cheap and the same value on every call; a failure shows up as the launch error
-    if (stage) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, UP_SMEM);
     kernel<<<tiles * tiles, stage && two ? UP_TILE / 2 : UP_TILE, smem, st>>>(sc, sph, s0, s1, accumulate, finalize, kw4,
                                                                             cones, ph, lin, Uf, U, counters, kcmp, chunk,
                                                                             counted_chunk, cap);
