@@ -378,6 +378,7 @@ static bs_status derive(bs_ctx* c) {
         S.tsc = (float)tsc;
         S.hp_hi = (float)hp;
         S.hp_lo = (float)(hp - (double)S.hp_hi);
+        for (int k = 0; k < 3; k++) S.rel[k] = (float)(sc.A[k] - S.p[k]);
         S.coef_off = coef;
         coef += S.Nl + 1;
         c->Lmax = std::max(c->Lmax, S.Nl + 1);

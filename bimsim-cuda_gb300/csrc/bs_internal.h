@@ -67,7 +67,7 @@ struct Sphere {
     double xs_usp, xs_uip;   // (dR - 1) / (dmax - r0) and (aR - 1) / (a - dmin): radial index scales
     float tsc;               // table columns per radian, (thetaR - 1) / PI_REF
     float hp_hi, hp_lo;      // pi / 2 in columns, rounded, and the rest
-    float pad_;
+    float rel[3];            // the slice's corner A from the sphere's centre, its difference formed in double
 };
 
 // Host helpers (bs_host.cpp).

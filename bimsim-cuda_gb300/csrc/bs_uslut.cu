@@ -94,7 +94,7 @@ struct SwShared {
     int4 band[SW_GROUPS];      // the band that starts at a group, see plan_bands
     float2 acc[8][2][32];      // Kahan sum and compensation of the warps' rows
     float rdist[8][2];         // 1 / distance of the rows' centres from the sphere
-    float3 A, X, Y;            // the slice in single precision (bounds and node directions)
+    float3 X, Y;               // the slice's axes in single precision (bounds and node directions)
     float iR, half;            // 1 / R; half a row, um
     PixRow px[8][32];
     float4 dir[8][2][16];      // pixel directions, pixels i and 15 - i together: {x, x', y, y'}, {z, z', cb, cb'}
@@ -306,7 +306,6 @@ __global__ void __launch_bounds__(SW_NT, 2)
         sm.acc[warp][r][lane] = a;
     }
     if (threadIdx.x == 0) {
-        sm.A = make_float3((float)sc.A[0], (float)sc.A[1], (float)sc.A[2]);
         sm.X = make_float3((float)sc.X[0], (float)sc.X[1], (float)sc.X[2]);
         sm.Y = make_float3((float)sc.Y[0], (float)sc.Y[1], (float)sc.Y[2]);
         sm.iR = 1.f / (float)sc.R;
@@ -368,11 +367,13 @@ __global__ void __launch_bounds__(SW_NT, 2)
             float3 ctr;
             float gam, tile_rdist = 0.f;  // 1 / distance of the tile's centre
             {
-                const float3 A = sm.A, X = sm.X, Y = sm.Y, P = make_float3((float)S.p[0], (float)S.p[1], (float)S.p[2]);
+                // from the sphere's centre: differences of absolute positions in single precision would lose the
+                // angles of a slice far from the origin
+                const float3 A = make_float3(S.rel[0], S.rel[1], S.rel[2]), X = sm.X, Y = sm.Y;
                 const float iR = sm.iR;
                 auto at = [&](float u, float v) {
-                    return make_float3(fmaf(X.x, u * iR, fmaf(Y.x, v * iR, A.x - P.x)), fmaf(X.y, u * iR, fmaf(Y.y, v * iR, A.y - P.y)),
-                                       fmaf(X.z, u * iR, fmaf(Y.z, v * iR, A.z - P.z)));
+                    return make_float3(fmaf(X.x, u * iR, fmaf(Y.x, v * iR, A.x)), fmaf(X.y, u * iR, fmaf(Y.y, v * iR, A.y)),
+                                       fmaf(X.z, u * iR, fmaf(Y.z, v * iR, A.z)));
                 };
                 ctr = at((float)tu + 7.5f, (float)tv + 7.5f);
                 const float cl2 = ctr.x * ctr.x + ctr.y * ctr.y + ctr.z * ctr.z;
