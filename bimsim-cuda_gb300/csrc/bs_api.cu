@@ -768,14 +768,17 @@ static void sort_waves(std::vector<double>& w, int chunk) {
 }
 
 // Bounding cone (unit axis, half-angle in radians, at most 2.9) of all directions; half-angle pi
-// if one of them is not a unit vector, which turns the mixed LUT kernel's angle bounds off.
-static float4 wave_cone(const std::vector<double>& w) {
-    double m[3] = {0, 0, 0};
+// if one of them is not a unit vector, which turns the mixed LUT kernel's angle bounds off.  A length of
+// 1 + e, e <= 1e-6, moves an angle by up to acos(1 / (1 + e)) < sqrt(2 e) at the poles: added to `margin`.
+static float4 wave_cone(const std::vector<double>& w, float& margin) {
+    double m[3] = {0, 0, 0}, off = 0;
     for (size_t i = 0; i < w.size(); i += 3) {
         const double l = std::sqrt(w[i] * w[i] + w[i + 1] * w[i + 1] + w[i + 2] * w[i + 2]);
         if (!(std::fabs(l - 1.0) <= 1e-6)) return make_float4(0.f, 0.f, 1.f, (float)TRUE_PI);
+        off = std::max(off, std::fabs(l - 1.0));
         for (int k = 0; k < 3; k++) m[k] += w[i + k];
     }
+    margin += (float)std::sqrt(2 * off);
     const double ml = std::sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
     if (!(ml > 1e-3)) return make_float4(0.f, 0.f, 1.f, 2.9f);
     double c = 1;
@@ -1023,6 +1026,7 @@ static bs_status run_nearfield(bs_ctx* c) {
     const bool plain = mixed_lut && lut_plain(ns), few = mixed_lut && lut_few(ns, nk);
     const bool split = mixed_lut && !plain;  // tables of the split single-precision build
     float4 cone = make_float4(0.f, 0.f, 1.f, (float)TRUE_PI);
+    float margin = LUT_STAGE_MARGIN;
     std::vector<float4> cones;
     double predicted = 0;
     if (p.plane_wave) w.assign(p.k_dir, p.k_dir + 3);
@@ -1033,7 +1037,7 @@ static bs_status run_nearfield(bs_ctx* c) {
         cones.swap(cp.cones);
         predicted = cp.predicted;
     } else if (split) {
-        cone = wave_cone(w);  // ordered per tile on the device
+        cone = wave_cone(w, margin);  // ordered per tile on the device
     } else if (!p.plane_wave) {
         sort_waves(w, WAVE_CHUNK_MAX);
     }
@@ -1310,7 +1314,8 @@ static bs_status run_nearfield(bs_ctx* c) {
                                         (const cpx<float>*)Uf, (cpx<float>*)U,
                                         ns > 0 ? c->d_cnt.as<unsigned long long>() : nullptr,
                                         carry ? c->d_kcmp.as<float2>() : nullptr,
-                                        shares > 1 ? c->d_part.as<float>() : nullptr, use_stage, chunk, cone, c->st);
+                                        shares > 1 ? c->d_part.as<float>() : nullptr, use_stage, chunk, cone, margin,
+                                        c->st);
                     if (!last) LAUNCHED(c);
                 }
                 if (shares > 1 && finalize) c->launches++;

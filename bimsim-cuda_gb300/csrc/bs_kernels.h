@@ -94,11 +94,11 @@ void launch_us_lut_f64(const Scene& sc, const Sphere* sph, int s0, int s1, int a
 // compensation from one sphere chunk's launch to the next, so that chunked
 // tables give the bits of one launch over all spheres;
 // stage = false reads every cell from the tables; cone: axis and half-angle of a cone that holds
-// every direction (half-angle pi: directions that are not unit vectors)
+// every direction (half-angle pi: directions that are not unit vectors); margin: added to the tiles' angular radii
 void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
                          const float4* kw4, const cpx<float>* ph, const float2* lin, const cpx<float>* Uf,
                          cpx<float>* U, unsigned long long* counters, float2* kcmp, float* part, bool stage, int chunk,
-                         float4 cone, cudaStream_t st);
+                         float4 cone, float margin, cudaStream_t st);
 // the same field by the plain kernel (lut_plain, lut_few): the waves in chunks of `chunk`, one bounding cone {axis,
 // half-angle} per chunk (read with `stage` only); counters in chunks of counted_chunk waves
 void launch_us_lut_plain(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,

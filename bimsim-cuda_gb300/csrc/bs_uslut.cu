@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
                          const float4* __restrict__ kw4, const cpx<float>* __restrict__ ph,
                          const float2* __restrict__ lin, const cpx<float>* __restrict__ Uf, cpx<float>* __restrict__ U,
                          unsigned long long* __restrict__ counters, float2* __restrict__ kcmp,
-                         float* __restrict__ part, int chunk, float4 cone) {
+                         float* __restrict__ part, int chunk, float4 cone, float margin) {
     extern __shared__ __align__(1024) unsigned char sw_smem[];
     SwShared& sm = *reinterpret_cast<SwShared*>(sw_smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(SW_NT, 2)
                     const float qi = 1.f / sqrtf(q.x * q.x + q.y * q.y + q.z * q.z);
                     const float ex = fmaf(q.x, qi, -ctr.x), ey = fmaf(q.y, qi, -ctr.y), ez = fmaf(q.z, qi, -ctr.z);
                     const float ch = sqrtf(ex * ex + ey * ey + ez * ez);
-                    const float a = ch <= 1.3f ? fmaf(ch * ch, 0.06f * ch, ch) + LUT_STAGE_MARGIN : (float)TRUE_PI;
+                    const float a = ch <= 1.3f ? fmaf(ch * ch, 0.06f * ch, ch) + margin : (float)TRUE_PI;
                     gam = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(a)));
                 } else {
                     ctr = make_float3(0.f, 0.f, 1.f);
@@ -701,14 +701,14 @@ int lut_ranges(int R, int ns, int nk, size_t table_bytes) {
 void launch_us_lut_mixed(const Scene& sc, const Sphere* sph, int s0, int s1, int accumulate, int finalize,
                          const float4* kw4, const cpx<float>* ph, const float2* lin, const cpx<float>* Uf,
                          cpx<float>* U, unsigned long long* counters, float2* kcmp, float* part, bool stage, int chunk,
-                         float4 cone, cudaStream_t st) {
+                         float4 cone, float margin, cudaStream_t st) {
     const unsigned tiles = (sc.R + 15) / 16;
     const int shares = part ? lut_splits(sc.R, sc.ns, sc.nk) : 1;
     // per device and cheap; a failure shows up as the launch error
     auto kernel = stage ? us_lut_sorted_kernel<true> : us_lut_sorted_kernel<false>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM);
     kernel<<<dim3(tiles * tiles, shares), SW_NT, SW_SMEM, st>>>(sc, sph, s0, s1, accumulate, finalize, kw4, ph,
-                                                                         lin, Uf, U, counters, kcmp, part, chunk, cone);
+                                                                         lin, Uf, U, counters, kcmp, part, chunk, cone, margin);
     if (part && finalize)
         us_lut_join_kernel<<<(sc.R * sc.R + 127) / 128, 128, 0, st>>>(sc, sph, shares, part, Uf, U);
 }

@@ -38,3 +38,14 @@ def test_slices_far_from_the_origin(far, ns):
     s = [(o[0] + 1.1 * (i % 3) - 1.2, o[1] + 1.3 * (i // 3) - 1.1, o[2] - 15.0 + 0.2 * (i % 2), 0.3 + 0.02 * i, 1.35, 0.01)
          for i in range(ns)]
     check(p, s, scenes.mc_waves(400, 0, 0.5, seed=7))
+
+
+# directions up to 1e-6 longer or shorter than 1, as decimal files hold them, along the lines from spheres to pixels,
+# in tables of 0.0001 rad a column: the angle of a direction of length 1.000001 is off by up to 13 columns
+@pytest.mark.parametrize("length", [1.0, 1 + 9.9e-7, 1 - 9.9e-7])
+@pytest.mark.parametrize("ns", [8, 9])
+def test_directions_of_almost_unit_length(length, ns):
+    p = abi.make_params(lam=2.5, condenser=(0, 0.004), objective=(0, 0.5), resolution=32, padding=1, supersample=1,
+                        us_lut_r=20, us_lut_theta=30000, xy=(0.08, 15.0))
+    s = [(0.01 * (i % 3) - 0.01, 0.01 * (i // 3) - 0.01, 0.5 * i - 2.0, 0.2 + 0.01 * i, 1.35, 0.01) for i in range(ns)]
+    check(p, s, length * scenes.mc_waves(256, 0, 0.004, seed=8))
