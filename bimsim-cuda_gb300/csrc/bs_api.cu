@@ -621,14 +621,12 @@ static bs_status run_detector(bs_ctx* c, bool accumulate) {
 // thetaR + 1 entries (the last column repeated, rounded up to an even count
 // for 16-byte rows; a Uip of one row is stored twice).
 static bs_status plan_tables(std::vector<Sphere>& hs, bool mixed, size_t budget, std::vector<int>& chunk_start,
-                             size_t& pool, size_t& maxrows, size_t& maxL) {
+                             size_t& pool) {
     const size_t patch = mixed ? sizeof(float2) : sizeof(Patch<double>);
     const int ns = (int)hs.size();
     chunk_start.clear();
     size_t acc = 0;
     pool = 0;
-    maxrows = 0;
-    maxL = 0;
     for (int i = 0; i < ns; i++) {
         Sphere& S = hs[i];
         S.lin_stride = mixed ? ((S.thetaR + 2) & ~1) : S.thetaR;
@@ -644,8 +642,6 @@ static bs_status plan_tables(std::vector<Sphere>& hs, bool mixed, size_t budget,
         S.uip_off = S.usp_off + (int64_t)S.dR * S.lin_stride;
         acc += need;
         pool = std::max(pool, acc);
-        maxrows = std::max(maxrows, (size_t)(S.dR + S.aR));
-        maxL = std::max(maxL, (size_t)(S.Nl + 1));
     }
     chunk_start.push_back(ns);
     return BS_OK;
@@ -690,15 +686,14 @@ static std::vector<CoefBatch> coef_batches(const std::vector<Sphere>& hs, const 
     return out;
 }
 
-static bs_status plan_luts(bs_ctx* c, bool mixed, std::vector<int>& chunk_start, size_t& pool, size_t& maxrows,
-                           size_t& maxL) {
+static bs_status plan_luts(bs_ctx* c, bool mixed, std::vector<int>& chunk_start, size_t& pool) {
     size_t budget = c->budget;
     if (!budget) {
         size_t free_b = 0, total_b = 0;
         CK(cudaMemGetInfo(&free_b, &total_b));
         budget = (size_t)(0.80 * (double)(free_b + c->d_lut.n));
     }
-    return plan_tables(c->hs, mixed, budget, chunk_start, pool, maxrows, maxL);
+    return plan_tables(c->hs, mixed, budget, chunk_start, pool);
 }
 
 // Order plane waves in compact groups of `chunk`: their projections on the
@@ -1094,9 +1089,9 @@ static bs_status run_nearfield(bs_ctx* c) {
     // ---- LUT placement (before the sphere table goes to the device) ----
     std::vector<int> chunk_start;
     std::vector<CoefBatch> batches;
-    size_t pool = 0, maxrows = 0, maxL = 0;
+    size_t pool = 0;
     if (p.scalar && p.lut_us && ns > 0) {
-        bs_status pst = plan_luts(c, !fp64, chunk_start, pool, maxrows, maxL);
+        bs_status pst = plan_luts(c, !fp64, chunk_start, pool);
         if (pst != BS_OK) return pst;
         batches = coef_batches(c->hs, chunk_start);
     }
@@ -1362,8 +1357,8 @@ static size_t estimate_bytes(bs_ctx* c, bool fp64, size_t lut_budget) {
     if (p.scalar && p.lut_us && ns > 0) {
         std::vector<Sphere> hs = c->hs;
         std::vector<int> cs;
-        size_t pool = 0, maxrows = 0, maxL = 0;
-        if (plan_tables(hs, !fp64, lut_budget ? lut_budget : SIZE_MAX / 4, cs, pool, maxrows, maxL) != BS_OK)
+        size_t pool = 0;
+        if (plan_tables(hs, !fp64, lut_budget ? lut_budget : SIZE_MAX / 4, cs, pool) != BS_OK)
             return 0;
         const size_t thetaR = hs[0].thetaR;
         long long maxcoef = 0, maxstarts = 0, maxrow = 0;

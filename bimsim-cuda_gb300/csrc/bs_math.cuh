@@ -1,5 +1,5 @@
 // bs_math.cuh -- device arithmetic: complex numbers, the reference's
-// recurrences (rts/math/legendre.h, rts/math/spherical_bessel.h) and
+// Legendre recurrence (rts/math/legendre.h) and
 // double-precision spherical Bessel functions for the Mie coefficients and
 // the lookup tables.
 #pragma once
@@ -46,8 +46,6 @@ __host__ __device__ __forceinline__ cpx<T> operator/(cpx<T> a, cpx<T> b) {
     T r = b.re / b.im, den = b.re * r + b.im;
     return mk((a.re * r + a.im) / den, (a.im * r - a.re) / den);
 }
-template <class T>
-__host__ __device__ __forceinline__ T cabs2(cpx<T> a) { return a.re * a.re + a.im * a.im; }
 
 __device__ __forceinline__ double zabs(zd a) { return hypot(a.re, a.im); }
 
@@ -66,41 +64,13 @@ __device__ __forceinline__ zd ipow(int l) {
 }
 
 // ---------------------------------------------------------------------------
-// The reference's three-term recurrences
+// The reference's three-term recurrence
 // ---------------------------------------------------------------------------
 // P_n from P_{n-1}, P_{n-2} (rts/math/legendre.h:17-25)
 __device__ __forceinline__ void legendre_step(int n, double x, double& P0, double& P1) {
     double Pn = ((2 * n - 1) * x * P1 - (n - 1) * P0) / n;
     P0 = P1;
     P1 = Pn;
-}
-
-// j_n upward with the "convergence" clamp of spherical_bessel.h:102-119:
-// once n > x, a value outside [0.0145, 0.4] is replaced by zero.
-__device__ __forceinline__ void sbesselj_step(int n, double x, double& b0, double& b1) {
-    double bn = ((2 * n - 1) * b1) / x - b0;
-    if (n > x && (bn < CONV_MIN || bn > CONV_MAX)) bn = 0.0;
-    b0 = b1;
-    b1 = bn;
-}
-
-// complex-argument version: the clamp tests the real parts
-__device__ __forceinline__ void sbesselj_step_c(int n, zd x, zd& b0, zd& b1) {
-    zd bn = (((double)(2 * n - 1)) * b1) / x - b0;
-    if (n > x.re && (bn.re < CONV_MIN || bn.re > CONV_MAX)) bn = mk(0.0, 0.0);
-    b0 = b1;
-    b1 = bn;
-}
-
-// y_n upward with the floor/sign clamp of spherical_bessel.h:121-141
-__device__ __forceinline__ void sbessely_step(int n, double x, double& b0, double& b1) {
-    double bn = ((2 * n - 1) * b1) / x - b0;
-    if (bn < Y_FLOOR || (n > x && bn > 0)) {
-        bn = 0;
-        b1 = 0;
-    }
-    b0 = b1;
-    b1 = bn;
 }
 
 // ---------------------------------------------------------------------------

@@ -37,7 +37,7 @@ __device__ __forceinline__ double mie_scale(int d) { return d == 0 ? 1.0 : (d ==
 
 // A_l, B_l for l = 0 .. N (N <= MAX_ORDER); called by all MIE_NT threads of a block.
 __device__ inline void mie_block(MieShared& sm, int N, double a, zd n, double k, zd* __restrict__ A, zd* __restrict__ B) {
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const double ka = k * a, cs = sqrt(PI_BES / TRUE_PI);
     const zd kna = (n * k) * a;
     const double az = fabs(ka), anz = zabs(kna);

@@ -35,14 +35,15 @@ struct UfLegendre {  // u_l(x), l = 0, 1, 2, ... in turn
     }
 };
 
-// The clamp of sbesselj_step off the FP64 pipe: the high words of CONV_MIN and CONV_MAX decide, but where they are equal.
+// The "convergence" clamp of the upward j_l (spherical_bessel.h:102-119: once l > x, a value outside [0.0145, 0.4] is
+// replaced by zero) off the FP64 pipe: the high words of CONV_MIN and CONV_MAX decide, but where they are equal.
 __device__ __forceinline__ double clamp_j(double j, bool beyond) {
     constexpr int LO = 0x3f8db22d, HI = 0x3fd99999;
     const int h = __double2hiint(j);
     return beyond && (h <= LO || h >= HI) && (h < LO || h > HI || j < CONV_MIN || j > CONV_MAX) ? 0.0 : j;
 }
 
-// The clamped upward j_l recurrence (sbesselj_step), one reciprocal for all quotients and orders.
+// The clamped upward j_l recurrence, one reciprocal for all quotients and orders.
 __device__ zd uf_direct(const Scene& sc, const UfOrder* __restrict__ w, const double p[3]) {
     double r[3];
     double d = dist_exact(p, sc.focus, r);
@@ -715,7 +716,7 @@ __global__ void __launch_bounds__(SC_I* SC_W) sh_coef_kernel(Scene sc, ShFrame f
 }
 
 // The radial functions of one (pixel, sphere) pair, order after order:
-//   outside (d > a):  j_l + i y_l (k d)   with the reference clamps
+//   outside (d > a):  j_l + i y_l (k d)   with the reference clamps (spherical_bessel.h:102-141)
 //   inside  (d <= a): j_l(k n d)          (1 for l = 0 and else 0 when Re(k n d) < 1e-6)
 // (--recursive; nfScalarUs.cu:17-95, 201-245, 333-491); their factors B_l and A_l are in the coefficients.
 // They depend on (pixel, sphere) only; the reference re-runs them for every wave (nfScalarUs.cu:69-93).
