@@ -549,9 +549,10 @@ def run_gb300(args):
                      "staged_fraction": staged, "wave_chunk": wave_chunk,
                      "hbm_peak_gbs": peaks.get("hbm_gbs"), "fp64_peak_tflops": fp64_tf,
                      "why_not_hbm_or_tensor": "no step is a dense contraction (no tensor-core use) and the kernel "
-                                              "reads ~0.013 TB/s of DRAM: it is bound by instruction issue, half of "
-                                              "it FP32 arithmetic, so the roofline is the measured FP32 FMA peak; "
-                                              "the DRAM view is roofline_hbm, the shared-memory pipe roofline_l1"},
+                                              "reads ~0.013 TB/s of DRAM, so the roofline is the measured FP32 FMA "
+                                              "peak; what limits it is the L1 data pipe (78 % busy with shared-memory "
+                                              "reads and staging on a small case) and its latency, issue being at "
+                                              "59 %: roofline_l1; the DRAM view is roofline_hbm"},
         "roofline_hbm": (None if not (profile_traffic() and peaks.get("hbm_gbs")) else
                          {"bound": "hbm", "kernel": "us_lut_sorted_kernel", "unit": "GB/s",
                           "achieved": profile_traffic() / us_s / 1e9, "peak": peaks["hbm_gbs"],

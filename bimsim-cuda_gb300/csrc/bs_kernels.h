@@ -26,8 +26,9 @@ constexpr int LUT_PLAIN_SPHERES = 8;
 inline bool lut_plain(int ns) { return ns <= LUT_PLAIN_SPHERES; }
 // More spheres with few directions: the plain kernel too, without windows and from the sorted kernel's tables.  Two
 // groups of 32 directions do not pay for the sorted kernel's ordering and blending; scattered field plain and sorted,
-// 20 spheres, 1536^2 pixels, 33, 64 and 96 directions: 6.5 and 18.3, 11.1 and 16.8, (17) and 19.5 ms; 768^2: 1.8 and
-// 4.5, 3.0 and 4.3, (4.5) and 5.0 ms; 192^2: 0.25 and 0.35, 0.38 and 0.34, (0.55) and 0.39 ms.
+// 20 spheres, 1536^2 pixels, 33 and 64 directions: 6.5 and 18.3, 11.1 and 16.8 ms; 768^2: 1.8 and 4.5, 3.0 and
+// 4.3 ms; 192^2: 0.25 and 0.35, 0.38 and 0.34 ms.  Each direction more adds 1/64 of the plain figure, 32 more less
+// than a sixth of the sorted one.
 constexpr int LUT_FEW_WAVES = 64;
 inline bool lut_few(int ns, int nk) { return !lut_plain(ns) && nk <= LUT_FEW_WAVES; }
 // Float2 values of the plain kernel's staged windows: 51 KB with 64-wave chunks (4 blocks per SM), 72 KB (3) with

@@ -354,7 +354,10 @@ bs_status bs_release_buffers(bs_ctx* ctx);
 
 /* Device bytes a context would hold after bs_simulate of this scene: near
  * fields, detector transform, tables (capped by lut_budget when it is > 0, as
- * bs_set_lut_budget does) and the per-sphere and per-wave arrays.  Host-only;
+ * bs_set_lut_budget does) and the per-sphere and per-wave arrays.  Among them,
+ * for mixed table slices of more than 8 spheres and 64 waves, the sums of the
+ * spheres' shares: 16 bytes per near-field pixel and share, up to 16 shares on
+ * small grids, about 110 MB at most.  Host-only;
  * the serving front end admits requests with it.  No reference counterpart. */
 bs_status bs_estimate_bytes(const bs_params* params, const bs_sphere* spheres, int32_t n_spheres, int32_t n_waves,
                             bs_precision prec, uint64_t lut_budget, uint64_t* bytes);
