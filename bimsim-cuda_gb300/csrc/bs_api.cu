@@ -702,9 +702,9 @@ static bs_status plan_luts(bs_ctx* c, bool mixed, std::vector<int>& chunk_start,
 // allows), so every group but one holds `chunk` waves and the one short
 // group goes last.  The sum over waves does not depend on the order (up to
 // rounding); compact groups have narrow bounding cones, so each tile's table
-// window per group stays small enough for shared memory (on the config-2 scene
-// 98-99.7 % of windows fit, against 60-86 % for chunks cut from a Hilbert
-// curve order, whose chunks can straddle the curve's jumps).
+// window per group stays small enough for shared memory (3072^2 pixels, 50
+// spheres, 1000 directions: 98-99.7 % of windows fit, against 60-86 % for
+// chunks cut from a Hilbert curve order, which can straddle the curve's jumps).
 static void group_split(std::vector<size_t>& idx, size_t lo, size_t hi, const std::vector<double>& px,
                         const std::vector<double>& py, size_t chunk, std::vector<std::pair<size_t, size_t>>& groups) {
     const size_t n = hi - lo;
